@@ -398,7 +398,8 @@ def main():
     S, m = measure(args.storage, args.case, args.repeats, args.seconds)
     case, cells, ms, mlups = m["case"], m["cells"], m["ms"], m["mlups"]
     tiling = m["tiling"]
-    kname = "k_fused_pipe" if tiling["pipelined"] else "k_fused"  # the fused-step kernel that ran
+    # the kernel(s) of the step that ran
+    kname = {0: "k_fused", 1: "k_fused_pipe", 2: "k_fused_bulk", 3: "k_step_pull+k_step_interface"}[tiling["pipelined"]]
     codec = "CodecF32" if args.storage == "f32" else "CodecF16"
     traffic, traffic_src = traffic_per_launch(cells, f"{kname}<{codec}>")
     roofline = {"bound": "hbm", "kernel": kname, "achieved": round(m["achieved"], 1), "peak": hbm_peak,

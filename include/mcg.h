@@ -191,14 +191,17 @@ mcg_status mcg_step_profiled(mcg_handle *h, int32_t nsteps, float *ms_total, flo
 mcg_status mcg_get_step(const mcg_handle *h, int64_t *step);
 /* Kernel launches issued by this handle since creation. */
 mcg_status mcg_launch_count(const mcg_handle *h, uint64_t *count);
-/* Launch shape of the fused step (no counterpart in the reference, whose
- * launch configuration is fixed): out[0..7] = rows per tile, planes per
- * z chunk, threads per row, y tiles, z chunks, shared memory bytes per CTA,
- * march (0: k_fused, block-synchronous; 1: k_fused_pipe, pipelined;
- * 2: k_fused_bulk, pipelined with each pulled row staged in shared memory by
- * bulk copies; chosen only when the environment sets MCG_FUSED_BULK=1, as it
- * measured slower), row length the kernel is compiled for (0: runtime
- * geometry). */
+/* Launch shape of the step (no counterpart in the reference, whose launch
+ * configuration is fixed): out[0..7] = rows per tile, planes per z chunk,
+ * threads per row, y tiles, z chunks, shared memory bytes per CTA, how the step
+ * runs, row length the kernel is compiled for (0: runtime geometry).
+ * How the step runs: 3, the default, in two launches (k_step_pull,
+ * k_step_interface), whose tiles are the rows of one CTA and z chunks single
+ * planes; otherwise as a march over z in one launch: 0 k_fused,
+ * block-synchronous (MCG_FUSED_PIPE=0 in the environment), 1 k_fused_pipe,
+ * pipelined (MCG_FUSED_PIPE=1), 2 k_fused_bulk, pipelined with each pulled row
+ * staged in shared memory by bulk copies (MCG_FUSED_BULK=1, rows of 128
+ * columns).  The results are the same bit for bit. */
 #define MCG_TILING_FIELDS 8
 mcg_status mcg_get_tiling(const mcg_handle *h, int32_t *out);
 /* k_fused_bulk waits for each staged row at most `tries` times (about 1 us

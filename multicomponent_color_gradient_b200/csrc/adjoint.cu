@@ -167,6 +167,7 @@ struct Run {
             void *b = (k == n - 1 && dst) ? dst : work[k & 1];
             ADJ_LAUNCH(h, mcg::launch_fused(with(a, b), h->tiling, 0, step0 + t0 + k, false, h->stream),
                        "adjoint: forward step");
+            h->launches += mcg::fused_launches(h->tiling) - 1;
             a = b;
         }
         *result = a;
@@ -202,6 +203,7 @@ struct Run {
             mcg::DeviceState d = with(a, work[t & 1]);
             d.tape = tape + size_t(t) * record_floats;
             ADJ_LAUNCH(h, mcg::launch_fused(d, h->tiling, 0, step0 + t, false, h->stream), "adjoint: forward step");
+            h->launches += mcg::fused_launches(h->tiling) - 1;
             a = work[t & 1];
         }
         {
@@ -226,6 +228,7 @@ struct Run {
             mcg::DeviceState d = with(a, work[k & 1]);
             d.tape = seg_tape + size_t(k) * record_floats;
             ADJ_LAUNCH(h, mcg::launch_fused(d, h->tiling, 0, step0 + t0 + k, false, h->stream), "adjoint: forward step");
+            h->launches += mcg::fused_launches(h->tiling) - 1;
             a = work[k & 1];
         }
         if (mcg_status s = op(a, t0 + n - 1)) return s;
@@ -358,6 +361,9 @@ mcg_status mcg_adjoint_run(mcg_handle *h, const float *psi_target, int32_t nstep
         run.lmom = static_cast<float *>(p);
         ADJ_CUDA(buf.alloc(&p, 3 * N * sizeof(float)), "adjoint gradient adjoints");
         run.lf = static_cast<float *>(p);
+        // the forward steps' psi of the tape (the handle's stays as it is): lf is
+        // free until the reverse sweep
+        if (tape_mode) run.base.psi[0] = run.base.psi[1] = run.lf;
         ADJ_CUDA(buf.alloc(&p, 3 * N * sizeof(float)), "adjoint du0");
         float *du0 = static_cast<float *>(p);
         ADJ_CUDA(buf.alloc(&p, N * sizeof(float)), "adjoint target");
@@ -567,6 +573,7 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
             d.tape = rec;
         }
         ADJ_LAUNCH(h, mcg::launch_fused(d, h->tiling, 0, step0 + t, stats, h->stream), "jet adjoint: forward step");
+        h->launches += mcg::fused_launches(h->tiling) - 1;
         d.tape = nullptr;
         if (!h->tiling.boundary)
             ADJ_LAUNCH(h, mcg::launch_boundary(d, 1, step0 + t, -1, true, h->stream), "jet adjoint: boundary");

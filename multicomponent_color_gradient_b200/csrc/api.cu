@@ -155,11 +155,13 @@ size_t pop_buffer_bytes(const mcg_params &p) {
     return p.storage == MCG_STORAGE_F16 ? size_t(mcg::kQ) * N * 4 : size_t(2 * mcg::kQ) * N * 4;
 }
 
+size_t piece_flag_bytes(const mcg_params &p) { return size_t(p.NY) * p.NZ * ((p.NX + 31) / 32); }
+
 void release(mcg_handle *h) {
     mcg::async_release(h);
     mcg::io_close(h);
     void *ptrs[] = {h->s.pops[0], h->s.pops[1], h->s.mom,      h->s.psi[0], h->s.psi[1], h->s.radial,
-                    h->s.uy_avg,  h->s.partials, h->s.flag, h->d_scalar, h->s.bmom,  h->d_inlet_profile, h->d_vti_text};
+                    h->s.uy_avg,  h->s.partials, h->s.piece_flags, h->s.flag, h->d_scalar, h->s.bmom,  h->d_inlet_profile, h->d_vti_text};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     if (h->h_vti_text) cudaFreeHost(h->h_vti_text);
@@ -209,12 +211,14 @@ bool stats_for_step(mcg_handle *h) {
     return h->stats_started;
 }
 
-// One fused step (k_fused, then k_boundary for the jet).  The moment planes in
-// HBM are not written by the fused kernel; they are refreshed on demand.
+// One step (fused.cuh), then k_boundary for the jet unless the step's launches
+// write the boundary themselves.  The moment planes in HBM are not written by
+// the step; they are refreshed on demand.
 mcg_status one_fused_step(mcg_handle *h, bool *ran_boundary) {
     const bool jet = h->p.boundary == MCG_BOUNDARY_JET;
     const bool stats = stats_for_step(h);
     MCG_LAUNCH(h, mcg::launch_fused(h->s, h->tiling, h->cur, h->step, stats, h->stream), "fused step kernel");
+    h->launches += mcg::fused_launches(h->tiling) - 1;
     if (stats) ++h->stats_samples;
     if (jet && !h->tiling.boundary)
         MCG_LAUNCH(h, mcg::launch_boundary(h->s, h->cur ^ 1, h->step, -1, true, h->stream), "boundary kernel");
@@ -229,7 +233,7 @@ mcg_status one_fused_step(mcg_handle *h, bool *ran_boundary) {
 // out since the last check (the kernel sets flag[1] and finishes its march on
 // stale rows, so the state is then invalid).  The flag is cleared.
 mcg_status check_stage_waits(mcg_handle *h) {
-    if (!h->tiling.bulk) return MCG_OK;
+    if (h->tiling.march != mcg::kMarchBulk) return MCG_OK;
     int flag = 0;
     MCG_CUDA(cudaMemcpyAsync(&flag, h->s.flag + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream),
              "download wait flag");
@@ -355,6 +359,7 @@ mcg_status mcg_create(const mcg_params *p, mcg_handle **out) {
         g.boundary = p->boundary;
         g.storage = p->storage;
         g.slots = mcg::kQ;  // one element (both colours) per direction: float2 or half2
+        g.px = p->NX;
         fill_physics(h);
         compute_ncols(h);
         const size_t N = g.N;
@@ -369,7 +374,8 @@ mcg_status mcg_create(const mcg_params *p, mcg_handle **out) {
         if (e == cudaSuccess) e = alloc_zero(&h->s.radial, 5 * M * 8);
         if (e == cudaSuccess) e = alloc_zero(&h->s.bmom, size_t(2) * p->NZ * mcg::kMomCount * p->NX * 4);
         h->tiling = mcg::fused_tiling(g, kFusedSmemPerBlock);
-        if (e == cudaSuccess) e = mcg::fused_configure(h->tiling.smem_bytes);
+        if (e == cudaSuccess) e = mcg::fused_configure(g, h->tiling);
+        if (e == cudaSuccess) e = alloc_zero(&h->s.piece_flags, piece_flag_bytes(*p));
         if (e == cudaSuccess) e = alloc_zero(&h->s.uy_avg, N * 4);
         h->s.partials_cap = mcg::conservation_blocks(g);
         if (e == cudaSuccess) e = alloc_zero(&h->s.partials, size_t(h->s.partials_cap) * 5 * 8);
@@ -447,7 +453,7 @@ mcg_status mcg_device_bytes(const mcg_handle *h, uint64_t *out) {
         MCG_REQUIRE(out != nullptr, "out is null");
         const size_t N = h->s.g.N, M = size_t(h->p.NY) * (h->p.NX / 2);
         *out = 2 * pop_buffer_bytes(h->p) + size_t(mcg::kMomCount) * N * 4 + 2 * N * 4 + 5 * M * 8 + N * 4 +
-               size_t(h->s.partials_cap) * 40 + 16 + 64;
+               size_t(h->s.partials_cap) * 40 + 16 + 64 + piece_flag_bytes(h->p);
         return MCG_OK;
     });
 }
@@ -570,8 +576,7 @@ mcg_status mcg_get_tiling(const mcg_handle *h, int32_t *out) {
         if (mcg_status s = check_handle(h)) return s;
         MCG_REQUIRE(out != nullptr, "out is null");
         const mcg::FusedTiling &t = h->tiling;
-        const int32_t march = t.bulk ? 2 : t.pipe;
-        const int32_t v[MCG_TILING_FIELDS] = {t.ty, t.lz, t.tpr, t.ny_tiles, t.nz_chunks, t.smem_bytes, march, t.fixed_nx};
+        const int32_t v[MCG_TILING_FIELDS] = {t.ty, t.lz, t.tpr, t.ny_tiles, t.nz_chunks, t.smem_bytes, t.march, t.fixed_nx};
         for (int k = 0; k < MCG_TILING_FIELDS; ++k) out[k] = v[k];
         return MCG_OK;
     });
@@ -834,6 +839,7 @@ mcg_status mcg_step_profiled(mcg_handle *h, int32_t nsteps, float *ms_total, flo
         for (int32_t n = 0; n < nsteps; ++n) {
             const bool stats = stats_for_step(h);
             MCG_LAUNCH(h, mcg::launch_fused(h->s, h->tiling, h->cur, h->step, stats, h->stream), "fused step kernel");
+            h->launches += mcg::fused_launches(h->tiling) - 1;
             if (stats) ++h->stats_samples;
             MCG_CUDA(cudaEventRecord(h->prof_events[ev++], h->stream), "event record");
             kind.push_back(0);

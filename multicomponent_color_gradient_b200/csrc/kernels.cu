@@ -1,1536 +1,12 @@
-// kernels.cu - the D3Q27 colour-gradient step on B200 (sm_100a).
-//
-// The step is one HBM pass, one launch (k_fused, or its pipelined forms
-// k_fused_pipe and k_fused_bulk):
-//   k_fused    a CTA owns a tile of rows (y) and marches a chunk of z planes.
-//              For each plane it pulls f(t) for its rows plus a one-row halo
-//              from the population buffer (row-blocked layout, so a pulled row
-//              is nine contiguous segments), forms rho_r, rho_b, u, Pi^neq
-//              (lbm.cuh:82-165) and psi into shared memory, accumulates the
-//              radial statistics (kernels.cu:188-233) with warp segmented
-//              reductions, and then relaxes the previous plane
-//              (lbm.cuh:184-293): Hermite-regularised BGK, colour-gradient
-//              perturbation and recolouring, with the gradient taken from the
-//              same step's psi in shared memory (the reference needs a kernel
-//              boundary for this), storing the post-collision values at each
-//              node (pull layout, coalesced rows).  Moments never go to HBM.
-//              The CTAs whose tiles hold the fluid rows 1 and NY-2 then write
-//              the jet's inlet (jet/boundary_conditions.cuh:17-85) and
-//              convective outlet (:163-233) columns of their chunk into the y
-//              ghost planes of the new buffer (fused_boundary).
-//   k_boundary the same boundary as a launch of its own, one thread per
-//              column, from the fluid-plane moments the step leaves in bmom
-//              (the granular sequence, and MCG_FUSED_BOUNDARY=0).
-// The granular launch sequence of the reference (k_moments, k_collide,
-// k_boundary, k_accumulate_radial) is kept for callers that drive the
-// launchers one by one; it writes the moment planes to HBM like the reference.
-// The reference's in-place push buffer becomes a ping-pong pull pair; the
-// populations a reference step never rewrites (y=1 slots fed by non-jet
-// inlet columns, y=NY-2 slots fed by ghost columns) are ghost-plane values of
-// both buffers that no kernel writes, so results are the same.
-#include <type_traits>
-#include <cuda_fp16.h>
-
-#include <algorithm>
-#include <cstdlib>
-#include <cstring>
-
-#include "kernels.cuh"
-#include "lattice.cuh"
+// kernels.cu - the kernels around the fused step (fused.cuh) on B200 (sm_100a):
+// the granular launch sequence of the reference (k_moments, k_collide,
+// k_boundary, k_accumulate_radial) for callers that drive the launchers one by
+// one, which writes the moment planes to HBM like the reference; initial
+// states, state transfer, diagnostics, outputs and the discrete adjoint.
+#include "step.cuh"
 
 namespace mcg {
 namespace {
-
-constexpr unsigned kFull = 0xffffffffu;
-
-// ------------------------------------------------------------------ storage codecs
-
-// Float32 element per (direction, node): the pair (fr, fb), so a pull or a
-// store of both colours is one 8-byte access.
-struct CodecF32 {
-    using Elem = float2;
-    static constexpr int kGroupSlots = 3;
-    static constexpr bool kSumDiff = false;  // pulls form sum fr and sum fb (reference order)
-    // store_bulk takes P_i itself (collision_poly without a shift)
-    static constexpr bool kShiftPoly = false;
-    __device__ __forceinline__ float poly_shift() const { return 0.0f; }
-    const float2 *__restrict__ rd;
-    float2 *__restrict__ wr;
-    int NX;
-    // store through `wrow` = the node's row in the written buffer, offset by x
-    template <int I>
-    __device__ __forceinline__ void store_row(float2 *wrow, float r, float b) const {
-        wrow[slot_pair(I) * NX] = make_float2(r, b);
-    }
-    // bulk node: fr_i = aR w_i P_i, fb_i = aB w_i P_i (lbm.cuh:216-247)
-    __device__ __forceinline__ void store_bulk(float2 *wrow, float aR, float aB, const float (&P)[kQ]) const {
-        static_for<kQ>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            // both colours in one packed multiply and one store
-            wrow[slot_pair(i) * NX] = __fmul2_rn(make_float2(aR * Dir<i>::w, aB * Dir<i>::w), make_float2(P[i], P[i]));
-        });
-    }
-    // pull in two halves: the raw pair at `p` = the source node's element of
-    // direction I, then the pair the colour sums add and the total gi
-    using Raw = float2;
-    template <int I>
-    __device__ __forceinline__ Raw load_raw(const float2 *p) const {
-        return __ldg(p);
-    }
-    template <int I>
-    __device__ __forceinline__ float2 decode(Raw v, float &gi) const {
-        gi = v.x + v.y;
-        return v;
-    }
-    template <int I>
-    __device__ __forceinline__ void store(size_t row, int x, float r, float b) const {
-        wr[row + size_t(slot_pair(I)) * NX + x] = make_float2(r, b);
-    }
-    __device__ __forceinline__ static void store_to(void *buf, const Geometry &g, int i, int x, int y, int z, float r,
-                                                    float b, float) {
-        static_cast<float2 *>(buf)[pop_index(g, slot_pair(i), x, y, z)] = make_float2(r, b);
-    }
-    // the colour pair of a pulled element
-    template <int I>
-    __device__ __forceinline__ void unpack(Raw v, float &r, float &b) const {
-        r = v.x;
-        b = v.y;
-    }
-    __device__ __forceinline__ static void load_from(const void *buf, const Geometry &g, int i, int x, int y, int z,
-                                                     float &r, float &b, float) {
-        const float2 v = static_cast<const float2 *>(buf)[pop_index(g, slot_pair(i), x, y, z)];
-        r = v.x;
-        b = v.y;
-    }
-};
-
-// F16 word per (direction, node): x = g/w_i - rho0 (total offset by the rest
-// equilibrium and scaled by 1/w_i), y = q, the minority-colour fraction
-// 2 min(fr,fb)/g carrying the sign of fr-fb.  Pure nodes store q = +-0
-// exactly, so a single-colour region keeps exactly zero of the other colour.
-__device__ __forceinline__ __half2 f16_encode(float r, float b, float inv_w, float rho0) {
-    // rounded operation by operation, so that every kernel that inlines it
-    // (the jet boundary is written from several) gives the same word
-    const float g = __fadd_rn(r, b);
-    const float h0 = __fsub_rn(__fmul_rn(g, inv_w), rho0);
-    const float mn = fminf(r, b);
-    float q = (g > 0.0f) ? __fdividef(2.0f * mn, g) : 0.0f;
-    q = copysignf(fmaxf(q, 0.0f), r - b);
-    return __floats2half2_rn(h0, q);
-}
-__device__ __forceinline__ void f16_decode(__half2 h, float w, float rho0, float &r, float &b) {
-    const float2 v = __half22float2(h);
-    const float g = w * (rho0 + v.x);
-    const float minor = 0.5f * g * fabsf(v.y);
-    const bool red_major = !signbit(v.y);
-    r = red_major ? g - minor : minor;
-    b = red_major ? minor : g - minor;
-}
-
-struct CodecF16 {
-    using Elem = __half2;
-    static constexpr int kGroupSlots = 3;
-    static constexpr bool kSumDiff = true;  // pulls form sum (fr+fb) and sum (fr-fb)
-    // store_bulk takes P_i - rho0, formed by collision_poly's constant term
-    static constexpr bool kShiftPoly = true;
-    __device__ __forceinline__ float poly_shift() const { return rho0; }
-    const __half2 *__restrict__ rd;
-    __half2 *__restrict__ wr;
-    int NX;
-    float rho0;
-    template <int I>
-    __device__ __forceinline__ void store_row(__half2 *wrow, float r, float b) const {
-        wrow[slot_pair(I) * NX] = f16_encode(r, b, 1.0f / Dir<I>::w, rho0);
-    }
-    // bulk node: every direction splits its total g_i = w_i P_i in the same
-    // proportion aR : aB, so the word is (P_i - rho0, q) (Ps = P - rho0 from
-    // collision_poly) with one signed
-    // minority fraction q = 2 min(aR, aB) for the node - the value f16_encode
-    // forms from fr_i, fb_i up to float rounding, and exactly +-0 at a pure
-    // node (aB or aR is exactly 0 there).
-    __device__ __forceinline__ void store_bulk(__half2 *wrow, float aR, float aB, const float (&Ps)[kQ]) const {
-        const float q = copysignf(fmaxf(2.0f * fminf(aR, aB), 0.0f), aR - aB);
-        static_for<kQ>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            wrow[slot_pair(i) * NX] = __floats2half2_rn(Ps[i], q);
-        });
-    }
-    // pull in two halves: the raw word, then the total g = fr + fb and the
-    // difference d = fr - fb.  With q the signed minority fraction, fr - fb =
-    // g (1 - q) when red is the majority and -g (1 + q) otherwise, i.e.
-    // g (sign(q) - q).
-    // The read-only load asks L2 to fetch 256-byte blocks on a miss: the words
-    // of a pulled row segment are then in L2 for the neighbouring warps'
-    // loads (measured +0.3 % on the 128x256x128 jet, +1.2 % on 256-column
-    // rows; no change in float32).
-    using Raw = __half2;
-    template <int I>
-    __device__ __forceinline__ Raw load_raw(const __half2 *p) const {
-        uint32_t u;
-        asm("ld.global.nc.L2::256B.b32 %0, [%1];" : "=r"(u) : "l"(p));
-        __half2 h;
-        memcpy(&h, &u, sizeof h);
-        return h;
-    }
-    template <int I>
-    __device__ __forceinline__ float2 decode(Raw h, float &gi) const {
-        const float2 v = __half22float2(h);
-        const float gs = fmaf(Dir<I>::w, v.x, Dir<I>::w * rho0);
-        gi = gs;
-        return make_float2(gs, fmaf(-gs, v.y, copysignf(gs, v.y)));
-    }
-    template <int I>
-    __device__ __forceinline__ void store(size_t row, int x, float r, float b) const {
-        wr[row + size_t(slot_pair(I)) * NX + x] = f16_encode(r, b, 1.0f / Dir<I>::w, rho0);
-    }
-    __device__ __forceinline__ static void store_to(void *buf, const Geometry &g, int i, int x, int y, int z, float r,
-                                                    float b, float rho0) {
-        static_cast<__half2 *>(buf)[pop_index(g, slot_pair(i), x, y, z)] = f16_encode(r, b, 1.0f / dir_w(i), rho0);
-    }
-    template <int I>
-    __device__ __forceinline__ void unpack(Raw h, float &r, float &b) const {
-        f16_decode(h, Dir<I>::w, rho0, r, b);
-    }
-    __device__ __forceinline__ static void load_from(const void *buf, const Geometry &g, int i, int x, int y, int z,
-                                                     float &r, float &b, float rho0) {
-        f16_decode(static_cast<const __half2 *>(buf)[pop_index(g, slot_pair(i), x, y, z)], dir_w(i), rho0, r, b);
-    }
-};
-
-template <class C>
-__host__ __device__ C make_codec(const DeviceState &s, int cur);
-template <>
-__host__ __device__ CodecF32 make_codec<CodecF32>(const DeviceState &s, int cur) {
-    return CodecF32{static_cast<const float2 *>(s.pops[cur]), static_cast<float2 *>(s.pops[cur ^ 1]), s.g.NX};
-}
-template <>
-__host__ __device__ CodecF16 make_codec<CodecF16>(const DeviceState &s, int cur) {
-    return CodecF16{static_cast<const __half2 *>(s.pops[cur]), static_cast<__half2 *>(s.pops[cur ^ 1]), s.g.NX,
-                    s.ph.f16_rho0};
-}
-
-// ------------------------------------------------------------------ helpers
-
-__device__ __forceinline__ float psi_of(float a, float b) { return (a - b) / (a + b); }  // mathUtilities.cuh:24-28
-
-__device__ __forceinline__ float clamp01(float v) { return fminf(fmaxf(v, 0.0f), 1.0f); }
-
-// Relaxation rate at height y (mathUtilities.cuh:56-90); constant when K == 0.
-__device__ __forceinline__ float omega_at(const Physics &ph, int y) {
-    if (!ph.sponge) return ph.omega;
-    const float s = clamp01((float(y) - ph.sponge_y_start) * ph.sponge_inv_width);
-    const float nus = ph.nu * (1.0f + ph.sponge_K * (s * s * s));
-    return 1.0f / (0.5f + nus * kInvCs2);
-}
-
-__device__ __forceinline__ bool is_jet_column(const Physics &ph, int x, int z) {  // mathUtilities.cuh:14-21
-    const float dx = float(x) - ph.jet_x0, dz = float(z) - ph.jet_z0;
-    return __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dz, dz)) <= ph.jet_r2;
-}
-
-// Inlet velocity of jet column (x, z): the top-hat U (boundary_conditions.cuh:62),
-// times the column's profile multiplier when a radial profile is set, times
-// the seeded perturbation when inlet_noise != 0.
-__device__ __forceinline__ float inlet_velocity(const DeviceState &s, int64_t step, int x, int z) {
-    const Physics &ph = s.ph;
-    float U = ph.jet_velocity;
-    if (s.inlet_profile) U *= s.inlet_profile[x + s.g.NX * z];
-    if (ph.inlet_noise == 0.0f) return U;
-    const float u = hash_uniform(ph.seed, 0x1A1E7ull ^ uint64_t(step), uint64_t(x), uint64_t(z));
-    return __fmul_rn(U, __fadd_rn(1.0f, __fmul_rn(__fsub_rn(2.0f * u, 1.0f), ph.inlet_noise)));
-}
-
-__host__ __device__ __forceinline__ int wrap_interior(int v, int n) { return v == 0 ? n - 2 : (v == n - 1 ? 1 : v); }
-
-// Pull sources of interior node (x,y,z).  x and z are periodic over the
-// interior through the ghost shell (the push side wraps with
-// bounds.cuh:23-60); y sources on a ghost plane are the boundary's slots and
-// are not wrapped laterally (boundary writes are unwrapped,
-// boundary_conditions.cuh:73,137); in the periodic box y wraps too.
-template <class C>
-struct PullMap {
-    long long own_row;              // offset of row (y,z)
-    long long step_y, step_z;       // row offsets of y+1, z+1
-    long long wzp, wzm, wyp, wym;   // wrap corrections (row offsets)
-    int wxp, wxm;                   // wrap corrections (x)
-    int NX;
-    bool gy_p, gy_m;
-    __device__ __forceinline__ PullMap(const Geometry &g, int x, int y, int z, bool periodic) {
-        NX = g.NX;
-        own_row = (long long)pop_row(g, y, z);
-        step_y = (long long)g.slots * g.NX;
-        step_z = step_y * g.NY;
-        wxp = (x == 1) ? (g.NX - 2) : 0;
-        wxm = (x == g.NX - 2) ? -(g.NX - 2) : 0;
-        wzp = (z == 1) ? step_z * (g.NZ - 2) : 0;
-        wzm = (z == g.NZ - 2) ? -step_z * (g.NZ - 2) : 0;
-        wyp = (periodic && y == 1) ? step_y * (g.NY - 2) : 0;
-        wym = (periodic && y == g.NY - 2) ? -step_y * (g.NY - 2) : 0;
-        gy_p = !periodic && y == 1;
-        gy_m = !periodic && y == g.NY - 2;
-    }
-    // offset of the group segment of direction I's source row, and source x
-    template <int I>
-    __device__ __forceinline__ void src(int x, size_t &grow, int &xs) const {
-        using D = Dir<I>;
-        const long long o = own_row - D::cy * step_y - D::cz * step_z;
-        bool ghost = false;
-        if constexpr (D::cy == 1) ghost = gy_p;
-        if constexpr (D::cy == -1) ghost = gy_m;
-        int xc = 0;
-        long long oc = 0;
-        if constexpr (D::cx == 1) xc = wxp;
-        if constexpr (D::cx == -1) xc = wxm;
-        if constexpr (D::cz == 1) oc = wzp;
-        if constexpr (D::cz == -1) oc = wzm;
-        if (ghost) {
-            xc = 0;
-            oc = 0;
-        }
-        if constexpr (D::cy == 1) oc += wyp;
-        if constexpr (D::cy == -1) oc += wym;
-        grow = size_t(o + oc) + size_t(dir_group(I) * C::kGroupSlots) * size_t(NX);
-        xs = x - D::cx + xc;
-    }
-    // the source's first slot of direction I (red for float32)
-    template <int I>
-    __device__ __forceinline__ const typename C::Elem *ptr(const C &codec, int x) const {
-        size_t grow;
-        int xs;
-        src<I>(x, grow, xs);
-        return codec.rd + grow + size_t(dir_cx(I) + 1) * size_t(NX) + xs;
-    }
-};
-
-// Pull sources of a node in rows y = 2 .. NY-3: no source lies on a y ghost
-// plane or wraps in y, so the only corrections are the z wrap, the same for
-// all directions of one cz, and the x wrap of columns 1 and NX-2.  One base
-// pointer per cz (z wrap applied, offset by x) then serves nine directions,
-// each a load at a constant offset from it, plus the x wrap for cx = +-1.
-// The addresses are those of PullMap.
-template <class C>
-struct FastPullMap {
-    const typename C::Elem *base[3];  // cz = -1, 0, +1
-    long long step_y;
-    int xwp, xwm;  // x wrap of cx = +1 (column 1) and cx = -1 (column NX-2)
-    int NX;
-    __device__ __forceinline__ FastPullMap(const Geometry &g, const C &codec, int x, int y, int z) {
-        NX = g.NX;
-        step_y = (long long)g.slots * g.NX;
-        const long long step_z = step_y * g.NY;
-        const typename C::Elem *own = codec.rd + pop_row(g, y, z) + x;
-        base[0] = own + step_z + ((z == g.NZ - 2) ? -step_z * (g.NZ - 2) : 0);  // cz = -1: source plane z+1
-        base[1] = own;
-        base[2] = own - step_z + ((z == 1) ? step_z * (g.NZ - 2) : 0);          // cz = +1: source plane z-1
-        xwp = (x == 1) ? (g.NX - 2) : 0;
-        xwm = (x == g.NX - 2) ? -(g.NX - 2) : 0;
-    }
-    template <int I>
-    __device__ __forceinline__ const typename C::Elem *ptr(const C &, int) const {
-        using D = Dir<I>;
-        const typename C::Elem *b = base[D::cz + 1];
-        if constexpr (D::cx == 1) b += xwp;
-        if constexpr (D::cx == -1) b += xwm;
-        return b + (-(long long)D::cy * step_y + (long long)(dir_group(I) * C::kGroupSlots + D::cx + 1) * NX - D::cx);
-    }
-};
-
-// Runtime-direction pull source (init/gather/diagnostic kernels): source
-// coordinates of direction i for interior node (x,y,z).
-__device__ __forceinline__ void pull_src_rt(const Geometry &g, int x, int y, int z, int i, int &xs, int &ys, int &zs) {
-    const bool periodic = g.boundary == kBoundaryPeriodic;
-    xs = x - dir_cx(i);
-    ys = y - dir_cy(i);
-    zs = z - dir_cz(i);
-    const bool ghost_plane = !periodic && (ys == 0 || ys == g.NY - 1);
-    if (!ghost_plane) {
-        xs = wrap_interior(xs, g.NX);
-        zs = wrap_interior(zs, g.NZ);
-    }
-    if (periodic) ys = wrap_interior(ys, g.NY);
-}
-
-// ------------------------------------------------------------------ per-node pieces
-
-// First of the opposite pairs (i, i+1), i = 2p+1, whose direction has a
-// nonzero c_a c_b (a == b: c_a != 0); the moment sums start there.
-__host__ __device__ constexpr int dir_comp(int i, int a) { return a == 0 ? dir_cx(i) : (a == 1 ? dir_cy(i) : dir_cz(i)); }
-__host__ __device__ constexpr int first_pair(int a, int b) {
-    for (int p = 0; p < (kQ - 1) / 2; ++p)
-        if (dir_comp(2 * p + 1, a) * dir_comp(2 * p + 1, b) != 0) return p;
-    return (kQ - 1) / 2;
-}
-template <bool kFirst>
-__device__ __forceinline__ void moment_add(float &acc, float v) {
-    if constexpr (kFirst)
-        acc = v;
-    else
-        acc += v;
-}
-
-// A node's pull in two halves: pull_issue loads the 27 raw elements (float2
-// or half2) into registers; densities_from / moments_from decode and sum them.
-// Between the two a warp can do other work while the loads are in flight.
-template <class C>
-struct RawPull {
-    typename C::Raw v[kQ];
-};
-
-template <class C, class Map>
-__device__ __forceinline__ void pull_issue_map(const Map &pm, const C &codec, int x, RawPull<C> &raw) {
-    static_for<kQ>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        raw.v[i] = codec.template load_raw<i>(pm.template ptr<i>(codec, x));
-    });
-}
-
-// Colour densities only of interior node (x,y,z): the colour sums of
-// pull_moments below in the same order (direction index), so psi formed from
-// either is bit-identical.  Nodes whose psi is all that is needed (halo rows
-// and planes of a tile) take this.
-// The pulled pairs come from `src.get<I>(gi)`: decoded from words already in
-// registers (RawSource) or loaded and decoded on the spot (DecodedPull).
-template <class C>
-struct RawSource {
-    const C &codec;
-    const RawPull<C> &raw;
-    template <int I>
-    __device__ __forceinline__ float2 get(float &gi) const {
-        return codec.template decode<I>(raw.v[I], gi);
-    }
-};
-
-template <class Src>
-__device__ __forceinline__ void densities_from(const Src &src, float &rr, float &rb) {
-    using C = std::remove_cv_t<std::remove_reference_t<decltype(src.codec)>>;
-    float2 sum = make_float2(0.f, 0.f);  // (sum fr, sum fb); C::kSumDiff: (sum fr+fb, sum fr-fb)
-    static_for<kQ>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        float gi;
-        sum = __fadd2_rn(sum, src.template get<i>(gi));  // both colours in one packed add
-    });
-    if constexpr (C::kSumDiff) {
-        rr = 0.5f * (sum.x + sum.y);
-        rb = 0.5f * (sum.x - sum.y);
-    } else {
-        rr = sum.x;
-        rb = sum.y;
-    }
-}
-
-// Pull the 54 populations of interior node (x,y,z) and form its moments
-// (lbm.cuh:106-164: densities, velocity, second-order Hermite moments minus
-// the equilibrium part).  The loads are issued in direction-index order
-// (measured: issuing them group by group was 5-20 % slower) into registers;
-// the moments are then formed from the sums and differences of opposite
-// pairs, about 100 operations instead of one multiply-add per direction and
-// moment.
-template <class Src>
-__device__ __forceinline__ NodeMoments moments_from(const Src &src) {
-    using C = std::remove_cv_t<std::remove_reference_t<decltype(src.codec)>>;
-    float2 sum = make_float2(0.f, 0.f);  // (sum fr, sum fb); C::kSumDiff: (sum fr+fb, sum fr-fb)
-    float gv[kQ];                        // totals fr + fb per direction
-    static_for<kQ>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        sum = __fadd2_rn(sum, src.template get<i>(gv[i]));
-    });
-    // Moments over the 13 opposite pairs (i, i+1), i odd: d = g_i - g_opp
-    // carries the first moments, s = g_i + g_opp the second.  Near equilibrium
-    // the two members of a pair are within a factor of two, so d is exact and
-    // the momentum sums add small numbers.  The diagonal stresses take s times
-    // the Hermite constants H_aa = c_a^2 - cs^2 (multiply-adds, as lbm.cuh
-    // forms them): the rounding of the two constants cancels at rest, whereas
-    // sum c_a^2 g - rho * float(1/3) is biased by 1e-8 rho at every node and
-    // step, which accumulated to 3x the float32 error of the reference's
-    // arithmetic in the kinetic energy.  (Summing whole (cy, cz) groups
-    // before differencing lost digits of the momentum.)
-    float Jx, Jy, Jz, Qxy, Qxz, Qyz;
-    float Axx = gv[0] * Dir<0>::Hxx, Ayy = gv[0] * Dir<0>::Hyy, Azz = gv[0] * Dir<0>::Hzz;
-    static_for<(kQ - 1) / 2>([&](auto P) {
-        constexpr int p = decltype(P)::value, i = 2 * p + 1;
-        using D = Dir<i>;
-        static_assert(Dir<i + 1>::cx == -D::cx && Dir<i + 1>::cy == -D::cy && Dir<i + 1>::cz == -D::cz,
-                      "directions i, i+1 (i odd) are opposite");
-        const float d = gv[i] - gv[i + 1], sp = gv[i] + gv[i + 1];
-        if constexpr (D::cx != 0) moment_add<p == first_pair(0, 0)>(Jx, D::cx > 0 ? d : -d);
-        if constexpr (D::cy != 0) moment_add<p == first_pair(1, 1)>(Jy, D::cy > 0 ? d : -d);
-        if constexpr (D::cz != 0) moment_add<p == first_pair(2, 2)>(Jz, D::cz > 0 ? d : -d);
-        Axx = fmaf(sp, D::Hxx, Axx);
-        Ayy = fmaf(sp, D::Hyy, Ayy);
-        Azz = fmaf(sp, D::Hzz, Azz);
-        if constexpr (D::cx * D::cy != 0) moment_add<p == first_pair(0, 1)>(Qxy, D::cx * D::cy > 0 ? sp : -sp);
-        if constexpr (D::cx * D::cz != 0) moment_add<p == first_pair(0, 2)>(Qxz, D::cx * D::cz > 0 ? sp : -sp);
-        if constexpr (D::cy * D::cz != 0) moment_add<p == first_pair(1, 2)>(Qyz, D::cy * D::cz > 0 ? sp : -sp);
-    });
-    float sumr = sum.x, sumb = sum.y;
-    if constexpr (C::kSumDiff) {
-        sumr = 0.5f * (sum.x + sum.y);
-        sumb = 0.5f * (sum.x - sum.y);
-    }
-    NodeMoments m;
-    const float rho = sumr + sumb;
-    const float inv = 1.0f / rho;
-    m.rr = sumr;
-    m.rb = sumb;
-    m.ux = Jx * inv;
-    m.uy = Jy * inv;
-    m.uz = Jz * inv;
-    m.pxx = Axx - rho * m.ux * m.ux;
-    m.pxy = Qxy - rho * m.ux * m.uy;
-    m.pyy = Ayy - rho * m.uy * m.uy;
-    m.pyz = Qyz - rho * m.uy * m.uz;
-    m.pzz = Azz - rho * m.uz * m.uz;
-    m.pxz = Qxz - rho * m.ux * m.uz;
-    return m;
-}
-
-// Rows 2 .. NY-3 take FastPullMap, the two edge rows PullMap (ghost planes,
-// y wrap); y is uniform over a warp at every call site, so the branch is too.
-template <class C, bool kPeriodic>
-__device__ __forceinline__ void pull_issue(const Geometry &g, const C &codec, int x, int y, int z, RawPull<C> &raw) {
-    if (y >= 2 && y <= g.NY - 3)
-        pull_issue_map(FastPullMap<C>(g, codec, x, y, z), codec, x, raw);
-    else
-        pull_issue_map(PullMap<C>(g, x, y, z, kPeriodic), codec, x, raw);
-}
-// One-piece pulls: each load is decoded where it is issued, which lets the
-// compiler consume the words as they arrive (measured 2 % faster at 80
-// registers than issuing all of them first).  The arithmetic and its order
-// are the same either way, so the results are bit-identical.
-template <class C, class Map>
-struct DecodedPull {
-    const Map &pm;
-    const C &codec;
-    int x;
-    template <int I>
-    __device__ __forceinline__ float2 get(float &gi) const {
-        return codec.template decode<I>(codec.template load_raw<I>(pm.template ptr<I>(codec, x)), gi);
-    }
-};
-template <class C, class Map>
-__device__ __forceinline__ void pull_densities_map(const Map &pm, const C &codec, int x, float &rr, float &rb) {
-    densities_from(DecodedPull<C, Map>{pm, codec, x}, rr, rb);
-}
-template <class C, class Map>
-__device__ __forceinline__ NodeMoments pull_moments_map(const Map &pm, const C &codec, int x) {
-    return moments_from(DecodedPull<C, Map>{pm, codec, x});
-}
-template <class C, bool kPeriodic>
-__device__ __forceinline__ void pull_densities(const Geometry &g, const C &codec, int x, int y, int z, float &rr,
-                                               float &rb) {
-    if (y >= 2 && y <= g.NY - 3)
-        pull_densities_map(FastPullMap<C>(g, codec, x, y, z), codec, x, rr, rb);
-    else
-        pull_densities_map(PullMap<C>(g, x, y, z, kPeriodic), codec, x, rr, rb);
-}
-template <class C, bool kPeriodic>
-__device__ __forceinline__ NodeMoments pull_moments(const Geometry &g, const C &codec, int x, int y, int z) {
-    if (y >= 2 && y <= g.NY - 3) return pull_moments_map(FastPullMap<C>(g, codec, x, y, z), codec, x);
-    return pull_moments_map(PullMap<C>(g, x, y, z, kPeriodic), codec, x);
-}
-
-// Relax one node and store its 54 post-collision values (lbm.cuh:184-293).
-// The bulk part feq + (1-omega) fneq of all 27 directions comes from
-// collision_poly (lattice.cuh).  At interface nodes the perturbation Omega2
-// (even in c: one evaluation per opposite pair) and the recolouring Delta
-// (odd) are added per direction.  psi_at(cx,cy,cz) returns the neighbour's
-// psi, read unwrapped like forces.cuh:31 (ghost psi is what the reference
-// sees there).
-template <class C, class PsiAt>
-__device__ __forceinline__ void collide_node(const Geometry &g, const Physics &ph, const C &codec, size_t row, int x,
-                                             int y, int z, const NodeMoments &m, PsiAt &&psi_at) {
-    const NeqTerms n = make_neq(m.pxx, m.pxy, m.pyy, m.pyz, m.pzz, m.pxz, m.ux, m.uy, m.uz);
-    const float rr = m.rr, rb = m.rb;
-    const float rT = rr + rb;
-    const float invrT = 1.0f / rT;
-    const float aR = rr * invrT, aB = rb * invrT;
-    const float oms = 1.0f - omega_at(ph, y);
-    const float Iind = 4.0f * rr * rb * invrT * invrT;
-    float P[kQ];  // P_i - shift, shift = 0 (float32) or rho0 (float16)
-    const float shift = codec.poly_shift();
-    collision_poly(rT, m.ux, m.uy, m.uz, n, oms, P, shift);
-    auto full = [&](float p) {  // P_i from P_i - shift
-        if constexpr (C::kShiftPoly)
-            return p + shift;
-        else
-            return p;
-    };
-    typename C::Elem *const wrow = codec.wr + row + x;
-    if (Iind <= 1e-4f) {  // bulk (lbm.cuh:216-247)
-        codec.store_bulk(wrow, aR, aB, P);
-        return;
-    }
-    // interface (lbm.cuh:249-292): colour gradient over the 26 neighbours
-    float sx = 0.f, sy = 0.f, sz = 0.f;
-    static_for<kQ - 1>([&](auto I) {
-        constexpr int i = decltype(I)::value + 1;
-        using D = Dir<i>;
-        const float wp = D::w * psi_at(D::cx, D::cy, D::cz);
-        if constexpr (D::cx == 1) sx += wp;
-        if constexpr (D::cx == -1) sx -= wp;
-        if constexpr (D::cy == 1) sy += wp;
-        if constexpr (D::cy == -1) sy -= wp;
-        if constexpr (D::cz == 1) sz += wp;
-        if constexpr (D::cz == -1) sz -= wp;
-    });
-    InterfaceTerms t;
-    t.Fx = kInvCs2 * sx;
-    t.Fy = kInvCs2 * sy;
-    t.Fz = kInvCs2 * sz;
-    t.absF = sqrtf(t.Fx * t.Fx + t.Fy * t.Fy + t.Fz * t.Fz);
-    t.has_dir = !(t.absF <= 1.0e-4f);
-    t.inv_absF = 1.0f / t.absF;
-    t.inv_absF2 = 1.0f / (t.absF * t.absF);
-    t.Ah_absF = ph.Ah * t.absF;
-    t.coeff_rho = ph.beta * ((rr * rb) / (rT * rT)) * rT;
-    {
-        const float g0 = Dir<0>::w * full(P[0]) + omega2<0>(t);
-        codec.template store_row<0>(wrow, aR * g0, aB * g0);
-    }
-    static_for<(kQ - 1) / 2>([&](auto Q) {
-        constexpr int i = 2 * decltype(Q)::value + 1;
-        const float o2 = omega2<i>(t);  // even: the same for i and its opposite
-        const float gi = Dir<i>::w * full(P[i]) + o2, go = Dir<i + 1>::w * full(P[i + 1]) + o2;
-        const float d = recolour<i>(t);  // odd: -d for the opposite
-        codec.template store_row<i>(wrow, aR * gi + d, aB * gi - d);
-        codec.template store_row<i + 1>(wrow, aR * go - d, aB * go + d);
-    });
-}
-
-// ------------------------------------------------------------------ radial statistics
-
-// Warp-collective: one warp = 32 consecutive x at fixed (y,z).  Lanes with the
-// same radial bin form contiguous runs once split by the side of the jet axis
-// (the bin is monotone in |x - x0| on each side), so a segmented scan leaves
-// each run's sums in its last lane, which issues one float64 atomic per sum.
-// Counts are not accumulated per node: every sample adds the fixed number of
-// interior columns of a bin, so they are materialised on read.
-__device__ __forceinline__ void radial_accumulate_warp(const DeviceState &s, int x, int y, int z, bool active,
-                                                       float ux, float uy, float uz) {
-    const Physics &ph = s.ph;
-    const int lane = threadIdx.x & 31;
-    unsigned key = 0xffffffffu;
-    float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f, v4 = 0.f;
-    if (active) {
-        const float dx = float(x) - ph.jet_x0, dz = float(z) - ph.jet_z0;
-        const float r = sqrtf(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dz, dz)));
-        const unsigned rb = unsigned(r);
-        if (rb < unsigned(ph.NRB)) {
-            key = (rb << 1) | (dx < 0.0f ? 1u : 0u);
-            float ur = 0.0f;
-            if (r > 1.0e-12f) ur = (ux * dx + uz * dz) / r;
-            v0 = uy;
-            v1 = uy * uy;
-            v2 = ur;
-            v3 = ur * ur;
-            v4 = ur * uy;
-        }
-    }
-    if (__all_sync(kFull, key == 0xffffffffu)) return;
-    // run sums in float32 (a run is at most 32 nodes of one row); the run
-    // totals go into the float64 accumulators
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned ok = __shfl_up_sync(kFull, key, d);
-        const float o0 = __shfl_up_sync(kFull, v0, d);
-        const float o1 = __shfl_up_sync(kFull, v1, d);
-        const float o2 = __shfl_up_sync(kFull, v2, d);
-        const float o3 = __shfl_up_sync(kFull, v3, d);
-        const float o4 = __shfl_up_sync(kFull, v4, d);
-        if (lane >= d && ok == key) {
-            v0 += o0; v1 += o1; v2 += o2; v3 += o3; v4 += o4;
-        }
-    }
-    const unsigned next = __shfl_down_sync(kFull, key, 1);
-    const bool tail = (lane == 31) || (next != key);
-    if (tail && key != 0xffffffffu) {
-        const size_t M = size_t(s.g.NY) * ph.NRB;
-        const size_t mi = size_t(y) * ph.NRB + (key >> 1);
-        atomicAdd(s.radial + mi, double(v0));
-        atomicAdd(s.radial + M + mi, double(v1));
-        atomicAdd(s.radial + 2 * M + mi, double(v2));
-        atomicAdd(s.radial + 3 * M + mi, double(v3));
-        atomicAdd(s.radial + 4 * M + mi, double(v4));
-    }
-}
-
-// ------------------------------------------------------------------ boundary arithmetic
-
-// The jet boundary columns are written from every fused kernel (and from
-// k_boundary).  Their arithmetic is rounded operation by operation (no
-// contraction into fused multiply-adds, which the compiler chooses per
-// kernel), so that every kernel writes the same bits.  Same formulas as
-// make_eq, make_neq, feq and fneq (lbm.cuh:16-78).
-__device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float rsub(float a, float b) { return __fsub_rn(a, b); }
-
-__device__ __forceinline__ EqTerms bnd_eq(float ux, float uy, float uz) {
-    return EqTerms{ux, uy, uz, radd(radd(rmul(ux, ux), rmul(uy, uy)), rmul(uz, uz))};
-}
-__device__ __forceinline__ NeqTerms bnd_neq(const NodeMoments &m) {
-    NeqTerms n;
-    n.pxx = m.pxx; n.pxy = m.pxy; n.pyy = m.pyy; n.pyz = m.pyz; n.pzz = m.pzz; n.pxz = m.pxz;
-    n.a3xxy = radd(rmul(m.pxx, m.uy), rmul(2.0f * m.pxy, m.ux));
-    n.a3xxz = radd(rmul(m.pxx, m.uz), rmul(2.0f * m.pxz, m.ux));
-    n.a3xyy = radd(rmul(m.pyy, m.ux), rmul(2.0f * m.pxy, m.uy));
-    n.a3xzz = radd(rmul(m.pzz, m.ux), rmul(2.0f * m.pxz, m.uz));
-    n.a3yyz = radd(rmul(m.pyy, m.uz), rmul(2.0f * m.pyz, m.uy));
-    n.a3yzz = radd(rmul(m.pzz, m.uy), rmul(2.0f * m.pyz, m.uz));
-    n.a3xyz = radd(radd(rmul(m.pxy, m.uz), rmul(m.pxz, m.uy)), rmul(m.pyz, m.ux));
-    return n;
-}
-template <int I>
-__device__ __forceinline__ float bnd_feq(float rho, const EqTerms &e) {
-    using D = Dir<I>;
-    float cu = 0.0f;
-    if constexpr (D::cx != 0) cu = radd(cu, D::fx * e.ux);
-    if constexpr (D::cy != 0) cu = radd(cu, D::fy * e.uy);
-    if constexpr (D::cz != 0) cu = radd(cu, D::fz * e.uz);
-    const float cu2 = rmul(cu, cu);
-    const float A2 = radd(rsub(rmul(cu2, kInv2Cs4), rmul(e.usq, kInv2Cs2)), rmul(cu, kInvCs2));
-    const float A3 = rmul(cu, rsub(rmul(cu2, kInv6Cs6), rmul(e.usq, kInv2Cs4)));
-    return rmul(rmul(D::w, rho), radd(radd(1.0f, A2), A3));
-}
-template <int I>
-__device__ __forceinline__ float bnd_fneq(const NeqTerms &n) {
-    using D = Dir<I>;
-    float A2 = 0.0f;
-    if constexpr (D::Hxx != 0.0f) A2 = radd(A2, rmul(n.pxx, D::Hxx));
-    if constexpr (D::Hxy != 0.0f) A2 = radd(A2, rmul(2.0f * n.pxy, D::Hxy));
-    if constexpr (D::Hyy != 0.0f) A2 = radd(A2, rmul(n.pyy, D::Hyy));
-    if constexpr (D::Hyz != 0.0f) A2 = radd(A2, rmul(2.0f * n.pyz, D::Hyz));
-    if constexpr (D::Hzz != 0.0f) A2 = radd(A2, rmul(n.pzz, D::Hzz));
-    if constexpr (D::Hxz != 0.0f) A2 = radd(A2, rmul(2.0f * n.pxz, D::Hxz));
-    A2 = rmul(A2, kInv2Cs4);
-    float A3 = 0.0f;
-    if constexpr (D::Hxxy != 0.0f) A3 = radd(A3, rmul(n.a3xxy, D::Hxxy));
-    if constexpr (D::Hxxz != 0.0f) A3 = radd(A3, rmul(n.a3xxz, D::Hxxz));
-    if constexpr (D::Hxyy != 0.0f) A3 = radd(A3, rmul(n.a3xyy, D::Hxyy));
-    if constexpr (D::Hxzz != 0.0f) A3 = radd(A3, rmul(n.a3xzz, D::Hxzz));
-    if constexpr (D::Hyyz != 0.0f) A3 = radd(A3, rmul(n.a3yyz, D::Hyyz));
-    if constexpr (D::Hyzz != 0.0f) A3 = radd(A3, rmul(n.a3yzz, D::Hyzz));
-    if constexpr (D::Hxyz != 0.0f) A3 = radd(A3, rmul(2.0f * n.a3xyz, D::Hxyz));
-    return rmul(D::w, radd(A2, rmul(A3, kInv2Cs6)));
-}
-// omega_at with the same rounding rule (the outlet's fluid plane)
-__device__ __forceinline__ float bnd_omega_at(const Physics &ph, int y) {
-    if (!ph.sponge) return ph.omega;
-    const float s = clamp01(rmul(float(y) - ph.sponge_y_start, ph.sponge_inv_width));
-    const float nus = rmul(ph.nu, radd(1.0f, rmul(ph.sponge_K, rmul(rmul(s, s), s))));
-    return 1.0f / radd(0.5f, rmul(nus, kInvCs2));
-}
-
-__device__ __forceinline__ NodeMoments load_moments(const float *m, size_t stride, size_t id) {
-    NodeMoments r;
-    r.rr = m[kMomRR * stride + id]; r.rb = m[kMomRB * stride + id];
-    r.ux = m[kMomUX * stride + id]; r.uy = m[kMomUY * stride + id]; r.uz = m[kMomUZ * stride + id];
-    r.pxx = m[kMomPXX * stride + id]; r.pxy = m[kMomPXY * stride + id]; r.pyy = m[kMomPYY * stride + id];
-    r.pyz = m[kMomPYZ * stride + id]; r.pzz = m[kMomPZZ * stride + id]; r.pxz = m[kMomPXZ * stride + id];
-    return r;
-}
-
-// ------------------------------------------------------------------ boundary pieces
-
-// Inlet column (x,z): density mask at y=0 and, for disc columns, the nine
-// cy=+1 populations entering y=1 (jet/boundary_conditions.cuh:17-85).  They
-// are stored in the ghost plane y=0 of `dst` at (x,0,z), where the y=1 nodes
-// (x+cx, 1, z+cz) pull them.  `m` are the moments of fluid node (x,1,z).
-template <class C>
-__device__ __forceinline__ void inlet_column(const DeviceState &s, void *dst, float *psi_dst, int x, int z,
-                                             int64_t step, const NodeMoments &m) {
-    const Geometry &g = s.g;
-    const Physics &ph = s.ph;
-    const uint32_t idB = uint32_t(x) + uint32_t(g.sz) * uint32_t(z);
-    const bool jet = is_jet_column(ph, x, z);
-    const float rrB = (1.0f - (jet ? 1.0f : 0.0f)) * ph.rhor0;
-    const float rbB = (jet ? 1.0f : 0.0f) * ph.rhob0;
-    s.mom[size_t(kMomRR) * g.N + idB] = rrB;
-    s.mom[size_t(kMomRB) * g.N + idB] = rbB;
-    psi_dst[idB] = psi_of(rrB, rbB);
-    if (!jet) return;
-    const float rT = radd(rrB, rbB);
-    const float aR = rmul(rrB, 1.0f / rT), aB = rmul(rbB, 1.0f / rT);
-    const float oms = rsub(1.0f, ph.omega_b);
-    const EqTerms e = bnd_eq(0.0f, inlet_velocity(s, step, x, z), 0.0f);
-    const NeqTerms n = bnd_neq(m);
-    static_for<kQ>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        if constexpr (Dir<i>::cy == 1) {
-            const float gi = radd(bnd_feq<i>(rT, e), rmul(oms, bnd_fneq<i>(n)));
-            C::store_to(dst, g, i, x, 0, z, rmul(aR, gi), rmul(aB, gi), ph.f16_rho0);
-        }
-    });
-}
-
-// Outlet column (x,z): convective update of the y=NY-1 state from fluid node
-// F=(x,NY-2,z) and the nine cy=-1 populations entering y=NY-2
-// (jet/boundary_conditions.cuh:163-233), stored in ghost plane y=NY-1 of dst.
-template <class C>
-__device__ __forceinline__ void outlet_column(const DeviceState &s, void *dst, float *psi_dst, int x, int z,
-                                              const NodeMoments &m) {
-    const Geometry &g = s.g;
-    const Physics &ph = s.ph;
-    const uint32_t idB = uint32_t(x) + uint32_t(g.sy) * uint32_t(g.NY - 1) + uint32_t(g.sz) * uint32_t(z);
-    float *mom = s.mom;
-    const size_t N = g.N;
-    const float uc = clamp01(m.uy);
-    auto conv = [uc](float b, float f) { return rsub(b, rmul(uc, rsub(b, f))); };
-    const float rrB = conv(mom[kMomRR * N + idB], m.rr);
-    const float rbB = conv(mom[kMomRB * N + idB], m.rb);
-    const float uxB = conv(mom[kMomUX * N + idB], m.ux);
-    const float uyB = conv(mom[kMomUY * N + idB], m.uy);
-    const float uzB = conv(mom[kMomUZ * N + idB], m.uz);
-    mom[kMomRR * N + idB] = rrB;
-    mom[kMomRB * N + idB] = rbB;
-    mom[kMomUX * N + idB] = uxB;
-    mom[kMomUY * N + idB] = uyB;
-    mom[kMomUZ * N + idB] = uzB;
-    psi_dst[idB] = psi_of(rrB, rbB);
-    const float rhoT = radd(rrB, rbB);
-    const float inv = 1.0f / rhoT;
-    const float aR = rmul(rrB, inv), aB = rmul(rbB, inv);
-    const float oms = rsub(1.0f, bnd_omega_at(ph, g.NY - 2));
-    const EqTerms e = bnd_eq(uxB, uyB, uzB);
-    const NeqTerms n = bnd_neq(m);
-    static_for<kQ>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        if constexpr (Dir<i>::cy == -1) {
-            const float gi = radd(bnd_feq<i>(rhoT, e), rmul(oms, bnd_fneq<i>(n)));
-            C::store_to(dst, g, i, x, g.NY - 1, z, rmul(aR, gi), rmul(aB, gi), ph.f16_rho0);
-        }
-    });
-}
-
-// ------------------------------------------------------------------ the fused step
-
-constexpr int kFusedThreads = 256;
-// Row lengths the fused kernels are specialised for (the 128-column rows of
-// the 128x256x128 jet, the 256-column rows of the 256x512x256 one); other
-// row lengths take the runtime-geometry kernels.
-constexpr int kFusedNX = 128;
-constexpr int kFusedNX2 = 256;
-
-#ifndef MCG_FUSED_MIN_BLOCKS
-#define MCG_FUSED_MIN_BLOCKS 3  // CTAs per SM the register budget is sized for
-#endif
-
-// First row of this CTA's y-tile.  With the jet boundary in the step the
-// tiles are numbered from the outlet end: the outlet tile's CTAs, which also
-// write the outlet columns, then start first in each chunk instead of last.
-// Neighbouring CTAs still hold neighbouring tiles.
-__device__ __forceinline__ int tile_y0(const FusedTiling &T) {
-    const int t = T.boundary ? T.ny_tiles - 1 - int(blockIdx.x) : int(blockIdx.x);
-    return 1 + t * T.ty;
-}
-
-// Own-row results of a pulled node: the moments into the stage row, the
-// fluid-plane moments for the boundary (fused_boundary or k_boundary), the
-// adjoint's moment record.
-template <class C>
-__device__ __forceinline__ void tile_store_moments(const DeviceState &s, int x, int y, int zp, const NodeMoments &m,
-                                                   float ps, float *msm_row, int tpr) {
-    const Geometry &g = s.g;
-    float *q = msm_row + x;
-    q[kMomRR * tpr] = m.rr;
-    q[kMomRB * tpr] = m.rb;
-    q[kMomUX * tpr] = m.ux;
-    q[kMomUY * tpr] = m.uy;
-    q[kMomUZ * tpr] = m.uz;
-    q[kMomPXX * tpr] = m.pxx;
-    q[kMomPXY * tpr] = m.pxy;
-    q[kMomPYY * tpr] = m.pyy;
-    q[kMomPYZ * tpr] = m.pyz;
-    q[kMomPZZ * tpr] = m.pzz;
-    q[kMomPXZ * tpr] = m.pxz;
-    if (g.boundary == kBoundaryJet && (y == 1 || y == g.NY - 2)) {
-        // fluid-plane moments for the boundary launch
-        float *b = s.bmom + ((size_t(y == 1 ? 0 : 1) * g.NZ + zp) * kMomCount) * g.NX + x;
-        const float v[kMomCount] = {m.rr, m.rb, m.ux, m.uy, m.uz, m.pxx, m.pxy, m.pyy, m.pyz, m.pzz, m.pxz};
-#pragma unroll
-        for (int k = 0; k < kMomCount; ++k) b[size_t(k) * g.NX] = v[k];
-    }
-    if (s.tape) {
-        // moment record of the pulled state (the adjoint sweep reads it)
-        float *t = s.tape + (uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(zp));
-        const size_t N = g.N;
-        const float v[kTapePlanes] = {m.rr, m.rb, m.ux, m.uy, m.uz, m.pxx, m.pxy, m.pyy, m.pyz, m.pzz, m.pxz, ps};
-#pragma unroll
-        for (int k = 0; k < kTapePlanes; ++k) t[size_t(k) * N] = v[k];
-    }
-}
-
-// One node of a tile row in plane zp, pulled in two halves.  tile_pull_issue
-// loads the node's words (at a position that is not pulled, its psi);
-// tile_pull_finish puts psi into `ring_row` (all columns, halo rows
-// included), and for own rows the moments into `msm_row`, the fluid-plane
-// moments for the boundary launch, the adjoint's moment record, and the
-// radial statistics.  tile_pull_finish is warp-collective when kStats: all
-// 32 lanes of a warp (one row) call it together.  TilePull holds the loads
-// between the two.
-template <class C>
-struct TilePull {
-    RawPull<C> raw;  // the node's pulled words, when `pull`
-    float ps;        // psi of a position that is not pulled (ghost)
-    bool pull;
-};
-
-template <class C, bool kPeriodic>
-__device__ __forceinline__ void tile_pull_issue(const DeviceState &s, const C &codec, const float *__restrict__ psi_g,
-                                                int x, int y, int zp, TilePull<C> &t) {
-    const Geometry &g = s.g;
-    t.pull = false;
-    if (x >= g.NX) return;
-    int xn = x, yn = y, zn = zp;
-    if constexpr (kPeriodic) {
-        xn = wrap_interior(x, g.NX);
-        yn = wrap_interior(y, g.NY);
-        zn = wrap_interior(zp, g.NZ);
-        t.pull = true;
-    } else {
-        t.pull = x >= 1 && x <= g.NX - 2 && y >= 1 && y <= g.NY - 2 && zp >= 1 && zp <= g.NZ - 2;
-    }
-    if (t.pull)
-        pull_issue<C, kPeriodic>(g, codec, xn, yn, zn, t.raw);
-    else
-        t.ps = psi_g[uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(zp)];
-}
-
-// A node's statistics sample held for a later radial_accumulate_warp call.
-struct RadialSample {
-    float ux, uy, uz;
-    int y, z;
-    bool active;
-};
-
-template <class C, bool kStats, bool kPeriodic>
-__device__ __forceinline__ void tile_pull_finish(const DeviceState &s, const C &codec, int x, int y, int zp,
-                                                 bool own_row, const TilePull<C> &t, float *ring_row, float *msm_row,
-                                                 int tpr, RadialSample *defer = nullptr) {
-    const Geometry &g = s.g;
-    const bool xin = x >= 1 && x <= g.NX - 2;
-    NodeMoments m{};
-    bool have = false;
-    if (x < g.NX) {
-        float ps;
-        if (t.pull && own_row) {  // own_row is uniform per warp: a warp covers part of one row
-            m = moments_from(RawSource<C>{codec, t.raw});
-            have = true;
-            ps = psi_of(m.rr, m.rb);
-        } else if (t.pull) {
-            float rr, rb;
-            densities_from(RawSource<C>{codec, t.raw}, rr, rb);
-            ps = psi_of(rr, rb);
-        } else {
-            ps = t.ps;
-        }
-        ring_row[x] = ps;
-        if (own_row && xin) tile_store_moments<C>(s, x, y, zp, m, ps, msm_row, tpr);
-    }
-    if constexpr (kStats) {
-        if (defer) {
-            *defer = RadialSample{m.ux, m.uy, m.uz, y, zp, have && xin};
-        } else if (own_row) {
-            radial_accumulate_warp(s, x, y, zp, have && xin, m.ux, m.uy, m.uz);
-        }
-    }
-}
-
-// tile_pull_issue + tile_pull_finish in one piece, for marches with nothing
-// to overlap: the own-row / halo branch comes before the loads, so each
-// branch consumes its loads as they arrive (issuing all of them before the
-// branch keeps every word live at once and spills at 80 registers).
-template <class C, bool kStats, bool kPeriodic>
-__device__ __forceinline__ void tile_pull(const DeviceState &s, const C &codec, const float *__restrict__ psi_g, int x,
-                                          int y, int zp, bool own_row, float *ring_row, float *msm_row, int tpr) {
-    const Geometry &g = s.g;
-    const bool xin = x >= 1 && x <= g.NX - 2;
-    NodeMoments m{};
-    bool have = false;
-    if (x < g.NX) {
-        int xn = x, yn = y, zn = zp;
-        bool pull;
-        if constexpr (kPeriodic) {
-            xn = wrap_interior(x, g.NX);
-            yn = wrap_interior(y, g.NY);
-            zn = wrap_interior(zp, g.NZ);
-            pull = true;
-        } else {
-            pull = xin && y >= 1 && y <= g.NY - 2 && zp >= 1 && zp <= g.NZ - 2;
-        }
-        float ps;
-        if (pull && own_row) {  // uniform per warp: a warp covers part of one row
-            m = pull_moments<C, kPeriodic>(g, codec, xn, yn, zn);
-            have = true;
-            ps = psi_of(m.rr, m.rb);
-        } else if (pull) {
-            float rr, rb;
-            pull_densities<C, kPeriodic>(g, codec, xn, yn, zn, rr, rb);
-            ps = psi_of(rr, rb);
-        } else {
-            ps = psi_g[uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(zp)];
-        }
-        ring_row[x] = ps;
-        if (own_row && xin) tile_store_moments<C>(s, x, y, zp, m, ps, msm_row, tpr);
-    }
-    if constexpr (kStats) {
-        if (own_row) radial_accumulate_warp(s, x, y, zp, have && xin, m.ux, m.uy, m.uz);
-    }
-}
-
-// Relax interior node (x, y, zc) of a tile: moments from the stage row
-// `msm_row`, psi of planes zc-1, zc, zc+1 from the ring planes pm, p0, pp at
-// ring row r.
-template <class C>
-__device__ __forceinline__ void tile_collide(const DeviceState &s, const C &codec, int x, int y, int zc, int r,
-                                             const float *msm_row, const float *pm, const float *p0, const float *pp,
-                                             int tpr) {
-    const Geometry &g = s.g;
-    const float *q = msm_row + x;
-    NodeMoments m;
-    m.rr = q[kMomRR * tpr];
-    m.rb = q[kMomRB * tpr];
-    m.ux = q[kMomUX * tpr];
-    m.uy = q[kMomUY * tpr];
-    m.uz = q[kMomUZ * tpr];
-    m.pxx = q[kMomPXX * tpr];
-    m.pxy = q[kMomPXY * tpr];
-    m.pyy = q[kMomPYY * tpr];
-    m.pyz = q[kMomPYZ * tpr];
-    m.pzz = q[kMomPZZ * tpr];
-    m.pxz = q[kMomPXZ * tpr];
-    const int base = r * tpr + x;
-    auto psi_at = [&](int cx, int cy, int cz) {
-        const float *pl = cz < 0 ? pm : (cz > 0 ? pp : p0);
-        return pl[base + cy * tpr + cx];
-    };
-    collide_node(g, s.ph, codec, pop_row(g, y, zc), x, y, zc, m, psi_at);
-}
-
-// The jet boundary of a fused step, from the CTAs whose tile holds fluid row
-// 1 (inlet) or NY-2 (outlet), once their march is over: every column of the
-// chunk from the fluid-plane moments the march left in bmom (written by this
-// CTA's threads, visible after the barrier), into the ghost planes of the
-// buffer the step writes and the next step's psi.  A column touches only its
-// own ghost nodes and the outlet state it carries, which no other CTA of the
-// launch reads.  Kept out of the march, where it added its instructions to
-// every row.  The condition is uniform over the CTA.
-template <class C>
-__device__ __forceinline__ void fused_boundary(const DeviceState &s, const FusedTiling &T, int y0, int ty, int z0,
-                                               int lz) {
-    const Geometry &g = s.g;
-    const bool inlet = y0 == 1, outlet = y0 + ty - 1 == g.NY - 2;
-    if (!T.boundary || !(inlet || outlet)) return;
-    __syncthreads();
-    const int nx = g.NX - 2;
-    for (int side = 0; side < 2; ++side) {
-        if (!(side == 0 ? inlet : outlet)) continue;
-        for (int i = threadIdx.x; i < lz * nx; i += blockDim.x) {
-            const int x = 1 + i % nx, z = z0 + i / nx;
-            const NodeMoments m =
-                load_moments(s.bmom + (size_t(side) * g.NZ + z) * kMomCount * g.NX, size_t(g.NX), size_t(x));
-            if (side == 0)
-                inlet_column<C>(s, T.bnd_dst, T.bnd_psi, x, z, int64_t(T.bnd_step), m);
-            else
-                outlet_column<C>(s, T.bnd_dst, T.bnd_psi, x, z, m);
-        }
-    }
-}
-
-// Geometry of a fused launch: with kNX > 0 (rows of exactly kNX columns, one
-// thread per column) the row length and slot counts are compile-time
-// constants, so population, slot and shared-memory offsets fold into the
-// loads' immediate offsets.
-template <class C, int kNX>
-__device__ __forceinline__ DeviceState fused_state(const DeviceState &s) {
-    DeviceState l = s;
-    if constexpr (kNX > 0) {
-        l.g.NX = kNX;
-        l.g.sy = kNX;
-        l.g.slots = 9 * C::kGroupSlots;
-    }
-    return l;
-}
-template <class C, int kNX>
-__device__ __forceinline__ C fused_codec(const DeviceState &s, int cur) {
-    C c = make_codec<C>(s, cur);
-    if constexpr (kNX > 0) c.NX = kNX;
-    return c;
-}
-
-template <class C, bool kStats, bool kPeriodic, int kNX>
-__global__ void __launch_bounds__(kFusedThreads, MCG_FUSED_MIN_BLOCKS) k_fused(const DeviceState s_arg,
-                                                                              const FusedTiling T, int cur,
-                                                                              int64_t step) {
-    extern __shared__ float sm[];
-    const DeviceState s = fused_state<C, kNX>(s_arg);
-    const Geometry &g = s.g;
-    const int tpr = kNX > 0 ? kNX : T.tpr;
-    const int rpt = kFusedThreads / tpr;
-    // row group of this thread; groups beyond rpt (when tpr does not divide
-    // the block) start past every row and only take part in the barriers
-    const int lr0 = threadIdx.x / tpr;
-    const int lr = lr0 < rpt ? lr0 : T.ty + 2;
-    const int x = threadIdx.x - lr0 * tpr;
-    const int y0 = tile_y0(T);
-    const int ty = min(T.ty, g.NY - 1 - y0);
-    const int z0 = 1 + int(blockIdx.y) * T.lz;
-    const int lz = min(T.lz, g.NZ - 1 - z0);
-    const int pstride = (T.ty + 2) * tpr;  // one psi plane of the ring
-    float *ring = sm;                      // [3][ty+2][tpr]
-    float *msm = sm + 3 * pstride;         // [2][ty][11][tpr]
-    const int mplane = T.ty * kMomCount * tpr;
-    const C codec = fused_codec<C, kNX>(s_arg, cur);
-    const float *__restrict__ psi_g = s_arg.psi[step & 1];  // indexed on the parameter, not the local copy
-    const bool xin = x >= 1 && x <= g.NX - 2;
-    // Odd chunks march down: the plane two neighbouring chunks both pull (one
-    // as its halo, one as its own) is then pulled by both at the same end of
-    // their marches, close in time, and the second pull finds it in L2.
-    const bool down = T.alternate && (blockIdx.y & 1);
-    for (int k = 0; k <= lz + 1; ++k) {
-        const int zp = down ? z0 + lz - k : z0 - 1 + k;
-        float *ringp = ring + (zp % 3) * pstride;
-        float *msmp = msm + (zp & 1) * mplane;
-        const bool own_plane = zp >= z0 && zp < z0 + lz;
-        // ---- pull plane zp: psi for rows y0-1 .. y0+ty, moments for own rows
-        for (int r = lr; r < ty + 2; r += rpt) {
-            tile_pull<C, kStats, kPeriodic>(s, codec, psi_g, x, y0 - 1 + r, zp, own_plane && r >= 1 && r <= ty,
-                                            ringp + r * tpr, msmp + (r - 1) * kMomCount * tpr, tpr);
-        }
-        __syncthreads();
-        // ---- relax the plane behind the march front, whose neighbours are all pulled
-        const int zc = down ? zp + 1 : zp - 1;
-        if (zc >= z0 && zc < z0 + lz) {
-            const float *pm = ring + ((zc + 2) % 3) * pstride;  // plane zc-1
-            const float *p0 = ring + (zc % 3) * pstride;        // plane zc
-            const float *pp = ring + ((zc + 1) % 3) * pstride;  // plane zc+1
-            const float *mc = msm + (zc & 1) * mplane;
-            for (int r = 1 + lr; r <= ty; r += rpt) {
-                if (!xin) continue;
-                tile_collide(s, codec, x, y0 - 1 + r, zc, r, mc + (r - 1) * kMomCount * tpr, pm, p0, pp, tpr);
-            }
-        }
-        __syncthreads();
-    }
-    fused_boundary<C>(s, T, y0, ty, z0, lz);
-}
-
-// ------------------------------------------------------------------ software-pipelined fused step
-
-// The tile march of k_fused with the pull and the relaxation in the same
-// phase: iteration k pulls march plane k and relaxes march plane k-2, whose
-// psi neighbours (planes k-3 .. k-1) and moments were pulled in earlier
-// iterations.  The pull writes ring slot k mod 4 and stage slot k mod 3; the
-// relaxation reads ring slots k-3 .. k-1 and stage slot k-2 - all different -
-// so one __syncthreads per iteration suffices.  Between barriers the warps of
-// a CTA drift apart, and the memory-bound pull of one warp overlaps the
-// ALU-bound relaxation of another.
-constexpr int kPipeRing = 4, kPipeStage = 3;
-// CTAs per SM the pipelined kernel's register budget is sized for: float32
-// (3-row tiles, 3 CTAs, 80 registers) measured faster than 2 CTAs at 128
-// registers; float16 keeps 2 (its words in flight across the relaxation need
-// the registers).
-template <class C>
-struct PipeBlocks {
-    static constexpr int value = std::is_same<C, CodecF16>::value ? 2 : 3;
-};
-
-template <class C, bool kStats, bool kPeriodic, int kNX>
-__global__ void __launch_bounds__(kFusedThreads, PipeBlocks<C>::value) k_fused_pipe(const DeviceState s_arg,
-                                                                                  const FusedTiling T, int cur,
-                                                                                  int64_t step) {
-    extern __shared__ float sm[];
-    const DeviceState s = fused_state<C, kNX>(s_arg);
-    const Geometry &g = s.g;
-    const int tpr = kNX > 0 ? kNX : T.tpr;
-    const int rpt = kFusedThreads / tpr;
-    const int lr0 = threadIdx.x / tpr;
-    const int lr = lr0 < rpt ? lr0 : T.ty + 2;  // idle groups (tpr not dividing the block) skip every row
-    const int x = threadIdx.x - lr0 * tpr;
-    const int pstride = (T.ty + 2) * tpr;
-    const int mplane = T.ty * kMomCount * tpr;
-    float *ring = sm;                        // [4][ty+2][tpr]
-    float *msm = sm + kPipeRing * pstride;   // [3][ty][11][tpr]
-    const C codec = fused_codec<C, kNX>(s_arg, cur);
-    const float *__restrict__ psi_g = s_arg.psi[step & 1];  // indexed on the parameter, not the local copy
-    const bool xin = x >= 1 && x <= g.NX - 2;
-    // Float16 words (27 registers a node) stay in flight across the relaxation
-    // of another row: measured +4 % on 128x256x128.  Float32 (27 float2, 54
-    // registers) pulls then relaxes: its 3-CTA, 80-register default is faster
-    // than the overlap, which spills there.
-    constexpr bool kOverlap = std::is_same<C, CodecF16>::value;
-    // One CTA per y-tile (blockIdx.x) and z chunk (blockIdx.y): CTAs of
-    // neighbouring y-tiles run the same planes at about the same time, so the
-    // halo rows one pulls are the own rows another pulled and hit L2.  Odd
-    // chunks march down: two neighbouring chunks then pull their shared
-    // boundary plane at the same end of their marches (L2 again).
-    {
-        const int y0 = tile_y0(T);
-        const int z0 = 1 + int(blockIdx.y) * T.lz;
-        const int lz = min(T.lz, g.NZ - 1 - z0);
-        const bool down = T.alternate && (blockIdx.y & 1);
-        const int ty = min(T.ty, g.NY - 1 - y0);
-        auto plane = [&](int k) { return down ? z0 + lz - k : z0 - 1 + k; };
-        RadialSample held{};   // statistics of this warp's last own row, taken
-        bool pending = false;  // after the next row's loads are issued
-        for (int k = 0; k <= lz + 2; ++k) {
-            const bool do_pull = k <= lz + 1;
-            const int c = k - 2;  // march index of the plane relaxed in this iteration
-            const bool do_relax = c >= 1 && c <= lz;
-            const int zp = plane(k);
-            float *ringp = ring + (k % kPipeRing) * pstride;
-            float *msmp = msm + (k % kPipeStage) * mplane;
-            const bool own_plane = k >= 1 && k <= lz;
-            const int zc = plane(c);
-            const float *pm = ring + (((down ? c + 1 : c - 1) + kPipeRing) % kPipeRing) * pstride;  // plane zc-1
-            const float *p0 = ring + ((c + kPipeRing) % kPipeRing) * pstride;                       // plane zc
-            const float *pp = ring + (((down ? c - 1 : c + 1) + kPipeRing) % kPipeRing) * pstride;  // plane zc+1
-            const float *mc = msm + ((c + kPipeStage) % kPipeStage) * mplane;
-            // rows of this thread: pull rows lr, lr+rpt, ... (< ty+2) and relax rows
-            // 1+lr, 1+lr+rpt, ... (<= ty), interleaved so that a warp has loads of
-            // one row in flight while it relaxes another.  With one row group (rows
-            // of 256 columns) the upper half of the row's threads takes the rows in
-            // a rotated order, so that one half pulls while the other relaxes, as
-            // two row groups do; the order of the rows within an iteration is free.
-            // (split at a warp boundary: the statistics are warp-collective)
-            const int rot = (rpt == 1 && x >= (tpr / 64) * 32) ? (ty + 2) / 2 : 0;
-            for (int ri = lr; ri < ty + 2; ri += rpt) {
-                const int r = rot ? (ri + rot) % (ty + 2) : ri;
-                const bool own = own_plane && r >= 1 && r <= ty;
-                const int rc = r + 1;
-                if constexpr (kOverlap) {
-                    // the loads of row r are in flight while this warp takes the
-                    // statistics of its previous own row and relaxes row r+1
-                    TilePull<C> tp;
-                    if (do_pull) tile_pull_issue<C, kPeriodic>(s, codec, psi_g, x, y0 - 1 + r, zp, tp);
-                    if constexpr (kStats) {
-                        if (pending) {  // warp-uniform
-                            radial_accumulate_warp(s, x, held.y, held.z, held.active, held.ux, held.uy, held.uz);
-                            pending = false;
-                        }
-                    }
-                    if (do_relax && rc <= ty && xin)
-                        tile_collide(s, codec, x, y0 - 1 + rc, zc, rc, mc + (rc - 1) * kMomCount * tpr, pm, p0, pp,
-                                     tpr);
-                    if (do_pull) {
-                        tile_pull_finish<C, kStats, kPeriodic>(s, codec, x, y0 - 1 + r, zp, own, tp, ringp + r * tpr,
-                                                               msmp + (r - 1) * kMomCount * tpr, tpr,
-                                                               kStats && own ? &held : nullptr);
-                        if (kStats && own) pending = true;
-                    }
-                } else {
-                    if (do_pull)
-                        tile_pull<C, kStats, kPeriodic>(s, codec, psi_g, x, y0 - 1 + r, zp, own, ringp + r * tpr,
-                                                        msmp + (r - 1) * kMomCount * tpr, tpr);
-                    if (do_relax && rc <= ty && xin)
-                        tile_collide(s, codec, x, y0 - 1 + rc, zc, rc, mc + (rc - 1) * kMomCount * tpr, pm, p0, pp,
-                                     tpr);
-                }
-            }
-            __syncthreads();
-        }
-        if constexpr (kStats) {
-            if (pending) radial_accumulate_warp(s, x, held.y, held.z, held.active, held.ux, held.uy, held.uz);
-        }
-        fused_boundary<C>(s, T, y0, ty, z0, lz);
-    }
-}
-
-// ------------------------------------------------------------------ bulk-staged pipelined fused step
-
-// One-dimensional bulk copies (cp.async.bulk, no multicast) into shared
-// memory, completed on an mbarrier; one GPU, the CTA's own shared memory.
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-// Waits for the phase of parity `parity` of `bar` to complete: at most
-// `limit` tries, each suspending the thread for about a microsecond at most.
-// Returns false when the limit ran out (limit 0: at once).
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32_t limit) {
-    for (uint32_t i = 0; i < limit; ++i) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-// Barrier of the `count` threads of one row group (named barrier `id` > 0);
-// returns the OR of `pred` over them.
-__device__ __forceinline__ bool group_barrier_or(int id, int count, bool pred) {
-    uint32_t out;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, %2, %3, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(out)
-        : "r"(uint32_t(pred)), "r"(id), "r"(count)
-        : "memory");
-    return out != 0;
-}
-
-// Row image of a staged pull: the 9 (cy, cz) source segments of row (y, z)
-// (3 slots x NX elements each, group g = dir_group at g*3*NX), copied
-// verbatim from the population buffer.  Direction I of node x reads slot
-// (g, cx+1) at column x - cx, with the lateral wrap of PullMap: columns 1
-// and NX-2 wrap for cx = +1 / -1, except in a segment that comes from a y
-// ghost plane (the boundary's unwrapped slots).
-template <class C, int kNX>
-struct StagedRow {
-    const typename C::Elem *img;
-    int x;
-    int wxp, wxm;
-    bool gy_p, gy_m;
-    __device__ __forceinline__ StagedRow(const typename C::Elem *img_, int x_, int y, const Geometry &g, bool periodic)
-        : img(img_), x(x_) {
-        wxp = (x == 1) ? (kNX - 2) : 0;
-        wxm = (x == kNX - 2) ? -(kNX - 2) : 0;
-        gy_p = !periodic && y == 1;
-        gy_m = !periodic && y == g.NY - 2;
-    }
-    template <int I>
-    __device__ __forceinline__ typename C::Raw load() const {
-        using D = Dir<I>;
-        int xc = 0;
-        if constexpr (D::cx == 1) xc = wxp;
-        if constexpr (D::cx == -1) xc = wxm;
-        if constexpr (D::cy == 1) xc = gy_p ? 0 : xc;
-        if constexpr (D::cy == -1) xc = gy_m ? 0 : xc;
-        return img[(dir_group(I) * C::kGroupSlots + D::cx + 1) * kNX + x - D::cx + xc];
-    }
-};
-
-// Issues the 9 segment copies of pulled row (y, z) (own coordinates, wrapped
-// for the periodic box) into `img`, completing on `bar`.
-template <class C, int kNX>
-__device__ __forceinline__ void stage_row(const Geometry &g, const C &codec, bool periodic, int y, int z,
-                                          typename C::Elem *img, uint64_t *bar) {
-    constexpr uint32_t seg = uint32_t(C::kGroupSlots * kNX * sizeof(typename C::Elem));
-    mbar_expect_tx(bar, 9 * seg);
-    for (int grp = 0; grp < 9; ++grp) {
-        const int cy = grp / 3 - 1, cz = grp % 3 - 1;
-        int ys = y - cy, zs = z - cz;
-        const bool ghost = !periodic && (ys == 0 || ys == g.NY - 1);
-        if (!ghost) {
-            zs = wrap_interior(zs, g.NZ);
-            if (periodic) ys = wrap_interior(ys, g.NY);
-        }
-        const typename C::Elem *src =
-            codec.rd + ((size_t(zs) * g.NY + ys) * kQ + size_t(grp) * C::kGroupSlots) * kNX;
-        bulk_copy_g2s(img + grp * C::kGroupSlots * kNX, src, seg, bar);
-    }
-}
-
-// The pipelined march of k_fused_pipe with each pulled row staged: the 9
-// source segments of a row (3 KB each in float32 at 128 columns) arrive in
-// shared memory by bulk copies while the row group (the 128 threads of one
-// row, 4 warps) finishes its previous row and relaxes another.  Each row
-// group owns one row image and one mbarrier; after its threads have read the
-// image into registers (a barrier of the group), its first thread issues the
-// copies of the group's next pulled row.  Pulls therefore hold no global
-// loads in registers.  Ghost rows and planes are not pulled (psi from HBM).
-// The pulled words, their order and the arithmetic are those of
-// k_fused_pipe, so the results are bit-identical.
-// Every wait has an iteration limit (T.wait_limit tries of about 1 us): when
-// it runs out, the group sets flag[1], issues nothing more and finishes the
-// march on whatever its image holds; before it exits, the group's first
-// thread waits (again bounded) for the copies it has in flight.
-constexpr int kBulkBarBytes = 128;  // mbarriers at the start of the shared memory
-template <class C>
-constexpr int bulk_image_bytes() { return kQ * kFusedNX * int(sizeof(typename C::Elem)); }
-
-template <class C, bool kStats, bool kPeriodic>
-__global__ void __launch_bounds__(kFusedThreads, 2) k_fused_bulk(const DeviceState s_arg, const FusedTiling T,
-                                                                 int cur, int64_t step) {
-    constexpr int kNX = kFusedNX;
-    constexpr int tpr = kNX;
-    constexpr int rpt = kFusedThreads / tpr;  // row groups
-    using E = typename C::Elem;
-    extern __shared__ __align__(128) unsigned char smb[];
-    const DeviceState s = fused_state<C, kNX>(s_arg);
-    const Geometry &g = s.g;
-    const int grp = threadIdx.x / tpr;
-    const int x = threadIdx.x - grp * tpr;
-    const bool leader = x == 0;
-    const int pstride = (T.ty + 2) * tpr;
-    const int mplane = T.ty * kMomCount * tpr;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smb) + grp;
-    E *img = reinterpret_cast<E *>(smb + kBulkBarBytes) + grp * (kQ * kNX);
-    float *ring = reinterpret_cast<float *>(smb + kBulkBarBytes + rpt * bulk_image_bytes<C>());  // [4][ty+2][tpr]
-    float *msm = ring + kPipeRing * pstride;                                                    // [3][ty][11][tpr]
-    const C codec = fused_codec<C, kNX>(s_arg, cur);
-    const float *__restrict__ psi_g = s_arg.psi[step & 1];
-    const bool xin = x >= 1 && x <= kNX - 2;
-    const int y0 = tile_y0(T);
-    const int z0 = 1 + int(blockIdx.y) * T.lz;
-    const int lz = min(T.lz, g.NZ - 1 - z0);
-    const bool down = T.alternate && (blockIdx.y & 1);
-    const int ty = min(T.ty, g.NY - 1 - y0);
-    auto plane = [&](int k) { return down ? z0 + lz - k : z0 - 1 + k; };
-    // a row of the march that is pulled (the periodic box pulls every row,
-    // ghost rows as their wrapped interior rows)
-    auto pulled = [&](int k, int r) {
-        if constexpr (kPeriodic) return true;
-        const int y = y0 - 1 + r, z = plane(k);
-        return y >= 1 && y <= g.NY - 2 && z >= 1 && z <= g.NZ - 2;
-    };
-    // the group's next pulled row after (k, r); k > lz+1 when there is none
-    auto next_pull = [&](int &k, int &r) {
-        do {
-            r += rpt;
-            if (r >= ty + 2) {
-                r = grp;
-                ++k;
-            }
-        } while (k <= lz + 1 && !pulled(k, r));
-    };
-    auto issue = [&](int k, int r) {
-        int y = y0 - 1 + r, z = plane(k);
-        if constexpr (kPeriodic) {
-            y = wrap_interior(y, g.NY);
-            z = wrap_interior(z, g.NZ);
-        }
-        stage_row<C, kNX>(g, codec, kPeriodic, y, z, img, bar);
-    };
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < rpt; ++k) mbar_init(reinterpret_cast<uint64_t *>(smb) + k, 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    const uint32_t limit = uint32_t(T.wait_limit);
-    bool failed = false;    // uniform over the row group
-    bool in_flight = false; // leader: copies issued and not yet waited for
-    uint32_t parity = 0;     // of the next phase this thread waits for
-    if (leader && grp < ty + 2) {
-        int k = 0, r = grp;
-        if (!pulled(k, r)) next_pull(k, r);
-        if (k <= lz + 1) {
-            issue(k, r);
-            in_flight = true;
-        }
-    }
-    for (int k = 0; k <= lz + 2; ++k) {
-        const bool do_pull = k <= lz + 1;
-        const int c = k - 2;
-        const bool do_relax = c >= 1 && c <= lz;
-        const int zp = plane(k);
-        float *ringp = ring + (k % kPipeRing) * pstride;
-        float *msmp = msm + (k % kPipeStage) * mplane;
-        const bool own_plane = k >= 1 && k <= lz;
-        const int zc = plane(c);
-        const float *pm = ring + (((down ? c + 1 : c - 1) + kPipeRing) % kPipeRing) * pstride;
-        const float *p0 = ring + ((c + kPipeRing) % kPipeRing) * pstride;
-        const float *pp = ring + (((down ? c - 1 : c + 1) + kPipeRing) % kPipeRing) * pstride;
-        const float *mc = msm + ((c + kPipeStage) % kPipeStage) * mplane;
-        for (int r = grp; r < ty + 2; r += rpt) {
-            const bool own = own_plane && r >= 1 && r <= ty;
-            const int y = y0 - 1 + r;
-            if (do_pull) {
-                if (pulled(k, r)) {
-                    bool late = false;
-                    if (!failed) {
-                        late = !mbar_wait(bar, parity, limit);
-                        if (!late) {
-                            parity ^= 1u;
-                            if (leader) in_flight = false;  // the copies have landed
-                        }
-                    }
-                    int xn = x, yn = y, zn = zp;
-                    if constexpr (kPeriodic) {
-                        xn = wrap_interior(x, kNX);
-                        yn = wrap_interior(y, g.NY);
-                        zn = wrap_interior(zp, g.NZ);
-                    }
-                    const bool pull = kPeriodic || xin;
-                    RawPull<C> raw;
-                    if (pull) {
-                        const StagedRow<C, kNX> src(img, xn, yn, g, kPeriodic);
-                        static_for<kQ>([&](auto I) {
-                            constexpr int i = decltype(I)::value;
-                            raw.v[i] = src.template load<i>();
-                        });
-                    }
-                    // every thread of the group has read the image
-                    const bool now_failed = group_barrier_or(1 + grp, tpr, late);
-                    if (now_failed && !failed) {
-                        failed = true;
-                        if (leader) atomicExch(s.flag + 1, 1);
-                    }
-                    if (leader && !failed) {
-                        int kn = k, rn = r;
-                        next_pull(kn, rn);
-                        if (kn <= lz + 1) {
-                            issue(kn, rn);
-                            in_flight = true;
-                        }
-                    }
-                    NodeMoments m{};
-                    float ps = 0.0f;
-                    if (pull && own) {  // own is uniform per warp
-                        m = moments_from(RawSource<C>{codec, raw});
-                        ps = psi_of(m.rr, m.rb);
-                    } else if (pull) {
-                        float rr, rb;
-                        densities_from(RawSource<C>{codec, raw}, rr, rb);
-                        ps = psi_of(rr, rb);
-                    } else {
-                        ps = psi_g[uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(zp)];
-                    }
-                    ringp[r * tpr + x] = ps;
-                    if (own && xin)
-                        tile_store_moments<C>(s, x, y, zp, m, ps, msmp + (r - 1) * kMomCount * tpr, tpr);
-                    if constexpr (kStats) {
-                        if (own) radial_accumulate_warp(s, x, y, zp, pull && xin, m.ux, m.uy, m.uz);
-                    }
-                } else {
-                    ringp[r * tpr + x] =
-                        psi_g[uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(zp)];
-                }
-            }
-            const int rc = r + 1;
-            if (do_relax && rc <= ty && xin)
-                tile_collide(s, codec, x, y0 - 1 + rc, zc, rc, mc + (rc - 1) * kMomCount * tpr, pm, p0, pp, tpr);
-        }
-        __syncthreads();
-    }
-    // copies still in flight after a wait ran out land before the CTA exits
-    if (leader && in_flight) mbar_wait(bar, parity, limit > 0 ? limit : kBulkDrainLimit);
-    fused_boundary<C>(s, T, y0, ty, z0, lz);
-}
-
-// Shared memory of k_fused_bulk with `ty`-row tiles: mbarriers, one row image
-// per row group, the psi ring and the moment stage of k_fused_pipe.
-template <class C>
-constexpr int bulk_smem_for(int ty) {
-    return kBulkBarBytes + (kFusedThreads / kFusedNX) * bulk_image_bytes<C>() +
-           (kPipeRing * (ty + 2) + kPipeStage * kMomCount * ty) * kFusedNX * 4;
-}
-// rows per tile of k_fused_bulk: float32 2 (3 KB segments, 27 KB images),
-// float16 4; both fit two CTAs per SM
-template <class C>
-constexpr int bulk_rows() { return std::is_same<C, CodecF16>::value ? 4 : 2; }
-template <class C>
-constexpr int bulk_smem_bytes() { return bulk_smem_for<C>(bulk_rows<C>()); }
 
 // ------------------------------------------------------------------ granular sequence
 
@@ -1601,7 +77,7 @@ __global__ void __launch_bounds__(kBX * kBY, 4) k_collide(const DeviceState s, c
     m.pxz = __ldg(mom + kMomPXZ * N + id);
     const float *__restrict__ psi = s.psi[step & 1];
     auto psi_at = [&](int cx, int cy, int cz) { return __ldg(psi + (int(id) + cx + g.sy * cy + g.sz * cz)); };
-    collide_node(g, s.ph, codec, pop_row(g, y, z), x, y, z, m, psi_at);
+    collide_node<false>(g, s.ph, codec, pop_row(g, y, z), x, y, z, m, psi_at);
 }
 
 
@@ -1946,59 +422,6 @@ unsigned grid1(const Geometry &g) {
 }
 
 
-template <class C, bool kStats, bool kPeriodic, int kNX>
-cudaError_t fused_attr_nx(int smem) {
-    cudaError_t e = cudaFuncSetAttribute(k_fused<C, kStats, kPeriodic, kNX>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_fused_pipe<C, kStats, kPeriodic, kNX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                smem);
-}
-
-template <class C, bool kStats, bool kPeriodic>
-cudaError_t fused_attr(int smem) {
-    cudaError_t e = fused_attr_nx<C, kStats, kPeriodic, 0>(smem);
-    if (e != cudaSuccess) return e;
-    e = fused_attr_nx<C, kStats, kPeriodic, kFusedNX>(smem);
-    if (e != cudaSuccess) return e;
-    e = fused_attr_nx<C, kStats, kPeriodic, kFusedNX2>(smem);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_fused_bulk<C, kStats, kPeriodic>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                bulk_smem_bytes<C>());
-}
-
-template <class C, bool kStats, bool kPeriodic, int kNX>
-cudaError_t fused_launch_nx(const DeviceState &s, const FusedTiling &t, int cur, int64_t step, cudaStream_t st) {
-    if constexpr (kNX == kFusedNX) {
-        if (t.bulk) {
-            k_fused_bulk<C, kStats, kPeriodic>
-                <<<dim3(t.ny_tiles, t.nz_chunks), dim3(kFusedThreads), size_t(t.smem_bytes), st>>>(s, t, cur, step);
-            return cudaGetLastError();
-        }
-    }
-    if (t.pipe) {
-        k_fused_pipe<C, kStats, kPeriodic, kNX>
-            <<<dim3(t.ny_tiles, t.nz_chunks), dim3(kFusedThreads), size_t(t.smem_bytes), st>>>(s, t, cur, step);
-        return cudaGetLastError();
-    }
-    k_fused<C, kStats, kPeriodic, kNX>
-        <<<dim3(t.ny_tiles, t.nz_chunks), dim3(kFusedThreads), size_t(t.smem_bytes), st>>>(s, t, cur, step);
-    return cudaGetLastError();
-}
-
-template <class C, bool kStats, bool kPeriodic>
-cudaError_t fused_launch(const DeviceState &s, const FusedTiling &t, int cur, int64_t step, cudaStream_t st) {
-    if (t.fixed_nx == kFusedNX) return fused_launch_nx<C, kStats, kPeriodic, kFusedNX>(s, t, cur, step, st);
-    if (t.fixed_nx == kFusedNX2) return fused_launch_nx<C, kStats, kPeriodic, kFusedNX2>(s, t, cur, step, st);
-    return fused_launch_nx<C, kStats, kPeriodic, 0>(s, t, cur, step, st);
-}
-
-template <class C, bool kStats>
-cudaError_t fused_dispatch(const DeviceState &s, const FusedTiling &t, int cur, int64_t step, cudaStream_t st) {
-    if (s.g.boundary == kBoundaryPeriodic) return fused_launch<C, kStats, true>(s, t, cur, step, st);
-    return fused_launch<C, kStats, false>(s, t, cur, step, st);
-}
-
 template <class C>
 cudaError_t moments_dispatch(const DeviceState &s, int cur, int64_t step, cudaStream_t st) {
     const C codec = make_codec<C>(s, cur);
@@ -2101,7 +524,7 @@ __global__ void __launch_bounds__(kBX * kBY) k_adj_terminal(const DeviceState s,
             size_t grow;
             int xs;
             pm.template src<i>(x, grow, xs);
-            reinterpret_cast<float2 *>(lam)[grow + size_t(dir_cx(i) + 1) * g.NX + xs] = make_float2(lrr, lrb);
+            reinterpret_cast<float2 *>(lam)[grow + size_t(dir_cx(i) + 1) * g.px + xs] = make_float2(lrr, lrb);
         });
     }
     const double r = block_sum_any(jloc, sh, kBX * kBY);
@@ -2244,7 +667,7 @@ __global__ void __launch_bounds__(kBX * kBY, 2) k_adj_collide(const DeviceState 
         const size_t row = pop_row(g, y, z);
         // (lambda_r, lambda_b) of a direction: one float2, as the populations
         auto lam_at = [&](int slot) {
-            return reinterpret_cast<const float2 *>(lam)[row + size_t(slot) * size_t(g.NX) + size_t(x)];
+            return reinterpret_cast<const float2 *>(lam)[row + size_t(slot) * size_t(g.px) + size_t(x)];
         };
         // Bulk part: g_i = w_i P(c_i) with P the collision polynomial, so the
         // sums over directions are the polynomial's coefficients dotted with
@@ -2498,7 +921,7 @@ __global__ void __launch_bounds__(kBX * kBY) k_adj_moments(const DeviceState s, 
                 size_t grow;
                 int xs;
                 pm.template src<i>(x, grow, xs);
-                reinterpret_cast<float2 *>(lam_out)[grow + size_t(dir_cx(i) + 1) * g.NX + xs] =
+                reinterpret_cast<float2 *>(lam_out)[grow + size_t(dir_cx(i) + 1) * g.px + xs] =
                     make_float2(lrr + lgi, lrb + lgi);
             });
         });
@@ -2779,7 +1202,7 @@ __global__ void __launch_bounds__(kBX * kBY) k_adj_initial(const DeviceState s, 
         size_t grow;
         int xs;
         pm.template src<i>(x, grow, xs);
-        const float2 l = reinterpret_cast<const float2 *>(lam0)[grow + size_t(dir_cx(i) + 1) * g.NX + xs];
+        const float2 l = reinterpret_cast<const float2 *>(lam0)[grow + size_t(dir_cx(i) + 1) * g.px + xs];
         const float lr = l.x, lb = l.y;
         float cu = 0.f;
         if constexpr (D::cx != 0) cu += D::fx * ux;
@@ -2801,120 +1224,6 @@ __global__ void __launch_bounds__(kBX * kBY) k_adj_initial(const DeviceState s, 
 }  // namespace
 
 // ---------------------------------------------------------------------- host side
-
-FusedTiling fused_tiling(const Geometry &g, int max_smem) {
-    FusedTiling t{};
-    t.tpr = ((g.NX + 31) / 32) * 32;
-    const int per_row = t.tpr * 4;
-    const int rpt = kFusedThreads / t.tpr;
-    if (const char *v = std::getenv("MCG_FUSED_SMEM_KB")) max_smem = std::atoi(v) * 1024;  // tuning sweeps
-    // software-pipelined march for rows of up to 128 columns (measured on
-    // 128x256x128: +5 % float32, and +2 % float16 with its loads in flight
-    // across the relaxation)
-    t.pipe = t.tpr <= 128;
-    // rows of 256 columns in float32 too, where one row group's upper half
-    // takes the rows in a rotated order, on 1-row tiles at 3 CTAs per SM
-    // (measured on 256x512x256: 11236 MLUPS at 24-plane chunks, against 10582
-    // on 2-row tiles at 2 CTAs per SM and 10336 for the block-synchronous
-    // march; float16 keeps the block-synchronous march on 2-row tiles, 16721
-    // against 13171 pipelined)
-    const bool pipe256 = t.tpr == 256 && g.storage == kStoreF32;
-    if (pipe256) t.pipe = 1;
-    if (const char *v = std::getenv("MCG_FUSED_PIPE")) t.pipe = std::atoi(v) != 0;  // tuning sweeps
-    if (t.pipe) max_smem = std::max(max_smem, 112 * 1024);  // 4 ring + 3 stage planes: two CTAs per SM
-    // rows per tile: at least one round of rows in parallel, 4 by default
-    // (measured best on 128x256x128), fewer if shared memory
-    // (3*(ty+2) + 2*11*ty) * tpr * 4 bytes does not fit
-    int ty = std::max(4, rpt);
-    // the float32 pipelined march runs 3 CTAs per SM (PipeBlocks) on one round
-    // of rows (2 rows for 128 columns; measured +1.5 % over 4-row tiles at 2 CTAs)
-    if (t.pipe && g.storage == kStoreF32) ty = std::max(2, rpt);
-    if (t.pipe && pipe256) ty = 1;
-    if (const char *v = std::getenv("MCG_FUSED_TY")) ty = std::max(1, std::atoi(v));  // tuning sweeps
-    auto smem_of = [&](int h) {
-        return (t.pipe ? kPipeRing * (h + 2) + kPipeStage * kMomCount * h : 3 * (h + 2) + 2 * kMomCount * h) * per_row;
-    };
-    while (ty > 1 && smem_of(ty) > max_smem) --ty;
-    if (ty > rpt) ty -= ty % rpt;  // whole rounds of rows in parallel
-    t.ty = ty;
-    t.ny_tiles = (g.NY - 2 + ty - 1) / ty;
-    // z chunks of the block-synchronous march: about thirteen CTAs per SM over
-    // the launch (measured on the 256x512x256 jet: 32-plane chunks, 2040 CTAs;
-    // float16 +2 %, float32 within 0.5 % of 51-plane ones)
-    const int target = 13 * 148;
-    int chunks = (target + t.ny_tiles - 1) / t.ny_tiles;
-    if (chunks < 1) chunks = 1;
-    int lz = (g.NZ - 2 + chunks - 1) / chunks;
-    if (lz < 4) lz = 4;
-    if (t.pipe) {
-        // Chunks of the pipelined march, measured on 128x256x128 over 8..16
-        // planes: float32 13 planes (10 chunks, 2.9 waves of 3 CTAs per SM;
-        // +4.5 % over 16), float16 10 planes (13 chunks, 2.8 waves of 2 CTAs
-        // per SM; +1 %).  The time follows the fill of the last wave more than
-        // the halo planes.  Grids that give fewer than 1.5 waves of 16-plane
-        // chunks keep the block-synchronous march, whose shorter chunks fill
-        // the GPU.
-        const int ctas16 = t.ny_tiles * ((g.NZ - 2 + 15) / 16);
-        if (ctas16 >= 3 * 148 && !std::getenv("MCG_FUSED_LZ")) lz = pipe256 ? 24 : (g.storage == kStoreF16 ? 10 : 13);
-        else if (!std::getenv("MCG_FUSED_PIPE")) t.pipe = 0;
-    }
-    if (const char *v = std::getenv("MCG_FUSED_LZ")) lz = std::max(1, std::atoi(v));  // tuning sweeps
-    t.lz = lz;
-    t.nz_chunks = (g.NZ - 2 + lz - 1) / lz;
-    t.smem_bytes = t.pipe ? (kPipeRing * (ty + 2) + kPipeStage * kMomCount * ty) * per_row
-                          : (3 * (ty + 2) + 2 * kMomCount * ty) * per_row;
-    t.alternate = 1;
-    if (const char *v = std::getenv("MCG_FUSED_ALTERNATE")) t.alternate = std::atoi(v) != 0;  // tuning sweeps
-    // compile-time row length for rows of exactly 128 or 256 columns (measured
-    // +5 % float32, +10 % float16 on 128x256x128); results are bit-identical
-    t.fixed_nx = ((g.NX == kFusedNX || g.NX == kFusedNX2) && t.tpr == g.NX) ? g.NX : 0;
-    if (const char *v = std::getenv("MCG_FUSED_FIXED_NX"))  // tuning sweeps and the equality test
-        if (std::atoi(v) == 0) t.fixed_nx = 0;
-    // rows staged by bulk copies (k_fused_bulk), on request only: the
-    // pipelined march on rows of 128 columns (16-byte segments).  Measured on
-    // 128x256x128 it is slower than the register-held pulls (float32 10868
-    // vs 11387 MLUPS, float16 12950 vs 16197): a 27 KB row image per row
-    // group leaves two CTAs per SM with one row in flight each.
-    t.wait_limit = kBulkWaitLimit;
-    // the jet's inlet and outlet columns from the fused step's own-row threads
-    // of rows 1 and NY-2, instead of a k_boundary launch after it
-    t.boundary = g.boundary == kBoundaryJet;
-    if (const char *v = std::getenv("MCG_FUSED_BOUNDARY")) t.boundary = t.boundary && std::atoi(v) != 0;  // tests
-    const bool f16 = g.storage == kStoreF16;
-    const bool bulk_ok = t.pipe && t.fixed_nx == kFusedNX &&
-                         t.ty <= (f16 ? bulk_rows<CodecF16>() : bulk_rows<CodecF32>());
-    t.bulk = 0;
-    if (const char *v = std::getenv("MCG_FUSED_BULK")) t.bulk = bulk_ok && std::atoi(v) != 0;
-    if (t.bulk) t.smem_bytes = f16 ? bulk_smem_for<CodecF16>(t.ty) : bulk_smem_for<CodecF32>(t.ty);
-    return t;
-}
-
-cudaError_t fused_configure(int smem) {
-    cudaError_t e;
-    if ((e = fused_attr<CodecF32, false, false>(smem)) != cudaSuccess) return e;
-    if ((e = fused_attr<CodecF32, true, false>(smem)) != cudaSuccess) return e;
-    if ((e = fused_attr<CodecF32, false, true>(smem)) != cudaSuccess) return e;
-    if ((e = fused_attr<CodecF32, true, true>(smem)) != cudaSuccess) return e;
-    if ((e = fused_attr<CodecF16, false, false>(smem)) != cudaSuccess) return e;
-    if ((e = fused_attr<CodecF16, true, false>(smem)) != cudaSuccess) return e;
-    if ((e = fused_attr<CodecF16, false, true>(smem)) != cudaSuccess) return e;
-    return fused_attr<CodecF16, true, true>(smem);
-}
-
-cudaError_t launch_fused(const DeviceState &s, const FusedTiling &t_in, int cur, int64_t step, bool stats,
-                         cudaStream_t st) {
-    FusedTiling t = t_in;
-    if (t.boundary) {
-        t.bnd_dst = s.pops[cur ^ 1];
-        t.bnd_psi = s.psi[(step + 1) & 1];
-        t.bnd_step = step;
-    }
-    if (s.g.storage == kStoreF16)
-        return stats ? fused_dispatch<CodecF16, true>(s, t, cur, step, st)
-                     : fused_dispatch<CodecF16, false>(s, t, cur, step, st);
-    return stats ? fused_dispatch<CodecF32, true>(s, t, cur, step, st)
-                 : fused_dispatch<CodecF32, false>(s, t, cur, step, st);
-}
 
 cudaError_t launch_moments(const DeviceState &s, int cur, int64_t step, bool stats, cudaStream_t st) {
     cudaError_t e = s.g.storage == kStoreF16 ? moments_dispatch<CodecF16>(s, cur, step, st)

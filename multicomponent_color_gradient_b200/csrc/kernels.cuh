@@ -2,9 +2,9 @@
 //
 // HBM layout (node index id = x + NX*(y + NY*z) for the per-node fields):
 //   pops[2]   two population buffers (ping-pong), row-blocked: row (y,z) holds
-//             `slots` = 27 x-rows of NX elements, grouped by pull source
+//             `slots` = 27 x-rows of px >= NX elements, grouped by pull source
 //             (lattice.cuh slot_pair); element (slot, x, y, z) is at
-//             ((z*NY + y)*27 + slot)*NX + x.  One element carries both colours
+//             ((z*NY + y)*27 + slot)*px + x.  One element carries both colours
 //             of a direction, so a pull or a store is one 8- or 4-byte access.
 //             A buffer holds, at node s and direction i, the value that streams
 //             OUT of s along c_i (post-collision, pull layout): node x reads
@@ -21,9 +21,10 @@
 //             not stream them; they are refreshed on demand (output steps,
 //             granular launch sequence).
 //   psi[2]    colour field psi = (rr-rb)/(rr+rb) per node, ping-pong by step
-//             parity; the fused step reads only its ghost nodes, which carry
-//             what the reference's unwrapped colour-gradient stencil reads
-//             there (forces.cuh:31-33).
+//             parity.  The ghost nodes carry what the reference's unwrapped
+//             colour-gradient stencil reads there (forces.cuh:31-33); the
+//             split step writes the interior for its interface launch, a march
+//             forms it in shared memory.
 //   bmom      moments of the first and last fluid planes (y=1, y=NY-2),
 //             [2][NZ][11][NX], for the boundary launch.
 #pragma once
@@ -48,13 +49,14 @@ struct Geometry {
     int boundary;
     int storage;
     int slots;   // x-rows per lattice row in the population buffers: 27 (one element per direction)
+    int px;      // row pitch of the population buffers in elements: >= NX
 };
 
 __host__ __device__ __forceinline__ size_t pop_row(const Geometry &g, int y, int z) {
-    return (size_t(z) * size_t(g.NY) + size_t(y)) * size_t(g.slots) * size_t(g.NX);
+    return (size_t(z) * size_t(g.NY) + size_t(y)) * size_t(g.slots) * size_t(g.px);
 }
 __host__ __device__ __forceinline__ size_t pop_index(const Geometry &g, int slot, int x, int y, int z) {
-    return pop_row(g, y, z) + size_t(slot) * size_t(g.NX) + size_t(x);
+    return pop_row(g, y, z) + size_t(slot) * size_t(g.px) + size_t(x);
 }
 
 struct Physics {
@@ -75,18 +77,24 @@ struct Physics {
     float f16_rho0;
 };
 
-// Tiling of the fused step: a CTA owns rows [y0, y0+ty) of every plane of a
+// How a step runs (the values mcg_get_tiling reports): a march in one launch
+// (block-synchronous k_fused, pipelined k_fused_pipe, with staged rows
+// k_fused_bulk), or the two launches of the split step.
+enum StepMarch : int { kMarchBlock = 0, kMarchPipe = 1, kMarchBulk = 2, kMarchSplit = 3 };
+
+// Launch shape of the step.  In a march a CTA owns rows [y0, y0+ty) of every plane of a
 // z-chunk [z0, z0+lz) and marches z (up, or down for odd chunks when
 // `alternate`); tpr threads per row (a multiple of 32,
 // >= NX), blockDim.x / tpr rows in parallel.
 struct FusedTiling {
     int ty, lz, tpr;
+    int threads;  // per CTA
     int ny_tiles, nz_chunks;
     int smem_bytes;
     int alternate; // odd z-chunks march down, so neighbouring chunks pull their shared planes together
-    int pipe;      // software-pipelined march (k_fused_pipe): one barrier per plane
+    int march;     // how a step runs (StepMarch)
+    int interface_ctas, boundary_ctas;  // CTAs of k_step_interface that relax pieces, and after them the jet columns
     int fixed_nx;  // row length the kernel is compiled for (0: runtime geometry)
-    int bulk;      // the pipelined march with rows staged by bulk copies (k_fused_bulk)
     int wait_limit;  // k_fused_bulk: tries (about 1 us each) of a wait for a staged row before it gives up
     int boundary;    // jet: the fused step writes the inlet and outlet columns itself (no k_boundary launch)
     // set by launch_fused for each launch when `boundary`: the buffer the step
@@ -112,6 +120,7 @@ struct DeviceState {
     float *uy_avg;    // [N]
     double *partials; // reduction scratch
     uint32_t partials_cap;
+    uint8_t *piece_flags;  // [NZ-2][NY-2][pieces of 32 columns]: the piece holds an interface node (this step)
     int *flag;        // device flags: [0] non-finite value, [1] a k_fused_bulk wait ran out
     float *tape;      // null, or [kTapePlanes][N]: the fused step records the moments and psi it pulls there
     const float *inlet_profile;  // null (top-hat), or [NZ][NX] multipliers of the inlet velocity per column
@@ -119,7 +128,8 @@ struct DeviceState {
 
 // ---- the fused step (moments + colour gradient + collision in one pass) ----
 FusedTiling fused_tiling(const Geometry &g, int max_smem_per_block);
-cudaError_t fused_configure(int max_smem);
+cudaError_t fused_configure(const Geometry &g, const FusedTiling &t);
+inline int fused_launches(const FusedTiling &t) { return t.march == kMarchSplit ? 2 : 1; }  // kernels of a step
 cudaError_t launch_fused(const DeviceState &s, const FusedTiling &t, int cur, int64_t step, bool stats,
                          cudaStream_t st);
 

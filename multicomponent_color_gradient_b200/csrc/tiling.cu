@@ -1,0 +1,109 @@
+// tiling.cu - launch shape of the fused step and its dispatch by row pitch.
+#include <algorithm>
+#include <cstdlib>
+
+#include "fused.cuh"
+
+namespace mcg {
+
+// The marches in one launch, on request only (MCG_FUSED_PIPE=0: k_fused, 1:
+// k_fused_pipe; with MCG_FUSED_BULK=1 k_fused_bulk, rows of 128 columns): each
+// is slower than the split step at every size measured, and they are kept as
+// independent forms of the same arithmetic that the tests compare.
+static void march_tiling(const Geometry &g, int max_smem, FusedTiling &t) {
+    const int rpt = kFusedThreads / t.tpr;
+    const bool f16 = g.storage == kStoreF16, pipe = t.march != kMarchBlock;
+    t.threads = kFusedThreads;
+    if (pipe) max_smem = std::max(max_smem, 112 * 1024);
+    // rows per tile: whole rounds of rows in parallel, fewer if shared memory does not fit
+    int ty = std::max(4, rpt);
+    if (pipe && !f16) ty = t.tpr == 256 ? 1 : std::max(2, rpt);
+    auto smem_of = [&](int h) {
+        return (pipe ? kPipeRing * (h + 2) + kPipeStage * kMomCount * h : 3 * (h + 2) + 2 * kMomCount * h) * t.tpr * 4;
+    };
+    while (ty > 1 && smem_of(ty) > max_smem) --ty;
+    if (ty > rpt) ty -= ty % rpt;
+    t.ty = ty;
+    t.smem_bytes = smem_of(ty);
+    t.ny_tiles = (g.NY - 2 + ty - 1) / ty;
+    if (t.march == kMarchBulk)
+        t.smem_bytes = f16 ? bulk_smem_for<CodecF16>(ty) : bulk_smem_for<CodecF32>(ty);
+    // z chunks: about thirteen CTAs per SM over the launch
+    const int chunks = std::max(1, (13 * 148 + t.ny_tiles - 1) / t.ny_tiles);
+    t.lz = std::max(4, (g.NZ - 2 + chunks - 1) / chunks);
+    if (const char *v = std::getenv("MCG_FUSED_LZ")) t.lz = std::max(1, std::atoi(v));
+    t.nz_chunks = (g.NZ - 2 + t.lz - 1) / t.lz;
+    t.alternate = 1;
+}
+
+// The split step: a warp per piece of 32 columns, a plane per blockIdx.y.
+static void split_tiling(const Geometry &g, FusedTiling &t) {
+    const int ppr = g.storage == kStoreF16 ? pieces_per_row<CodecF16>(g) : pieces_per_row<CodecF32>(g);
+    const int warps = kSplitThreads / 32;
+    t.threads = kSplitThreads;
+    t.ty = std::max(1, warps / ppr);
+    t.lz = 1;
+    t.ny_tiles = (ppr * (g.NY - 2) + warps - 1) / warps;
+    t.nz_chunks = g.NZ - 2;
+    // one wave of the interface launch, at most one warp per piece
+    const long long per = kInterfaceThreads / 32, pieces = (long long)ppr * (g.NY - 2) * (g.NZ - 2);
+    t.interface_ctas = int(std::min<long long>((pieces + per - 1) / per, 148 * kInterfaceBlocks));
+    const long long columns = 2ll * (g.NX - 2) * (g.NZ - 2);
+    t.boundary_ctas = int(std::min<long long>((columns + kInterfaceThreads - 1) / kInterfaceThreads, 148));
+}
+
+FusedTiling fused_tiling(const Geometry &g, int max_smem) {
+    FusedTiling t{};
+    t.tpr = ((g.NX + 31) / 32) * 32;
+    t.fixed_nx = (g.NX == kFusedNX || g.NX == kFusedNX2) ? g.NX : 0;
+    if (const char *v = std::getenv("MCG_FUSED_FIXED_NX"))  // tests
+        if (std::atoi(v) == 0) t.fixed_nx = 0;
+    t.wait_limit = kBulkWaitLimit;
+    t.march = kMarchSplit;
+    if (const char *v = std::getenv("MCG_FUSED_PIPE")) t.march = std::atoi(v) != 0 ? kMarchPipe : kMarchBlock;
+    if (const char *v = std::getenv("MCG_FUSED_BULK"))
+        if (std::atoi(v) != 0 && t.march != kMarchBlock && t.fixed_nx == kFusedNX) t.march = kMarchBulk;
+    // planes are blockIdx.y of the split step
+    if (t.march == kMarchSplit && g.NZ - 2 > 65535) t.march = kMarchBlock;
+    if (t.march == kMarchSplit)
+        split_tiling(g, t);
+    else
+        march_tiling(g, max_smem, t);
+    // the jet's inlet and outlet columns within the step's launches, instead of
+    // a k_boundary launch after them
+    t.boundary = g.boundary == kBoundaryJet;
+    if (const char *v = std::getenv("MCG_FUSED_BOUNDARY")) t.boundary = t.boundary && std::atoi(v) != 0;  // tests
+    return t;
+}
+
+// One object per row pitch instantiates these (fused.cu).
+extern template cudaError_t fused_configure_pitch<0>(const Geometry &, const FusedTiling &);
+extern template cudaError_t fused_configure_pitch<kFusedNX>(const Geometry &, const FusedTiling &);
+extern template cudaError_t fused_configure_pitch<kFusedNX2>(const Geometry &, const FusedTiling &);
+extern template cudaError_t fused_launch_pitch<0>(const DeviceState &, const FusedTiling &, int, int64_t, bool,
+                                                  cudaStream_t);
+extern template cudaError_t fused_launch_pitch<kFusedNX>(const DeviceState &, const FusedTiling &, int, int64_t, bool,
+                                                         cudaStream_t);
+extern template cudaError_t fused_launch_pitch<kFusedNX2>(const DeviceState &, const FusedTiling &, int, int64_t,
+                                                          bool, cudaStream_t);
+
+cudaError_t fused_configure(const Geometry &g, const FusedTiling &t) {
+    if (t.fixed_nx == kFusedNX) return fused_configure_pitch<kFusedNX>(g, t);
+    if (t.fixed_nx == kFusedNX2) return fused_configure_pitch<kFusedNX2>(g, t);
+    return fused_configure_pitch<0>(g, t);
+}
+
+cudaError_t launch_fused(const DeviceState &s, const FusedTiling &t_in, int cur, int64_t step, bool stats,
+                         cudaStream_t st) {
+    FusedTiling t = t_in;
+    if (t.boundary) {
+        t.bnd_dst = s.pops[cur ^ 1];
+        t.bnd_psi = s.psi[(step + 1) & 1];
+        t.bnd_step = step;
+    }
+    if (t.fixed_nx == kFusedNX) return fused_launch_pitch<kFusedNX>(s, t, cur, step, stats, st);
+    if (t.fixed_nx == kFusedNX2) return fused_launch_pitch<kFusedNX2>(s, t, cur, step, stats, st);
+    return fused_launch_pitch<0>(s, t, cur, step, stats, st);
+}
+
+}  // namespace mcg
