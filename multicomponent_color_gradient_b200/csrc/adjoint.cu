@@ -35,6 +35,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <vector>
 
 #include "internal.hpp"
@@ -122,20 +124,76 @@ int64_t forward_steps_of(const std::vector<Action> &acts) {
         ++(h)->launches;                                     \
     } while (0)
 
+// Device memory of one adjoint run.  Allocating and freeing a run's gigabytes
+// took longer than the run (2 GB in 17 blocks: 10-56 ms and 9-1000 ms), so the
+// blocks of the last run on a device are kept for the next one, up to 1/16 of
+// the device's memory, while any handle lives (workspace_release).  A run takes
+// the kept blocks out, so runs of several threads never share one, and returns
+// its own after its stream has finished with them.  Blocks come with whatever
+// they hold; a buffer that has to start at zero is cleared.
+struct Block {
+    void *p;
+    size_t bytes;
+};
+std::mutex g_kept_mutex;
+std::map<int, std::vector<Block>> g_kept;  // by device
+
 struct DeviceBuffers {
-    cudaStream_t stream;  // the run's stream: buffers are cleared in its order
-    std::vector<void *> ptrs;
-    explicit DeviceBuffers(cudaStream_t st) : stream(st) {}
-    ~DeviceBuffers() {
-        if (!ptrs.empty()) cudaStreamSynchronize(stream);
-        for (void *p : ptrs) cudaFree(p);
+    cudaStream_t stream;  // the run's stream
+    int device = 0;
+    std::vector<Block> used, spare;
+    explicit DeviceBuffers(cudaStream_t st) : stream(st) {
+        cudaGetDevice(&device);
+        std::lock_guard<std::mutex> lock(g_kept_mutex);
+        spare.swap(g_kept[device]);
     }
-    cudaError_t alloc(void **p, size_t bytes) {
+    ~DeviceBuffers() {
+        if (!used.empty()) cudaStreamSynchronize(stream);
+        drop_spare();
+        size_t total = 0, free_b = 0, total_b = 0;
+        for (const Block &b : used) total += b.bytes;
+        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && total <= total_b / 16) {
+            std::lock_guard<std::mutex> lock(g_kept_mutex);
+            if (g_kept[device].empty()) {
+                g_kept[device].swap(used);
+                return;
+            }
+        }
+        for (const Block &b : used) cudaFree(b.p);
+    }
+    void drop_spare() {
+        for (const Block &b : spare) cudaFree(b.p);
+        spare.clear();
+    }
+    size_t spare_bytes() const {
+        size_t s = 0;
+        for (const Block &b : spare) s += b.bytes;
+        return s;
+    }
+    cudaError_t alloc(void **p, size_t bytes, bool zero = false) {
         *p = nullptr;
-        cudaError_t e = cudaMalloc(p, bytes);
-        if (e != cudaSuccess) return e;
-        ptrs.push_back(*p);
-        return cudaMemsetAsync(*p, 0, bytes, stream);
+        size_t best = spare.size();
+        for (size_t k = 0; k < spare.size(); ++k)
+            if (spare[k].bytes >= bytes && spare[k].bytes <= bytes + bytes / 4 + 4096 &&
+                (best == spare.size() || spare[k].bytes < spare[best].bytes))
+                best = k;
+        used.reserve(used.size() + 1);
+        if (best < spare.size()) {
+            used.push_back(spare[best]);
+            spare.erase(spare.begin() + long(best));
+        } else {
+            void *q = nullptr;
+            cudaError_t e = cudaMalloc(&q, bytes);
+            if (e == cudaErrorMemoryAllocation && !spare.empty()) {
+                cudaGetLastError();
+                drop_spare();
+                e = cudaMalloc(&q, bytes);
+            }
+            if (e != cudaSuccess) return e;
+            used.push_back({q, bytes});
+        }
+        *p = used.back().p;
+        return zero ? cudaMemsetAsync(*p, 0, bytes, stream) : cudaSuccess;
     }
 };
 
@@ -258,6 +316,21 @@ struct Run {
 
 }  // namespace
 
+namespace mcg {
+void workspace_release(int device) noexcept {
+    std::vector<Block> blocks;
+    {
+        std::lock_guard<std::mutex> lock(g_kept_mutex);
+        blocks.swap(g_kept[device]);
+    }
+    int current = 0;
+    cudaGetDevice(&current);
+    if (current != device) cudaSetDevice(device);
+    for (const Block &b : blocks) cudaFree(b.p);
+    if (current != device) cudaSetDevice(current);
+}
+}  // namespace mcg
+
 extern "C" {
 
 mcg_status mcg_adjoint_plan_taped(int32_t nsteps, int32_t snapshots, int32_t tape, int64_t *forward_steps,
@@ -369,7 +442,7 @@ mcg_status mcg_adjoint_run(mcg_handle *h, const float *psi_target, int32_t nstep
         ADJ_CUDA(buf.alloc(&p, N * sizeof(float)), "adjoint target");
         run.target = static_cast<const float *>(p);
         ADJ_CUDA(cudaMemcpyAsync(p, psi_target, N * sizeof(float), cudaMemcpyHostToDevice, h->stream), "upload target");
-        ADJ_CUDA(buf.alloc(&p, 4 * sizeof(double)), "adjoint accumulators");
+        ADJ_CUDA(buf.alloc(&p, 4 * sizeof(double), true), "adjoint accumulators");
         run.acc = static_cast<double *>(p);
 
         ADJ_CUDA(cudaEventRecord(h->ev0, h->stream), "event");
@@ -407,7 +480,10 @@ mcg_status mcg_adjoint_run(mcg_handle *h, const float *psi_target, int32_t nstep
 
 
 namespace {
-// J0(alpha_k r / R) of every column, k < kInletBesselMax (the inlet profile's basis).
+// J0(alpha_k r / R), k < kInletBesselMax (the inlet profile's basis), of the
+// columns within a node of the jet's radius: only jet columns read it
+// (is_jet_column; the margin covers its float32 rounding).  All of a 64x64
+// plane took 14 ms.
 std::vector<float> bessel_basis(const mcg_params &p) {
     const int NX = p.NX, NZ = p.NZ, nb = mcg::kInletBesselMax;
     std::vector<float> b(size_t(nb) * NX * NZ);
@@ -422,6 +498,7 @@ std::vector<float> bessel_basis(const mcg_params &p) {
             for (int x = 0; x < NX; ++x) {
                 const double dx = double(float(x) - p.jet_x0), dz = double(float(z) - p.jet_z0);
                 const double r = std::sqrt(dx * dx + dz * dz);
+                if (r > std::fabs(double(p.jet_radius)) + 1.0) continue;
                 b[(size_t(k) * NZ + z) * NX + x] = float(std::cyl_bessel_j(0.0, a * r / double(p.jet_radius)));
             }
     }
@@ -489,7 +566,7 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
     ADJ_CUDA(buf.alloc(&p, size_t(2) * g.NZ * mcg::kMomCount * g.NX * sizeof(float)), "jet adjoint bmom");
     run.bmom = static_cast<float *>(p);
     // the run's own radial sums (the profile objective's time averages)
-    ADJ_CUDA(buf.alloc(&p, 5 * M * sizeof(double)), "jet adjoint radial sums");
+    ADJ_CUDA(buf.alloc(&p, 5 * M * sizeof(double), true), "jet adjoint radial sums");
     run.radial = static_cast<double *>(p);
     // segments of L steps: a snapshot (populations + outlet state) at the
     // start of each, and a tape of one segment's records
@@ -505,7 +582,8 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
     }
     float *lam[2];
     for (int k = 0; k < 2; ++k) {
-        ADJ_CUDA(buf.alloc(&p, lam_bytes), "jet adjoint lambda buffers");
+        // zero: lambda_T, and the slots that stream out of the domain
+        ADJ_CUDA(buf.alloc(&p, lam_bytes, true), "jet adjoint lambda buffers");
         lam[k] = static_cast<float *>(p);
     }
     ADJ_CUDA(buf.alloc(&p, size_t(mcg::kMomCount) * N * sizeof(float)), "jet adjoint moment adjoints");
@@ -514,7 +592,7 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
     float *lf = static_cast<float *>(p);
     float *LB[2];
     for (int k = 0; k < 2; ++k) {
-        ADJ_CUDA(buf.alloc(&p, 5 * NP * sizeof(float)), "jet adjoint outlet adjoints");
+        ADJ_CUDA(buf.alloc(&p, 5 * NP * sizeof(float), true), "jet adjoint outlet adjoints");
         LB[k] = static_cast<float *>(p);
     }
     const std::vector<float> basis = bessel_basis(h->p);
@@ -522,10 +600,10 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
     float *dbasis = static_cast<float *>(p);
     ADJ_CUDA(cudaMemcpyAsync(dbasis, basis.data(), basis.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream),
              "upload profile basis");
-    ADJ_CUDA(buf.alloc(&p, (2 + size_t(nb)) * sizeof(double)), "jet adjoint accumulators");
+    ADJ_CUDA(buf.alloc(&p, (2 + size_t(nb)) * sizeof(double), true), "jet adjoint accumulators");
     double *acc = static_cast<double *>(p);  // [0] J, [1] (unused), [2..] dJ/dc_k
     double *dacc_w = nullptr;
-    ADJ_CUDA(buf.alloc(&p, 2 * sizeof(double)), "jet adjoint parameter partials");
+    ADJ_CUDA(buf.alloc(&p, 2 * sizeof(double), true), "jet adjoint parameter partials");
     dacc_w = static_cast<double *>(p);
     float *table = nullptr;
     if (profile) {
@@ -542,6 +620,7 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
     {
         size_t free_b = 0, total_b = 0;
         ADJ_CUDA(cudaMemGetInfo(&free_b, &total_b), "device memory");
+        free_b += buf.spare_bytes();
         const size_t margin = std::max<size_t>(size_t(4) << 30, total_b / 20);
         const int64_t fit = free_b > margin ? int64_t((free_b - margin) / tape_bytes) : 0;
         const int64_t want = h->jet_adjoint_tapes > 0 ? int64_t(h->jet_adjoint_tapes) : nseg;

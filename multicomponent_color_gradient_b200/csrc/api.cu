@@ -6,6 +6,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -38,6 +40,29 @@ void radial_counts_for(const mcg_handle *h, uint32_t samples, uint64_t *count) {
 }
 
 void radial_counts(const mcg_handle *h, uint64_t *count) { radial_counts_for(h, h->stats_samples, count); }
+
+cudaError_t device_malloc(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    int device = 0;
+    cudaGetDevice(&device);
+    workspace_release(device);
+    return cudaMalloc(p, bytes);
+}
+
+namespace {
+std::mutex g_live_mutex;
+std::map<int, int> g_live;  // handles by device
+}
+static void handle_born(int device) {
+    std::lock_guard<std::mutex> lock(g_live_mutex);
+    ++g_live[device];
+}
+static void handle_gone(int device) {
+    std::lock_guard<std::mutex> lock(g_live_mutex);
+    if (--g_live[device] == 0) workspace_release(device);
+}
 
 StatsSnapshot stats_snapshot(const mcg_handle *h) {
     StatsSnapshot s;
@@ -179,7 +204,7 @@ void release(mcg_handle *h) {
 
 template <class T>
 cudaError_t alloc_zero(T **ptr, size_t bytes) {
-    cudaError_t e = cudaMalloc(reinterpret_cast<void **>(ptr), bytes);
+    cudaError_t e = mcg::device_malloc(reinterpret_cast<void **>(ptr), bytes);
     if (e != cudaSuccess) {
         *ptr = nullptr;
         return e;
@@ -397,6 +422,7 @@ mcg_status mcg_create(const mcg_params *p, mcg_handle **out) {
             delete h;
             return s;
         }
+        mcg::handle_born(h->device);
         h->stream = h->own_stream;
         *out = h;
         return MCG_OK;
@@ -407,8 +433,10 @@ mcg_status mcg_destroy(mcg_handle *h) {
     return mcg::guarded([&]() -> mcg_status {
         if (!h) return MCG_OK;
         cudaStreamSynchronize(h->stream);
+        const int device = h->device;
         release(h);
         delete h;
+        mcg::handle_gone(device);
         return MCG_OK;
     });
 }
@@ -560,7 +588,8 @@ mcg_status mcg_set_inlet_bessel(mcg_handle *h, const float *coeffs, int32_t n) {
                 prof[size_t(z) * NX + x] = float(m);
             }
         if (!h->d_inlet_profile)
-            MCG_CUDA(cudaMalloc(&h->d_inlet_profile, prof.size() * sizeof(float)), "inlet profile allocation");
+            MCG_CUDA(mcg::device_malloc(reinterpret_cast<void **>(&h->d_inlet_profile), prof.size() * sizeof(float)),
+                     "inlet profile allocation");
         MCG_CUDA(cudaMemcpyAsync(h->d_inlet_profile, prof.data(), prof.size() * sizeof(float), cudaMemcpyHostToDevice,
                                  h->stream),
                  "upload inlet profile");

@@ -99,6 +99,11 @@ StatsSnapshot stats_snapshot(const mcg_handle *h);
 // float64 device sum of this output step
 void tke_update(mcg_handle *h, int32_t step, double total);
 
+// adjoint.cu: frees the device memory kept between adjoint runs on `device`.
+void workspace_release(int device) noexcept;
+// cudaMalloc that first gives that memory back where it is in the way.
+cudaError_t device_malloc(void **p, size_t bytes);
+
 // io.cpp
 mcg_status io_open(mcg_handle *h, const char *root);
 mcg_status io_close(mcg_handle *h);
