@@ -197,6 +197,31 @@ struct DeviceBuffers {
     }
 };
 
+// A state's record: kTapePlanes planes, `extra` floats (the jet's outlet state),
+// and the flags of the pieces that hold an interface node.
+size_t record_flag_bytes(const mcg::Geometry &g) {
+    return (size_t((g.NX - 1 + 31) / 32) * size_t(g.NY - 2) * size_t(g.NZ - 2) + 255) / 256 * 256;
+}
+size_t record_size(const mcg::Geometry &g, size_t extra) {
+    return size_t(mcg::kTapePlanes) * g.N + extra + record_flag_bytes(g) / sizeof(float);
+}
+uint8_t *record_flags(const mcg::Geometry &g, float *rec, size_t extra) {
+    return reinterpret_cast<uint8_t *>(rec + size_t(mcg::kTapePlanes) * g.N + extra);
+}
+
+// A forward step of d (pops[0] -> pops[1]) that leaves the record of the state
+// it pulls in `rec`.
+mcg_status record_step(mcg_handle *h, mcg::DeviceState d, float *rec, size_t extra, int64_t step, bool stats) {
+    d.tape = rec;
+    uint8_t *flags = record_flags(d.g, rec, extra);
+    const bool split = h->tiling.march == mcg::kMarchSplit;  // its pull launch sets them
+    if (split) d.piece_flags = flags;
+    ADJ_LAUNCH(h, mcg::launch_fused(d, h->tiling, 0, step, stats, h->stream), "adjoint: forward step");
+    h->launches += mcg::fused_launches(h->tiling) - 1;
+    if (!split) ADJ_LAUNCH(h, mcg::launch_piece_flags(d, rec, flags, h->stream), "adjoint: flags");
+    return MCG_OK;
+}
+
 struct Run {
     mcg_handle *h = nullptr;
     mcg::DeviceState base{};   // the handle's state with the run's own moment / psi planes
@@ -206,6 +231,7 @@ struct Run {
     float *lam[2] = {nullptr, nullptr};
     int lc = 0;                // lam[lc]: adjoint of the latest state reached
     float *lmom = nullptr, *lf = nullptr;
+    uint8_t *near_flags = nullptr;
     const float *target = nullptr;
     double *acc = nullptr;     // [0] J, [1] dJ/domega, [2] dJ/d(A/2)
     int64_t step0 = 0, T = 0;
@@ -234,14 +260,17 @@ struct Run {
 
     // op t with the moment record M of S_t
     const float *last_record = nullptr;  // the record the latest op read (op 0's, after a sweep)
-    mcg_status op_record(const float *M, int64_t t) {
+    mcg_status op_record(float *M, int64_t t) {
         last_record = M;
         if (t == T) {
             ADJ_LAUNCH(h, mcg::launch_adj_terminal(base, M, target, lam[lc], acc, h->stream), "adjoint: terminal");
         } else {
-            ADJ_LAUNCH(h, mcg::launch_adj_step(base, M, lam[lc], lmom, lf, lam[lc ^ 1], acc + 1, h->stream),
-                       "adjoint: step");
-            h->launches += 1;  // two kernels
+            const uint8_t *flags = record_flags(base.g, M, 0);
+            ADJ_LAUNCH(h, mcg::launch_adj_relax(base, M, flags, near_flags, lam[lc], lmom, lf, lam[lc ^ 1], acc + 1,
+                                                mcg::AdjObjective{0.0f, 0, nullptr}, h->stream),
+                       "adjoint: relaxation part");
+            ADJ_LAUNCH(h, mcg::launch_adj_near(base, M, flags, near_flags, lmom, lf, lam[lc ^ 1], h->stream),
+                       "adjoint: moment part");
             lc ^= 1;
         }
         return MCG_OK;
@@ -250,6 +279,7 @@ struct Run {
     // op t on the state held in `state` (its record formed first)
     mcg_status op(void *state, int64_t t) {
         ADJ_LAUNCH(h, mcg::launch_moments(with(state, nullptr), 0, step0 + t, false, h->stream), "adjoint: moments");
+        ADJ_LAUNCH(h, mcg::launch_piece_flags(base, rec, record_flags(base.g, rec, 0), h->stream), "adjoint: flags");
         return op_record(rec, t);
     }
 
@@ -259,9 +289,7 @@ struct Run {
         void *a = slots[0];
         for (int64_t t = 0; t < T; ++t) {
             mcg::DeviceState d = with(a, work[t & 1]);
-            d.tape = tape + size_t(t) * record_floats;
-            ADJ_LAUNCH(h, mcg::launch_fused(d, h->tiling, 0, step0 + t, false, h->stream), "adjoint: forward step");
-            h->launches += mcg::fused_launches(h->tiling) - 1;
+            if (mcg_status s = record_step(h, d, tape + size_t(t) * record_floats, 0, step0 + t, false)) return s;
             a = work[t & 1];
         }
         {
@@ -270,6 +298,7 @@ struct Run {
             d.mom = M;
             d.psi[0] = d.psi[1] = M + size_t(mcg::kTapePsi) * base.g.N;
             ADJ_LAUNCH(h, mcg::launch_moments(d, 0, step0 + T, false, h->stream), "adjoint: moments");
+            ADJ_LAUNCH(h, mcg::launch_piece_flags(d, M, record_flags(d.g, M, 0), h->stream), "adjoint: flags");
         }
         for (int64_t t = T; t >= 0; --t)
             if (mcg_status s = op_record(tape + size_t(t) * record_floats, t)) return s;
@@ -284,9 +313,7 @@ struct Run {
         void *a = src;
         for (int64_t k = 0; k + 1 < n; ++k) {
             mcg::DeviceState d = with(a, work[k & 1]);
-            d.tape = seg_tape + size_t(k) * record_floats;
-            ADJ_LAUNCH(h, mcg::launch_fused(d, h->tiling, 0, step0 + t0 + k, false, h->stream), "adjoint: forward step");
-            h->launches += mcg::fused_launches(h->tiling) - 1;
+            if (mcg_status s = record_step(h, d, seg_tape + size_t(k) * record_floats, 0, step0 + t0 + k, false)) return s;
             a = work[k & 1];
         }
         if (mcg_status s = op(a, t0 + n - 1)) return s;
@@ -386,7 +413,7 @@ mcg_status mcg_adjoint_run(mcg_handle *h, const float *psi_target, int32_t nstep
         const mcg::Geometry &g = h->s.g;
         const size_t N = g.N;
         const size_t pop_bytes = size_t(2 * mcg::kQ) * N * sizeof(float);  // float32 populations or lambda
-        const size_t record_floats = size_t(mcg::kTapePlanes) * N;
+        const size_t record_floats = record_size(g, 0);
         const bool tape_mode = snapshots > nsteps;
         const int free_slots = tape_mode ? 0 : snapshots - 1;
         const int64_t seg = std::min<int64_t>(h->adjoint_tape, nsteps);  // records of a taped segment
@@ -437,6 +464,8 @@ mcg_status mcg_adjoint_run(mcg_handle *h, const float *psi_target, int32_t nstep
         // the forward steps' psi of the tape (the handle's stays as it is): lf is
         // free until the reverse sweep
         if (tape_mode) run.base.psi[0] = run.base.psi[1] = run.lf;
+        ADJ_CUDA(buf.alloc(&p, record_flag_bytes(g)), "adjoint piece flags");
+        run.near_flags = static_cast<uint8_t *>(p);
         ADJ_CUDA(buf.alloc(&p, 3 * N * sizeof(float)), "adjoint du0");
         float *du0 = static_cast<float *>(p);
         ADJ_CUDA(buf.alloc(&p, N * sizeof(float)), "adjoint target");
@@ -535,7 +564,7 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
     // its lambda arrays are float32 pairs
     const size_t state_bytes = g.storage == MCG_STORAGE_F16 ? size_t(mcg::kQ) * N * 4 : size_t(2 * mcg::kQ) * N * 4;
     const size_t lam_bytes = size_t(2 * mcg::kQ) * N * sizeof(float);
-    const size_t rec_floats = size_t(mcg::kTapePlanes) * N + 5 * NP;  // moments, psi with ghosts, outlet state
+    const size_t rec_floats = record_size(g, 5 * NP);  // moments, psi with ghosts, outlet state, flags
     const int nb = mcg::kInletBesselMax;
     const bool profile = objective.kind == 1;
 
@@ -590,6 +619,8 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
     float *lmom = static_cast<float *>(p);
     ADJ_CUDA(buf.alloc(&p, 3 * N * sizeof(float)), "jet adjoint gradient adjoints");
     float *lf = static_cast<float *>(p);
+    ADJ_CUDA(buf.alloc(&p, record_flag_bytes(g)), "jet adjoint piece flags");
+    uint8_t *near_flags = static_cast<uint8_t *>(p);
     float *LB[2];
     for (int k = 0; k < 2; ++k) {
         ADJ_CUDA(buf.alloc(&p, 5 * NP * sizeof(float), true), "jet adjoint outlet adjoints");
@@ -649,11 +680,11 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
                      "record psi");
             ADJ_LAUNCH(h, mcg::launch_copy_outlet_state(d, rec + size_t(mcg::kTapePlanes) * N, h->stream),
                        "jet adjoint: record outlet state");
-            d.tape = rec;
+            if (mcg_status st = record_step(h, d, rec, 5 * NP, step0 + t, stats)) return st;
+        } else {
+            ADJ_LAUNCH(h, mcg::launch_fused(d, h->tiling, 0, step0 + t, stats, h->stream), "jet adjoint: forward step");
+            h->launches += mcg::fused_launches(h->tiling) - 1;
         }
-        ADJ_LAUNCH(h, mcg::launch_fused(d, h->tiling, 0, step0 + t, stats, h->stream), "jet adjoint: forward step");
-        h->launches += mcg::fused_launches(h->tiling) - 1;
-        d.tape = nullptr;
         if (!h->tiling.boundary)
             ADJ_LAUNCH(h, mcg::launch_boundary(d, 1, step0 + t, -1, true, h->stream), "jet adjoint: boundary");
         ++fwd;
@@ -712,17 +743,20 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
                 if (mcg_status st = forward(t, tape + size_t(t - s0) * rec_floats, false)) return st;
         }
         for (int64_t t = s1 - 1; t >= s0; --t) {
-            const float *rec = tape + size_t(t - s0) * rec_floats;
+            float *rec = tape + size_t(t - s0) * rec_floats;
+            const uint8_t *flags = record_flags(g, rec, 5 * NP);
             const bool in_window = t >= t_begin && t <= t_end;
             mcg::AdjObjective obj{in_window && !profile ? 1.0f : 0.0f, objective.y_obs, profile ? nullptr : acc};
             if (profile && in_window) obj.table = table;
-            ADJ_LAUNCH(h, mcg::launch_adj_collide(run, rec, lam[lc], lmom, lf, dacc_w, obj, h->stream),
-                       "jet adjoint: collision");
+            ADJ_LAUNCH(h, mcg::launch_adj_relax(run, rec, flags, near_flags, lam[lc], lmom, lf, lam[lc ^ 1], dacc_w, obj,
+                                                h->stream),
+                       "jet adjoint: relaxation part");
             ADJ_LAUNCH(h,
                        mcg::launch_adj_boundary(run, step0 + t, rec, rec + size_t(mcg::kTapePlanes) * N, lam[lc], lf,
                                                 lmom, LB[lb], LB[lb ^ 1], dbasis, nb, acc + 2, h->stream),
                        "jet adjoint: boundary");
-            ADJ_LAUNCH(h, mcg::launch_adj_moments(run, rec, lmom, lf, lam[lc ^ 1], h->stream), "jet adjoint: moments");
+            ADJ_LAUNCH(h, mcg::launch_adj_near(run, rec, flags, near_flags, lmom, lf, lam[lc ^ 1], h->stream),
+                       "jet adjoint: moment part");
             lc ^= 1;
             lb ^= 1;
         }

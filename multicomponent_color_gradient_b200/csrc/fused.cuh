@@ -539,12 +539,6 @@ constexpr int kInterfaceThreads = 128, kInterfaceBlocks = 5;
 // 128x256x128 float16 jet, 2250 against 2328 for 256x512x256 float32).
 constexpr int kPieceGroup = 4;
 
-// Pieces of 32 columns that hold the stored columns of a row.
-template <class C>
-__host__ __device__ __forceinline__ int pieces_per_row(const Geometry &g) {
-    return (store_columns<C>(g) + 31) / 32;
-}
-
 // Moments of a node to and from its own element slots in the row it will
 // store: two floats an element in float32, one in float16.
 __device__ __forceinline__ void park_moments(float2 *wrow, int px, const NodeMoments &m) {
@@ -627,8 +621,8 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitBlocks) k_step_pull(const
         tile_record_moments(s, x, y, z, m, ps);
     }
     if constexpr (kStats) radial_accumulate_warp(s, x, y, z, xin, m.ux, m.uy, m.uz);
-    const bool interface = __any_sync(kFull, xin && !is_bulk(m.rr, m.rb));
-    if ((x & 31) == 0) s.piece_flags[(size_t(zi) * (g.NY - 2) + row) * ppr + w] = interface ? 1 : 0;
+    const unsigned interface = __ballot_sync(kFull, xin && !is_bulk(m.rr, m.rb));
+    if ((x & 31) == 0) s.piece_flags[(size_t(zi) * (g.NY - 2) + row) * ppr + w] = piece_flag(g, w, interface);
     const size_t at = pop_row(g, y, z);
     if (interface) {
         if (xin) park_moments(codec.wr + at + x, g.px, m);

@@ -448,8 +448,8 @@ cudaError_t boundary_dispatch(const DeviceState &s, int wbuf, int64_t step, int 
 //   f_i(x) = S_t,i(x - c_i); M(x) = moments(f(x)); psi(x) = psi(M(x));
 //   F(x) = (1/cs2) sum_j w_j c_j psi(x + c_j);  S_{t+1},i(x) = C_i(M(x), F(x)).
 // Given lambda_{t+1} = dJ/dS_{t+1} the adjoint forms lambda_t = dJ/dS_t in two
-// node-parallel passes: k_adj_collide takes C's Jacobian (moments and F of the
-// node), k_adj_moments gathers the F-adjoints of the neighbours into the
+// node-parallel parts: adj_collide_node takes C's Jacobian (moments and F of the
+// node), adj_moments_node gathers the F-adjoints of the neighbours into the
 // node's psi-adjoint, goes back through the moments and scatters along the
 // transposed streaming.  The bulk/interface switch (I <= 1e-4) and the
 // |F| <= 1e-4 cut-off are taken as in the forward step (derivatives inside
@@ -595,9 +595,15 @@ __device__ __forceinline__ PolyAdjoint poly_adjoint(const float (&T)[17], float 
     return r;
 }
 
-// Per node: lambda_post (54 values at the node) -> adjoints of the node's
-// moments (11, to lmom) and colour gradient (3, to lf); float64 partials of
-// dJ/domega (acc[0]) and dJ/d(A/2) (acc[1]).
+// Adjoints of a node's moments (moment order) and of its colour gradient.
+struct NodeAdjoint {
+    float rr, rb, ux, uy, uz, pxx, pxy, pyy, pyz, pzz, pxz;
+    float Fx, Fy, Fz;
+};
+
+// Relaxation part of a node: lambda_post (54 values at the node) -> adjoints of
+// the node's moments and colour gradient; float64 parts of dJ/domega, dJ/d(A/2)
+// and J.  kInterface false: the caller knows that the node is bulk.
 //
 // Per direction the stored pair is r_i = aR g_i + D_i, b_i = aB g_i - D_i, so
 // with lg_i = aR lr_i + aB lb_i and ld_i = lr_i - lb_i the node's sums are
@@ -608,301 +614,233 @@ __device__ __forceinline__ PolyAdjoint poly_adjoint(const float (&T)[17], float 
 // Opposite directions i, i+1 are taken together: feq and fneq split into even
 // and odd parts, Omega2 is even and D odd, so every sum needs only
 // lg_i + lg_o, lg_i - lg_o, ld_i + ld_o and ld_i - ld_o.
-template <bool kPeriodic>
-__global__ void __launch_bounds__(kBX * kBY, 2) k_adj_collide(const DeviceState s, const float *__restrict__ M,
-                                                             const float *lam, float *lmom, float *lf, double *acc,
-                                                             AdjObjective obj) {
-    __shared__ double sh[3 * (kBX * kBY / 32)];  // block_sum3
+template <bool kPeriodic, bool kInterface>
+__device__ __forceinline__ void adj_collide_node(const DeviceState &s, const float *M, const float *lam,
+                                                 const AdjObjective &obj, int x, int y, int z, NodeAdjoint &o,
+                                                 double &a_omega, double &a_Ah, double &a_J) {
     const Geometry &g = s.g;
     const Physics &ph = s.ph;
-    const int x = blockIdx.x * kBX + threadIdx.x;
-    const int y = blockIdx.y * kBY + threadIdx.y;
-    const int z = blockIdx.z;
-    const bool in = x >= 1 && x <= g.NX - 2 && y >= 1 && y <= g.NY - 2 && z >= 1 && z <= g.NZ - 2;
-    double a_omega = 0.0, a_Ah = 0.0, a_J = 0.0;
-    if (in) {
-        const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
-        const size_t N = g.N;
-        const float *mom = M;
-        const float rr = mom[kMomRR * N + id], rb = mom[kMomRB * N + id];
-        const float ux = mom[kMomUX * N + id], uy = mom[kMomUY * N + id], uz = mom[kMomUZ * N + id];
-        const NeqTerms n = make_neq(mom[kMomPXX * N + id], mom[kMomPXY * N + id], mom[kMomPYY * N + id],
-                                    mom[kMomPYZ * N + id], mom[kMomPZZ * N + id], mom[kMomPXZ * N + id], ux, uy, uz);
-        const float rho = rr + rb;
-        const float invr = 1.0f / rho;
-        const float aR = rr * invr, aB = rb * invr;
-        const float oms = 1.0f - omega_at(ph, y);
-        const bool interface = !(4.0f * rr * rb * invr * invr <= 1e-4f);
-        float Fx = 0.f, Fy = 0.f, Fz = 0.f, absF = 0.f, K = 0.f;
-        bool has_dir = false;
-        if (interface) {
-            // periodic box: neighbours wrap over the interior; jet: the record's
-            // psi plane holds the ghost values the forward step read unwrapped
-            const float *psi = M + size_t(kTapePsi) * N;
-            const int xn[3] = {kPeriodic ? wrap_interior(x - 1, g.NX) : x - 1, x,
-                               kPeriodic ? wrap_interior(x + 1, g.NX) : x + 1};
-            const int yn[3] = {g.sy * (kPeriodic ? wrap_interior(y - 1, g.NY) : y - 1), g.sy * y,
-                               g.sy * (kPeriodic ? wrap_interior(y + 1, g.NY) : y + 1)};
-            const int zn[3] = {g.sz * (kPeriodic ? wrap_interior(z - 1, g.NZ) : z - 1), g.sz * z,
-                               g.sz * (kPeriodic ? wrap_interior(z + 1, g.NZ) : z + 1)};
-            float sx = 0.f, sy = 0.f, sz = 0.f;
-            static_for<kQ - 1>([&](auto I) {
-                constexpr int i = decltype(I)::value + 1;
-                using D = Dir<i>;
-                const float wp = D::w * psi[xn[D::cx + 1] + yn[D::cy + 1] + zn[D::cz + 1]];
-                if constexpr (D::cx != 0) sx += D::fx * wp;
-                if constexpr (D::cy != 0) sy += D::fy * wp;
-                if constexpr (D::cz != 0) sz += D::fz * wp;
+            const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
+            const size_t N = g.N;
+            const float *mom = M;
+            const float rr = mom[kMomRR * N + id], rb = mom[kMomRB * N + id];
+            const float ux = mom[kMomUX * N + id], uy = mom[kMomUY * N + id], uz = mom[kMomUZ * N + id];
+            const NeqTerms n = make_neq(mom[kMomPXX * N + id], mom[kMomPXY * N + id], mom[kMomPYY * N + id],
+                                        mom[kMomPYZ * N + id], mom[kMomPZZ * N + id], mom[kMomPXZ * N + id], ux, uy, uz);
+            const float rho = rr + rb;
+            const float invr = 1.0f / rho;
+            const float aR = rr * invr, aB = rb * invr;
+            const float oms = 1.0f - omega_at(ph, y);
+            const bool interface = kInterface && !is_bulk(rr, rb);
+            float Fx = 0.f, Fy = 0.f, Fz = 0.f, absF = 0.f, K = 0.f;
+            bool has_dir = false;
+            if (interface) {
+                // periodic box: neighbours wrap over the interior; jet: the record's
+                // psi plane holds the ghost values the forward step read unwrapped
+                const float *psi = M + size_t(kTapePsi) * N;
+                const int xn[3] = {kPeriodic ? wrap_interior(x - 1, g.NX) : x - 1, x,
+                                   kPeriodic ? wrap_interior(x + 1, g.NX) : x + 1};
+                const int yn[3] = {g.sy * (kPeriodic ? wrap_interior(y - 1, g.NY) : y - 1), g.sy * y,
+                                   g.sy * (kPeriodic ? wrap_interior(y + 1, g.NY) : y + 1)};
+                const int zn[3] = {g.sz * (kPeriodic ? wrap_interior(z - 1, g.NZ) : z - 1), g.sz * z,
+                                   g.sz * (kPeriodic ? wrap_interior(z + 1, g.NZ) : z + 1)};
+                float sx = 0.f, sy = 0.f, sz = 0.f;
+                static_for<kQ - 1>([&](auto I) {
+                    constexpr int i = decltype(I)::value + 1;
+                    using D = Dir<i>;
+                    const float wp = D::w * psi[xn[D::cx + 1] + yn[D::cy + 1] + zn[D::cz + 1]];
+                    if constexpr (D::cx != 0) sx += D::fx * wp;
+                    if constexpr (D::cy != 0) sy += D::fy * wp;
+                    if constexpr (D::cz != 0) sz += D::fz * wp;
+                });
+                Fx = kInvCs2 * sx;
+                Fy = kInvCs2 * sy;
+                Fz = kInvCs2 * sz;
+                absF = sqrtf(Fx * Fx + Fy * Fy + Fz * Fz);
+                has_dir = !(absF <= 1.0e-4f);
+                K = ph.beta * ((rr * rb) / (rho * rho)) * rho;
+            }
+            const float invF = has_dir ? 1.0f / absF : 0.0f;
+            const float invF2 = invF * invF;
+            [[maybe_unused]] const float Ah = ph.Ah;
+            const size_t row = pop_row(g, y, z);
+            // (lambda_r, lambda_b) of a direction: one float2, as the populations
+            auto lam_at = [&](int slot) {
+                return reinterpret_cast<const float2 *>(lam)[row + size_t(slot) * size_t(g.px) + size_t(x)];
+            };
+            // Bulk part: g_i = w_i P(c_i) with P the collision polynomial, so the
+            // sums over directions are the polynomial's coefficients dotted with
+            // the moments T_k = sum_i w_i lambda_g,i m_k(c_i) (and U_k with
+            // lambda_r - lambda_b for the colour split).  The moments are formed
+            // group by group: per (cy, cz) the three cx values reduce to
+            // (sum, sum cx, sum cx^2), which add into the 17 moments with the
+            // weights cy^b cz^c.
+            float Tm[17], Um[17];
+    #pragma unroll
+            for (int k = 0; k < 17; ++k) Tm[k] = Um[k] = 0.f;
+            static_for<9>([&](auto G) {
+                constexpr int cy = decltype(G)::value / 3 - 1, cz = decltype(G)::value % 3 - 1;
+                float mv[3], nv[3];
+                static_for<3>([&](auto X) {
+                    constexpr int cx = decltype(X)::value - 1;
+                    constexpr int i = dir_of(cx, cy, cz);
+                    const float2 l = lam_at(slot_pair(i));
+                    mv[cx + 1] = Dir<i>::w * (aR * l.x + aB * l.y);
+                    nv[cx + 1] = Dir<i>::w * (l.x - l.y);
+                });
+                const float m2 = mv[2] + mv[0], n2 = nv[2] + nv[0];
+                const float ms[3] = {m2 + mv[1], mv[2] - mv[0], m2};
+                const float ns[3] = {n2 + nv[1], nv[2] - nv[0], n2};
+                static_for<17>([&](auto K) {
+                    constexpr int k = decltype(K)::value;
+                    constexpr int wgt = ipow1(cy, poly_exp(k, 1)) * ipow1(cz, poly_exp(k, 2));
+                    constexpr int a = poly_exp(k, 0);
+                    if constexpr (wgt == 1) {
+                        Tm[k] += ms[a];
+                        Um[k] += ns[a];
+                    } else if constexpr (wgt == -1) {
+                        Tm[k] -= ms[a];
+                        Um[k] -= ns[a];
+                    }
+                });
             });
-            Fx = kInvCs2 * sx;
-            Fy = kInvCs2 * sy;
-            Fz = kInvCs2 * sz;
-            absF = sqrtf(Fx * Fx + Fy * Fy + Fz * Fz);
-            has_dir = !(absF <= 1.0e-4f);
-            K = ph.beta * ((rr * rb) / (rho * rho)) * rho;
-        }
-        const float invF = has_dir ? 1.0f / absF : 0.0f;
-        const float invF2 = invF * invF;
-        const float Ah = ph.Ah;
-        const size_t row = pop_row(g, y, z);
-        // (lambda_r, lambda_b) of a direction: one float2, as the populations
-        auto lam_at = [&](int slot) {
-            return reinterpret_cast<const float2 *>(lam)[row + size_t(slot) * size_t(g.px) + size_t(x)];
-        };
-        // Bulk part: g_i = w_i P(c_i) with P the collision polynomial, so the
-        // sums over directions are the polynomial's coefficients dotted with
-        // the moments T_k = sum_i w_i lambda_g,i m_k(c_i) (and U_k with
-        // lambda_r - lambda_b for the colour split).  The moments are formed
-        // group by group: per (cy, cz) the three cx values reduce to
-        // (sum, sum cx, sum cx^2), which add into the 17 moments with the
-        // weights cy^b cz^c.
-        float Tm[17], Um[17];
-#pragma unroll
-        for (int k = 0; k < 17; ++k) Tm[k] = Um[k] = 0.f;
-        static_for<9>([&](auto G) {
-            constexpr int cy = decltype(G)::value / 3 - 1, cz = decltype(G)::value % 3 - 1;
-            float mv[3], nv[3];
-            static_for<3>([&](auto X) {
-                constexpr int cx = decltype(X)::value - 1;
-                constexpr int i = dir_of(cx, cy, cz);
-                const float2 l = lam_at(slot_pair(i));
-                mv[cx + 1] = Dir<i>::w * (aR * l.x + aB * l.y);
-                nv[cx + 1] = Dir<i>::w * (l.x - l.y);
-            });
-            const float m2 = mv[2] + mv[0], n2 = nv[2] + nv[0];
-            const float ms[3] = {m2 + mv[1], mv[2] - mv[0], m2};
-            const float ns[3] = {n2 + nv[1], nv[2] - nv[0], n2};
-            static_for<17>([&](auto K) {
-                constexpr int k = decltype(K)::value;
-                constexpr int wgt = ipow1(cy, poly_exp(k, 1)) * ipow1(cz, poly_exp(k, 2));
-                constexpr int a = poly_exp(k, 0);
-                if constexpr (wgt == 1) {
-                    Tm[k] += ms[a];
-                    Um[k] += ns[a];
-                } else if constexpr (wgt == -1) {
-                    Tm[k] -= ms[a];
-                    Um[k] -= ns[a];
+            const PolyAdjoint pT = poly_adjoint(Tm, ux, uy, uz, n);
+            const PolyAdjoint pU = poly_adjoint(Um, ux, uy, uz, n);
+            const float(&S2)[6] = pT.S2;
+            const float(&S3)[7] = pT.S3;
+            const float l_rhoeq = rho * pT.Phi;  // sum lambda_g feq (feq is proportional to rho)
+            const float l_oms = pT.Psi;          // sum lambda_g fneq
+            float l_d = rho * pU.Phi + oms * pU.Psi;  // sum (lambda_r - lambda_b) g
+            // interface nodes: the perturbation and recolouring terms, direction by direction
+            float sAx = 0.f, sAy = 0.f, sAz = 0.f, sB = 0.f, sDx = 0.f, sDy = 0.f, sDz = 0.f, sE = 0.f, sBB = 0.f,
+                  l_Ah = 0.f;
+            if (interface) {
+                {  // rest direction: even only
+                    const float2 l0 = lam_at(slot_pair(0));
+                    const float lg = aR * l0.x + aB * l0.y, ld = l0.x - l0.y;
+                    const float o2A = -absF * Dir<0>::B;  // Omega2 / (A/2)
+                    l_d += ld * (Ah * o2A);
+                    sBB += lg * Dir<0>::B;
+                    l_Ah += lg * o2A;
                 }
-            });
-        });
-        const PolyAdjoint pT = poly_adjoint(Tm, ux, uy, uz, n);
-        const PolyAdjoint pU = poly_adjoint(Um, ux, uy, uz, n);
-        const float(&S2)[6] = pT.S2;
-        const float(&S3)[7] = pT.S3;
-        const float l_rhoeq = rho * pT.Phi;  // sum lambda_g feq (feq is proportional to rho)
-        const float l_oms = pT.Psi;          // sum lambda_g fneq
-        float l_d = rho * pU.Phi + oms * pU.Psi;  // sum (lambda_r - lambda_b) g
-        // interface nodes: the perturbation and recolouring terms, direction by direction
-        float sAx = 0.f, sAy = 0.f, sAz = 0.f, sB = 0.f, sDx = 0.f, sDy = 0.f, sDz = 0.f, sE = 0.f, sBB = 0.f,
-              l_Ah = 0.f;
-        if (interface) {
-            {  // rest direction: even only
-                const float2 l0 = lam_at(slot_pair(0));
-                const float lg = aR * l0.x + aB * l0.y, ld = l0.x - l0.y;
-                const float o2A = -absF * Dir<0>::B;  // Omega2 / (A/2)
-                l_d += ld * (Ah * o2A);
-                sBB += lg * Dir<0>::B;
-                l_Ah += lg * o2A;
+                static_for<(kQ - 1) / 2>([&](auto P) {
+                    constexpr int i = 2 * decltype(P)::value + 1;
+                    using D = Dir<i>;
+                    const float2 li = lam_at(slot_pair(i)), lo = lam_at(slot_pair(i + 1));
+                    const float lgi = aR * li.x + aB * li.y, lgo = aR * lo.x + aB * lo.y;
+                    const float ldi = li.x - li.y, ldo = lo.x - lo.y;
+                    const float gs = lgi + lgo, ds = ldi + ldo, dd = ldi - ldo;
+                    float fc = 0.f;
+                    if constexpr (D::cx != 0) fc += D::fx * Fx;
+                    if constexpr (D::cy != 0) fc += D::fy * Fy;
+                    if constexpr (D::cz != 0) fc += D::fz * Fz;
+                    const float o2A = absF * (D::w * (fc * fc) * invF2 - D::B);  // Omega2 / (A/2), even
+                    l_d += ds * (Ah * o2A);
+                    sBB += gs * D::B;
+                    l_Ah += gs * o2A;
+                    const float a = gs * D::w * fc, d = dd * D::w * D::invc;
+                    if constexpr (D::cx != 0) { sAx += D::fx * a; sDx += D::fx * d; }
+                    if constexpr (D::cy != 0) { sAy += D::fy * a; sDy += D::fy * d; }
+                    if constexpr (D::cz != 0) { sAz += D::fz * a; sDz += D::fz * d; }
+                    sB += a * fc;
+                    sE += d * fc;
+                });
             }
-            static_for<(kQ - 1) / 2>([&](auto P) {
-                constexpr int i = 2 * decltype(P)::value + 1;
-                using D = Dir<i>;
-                const float2 li = lam_at(slot_pair(i)), lo = lam_at(slot_pair(i + 1));
-                const float lgi = aR * li.x + aB * li.y, lgo = aR * lo.x + aB * lo.y;
-                const float ldi = li.x - li.y, ldo = lo.x - lo.y;
-                const float gs = lgi + lgo, ds = ldi + ldo, dd = ldi - ldo;
-                float fc = 0.f;
-                if constexpr (D::cx != 0) fc += D::fx * Fx;
-                if constexpr (D::cy != 0) fc += D::fy * Fy;
-                if constexpr (D::cz != 0) fc += D::fz * Fz;
-                const float o2A = absF * (D::w * (fc * fc) * invF2 - D::B);  // Omega2 / (A/2), even
-                l_d += ds * (Ah * o2A);
-                sBB += gs * D::B;
-                l_Ah += gs * o2A;
-                const float a = gs * D::w * fc, d = dd * D::w * D::invc;
-                if constexpr (D::cx != 0) { sAx += D::fx * a; sDx += D::fx * d; }
-                if constexpr (D::cy != 0) { sAy += D::fy * a; sDy += D::fy * d; }
-                if constexpr (D::cz != 0) { sAz += D::fz * a; sDz += D::fz * d; }
-                sB += a * fc;
-                sE += d * fc;
-            });
-        }
-        // fneq: Pi enters directly (H2) and through the third-order terms a3
-        const float c2 = oms * kInv2Cs4, c3 = oms * kInv2Cs6;
-        float lPxx = S2[0] * c2, lPxy = 2.0f * S2[1] * c2, lPyy = S2[2] * c2;
-        float lPyz = 2.0f * S2[3] * c2, lPzz = S2[4] * c2, lPxz = 2.0f * S2[5] * c2;
-        const float la_xxy = S3[0] * c3, la_xxz = S3[1] * c3, la_xyy = S3[2] * c3, la_xzz = S3[3] * c3;
-        const float la_yyz = S3[4] * c3, la_yzz = S3[5] * c3, la_xyz = 2.0f * S3[6] * c3;
-        lPxx += la_xxy * uy + la_xxz * uz;
-        lPyy += la_xyy * ux + la_yyz * uz;
-        lPzz += la_xzz * ux + la_yzz * uy;
-        lPxy += 2.0f * la_xxy * ux + 2.0f * la_xyy * uy + la_xyz * uz;
-        lPxz += 2.0f * la_xxz * ux + 2.0f * la_xzz * uz + la_xyz * uy;
-        lPyz += 2.0f * la_yyz * uy + 2.0f * la_yzz * uz + la_xyz * ux;
-        float lux = 2.0f * la_xxy * n.pxy + 2.0f * la_xxz * n.pxz + la_xyy * n.pyy + la_xzz * n.pzz + la_xyz * n.pyz;
-        float luy = la_xxy * n.pxx + 2.0f * la_xyy * n.pxy + 2.0f * la_yyz * n.pyz + la_yzz * n.pzz + la_xyz * n.pxz;
-        float luz = la_xxz * n.pxx + 2.0f * la_xzz * n.pxz + la_yyz * n.pyy + 2.0f * la_yzz * n.pyz + la_xyz * n.pxy;
-        // feq: rho times the u-gradient of the feq polynomial against T
-        lux += rho * pT.dPhi[0];
-        luy += rho * pT.dPhi[1];
-        luz += rho * pT.dPhi[2];
-        // colour gradient: perturbation and recolouring
-        float lFx = 0.f, lFy = 0.f, lFz = 0.f, lK = 0.f;
-        if (interface) {
-            if (has_dir) {
-                const float i3 = invF2 * invF;
-                lFx = Ah * (2.0f * invF * sAx - Fx * i3 * sB - Fx * invF * sBB) + K * (sDx * invF - Fx * i3 * sE);
-                lFy = Ah * (2.0f * invF * sAy - Fy * i3 * sB - Fy * invF * sBB) + K * (sDy * invF - Fy * i3 * sE);
-                lFz = Ah * (2.0f * invF * sAz - Fz * i3 * sB - Fz * invF * sBB) + K * (sDz * invF - Fz * i3 * sE);
-                lK = sE * invF;
-            } else if (absF > 0.0f) {
-                const float q = -Ah * sBB / absF;
-                lFx = q * Fx;
-                lFy = q * Fy;
-                lFz = q * Fz;
+            // fneq: Pi enters directly (H2) and through the third-order terms a3
+            const float c2 = oms * kInv2Cs4, c3 = oms * kInv2Cs6;
+            float lPxx = S2[0] * c2, lPxy = 2.0f * S2[1] * c2, lPyy = S2[2] * c2;
+            float lPyz = 2.0f * S2[3] * c2, lPzz = S2[4] * c2, lPxz = 2.0f * S2[5] * c2;
+            const float la_xxy = S3[0] * c3, la_xxz = S3[1] * c3, la_xyy = S3[2] * c3, la_xzz = S3[3] * c3;
+            const float la_yyz = S3[4] * c3, la_yzz = S3[5] * c3, la_xyz = 2.0f * S3[6] * c3;
+            lPxx += la_xxy * uy + la_xxz * uz;
+            lPyy += la_xyy * ux + la_yyz * uz;
+            lPzz += la_xzz * ux + la_yzz * uy;
+            lPxy += 2.0f * la_xxy * ux + 2.0f * la_xyy * uy + la_xyz * uz;
+            lPxz += 2.0f * la_xxz * ux + 2.0f * la_xzz * uz + la_xyz * uy;
+            lPyz += 2.0f * la_yyz * uy + 2.0f * la_yzz * uz + la_xyz * ux;
+            float lux = 2.0f * la_xxy * n.pxy + 2.0f * la_xxz * n.pxz + la_xyy * n.pyy + la_xzz * n.pzz + la_xyz * n.pyz;
+            float luy = la_xxy * n.pxx + 2.0f * la_xyy * n.pxy + 2.0f * la_yyz * n.pyz + la_yzz * n.pzz + la_xyz * n.pxz;
+            float luz = la_xxz * n.pxx + 2.0f * la_xzz * n.pxz + la_yyz * n.pyy + 2.0f * la_yzz * n.pyz + la_xyz * n.pxy;
+            // feq: rho times the u-gradient of the feq polynomial against T
+            lux += rho * pT.dPhi[0];
+            luy += rho * pT.dPhi[1];
+            luz += rho * pT.dPhi[2];
+            // colour gradient: perturbation and recolouring
+            float lFx = 0.f, lFy = 0.f, lFz = 0.f, lK = 0.f;
+            if (interface) {
+                if (has_dir) {
+                    const float i3 = invF2 * invF;
+                    lFx = Ah * (2.0f * invF * sAx - Fx * i3 * sB - Fx * invF * sBB) + K * (sDx * invF - Fx * i3 * sE);
+                    lFy = Ah * (2.0f * invF * sAy - Fy * i3 * sB - Fy * invF * sBB) + K * (sDy * invF - Fy * i3 * sE);
+                    lFz = Ah * (2.0f * invF * sAz - Fz * i3 * sB - Fz * invF * sBB) + K * (sDz * invF - Fz * i3 * sE);
+                    lK = sE * invF;
+                } else if (absF > 0.0f) {
+                    const float q = -Ah * sBB / absF;
+                    lFx = q * Fx;
+                    lFy = q * Fy;
+                    lFz = q * Fz;
+                }
             }
-        }
-        const float inv2 = invr * invr;
-        const float l_rho = l_rhoeq * invr;  // feq is proportional to rho
-        lmom[kMomRR * N + id] = l_rho + l_d * rb * inv2 + lK * ph.beta * rb * rb * inv2;
-        lmom[kMomRB * N + id] = l_rho - l_d * rr * inv2 + lK * ph.beta * rr * rr * inv2;
-        // the objective's source: J_t = (w/2) sum uy^2 over nodes with y >= y_obs,
-        // or the profile objective's dJ/duy of the node's radial bin (the bin of
-        // radial_accumulate_warp, same float arithmetic)
-        float lobj = 0.f;
-        if (obj.table) {
-            const float dx = float(x) - ph.jet_x0, dz = float(z) - ph.jet_z0;
-            const unsigned rbin = unsigned(sqrtf(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dz, dz))));
-            if (rbin < unsigned(ph.NRB)) lobj = obj.table[size_t(y) * ph.NRB + rbin];
-        } else if (obj.weight != 0.0f && y >= obj.y_obs) {
-            lobj = obj.weight * uy;
-            a_J = 0.5 * double(obj.weight) * double(uy) * double(uy);
-        }
-        lmom[kMomUX * N + id] = lux;
-        lmom[kMomUY * N + id] = luy + lobj;
-        lmom[kMomUZ * N + id] = luz;
-        lmom[kMomPXX * N + id] = lPxx;
-        lmom[kMomPXY * N + id] = lPxy;
-        lmom[kMomPYY * N + id] = lPyy;
-        lmom[kMomPYZ * N + id] = lPyz;
-        lmom[kMomPZZ * N + id] = lPzz;
-        lmom[kMomPXZ * N + id] = lPxz;
-        lf[0 * N + id] = lFx;
-        lf[1 * N + id] = lFy;
-        lf[2 * N + id] = lFz;
-        a_omega = -double(l_oms);  // oms = 1 - omega
-        a_Ah = double(l_Ah);
-    }
-    double r[3] = {a_omega, a_Ah, obj.J ? a_J : 0.0};
-    block_sum3(r, sh, kBX * kBY);
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        atomicAdd(acc, r[0]);
-        atomicAdd(acc + 1, r[1]);
-        if (obj.J) atomicAdd(obj.J, r[2]);
-    }
+            const float inv2 = invr * invr;
+            const float l_rho = l_rhoeq * invr;  // feq is proportional to rho
+            o.rr = l_rho + l_d * rb * inv2 + lK * ph.beta * rb * rb * inv2;
+    o.rb = l_rho - l_d * rr * inv2 + lK * ph.beta * rr * rr * inv2;
+    // the objective's source: J_t = (w/2) sum uy^2 over nodes with y >= y_obs,
+            // or the profile objective's dJ/duy of the node's radial bin (the bin of
+            // radial_accumulate_warp, same float arithmetic)
+            float lobj = 0.f;
+            if (obj.table) {
+                const float dx = float(x) - ph.jet_x0, dz = float(z) - ph.jet_z0;
+                const unsigned rbin = unsigned(sqrtf(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dz, dz))));
+                if (rbin < unsigned(ph.NRB)) lobj = obj.table[size_t(y) * ph.NRB + rbin];
+            } else if (obj.weight != 0.0f && y >= obj.y_obs) {
+                lobj = obj.weight * uy;
+                a_J += 0.5 * double(obj.weight) * double(uy) * double(uy);
+            }
+            o.ux = lux;
+    o.uy = luy + lobj;
+    o.uz = luz;
+    o.pxx = lPxx; o.pxy = lPxy; o.pyy = lPyy; o.pyz = lPyz; o.pzz = lPzz; o.pxz = lPxz;
+    o.Fx = lFx; o.Fy = lFy; o.Fz = lFz;
+    a_omega -= double(l_oms);  // oms = 1 - omega
+    if constexpr (kInterface) a_Ah += double(l_Ah);
 }
 
-// Per node: the psi-adjoint gathered from the neighbours' F-adjoints, then back
-// through the moments to the 54 pulled populations, stored at their pull
-// sources (transposed streaming) in lam_out.
+// Moment part of a node: the psi-adjoint lpsi and the adjoints of its moments
+// back through the moments to the 54 pulled populations, stored at their pull
+// sources (transposed streaming) in lam_out.  `node` false: a column that is
+// only stored (store_columns), to complete the sectors of the rows.
 template <bool kPeriodic>
-__global__ void __launch_bounds__(kBX * kBY) k_adj_moments(const DeviceState s, const float *__restrict__ M,
-                                                          const float *lmom, const float *lf, float *lam_out) {
-    // The block's F-adjoints with a one-node halo, [3][3 planes][kBY+2][kBX+2],
-    // so the 26-neighbour gather reads shared memory.  A halo position holds
-    // lf of the node whose psi it is: periodic neighbours wrap over the
-    // interior; otherwise a position off the interior holds 0 (only interior
-    // nodes relax, and read psi there).
-    constexpr int TX = kBX + 2, TY = kBY + 2, TP = TX * TY * 3;
-    __shared__ float tile[3 * TP];
+__device__ __forceinline__ void adj_moments_node(const DeviceState &s, const float *M, const NodeAdjoint &o,
+                                                 float lpsi, float *lam_out, int x, int y, int z, bool node) {
     const Geometry &g = s.g;
     const size_t N = g.N;
-    const int bx0 = int(blockIdx.x) * kBX - 1, by0 = int(blockIdx.y) * kBY - 1, bz0 = int(blockIdx.z) - 1;
-    for (int t = threadIdx.y * kBX + threadIdx.x; t < TP; t += kBX * kBY) {
-        const int xt = t % TX, yt = (t / TX) % TY, zt = t / (TX * TY);
-        int xn = bx0 + xt, yn = by0 + yt, zn = bz0 + zt;
-        bool ok;
-        if constexpr (kPeriodic) {
-            ok = xn >= 0 && xn <= g.NX - 1 && yn >= 0 && yn <= g.NY - 1 && zn >= 0 && zn <= g.NZ - 1;
-            xn = wrap_interior(xn, g.NX);
-            yn = wrap_interior(yn, g.NY);
-            zn = wrap_interior(zn, g.NZ);
-        } else {
-            ok = xn >= 1 && xn <= g.NX - 2 && yn >= 1 && yn <= g.NY - 2 && zn >= 1 && zn <= g.NZ - 2;
-        }
-        float v0 = 0.f, v1 = 0.f, v2 = 0.f;
-        if (ok) {
-            const uint32_t nid = uint32_t(xn) + uint32_t(g.sy) * uint32_t(yn) + uint32_t(g.sz) * uint32_t(zn);
-            v0 = lf[0 * N + nid];
-            v1 = lf[1 * N + nid];
-            v2 = lf[2 * N + nid];
-        }
-        tile[t] = v0;
-        tile[TP + t] = v1;
-        tile[2 * TP + t] = v2;
+    float lrr = 0.f, lrb = 0.f, k0 = 0.f, ljx = 0.f, ljy = 0.f, ljz = 0.f;
+    float lPxx = 0.f, lPxy = 0.f, lPyy = 0.f, lPyz = 0.f, lPzz = 0.f, lPxz = 0.f;
+    if (node) {
+        const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
+        const float rr = M[kMomRR * N + id], rb = M[kMomRB * N + id];
+        const float ux = M[kMomUX * N + id], uy = M[kMomUY * N + id], uz = M[kMomUZ * N + id];
+        const float rho = rr + rb;
+        const float inv2 = 1.0f / (rho * rho);
+        lrr = o.rr + lpsi * 2.0f * rb * inv2;
+        lrb = o.rb - lpsi * 2.0f * rr * inv2;
+        lPxx = o.pxx; lPxy = o.pxy; lPyy = o.pyy;
+        lPyz = o.pyz; lPzz = o.pzz; lPxz = o.pxz;
+        // Pi = A - rho u u
+        const float lux = o.ux - rho * (2.0f * ux * lPxx + uy * lPxy + uz * lPxz);
+        const float luy = o.uy - rho * (2.0f * uy * lPyy + ux * lPxy + uz * lPyz);
+        const float luz = o.uz - rho * (2.0f * uz * lPzz + ux * lPxz + uy * lPyz);
+        float lrho = -(lPxx * ux * ux + lPxy * ux * uy + lPyy * uy * uy + lPyz * uy * uz + lPzz * uz * uz + lPxz * ux * uz);
+        // u = j / rho
+        const float invr = 1.0f / rho;
+        ljx = lux * invr; ljy = luy * invr; ljz = luz * invr;
+        lrho -= (lux * ux + luy * uy + luz * uz) * invr;
+        // lambda_g,i = lrho + lj.c_i + lP:H2(c_i) is a quadratic polynomial in c_i:
+        // evaluated at the 27 directions by sum factorisation (per cz, then cy,
+        // then cx) instead of a Hermite sum per direction
+        k0 = lrho - kCs2 * (lPxx + lPyy + lPzz);
     }
-    __syncthreads();
-    const int x = blockIdx.x * kBX + threadIdx.x;
-    const int y = blockIdx.y * kBY + threadIdx.y;
-    const int z = blockIdx.z;
-    if (!(x >= 1 && x <= g.NX - 2 && y >= 1 && y <= g.NY - 2 && z >= 1 && z <= g.NZ - 2)) return;
-    const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
-    const float *mom = M;
-    const float rr = mom[kMomRR * N + id], rb = mom[kMomRB * N + id];
-    const float ux = mom[kMomUX * N + id], uy = mom[kMomUY * N + id], uz = mom[kMomUZ * N + id];
-    const float rho = rr + rb;
-    // psi(y) enters F(y - c_j) with weight w_j c_j / cs2
-    float lpsi = 0.f;
-    const int tc = (1 * TY + int(threadIdx.y) + 1) * TX + int(threadIdx.x) + 1;  // the node in the tile
-    static_for<kQ - 1>([&](auto I) {
-        constexpr int i = decltype(I)::value + 1;
-        using D = Dir<i>;
-        const int tn = tc - (D::cz * TY + D::cy) * TX - D::cx;
-        float dot = 0.f;
-        if constexpr (D::cx != 0) dot += D::fx * tile[tn];
-        if constexpr (D::cy != 0) dot += D::fy * tile[TP + tn];
-        if constexpr (D::cz != 0) dot += D::fz * tile[2 * TP + tn];
-        lpsi += D::w * dot;
-    });
-    lpsi *= kInvCs2;
-    const float inv2 = 1.0f / (rho * rho);
-    const float lrr = lmom[kMomRR * N + id] + lpsi * 2.0f * rb * inv2;
-    const float lrb = lmom[kMomRB * N + id] - lpsi * 2.0f * rr * inv2;
-    const float lPxx = lmom[kMomPXX * N + id], lPxy = lmom[kMomPXY * N + id], lPyy = lmom[kMomPYY * N + id];
-    const float lPyz = lmom[kMomPYZ * N + id], lPzz = lmom[kMomPZZ * N + id], lPxz = lmom[kMomPXZ * N + id];
-    // Pi = A - rho u u
-    const float lux = lmom[kMomUX * N + id] - rho * (2.0f * ux * lPxx + uy * lPxy + uz * lPxz);
-    const float luy = lmom[kMomUY * N + id] - rho * (2.0f * uy * lPyy + ux * lPxy + uz * lPyz);
-    const float luz = lmom[kMomUZ * N + id] - rho * (2.0f * uz * lPzz + ux * lPxz + uy * lPyz);
-    float lrho = -(lPxx * ux * ux + lPxy * ux * uy + lPyy * uy * uy + lPyz * uy * uz + lPzz * uz * uz + lPxz * ux * uz);
-    // u = j / rho
-    const float invr = 1.0f / rho;
-    const float ljx = lux * invr, ljy = luy * invr, ljz = luz * invr;
-    lrho -= (lux * ux + luy * uy + luz * uz) * invr;
-    // lambda_g,i = lrho + lj.c_i + lP:H2(c_i) is a quadratic polynomial in c_i:
-    // evaluated at the 27 directions by sum factorisation (per cz, then cy,
-    // then cx) instead of a Hermite sum per direction
-    const float k0 = lrho - kCs2 * (lPxx + lPyy + lPzz);
     const PullMap<CodecF32> pm(g, x, y, z, kPeriodic);
     static_for<3>([&](auto CZ) {
         constexpr int cz = decltype(CZ)::value - 1;
@@ -918,14 +856,235 @@ __global__ void __launch_bounds__(kBX * kBY) k_adj_moments(const DeviceState s, 
                 constexpr int cx = decltype(CX)::value - 1;
                 constexpr int i = dir_of(cx, cy, cz);
                 const float lgi = cx == 0 ? c0 : (cx > 0 ? c2 + c1 : c2 - c1);
+                // lanes of columns that are only stored write 0 to their own
+                // column of the rows, never to a y ghost plane
+                if (!node && !kPeriodic && ((cy == 1 && pm.gy_p) || (cy == -1 && pm.gy_m))) return;
                 size_t grow;
                 int xs;
-                pm.template src<i>(x, grow, xs);
+                pm.template src<i>(node ? x : x + cx, grow, xs);
                 reinterpret_cast<float2 *>(lam_out)[grow + size_t(dir_cx(i) + 1) * g.px + xs] =
                     make_float2(lrr + lgi, lrb + lgi);
             });
         });
     });
+}
+
+__device__ __forceinline__ void adj_write(const NodeAdjoint &o, float *lmom, size_t N, uint32_t id) {
+    const float v[kMomCount] = {o.rr, o.rb, o.ux, o.uy, o.uz, o.pxx, o.pxy, o.pyy, o.pyz, o.pzz, o.pxz};
+#pragma unroll
+    for (int k = 0; k < kMomCount; ++k) lmom[size_t(k) * N + id] = v[k];
+}
+__device__ __forceinline__ void adj_read(NodeAdjoint &o, const float *lmom, size_t N, uint32_t id) {
+    float v[kMomCount];
+#pragma unroll
+    for (int k = 0; k < kMomCount; ++k) v[k] = lmom[size_t(k) * N + id];
+    o = NodeAdjoint{v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], v[9], v[10], 0.f, 0.f, 0.f};
+}
+
+// The reverse step in the pieces of 32 columns of the split step (fused.cuh),
+// with the flags of the pieces that hold an interface node of the state.  Only
+// an interface node has a colour-gradient adjoint F, and a node's psi-adjoint
+// gathers F of its 26 neighbours, so a piece with no flagged piece around it is
+// taken from lambda_in to lambda_out in one pass:
+//   k_adj_relax  unflagged pieces: the relaxation part, and where no interface
+//                node is around the moment part too; otherwise the moments'
+//                adjoints go to lmom, and the piece is marked as left over.
+//                Flagged pieces: the relaxation part, to lmom and lf.
+//   k_adj_near   pieces left over: psi-adjoint from lf of the interface nodes
+//                around, moment part.
+// (The jet's boundary adjoint, between the two, adds to lmom in rows 1 and
+// NY-2, which are always left over.)
+// Bound by HBM: lambda 216 B read and 216 written, the moment record 48 read a
+// node; lmom and lf (56 B written and read) only near interfaces, where the
+// two-pass form moved them for every node.  Reverse step, before and after:
+// 96^3 bubble (a third of the pieces left over) 124 -> 109 us, jet 64x128x64
+// 101 -> 79 us (its boundary adjoint 26 -> 7 us of that).
+// CTAs per SM: 20 warps of 96 registers for k_adj_relax (which spill a little:
+// 9.33 ms for the 96^3 bubble's 40 steps against 9.86 at 16 warps that do not
+// and 9.44 at 24), 24 of 80 for k_adj_near (9.29 ms against 9.33 at 20).
+constexpr int kAdjThreads = 128, kAdjRelaxBlocks = 5, kAdjNearBlocks = 6;
+
+__host__ __device__ __forceinline__ int adj_pieces_per_row(const Geometry &g) { return pieces_per_row<CodecF32>(g); }
+
+// What piece (w, y, z) sees of the flags around it: bit 3 r + d, r = 3 (dy + 1)
+// + dz + 1 over the rows; d = 1: the row's piece at w holds an interface node;
+// d = 0, 2: the node before its first or after its last column is one.  The box
+// wraps when periodic; outside it nothing is flagged.  Warp-collective.
+template <bool kPeriodic>
+__device__ __forceinline__ unsigned flags_around(const Geometry &g, const uint8_t *flags, int w, int y, int z) {
+    const int ppr = adj_pieces_per_row(g), lane = int(threadIdx.x & 31);
+    bool hit = false;
+    if (lane < 27) {
+        int yy = y + lane / 9 - 1, zz = z + (lane / 3) % 3 - 1, ww = w + lane % 3 - 1;
+        if constexpr (kPeriodic) {
+            yy = wrap_interior(yy, g.NY);
+            zz = wrap_interior(zz, g.NZ);
+            // the piece of column NX-2 lies before column 1's, and after it
+            ww = ww < 0 ? (g.NX - 2) >> 5 : (ww * 32 > g.NX - 2 ? 0 : ww);
+        }
+        if (yy >= 1 && yy <= g.NY - 2 && zz >= 1 && zz <= g.NZ - 2 && ww >= 0 && ww < ppr)
+            hit = (flags[(size_t(zz - 1) * (g.NY - 2) + (yy - 1)) * ppr + ww] >> (lane % 3 == 1 ? 0 : lane % 3 == 0 ? 2 : 1)) & 1;
+    }
+    return __ballot_sync(kFull, hit);
+}
+
+// Calls f(w, y, z) with a whole warp for every piece set in `flags`, the pieces
+// spread over blocks 0 .. ctas-1 as in k_step_interface.
+template <class F>
+__device__ __forceinline__ void for_flagged_pieces(const Geometry &g, const uint8_t *flags, uint32_t ctas, F &&f) {
+    __shared__ uint32_t list[kAdjThreads];
+    __shared__ int found;
+    constexpr uint32_t kGroup = 4;
+    const int lane = int(threadIdx.x & 31), warp = int(threadIdx.x >> 5);
+    const uint32_t ppr = uint32_t(adj_pieces_per_row(g));
+    const uint32_t pieces = ppr * uint32_t(g.NY - 2) * uint32_t(g.NZ - 2);
+    for (uint32_t first = 0; first < pieces; first += ctas * kAdjThreads) {
+        if (threadIdx.x == 0) found = 0;
+        __syncthreads();
+        const uint64_t mine = (uint64_t(threadIdx.x / kGroup) * ctas + blockIdx.x) * kGroup + threadIdx.x % kGroup + first;
+        const bool flagged = mine < pieces && flags[mine];
+        const unsigned hits = __ballot_sync(kFull, flagged);
+        int base = 0;
+        if (lane == 0 && hits) base = atomicAdd(&found, __popc(hits));
+        base = __shfl_sync(kFull, base, 0);
+        if (flagged) list[base + __popc(hits & ((1u << lane) - 1u))] = uint32_t(mine);
+        __syncthreads();
+        for (int i = warp; i < found; i += kAdjThreads / 32) {
+            const uint32_t piece = list[i], row = piece / ppr, zi = row / uint32_t(g.NY - 2);
+            f(int(piece - row * ppr), 1 + int(row - zi * uint32_t(g.NY - 2)), 1 + int(zi));
+        }
+        __syncthreads();
+    }
+}
+
+// The two roles share a launch: its first `list_blocks` blocks take the flagged
+// pieces, each other block the unflagged ones among kAdjThreads / 32 neighbours.
+template <bool kPeriodic>
+__global__ void __launch_bounds__(kAdjThreads, kAdjRelaxBlocks) k_adj_relax(const DeviceState s,
+                                                                           const float *__restrict__ M,
+                                                                           const uint8_t *__restrict__ flags,
+                                                                           uint8_t *near_flags, const float *lam,
+                                                                           float *lmom, float *lf, float *lam_out,
+                                                                           double *acc, AdjObjective obj,
+                                                                           int list_blocks, int plane_blocks) {
+    __shared__ double sh[3 * (kAdjThreads / 32)];
+    const Geometry &g = s.g;
+    double a_omega = 0.0, a_Ah = 0.0, a_J = 0.0;
+    if (int(blockIdx.x) < list_blocks) {
+        for_flagged_pieces(g, flags, uint32_t(list_blocks), [&](int w, int y, int z) {
+            const int x = w * 32 + int(threadIdx.x & 31);
+            if (x < 1 || x > g.NX - 2) return;
+            NodeAdjoint o;
+            adj_collide_node<kPeriodic, true>(s, M, lam, obj, x, y, z, o, a_omega, a_Ah, a_J);
+            const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
+            adj_write(o, lmom, g.N, id);
+            lf[id] = o.Fx;
+            lf[size_t(g.N) + id] = o.Fy;
+            lf[size_t(2) * g.N + id] = o.Fz;
+        });
+    } else {
+        const int ppr = adj_pieces_per_row(g), block = int(blockIdx.x) - list_blocks, zi = block / plane_blocks;
+        const int piece = (block - zi * plane_blocks) * (kAdjThreads / 32) + int(threadIdx.x >> 5);
+        const int row = piece / ppr, y = 1 + row, z = 1 + zi;
+        if (y <= g.NY - 2) {  // uniform over the warp
+            const int w = piece - row * ppr, x = w * 32 + int(threadIdx.x & 31);
+            const unsigned around = flags_around<kPeriodic>(g, flags, w, y, z);
+            const bool near_one = around != 0 || (!kPeriodic && (y == 1 || y == g.NY - 2));
+            if ((x & 31) == 0) near_flags[(size_t(zi) * (g.NY - 2) + row) * ppr + w] = near_one ? 1 : 0;
+            const bool node = x >= 1 && x <= g.NX - 2;
+            if (!((around >> 13) & 1u)) {
+                NodeAdjoint o{};
+                if (node) adj_collide_node<kPeriodic, false>(s, M, lam, obj, x, y, z, o, a_omega, a_Ah, a_J);
+                if (!near_one) {
+                    if (x < store_columns<CodecF32>(g)) adj_moments_node<kPeriodic>(s, M, o, 0.0f, lam_out, x, y, z, node);
+                } else if (node) {
+                    const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
+                    adj_write(o, lmom, g.N, id);
+                    if (!kPeriodic && y == g.NY - 2)  // read by the boundary adjoint
+                        for (int k = 0; k < 3; ++k) lf[size_t(k) * g.N + id] = 0.0f;
+                }
+            }
+        }
+    }
+    double r[3] = {a_omega, a_Ah, obj.J ? a_J : 0.0};
+    block_sum3(r, sh, kAdjThreads);
+    if (threadIdx.x == 0) {
+        if (r[0] != 0.0) atomicAdd(acc, r[0]);
+        if (r[1] != 0.0) atomicAdd(acc + 1, r[1]);
+        if (r[2] != 0.0) atomicAdd(obj.J, r[2]);
+    }
+}
+
+template <bool kPeriodic>
+__global__ void __launch_bounds__(kAdjThreads, kAdjNearBlocks) k_adj_near(const DeviceState s, const float *__restrict__ M,
+                                                                const uint8_t *__restrict__ flags,
+                                                                const uint8_t *__restrict__ near_flags,
+                                                                const float *lmom, const float *lf, float *lam_out) {
+    const Geometry &g = s.g;
+    const size_t N = g.N;
+    for_flagged_pieces(g, near_flags, gridDim.x, [&](int w, int y, int z) {
+        const unsigned around = flags_around<kPeriodic>(g, flags, w, y, z);
+        const int x = w * 32 + int(threadIdx.x & 31);
+        if (x >= store_columns<CodecF32>(g)) return;
+        const bool node = x >= 1 && x <= g.NX - 2;
+        NodeAdjoint o{};
+        float lpsi = 0.f;
+        if (node) {
+            // psi(y) enters F(y - c_j) with weight w_j c_j / cs2
+            const int xs[3] = {kPeriodic ? wrap_interior(x - 1, g.NX) : x - 1, x,
+                               kPeriodic ? wrap_interior(x + 1, g.NX) : x + 1};
+            // the piece of the node before and after: bit offsets in a row of `around`
+            const int px[3] = {(x & 31) == 0 || x == 1 ? 0 : 1, 1, (x & 31) == 31 || x == g.NX - 2 ? 2 : 1};
+            static_for<kQ - 1>([&](auto I) {
+                constexpr int i = decltype(I)::value + 1;
+                using D = Dir<i>;
+                constexpr int r = 3 * (1 - D::cy) + (1 - D::cz);  // row (y - cy, z - cz)
+                float v0 = 0.f, v1 = 0.f, v2 = 0.f;
+                if ((around >> (3 * r + px[1 - D::cx])) & 1u) {
+                    const int yn = kPeriodic ? wrap_interior(y - D::cy, g.NY) : y - D::cy;
+                    const int zn = kPeriodic ? wrap_interior(z - D::cz, g.NZ) : z - D::cz;
+                    const uint32_t nid = uint32_t(xs[1 - D::cx]) + uint32_t(g.sy) * uint32_t(yn) + uint32_t(g.sz) * uint32_t(zn);
+                    if constexpr (D::cx != 0) v0 = lf[nid];
+                    if constexpr (D::cy != 0) v1 = lf[N + nid];
+                    if constexpr (D::cz != 0) v2 = lf[2 * N + nid];
+                }
+                float dot = 0.f;
+                if constexpr (D::cx != 0) dot += D::fx * v0;
+                if constexpr (D::cy != 0) dot += D::fy * v1;
+                if constexpr (D::cz != 0) dot += D::fz * v2;
+                lpsi += D::w * dot;
+            });
+            lpsi *= kInvCs2;
+            const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
+            adj_read(o, lmom, N, id);
+        }
+        adj_moments_node<kPeriodic>(s, M, o, lpsi, lam_out, x, y, z, node);
+    });
+}
+
+// One wave of blocks over the flagged pieces, at most a warp each.
+unsigned adj_list_blocks(const Geometry &g, int per_sm) {
+    const long long per = kAdjThreads / 32, pieces = (long long)adj_pieces_per_row(g) * (g.NY - 2) * (g.NZ - 2);
+    return unsigned(std::min<long long>((pieces + per - 1) / per, 148ll * per_sm));
+}
+
+// Flags of the pieces of a moment record (k_step_pull sets those of the states
+// it records).
+__global__ void __launch_bounds__(kRedThreads) k_piece_flags(const DeviceState s, const float *__restrict__ M,
+                                                            uint8_t *flags) {
+    const Geometry &g = s.g;
+    const int ppr = adj_pieces_per_row(g);
+    const int piece = int(blockIdx.x) * (kRedThreads / 32) + int(threadIdx.x >> 5);
+    const int row = piece / ppr, y = 1 + row, z = 1 + int(blockIdx.y);
+    if (y > g.NY - 2) return;
+    const int w = piece - row * ppr, x = w * 32 + int(threadIdx.x & 31);
+    bool interface = false;
+    if (x >= 1 && x <= g.NX - 2) {
+        const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
+        interface = !is_bulk(M[kMomRR * size_t(g.N) + id], M[kMomRB * size_t(g.N) + id]);
+    }
+    const unsigned lanes = __ballot_sync(kFull, interface);
+    if ((x & 31) == 0) flags[(size_t(blockIdx.y) * (g.NY - 2) + row) * ppr + w] = piece_flag(g, w, lanes);
 }
 
 // Adjoint of the regularised non-equilibrium part over a set of directions:
@@ -971,10 +1130,10 @@ __device__ __forceinline__ float inlet_noise_factor(const Physics &ph, int64_t s
     return 1.0f + (2.0f * u - 1.0f) * ph.inlet_noise;
 }
 
-// One thread per interior column (x, z): the outlet at y = NY-1 and, in a jet
-// column, the inlet at y = 0.  A ghost-plane slot enters only if an interior
+// One thread per interior column (x, z): the outlet at y = NY-1 (blockIdx.z 0)
+// or, in a jet column, the inlet at y = 0 (1).  A ghost-plane slot enters only if an interior
 // node pulls it (the boundary also writes slots nothing reads).
-__global__ void __launch_bounds__(256) k_adj_boundary(const DeviceState s, int64_t step, const float *__restrict__ M,
+__global__ void __launch_bounds__(32) k_adj_boundary(const DeviceState s, int64_t step, const float *__restrict__ M,
                                                       const float *__restrict__ Bt, const float *__restrict__ lam,
                                                       const float *__restrict__ lf, float *lmom,
                                                       const float *__restrict__ LB_in, float *LB_out,
@@ -991,7 +1150,25 @@ __global__ void __launch_bounds__(256) k_adj_boundary(const DeviceState s, int64
 #pragma unroll
     for (int k = 0; k < kInletBesselMax; ++k) dc[k] = 0.f;
     auto pulled = [&](int xp, int zp) { return xp >= 1 && xp <= g.NX - 2 && zp >= 1 && zp <= g.NZ - 2; };
-    if (col) {
+    // The values a side reads from memory come first, all in flight together;
+    // one after the other behind the branches they took 26 us a launch.
+    auto pulled_lambda = [&](auto CY, int y, float2 (&l)[9]) {
+        constexpr int cy = decltype(CY)::value;
+        static_for<9>([&](auto K) {
+            constexpr int k = decltype(K)::value, i = dir_of(k / 3 - 1, cy, k % 3 - 1);
+            l[k] = pulled(x + Dir<i>::cx, z + Dir<i>::cz)
+                       ? reinterpret_cast<const float2 *>(lam)[pop_index(g, slot_pair(i), x, y, z)]
+                       : make_float2(0.f, 0.f);
+        });
+    };
+    auto add_to = [&](uint32_t id, const float (&v)[kMomCount]) {
+        float m[kMomCount];
+#pragma unroll
+        for (int k = 0; k < kMomCount; ++k) m[k] = lmom[size_t(k) * N + id];
+#pragma unroll
+        for (int k = 0; k < kMomCount; ++k) lmom[size_t(k) * N + id] = m[k] + v[k];
+    };
+    if (col && blockIdx.z == 0) {
         // ---------------- outlet (boundary_conditions.cuh:163-233)
         const uint32_t idF = uint32_t(x) + uint32_t(g.sy) * uint32_t(g.NY - 2) + uint32_t(g.sz) * uint32_t(z);
         const float phi[5] = {M[kMomRR * N + idF], M[kMomRB * N + idF], M[kMomUX * N + idF], M[kMomUY * N + idF],
@@ -999,6 +1176,17 @@ __global__ void __launch_bounds__(256) k_adj_boundary(const DeviceState s, int64
         const NeqTerms nF = make_neq(M[kMomPXX * N + idF], M[kMomPXY * N + idF], M[kMomPYY * N + idF],
                                      M[kMomPYZ * N + idF], M[kMomPZZ * N + idF], M[kMomPXZ * N + idF], phi[2], phi[3],
                                      phi[4]);
+        float2 l9[9];
+        pulled_lambda(std::integral_constant<int, -1>{}, g.NY - 1, l9);
+        // colour-gradient adjoints of the nodes (x - cx, NY-2, z - cz)
+        float f9[9][3];
+        static_for<9>([&](auto K) {
+            constexpr int k = decltype(K)::value, cx = k / 3 - 1, cz = k % 3 - 1;
+            const bool in = pulled(x - cx, z - cz);
+            const uint32_t nid = in ? uint32_t(x - cx) + uint32_t(g.sy) * uint32_t(g.NY - 2) + uint32_t(g.sz) * uint32_t(z - cz)
+                                    : idF;
+            for (int c = 0; c < 3; ++c) f9[k][c] = in ? lf[size_t(c) * N + nid] : 0.f;
+        });
         float B[5], Bn[5];
         const float uc = clamp01(phi[3]);
 #pragma unroll
@@ -1017,8 +1205,7 @@ __global__ void __launch_bounds__(256) k_adj_boundary(const DeviceState s, int64
             constexpr int i = decltype(I)::value;
             using D = Dir<i>;
             if constexpr (D::cy == -1) {
-                if (!pulled(x + D::cx, z + D::cz)) return;
-                const float2 l = reinterpret_cast<const float2 *>(lam)[pop_index(g, slot_pair(i), x, g.NY - 1, z)];
+                const float2 l = l9[(D::cx + 1) * 3 + D::cz + 1];
                 const float lr = l.x, lb = l.y;
                 const float fe = feq<i>(rho, e), fn = fneq<i>(nF);
                 const float gi = fe + oms * fn;
@@ -1061,17 +1248,8 @@ __global__ void __launch_bounds__(256) k_adj_boundary(const DeviceState s, int64
         if (phi[3] > 0.0f && phi[3] < 1.0f) lphi[3] += luc;  // d clamp01 / d uy
         float lP[6], lu[3] = {0.f, 0.f, 0.f};
         neq_adjoint(S2, S3, nF, phi[2], phi[3], phi[4], lP, lu);
-        lmom[kMomRR * N + idF] += lphi[0];
-        lmom[kMomRB * N + idF] += lphi[1];
-        lmom[kMomUX * N + idF] += lphi[2] + lu[0];
-        lmom[kMomUY * N + idF] += lphi[3] + lu[1];
-        lmom[kMomUZ * N + idF] += lphi[4] + lu[2];
-        lmom[kMomPXX * N + idF] += lP[0];
-        lmom[kMomPXY * N + idF] += lP[1];
-        lmom[kMomPYY * N + idF] += lP[2];
-        lmom[kMomPYZ * N + idF] += lP[3];
-        lmom[kMomPZZ * N + idF] += lP[4];
-        lmom[kMomPXZ * N + idF] += lP[5];
+        add_to(idF, {lphi[0], lphi[1], lphi[2] + lu[0], lphi[3] + lu[1], lphi[4] + lu[2], lP[0], lP[1], lP[2], lP[3],
+                     lP[4], lP[5]});
         // psi(B) at (x, NY-1, z) entered the colour gradient of the step's
         // interior nodes (x, NY-2, z) - c over the cy = +1 directions
         float lpsi = 0.f;
@@ -1079,12 +1257,10 @@ __global__ void __launch_bounds__(256) k_adj_boundary(const DeviceState s, int64
             constexpr int i = decltype(I)::value;
             using D = Dir<i>;
             if constexpr (D::cy == 1) {
-                const int xn = x - D::cx, zn = z - D::cz;
-                if (!pulled(xn, zn)) return;
-                const uint32_t nid = uint32_t(xn) + uint32_t(g.sy) * uint32_t(g.NY - 2) + uint32_t(g.sz) * uint32_t(zn);
-                float dot = D::fy * lf[1 * N + nid];
-                if constexpr (D::cx != 0) dot += D::fx * lf[0 * N + nid];
-                if constexpr (D::cz != 0) dot += D::fz * lf[2 * N + nid];
+                const float(&v)[3] = f9[(D::cx + 1) * 3 + D::cz + 1];
+                float dot = D::fy * v[1];
+                if constexpr (D::cx != 0) dot += D::fx * v[0];
+                if constexpr (D::cz != 0) dot += D::fz * v[2];
                 lpsi += D::w * dot;
             }
         });
@@ -1095,8 +1271,12 @@ __global__ void __launch_bounds__(256) k_adj_boundary(const DeviceState s, int64
         lB[1] -= lpsi * 2.0f * B[0] * i2;
 #pragma unroll
         for (int c = 0; c < 5; ++c) LB_out[c * NP + ic] = lB[c];
+    }
+    if (col && blockIdx.z == 1) {
         // ---------------- inlet (boundary_conditions.cuh:17-85): jet columns only
         if (is_jet_column(ph, x, z)) {
+            float2 l9[9];
+            pulled_lambda(std::integral_constant<int, 1>{}, 0, l9);
             const uint32_t id1 = uint32_t(x) + uint32_t(g.sy) * 1u + uint32_t(g.sz) * uint32_t(z);
             const float u1x = M[kMomUX * N + id1], u1y = M[kMomUY * N + id1], u1z = M[kMomUZ * N + id1];
             const NeqTerms n1 = make_neq(M[kMomPXX * N + id1], M[kMomPXY * N + id1], M[kMomPYY * N + id1],
@@ -1111,8 +1291,7 @@ __global__ void __launch_bounds__(256) k_adj_boundary(const DeviceState s, int64
                 constexpr int i = decltype(I)::value;
                 using D = Dir<i>;
                 if constexpr (D::cy == 1) {
-                    if (!pulled(x + D::cx, z + D::cz)) return;
-                    const float lg = reinterpret_cast<const float2 *>(lam)[pop_index(g, slot_pair(i), x, 0, z)].y;  // red = 0 * g
+                    const float lg = l9[(D::cx + 1) * 3 + D::cz + 1].y;  // red = 0 * g
                     // d feq_i / d uy at u = (0, U, 0): w rho (c_y P - U Q), c.u = U
                     const float P = kInvCs2 + U * (2.0f * kInv2Cs4) + (U * U) * (3.0f * kInv6Cs6) - (U * U) * kInv2Cs4;
                     const float Q = kInvCs2 + U * (2.0f * kInv2Cs4);
@@ -1122,15 +1301,7 @@ __global__ void __launch_bounds__(256) k_adj_boundary(const DeviceState s, int64
             });
             float lP1[6], lu1[3] = {0.f, 0.f, 0.f};
             neq_adjoint(T2, T3, n1, u1x, u1y, u1z, lP1, lu1);
-            lmom[kMomUX * N + id1] += lu1[0];
-            lmom[kMomUY * N + id1] += lu1[1];
-            lmom[kMomUZ * N + id1] += lu1[2];
-            lmom[kMomPXX * N + id1] += lP1[0];
-            lmom[kMomPXY * N + id1] += lP1[1];
-            lmom[kMomPYY * N + id1] += lP1[2];
-            lmom[kMomPYZ * N + id1] += lP1[3];
-            lmom[kMomPZZ * N + id1] += lP1[4];
-            lmom[kMomPXZ * N + id1] += lP1[5];
+            add_to(id1, {0.f, 0.f, lu1[0], lu1[1], lu1[2], lP1[0], lP1[1], lP1[2], lP1[3], lP1[4], lP1[5]});
             // U = U0 (1 + sum_k c_k J0_k) (1 + noise): dU/dc_k = U0 (1 + noise) J0_k
             if (bessel) {
                 const float dU = ph.jet_velocity * inlet_noise_factor(ph, step, x, z);
@@ -1411,35 +1582,50 @@ cudaError_t launch_adj_terminal(const DeviceState &s, const float *M, const floa
     return cudaGetLastError();
 }
 
-cudaError_t launch_adj_collide(const DeviceState &s, const float *M, const float *lam_in, float *lmom, float *lf,
-                               double *acc, const AdjObjective &obj, cudaStream_t st) {
+namespace {
+template <bool kPeriodic>
+cudaError_t adj_relax(const DeviceState &s, const float *M, const uint8_t *flags, uint8_t *near_flags, const float *lam_in,
+                      float *lmom, float *lf, float *lam_out, double *acc, const AdjObjective &obj, cudaStream_t st) {
+    constexpr int kWarps = kAdjThreads / 32;
+    const int plane = (adj_pieces_per_row(s.g) * (s.g.NY - 2) + kWarps - 1) / kWarps;
+    const int list = int(adj_list_blocks(s.g, kAdjRelaxBlocks));
+    k_adj_relax<kPeriodic><<<list + plane * (s.g.NZ - 2), kAdjThreads, 0, st>>>(s, M, flags, near_flags, lam_in, lmom, lf,
+                                                                               lam_out, acc, obj, list, plane);
+    return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_adj_relax(const DeviceState &s, const float *M, const uint8_t *flags, uint8_t *near_flags,
+                             const float *lam_in, float *lmom, float *lf, float *lam_out, double *acc,
+                             const AdjObjective &obj, cudaStream_t st) {
+    return s.g.boundary == kBoundaryPeriodic
+               ? adj_relax<true>(s, M, flags, near_flags, lam_in, lmom, lf, lam_out, acc, obj, st)
+               : adj_relax<false>(s, M, flags, near_flags, lam_in, lmom, lf, lam_out, acc, obj, st);
+}
+
+cudaError_t launch_adj_near(const DeviceState &s, const float *M, const uint8_t *flags, const uint8_t *near_flags,
+                            const float *lmom, const float *lf, float *lam_out, cudaStream_t st) {
+    const unsigned n = adj_list_blocks(s.g, kAdjNearBlocks);
     if (s.g.boundary == kBoundaryPeriodic)
-        k_adj_collide<true><<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s, M, lam_in, lmom, lf, acc, obj);
+        k_adj_near<true><<<n, kAdjThreads, 0, st>>>(s, M, flags, near_flags, lmom, lf, lam_out);
     else
-        k_adj_collide<false><<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s, M, lam_in, lmom, lf, acc, obj);
+        k_adj_near<false><<<n, kAdjThreads, 0, st>>>(s, M, flags, near_flags, lmom, lf, lam_out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_adj_moments(const DeviceState &s, const float *M, const float *lmom, const float *lf,
-                               float *lam_out, cudaStream_t st) {
-    if (s.g.boundary == kBoundaryPeriodic)
-        k_adj_moments<true><<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s, M, lmom, lf, lam_out);
-    else
-        k_adj_moments<false><<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s, M, lmom, lf, lam_out);
+cudaError_t launch_piece_flags(const DeviceState &s, const float *M, uint8_t *flags, cudaStream_t st) {
+    constexpr int kWarps = kRedThreads / 32;
+    const int pieces = adj_pieces_per_row(s.g) * (s.g.NY - 2);
+    k_piece_flags<<<dim3((pieces + kWarps - 1) / kWarps, s.g.NZ - 2), kRedThreads, 0, st>>>(s, M, flags);
     return cudaGetLastError();
-}
-
-cudaError_t launch_adj_step(const DeviceState &s, const float *M, const float *lam_in, float *lmom, float *lf,
-                            float *lam_out, double *acc, cudaStream_t st) {
-    cudaError_t e = launch_adj_collide(s, M, lam_in, lmom, lf, acc, AdjObjective{0.0f, 0, nullptr}, st);
-    if (e != cudaSuccess) return e;
-    return launch_adj_moments(s, M, lmom, lf, lam_out, st);
 }
 
 cudaError_t launch_adj_boundary(const DeviceState &s, int64_t step, const float *M, const float *Bt,
                                 const float *lam_next, const float *lf, float *lmom, const float *LB_in,
                                 float *LB_out, const float *bessel, int nb, double *dJdc, cudaStream_t st) {
-    const dim3 block(32, 8), grid((s.g.NX + 31) / 32, (s.g.NZ + 7) / 8);
+    // one warp per block: a column is a long chain of dependent work, and blocks
+    // of 8 warps put the 62 x 62 columns of a 64-wide jet on 16 SMs
+    const dim3 block(32, 1), grid((s.g.NX + 31) / 32, s.g.NZ, 2);
     k_adj_boundary<<<grid, block, 0, st>>>(s, step, M, Bt, lam_next, lf, lmom, LB_in, LB_out, bessel, nb, dJdc);
     return cudaGetLastError();
 }

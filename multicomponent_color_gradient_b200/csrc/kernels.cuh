@@ -120,7 +120,7 @@ struct DeviceState {
     float *uy_avg;    // [N]
     double *partials; // reduction scratch
     uint32_t partials_cap;
-    uint8_t *piece_flags;  // [NZ-2][NY-2][pieces of 32 columns]: the piece holds an interface node (this step)
+    uint8_t *piece_flags;  // [NZ-2][NY-2][pieces of 32 columns]: interface nodes of this step (piece_flag)
     int *flag;        // device flags: [0] non-finite value, [1] a k_fused_bulk wait ran out
     float *tape;      // null, or [kTapePlanes][N]: the fused step records the moments and psi it pulls there
     const float *inlet_profile;  // null (top-hat), or [NZ][NX] multipliers of the inlet velocity per column
@@ -209,20 +209,23 @@ struct AdjObjective {
 // ---- discrete adjoint of the step (float32 populations) ----
 // lambda buffers share the population layout; M is the moment record
 // [kTapePlanes][N] of the state the pass belongs to (interior nodes).
-// Terminal condition for J = sum (psi_T - target)^2, one adjoint step
-// (lmom [11][N], lf [3][N] scratch; acc[0] += dJ/domega, acc[1] += dJ/d(A/2)),
-// and dJ/du0 of a state f0 = feq(rho_c, u0) (du0 [3][N]).
+// Terminal condition for J = sum (psi_T - target)^2, the adjoint step (lmom
+// [11][N], lf [3][N] scratch; acc[0] += dJ/domega, acc[1] += dJ/d(A/2)), and
+// dJ/du0 of a state f0 = feq(rho_c, u0) (du0 [3][N]).
 cudaError_t launch_adj_terminal(const DeviceState &s, const float *M, const float *target, float *lam, double *J,
                                 cudaStream_t st);
-cudaError_t launch_adj_step(const DeviceState &s, const float *M, const float *lam_in, float *lmom, float *lf,
-                            float *lam_out, double *acc, cudaStream_t st);
-// The same step in two parts for the jet, with the boundary adjoint between
-// them: the relaxation part (lam_in -> lmom, lf, objective source) and the
-// moment part (lmom, lf -> lam_out).
-cudaError_t launch_adj_collide(const DeviceState &s, const float *M, const float *lam_in, float *lmom, float *lf,
-                               double *acc, const AdjObjective &obj, cudaStream_t st);
-cudaError_t launch_adj_moments(const DeviceState &s, const float *M, const float *lmom, const float *lf,
-                               float *lam_out, cudaStream_t st);
+// The step in two parts, between which the jet's boundary adjoint comes: the
+// relaxation part (lam_in -> lmom, lf, objective source; lam_out of the pieces
+// with no interface around, near_flags marking the others) and the moment part
+// of those others (lmom, lf -> lam_out).  flags: the state's pieces that hold an
+// interface node (DeviceState::piece_flags as the step that recorded the state
+// set them, or launch_piece_flags).
+cudaError_t launch_adj_relax(const DeviceState &s, const float *M, const uint8_t *flags, uint8_t *near_flags,
+                             const float *lam_in, float *lmom, float *lf, float *lam_out, double *acc,
+                             const AdjObjective &obj, cudaStream_t st);
+cudaError_t launch_adj_near(const DeviceState &s, const float *M, const uint8_t *flags, const uint8_t *near_flags,
+                            const float *lmom, const float *lf, float *lam_out, cudaStream_t st);
+cudaError_t launch_piece_flags(const DeviceState &s, const float *M, uint8_t *flags, cudaStream_t st);
 // Adjoint of the jet boundary of step `step` (inlet and convective outlet,
 // jet/boundary_conditions.cuh:17-85,163-233) and of the outlet-plane psi the
 // step read.  M: the step's moment record; Bt: [5][NX*NZ] outlet state

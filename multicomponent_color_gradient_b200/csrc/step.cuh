@@ -528,6 +528,19 @@ __host__ __device__ __forceinline__ int store_columns(const Geometry &g) {
     return c < g.px ? c : g.px;
 }
 
+// Pieces of 32 columns that hold the stored columns of a row.
+template <class C>
+__host__ __device__ __forceinline__ int pieces_per_row(const Geometry &g) {
+    return (store_columns<C>(g) + 31) / 32;
+}
+
+// Flag of piece w of a row from the lanes that hold interface nodes: bit 0 any,
+// bit 1 its first interior column, bit 2 its last.
+__device__ __forceinline__ uint8_t piece_flag(const Geometry &g, int w, unsigned lanes) {
+    const int first = w == 0 ? 1 : 0, last = min(31, g.NX - 2 - 32 * w);
+    return uint8_t((lanes != 0 ? 1u : 0u) | (((lanes >> first) & 1u) << 1) | (((lanes >> last) & 1u) << 2));
+}
+
 // A node whose interface indicator (lbm.cuh:214-216) is at most 1e-4 takes the
 // bulk branch, which reads no psi.  A NaN is not bulk.
 __device__ __forceinline__ bool is_bulk(float rr, float rb) {
