@@ -34,6 +34,8 @@
 // handle's state is left untouched.
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -142,7 +144,9 @@ struct DeviceBuffers {
     cudaStream_t stream;  // the run's stream
     int device = 0;
     std::vector<Block> used, spare;
+    size_t total = 0, limit = SIZE_MAX;  // bytes in use, and the most a run may take (tests)
     explicit DeviceBuffers(cudaStream_t st) : stream(st) {
+        if (const char *v = std::getenv("MCG_ADJOINT_MEMORY_MB")) limit = size_t(std::atoll(v)) << 20;
         cudaGetDevice(&device);
         std::lock_guard<std::mutex> lock(g_kept_mutex);
         spare.swap(g_kept[device]);
@@ -150,8 +154,7 @@ struct DeviceBuffers {
     ~DeviceBuffers() {
         if (!used.empty()) cudaStreamSynchronize(stream);
         drop_spare();
-        size_t total = 0, free_b = 0, total_b = 0;
-        for (const Block &b : used) total += b.bytes;
+        size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && total <= total_b / 16) {
             std::lock_guard<std::mutex> lock(g_kept_mutex);
             if (g_kept[device].empty()) {
@@ -172,6 +175,7 @@ struct DeviceBuffers {
     }
     cudaError_t alloc(void **p, size_t bytes, bool zero = false) {
         *p = nullptr;
+        if (total + bytes > limit) return cudaErrorMemoryAllocation;
         size_t best = spare.size();
         for (size_t k = 0; k < spare.size(); ++k)
             if (spare[k].bytes >= bytes && spare[k].bytes <= bytes + bytes / 4 + 4096 &&
@@ -192,6 +196,7 @@ struct DeviceBuffers {
             if (e != cudaSuccess) return e;
             used.push_back({q, bytes});
         }
+        total += used.back().bytes;
         *p = used.back().p;
         return zero ? cudaMemsetAsync(*p, 0, bytes, stream) : cudaSuccess;
     }
@@ -358,6 +363,19 @@ void workspace_release(int device) noexcept {
 }
 }  // namespace mcg
 
+namespace {
+// A run that finds no room for buffers of padded rows runs with unpadded ones.
+template <class F>
+mcg_status with_rows_that_fit(mcg_handle *h, F &&run) {
+    const mcg_status st = run();
+    if (st != MCG_ERR_OOM || !h || h->s.g.px == h->p.NX) return st;
+    cudaGetLastError();
+    mcg::workspace_release(h->device);
+    if (mcg_status u = mcg::unpad_rows(h)) return u;
+    return run();
+}
+}  // namespace
+
 extern "C" {
 
 mcg_status mcg_adjoint_plan_taped(int32_t nsteps, int32_t snapshots, int32_t tape, int64_t *forward_steps,
@@ -400,8 +418,9 @@ mcg_status mcg_set_adjoint_tape(mcg_handle *h, int32_t records) {
     });
 }
 
-mcg_status mcg_adjoint_run(mcg_handle *h, const float *psi_target, int32_t nsteps, int32_t snapshots, double *J,
-                           double *dJ_dsigma, double *dJ_dtau, float *dJ_du0, int64_t *forward_steps, float *ms) {
+static mcg_status bubble_adjoint(mcg_handle *h, const float *psi_target, int32_t nsteps, int32_t snapshots, double *J,
+                                 double *dJ_dsigma, double *dJ_dtau, float *dJ_du0, int64_t *forward_steps,
+                                 float *ms) {
     return mcg::guarded([&]() -> mcg_status {
         if (!h) return fail(MCG_ERR_INVALID_ARG, "handle is null");
         if (!psi_target) return fail(MCG_ERR_INVALID_ARG, "psi_target is null");
@@ -412,7 +431,7 @@ mcg_status mcg_adjoint_run(mcg_handle *h, const float *psi_target, int32_t nstep
         if (h->p.sponge_K != 0.0f) return fail(MCG_ERR_UNSUPPORTED, "the adjoint needs a uniform relaxation rate");
         const mcg::Geometry &g = h->s.g;
         const size_t N = g.N;
-        const size_t pop_bytes = size_t(2 * mcg::kQ) * N * sizeof(float);  // float32 populations or lambda
+        const size_t pop_bytes = size_t(2 * mcg::kQ) * g.px * g.NY * g.NZ * sizeof(float);  // float32 populations or lambda
         const size_t record_floats = record_size(g, 0);
         const bool tape_mode = snapshots > nsteps;
         const int free_slots = tape_mode ? 0 : snapshots - 1;
@@ -507,6 +526,15 @@ mcg_status mcg_adjoint_run(mcg_handle *h, const float *psi_target, int32_t nstep
     });
 }
 
+mcg_status mcg_adjoint_run(mcg_handle *h, const float *psi_target, int32_t nsteps, int32_t snapshots, double *J,
+                           double *dJ_dsigma, double *dJ_dtau, float *dJ_du0, int64_t *forward_steps, float *ms) {
+    return mcg::guarded([&]() -> mcg_status {
+        return with_rows_that_fit(h, [&] {
+            return bubble_adjoint(h, psi_target, nsteps, snapshots, J, dJ_dsigma, dJ_dtau, dJ_du0, forward_steps, ms);
+        });
+    });
+}
+
 
 namespace {
 // J0(alpha_k r / R), k < kInletBesselMax (the inlet profile's basis), of the
@@ -562,8 +590,9 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
     // the forward states keep the handle's storage (float16 or float32); the
     // reverse sweep reads them only through their float32 moment records, and
     // its lambda arrays are float32 pairs
-    const size_t state_bytes = g.storage == MCG_STORAGE_F16 ? size_t(mcg::kQ) * N * 4 : size_t(2 * mcg::kQ) * N * 4;
-    const size_t lam_bytes = size_t(2 * mcg::kQ) * N * sizeof(float);
+    const size_t NP27 = size_t(mcg::kQ) * g.px * g.NY * g.NZ;
+    const size_t state_bytes = NP27 * (g.storage == MCG_STORAGE_F16 ? 4 : 8);
+    const size_t lam_bytes = NP27 * 8;
     const size_t rec_floats = record_size(g, 5 * NP);  // moments, psi with ghosts, outlet state, flags
     const int nb = mcg::kInletBesselMax;
     const bool profile = objective.kind == 1;
@@ -783,7 +812,9 @@ mcg_status mcg_adjoint_jet_run(mcg_handle *h, int32_t nsteps, int32_t t_begin, i
         JetObjective obj;
         obj.kind = 0;
         obj.y_obs = y_obs;
-        return jet_adjoint(h, nsteps, t_begin, t_end, segment, obj, J, dJ_dc, forward_steps, ms);
+        return with_rows_that_fit(h, [&] {
+            return jet_adjoint(h, nsteps, t_begin, t_end, segment, obj, J, dJ_dc, forward_steps, ms);
+        });
     });
 }
 
@@ -801,7 +832,9 @@ mcg_status mcg_adjoint_jet_profile_run(mcg_handle *h, int32_t nsteps, int32_t t_
         obj.y_hi = y_hi;
         obj.uc_target = uc_target;
         obj.rh_target = rhalf_target;
-        return jet_adjoint(h, nsteps, t_begin, t_end, segment, obj, J, dJ_dc, forward_steps, ms);
+        return with_rows_that_fit(h, [&] {
+            return jet_adjoint(h, nsteps, t_begin, t_end, segment, obj, J, dJ_dc, forward_steps, ms);
+        });
     });
 }
 

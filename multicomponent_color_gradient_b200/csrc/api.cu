@@ -5,6 +5,7 @@
 // queues work on one stream, returns status codes instead of exiting.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -175,14 +176,44 @@ void compute_ncols(mcg_handle *h) {
         }
 }
 
-size_t pop_buffer_bytes(const mcg_params &p) {
-    const size_t N = size_t(p.NX) * p.NY * p.NZ;
-    return p.storage == MCG_STORAGE_F16 ? size_t(mcg::kQ) * N * 4 : size_t(2 * mcg::kQ) * N * 4;
+size_t pop_buffer_bytes(const mcg_params &p, int px) {
+    return size_t(mcg::kQ) * px * p.NY * p.NZ * (p.storage == MCG_STORAGE_F16 ? 4 : 8);
+}
+size_t pop_buffer_bytes(const mcg_handle *h) { return pop_buffer_bytes(h->p, h->s.g.px); }
+
+// Row pitch of the population buffers: rows that are not whole pieces of 32
+// columns are padded to them, so that the step's kernels are compiled for the
+// pitch and rows start on 128 bytes (us a step: 97x75x131 float32 103 -> 78,
+// float16 73 -> 61, 24x40x24 10.5 -> 9.7).  Not where float32 rows are whole
+// sectors of 64 bytes already (200x301x183: 761 without, 782 with), nor where it
+// would cost more than a third more memory, nor beyond 1/128 of the device's
+// memory for all handles together.
+std::mutex g_pad_mutex;
+std::map<int, size_t> g_pad;  // bytes of padding in use, by device
+int row_pitch(const mcg_params &p, int device, size_t *padding) {
+    *padding = 0;
+    const int px = (p.NX + 31) / 32 * 32;
+    if (px == p.NX || 3 * px > 4 * p.NX || std::getenv("MCG_FUSED_FIXED_NX")) return p.NX;
+    if (p.storage == MCG_STORAGE_F32 && p.NX % 8 == 0 && p.NX >= 64) return p.NX;
+    const size_t extra = 2 * (pop_buffer_bytes(p, px) - pop_buffer_bytes(p, p.NX));
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return p.NX;
+    std::lock_guard<std::mutex> lock(g_pad_mutex);
+    if (g_pad[device] + extra > total_b / 128) return p.NX;
+    g_pad[device] += extra;
+    *padding = extra;
+    return px;
+}
+void give_back_padding(mcg_handle *h) {
+    std::lock_guard<std::mutex> lock(g_pad_mutex);
+    g_pad[h->device] -= h->padding;
+    h->padding = 0;
 }
 
 size_t piece_flag_bytes(const mcg_params &p) { return size_t(p.NY) * p.NZ * ((p.NX + 31) / 32); }
 
 void release(mcg_handle *h) {
+    give_back_padding(h);
     mcg::async_release(h);
     mcg::io_close(h);
     void *ptrs[] = {h->s.pops[0], h->s.pops[1], h->s.mom,      h->s.psi[0], h->s.psi[1], h->s.radial,
@@ -286,6 +317,23 @@ mcg_status ensure_moments(mcg_handle *h) {
 
 }  // namespace
 
+namespace mcg {
+// Takes the padding out of the rows of both population buffers (their memory
+// stays), for a call that finds no room for buffers of padded rows.
+mcg_status unpad_rows(mcg_handle *h) {
+    if (mcg_status s = ensure_moments(h)) return s;  // the spare buffer holds the last step's input
+    MCG_LAUNCH(h, launch_unpad_rows(h->s, h->cur, h->stream), "unpad rows");
+    h->s.g.px = h->p.NX;
+    MCG_CUDA(cudaMemcpyAsync(h->s.pops[h->cur], h->s.pops[h->cur ^ 1], pop_buffer_bytes(h), cudaMemcpyDeviceToDevice,
+                             h->stream),
+             "unpad rows");
+    MCG_CUDA(cudaStreamSynchronize(h->stream), "unpad rows");
+    h->tiling = fused_tiling(h->s.g, kFusedSmemPerBlock);
+    MCG_CUDA(fused_configure(h->s.g, h->tiling), "unpad rows");
+    return MCG_OK;
+}
+}  // namespace mcg
+
 extern "C" {
 
 int32_t mcg_abi_version(void) { return MCG_ABI_VERSION; }
@@ -384,13 +432,13 @@ mcg_status mcg_create(const mcg_params *p, mcg_handle **out) {
         g.boundary = p->boundary;
         g.storage = p->storage;
         g.slots = mcg::kQ;  // one element (both colours) per direction: float2 or half2
-        g.px = p->NX;
+        g.px = row_pitch(*p, h->device, &h->padding);
         fill_physics(h);
         compute_ncols(h);
         const size_t N = g.N;
         const size_t M = size_t(p->NY) * (p->NX / 2);
         cudaError_t e = cudaSuccess;
-        const size_t pb = pop_buffer_bytes(*p);
+        const size_t pb = pop_buffer_bytes(h);
         if (e == cudaSuccess) e = alloc_zero(&h->s.pops[0], pb);
         if (e == cudaSuccess) e = alloc_zero(&h->s.pops[1], pb);
         if (e == cudaSuccess) e = alloc_zero(&h->s.mom, size_t(mcg::kMomCount) * N * 4);
@@ -480,7 +528,7 @@ mcg_status mcg_device_bytes(const mcg_handle *h, uint64_t *out) {
         if (mcg_status s = check_handle(h)) return s;
         MCG_REQUIRE(out != nullptr, "out is null");
         const size_t N = h->s.g.N, M = size_t(h->p.NY) * (h->p.NX / 2);
-        *out = 2 * pop_buffer_bytes(h->p) + size_t(mcg::kMomCount) * N * 4 + 2 * N * 4 + 5 * M * 8 + N * 4 +
+        *out = 2 * pop_buffer_bytes(h->p, h->p.NX) + h->padding + size_t(mcg::kMomCount) * N * 4 + 2 * N * 4 + 5 * M * 8 + N * 4 +
                size_t(h->s.partials_cap) * 40 + 16 + 64 + piece_flag_bytes(h->p);
         return MCG_OK;
     });
@@ -648,7 +696,7 @@ XferPlan xfer_plan(const mcg_handle *h) {
     x.nchunks = (g.NZ + x.zc - 1) / x.zc;
     x.pitch = size_t(x.zc) * size_t(g.sz);
     x.slot_floats = 2 * size_t(mcg::kQ) * x.pitch;
-    const size_t cap = pop_buffer_bytes(h->p) / 4;
+    const size_t cap = pop_buffer_bytes(h) / 4;
     x.slots = int(std::min<size_t>(size_t(x.nchunks), cap / x.slot_floats));
     return x;
 }
@@ -683,7 +731,7 @@ mcg_status mcg_set_populations(mcg_handle *h, const float *fr, const float *fb) 
             MCG_CUDA(cudaEventRecord(h->xfer_kern[k], h->stream), "event record");
         }
         // both buffers carry the same ghost-plane slots (the ones no step rewrites)
-        MCG_CUDA(cudaMemcpyAsync(h->s.pops[1], h->s.pops[0], pop_buffer_bytes(h->p), cudaMemcpyDeviceToDevice, h->stream),
+        MCG_CUDA(cudaMemcpyAsync(h->s.pops[1], h->s.pops[0], pop_buffer_bytes(h), cudaMemcpyDeviceToDevice, h->stream),
                  "copy populations");
         h->cur = 0;
         MCG_CUDA(cudaStreamSynchronize(h->stream), "set populations");
@@ -722,7 +770,7 @@ mcg_status mcg_get_populations(mcg_handle *h, float *fr, float *fb) {
         }
         // the spare buffer again holds the ghost-plane slots of the current one
         MCG_CUDA(cudaStreamWaitEvent(h->stream, h->xfer_copy[x.nchunks - 1], 0), "stream wait");
-        MCG_CUDA(cudaMemcpyAsync(h->s.pops[rd ^ 1], h->s.pops[rd], pop_buffer_bytes(h->p), cudaMemcpyDeviceToDevice,
+        MCG_CUDA(cudaMemcpyAsync(h->s.pops[rd ^ 1], h->s.pops[rd], pop_buffer_bytes(h), cudaMemcpyDeviceToDevice,
                                  h->stream),
                  "restore spare buffer");
         MCG_CUDA(cudaStreamSynchronize(h->stream), "get populations");

@@ -528,11 +528,12 @@ __global__ void __launch_bounds__(kFusedThreads, PipeBlocks<C>::value) k_fused_p
 // (0.52).  With every node an interface node it is even: 128x256x128 float32
 // 360 against 352, float16 324 against 365.
 
-// Threads and CTAs per SM the register budgets are sized for: k_step_pull 80
-// registers, k_step_interface 96 (at 80 a periodic float16 run of 128^2 x 256
-// was 12 % slower, at 2 CTAs of 256 threads a float16 jet 13 %).  No variant
-// may spill: a few spilled bytes made such a kernel 40 % slower.
-constexpr int kSplitThreads = 256, kSplitBlocks = 3;
+// Threads and CTAs per SM the register budgets are sized for: k_step_pull 72
+// registers (64, with spills in float32, to 96 measured within 1 % in float32;
+// the float16 jet 128x256x128 takes 171 us a step at 72, 175 at 64 and 189 at
+// 80), k_step_interface 96 (at 80 a periodic float16 run of 128^2 x 256 was 12 %
+// slower, at 2 CTAs of 256 threads a float16 jet 13 %).
+constexpr int kSplitThreads = 128, kSplitBlocks = 7;
 constexpr int kInterfaceThreads = 128, kInterfaceBlocks = 5;
 // Neighbouring pieces that one CTA of k_step_interface takes together: whole
 // rows of 128 columns (4 against 1: 174 against 196 us a step for the

@@ -34,6 +34,7 @@ struct mcg_handle {
     int64_t step = 0;       // completed collisions
     uint64_t launches = 0;  // kernels launched through this handle
     mcg::FusedTiling tiling{};
+    size_t padding = 0;      // bytes of the population buffers that pad their rows
     bool mom_stale = false;  // moment planes lag the last fused step
 
     // radial statistics (meanF/memoryMeanFields.cuh:39-45)
@@ -99,6 +100,7 @@ StatsSnapshot stats_snapshot(const mcg_handle *h);
 // float64 device sum of this output step
 void tke_update(mcg_handle *h, int32_t step, double total);
 
+mcg_status unpad_rows(mcg_handle *h);  // api.cu
 // adjoint.cu: frees the device memory kept between adjoint runs on `device`.
 void workspace_release(int device) noexcept;
 // cudaMalloc that first gives that memory back where it is in the way.

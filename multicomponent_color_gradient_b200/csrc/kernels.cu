@@ -282,6 +282,13 @@ __global__ void k_gather_chunk(const DeviceState s, int cur, float *__restrict__
     }
 }
 
+template <class E>
+__global__ void k_unpad_rows(const E *__restrict__ src, E *__restrict__ dst, int NX, int px, size_t rows) {
+    const size_t warps = size_t(gridDim.x) * (blockDim.x / 32);
+    for (size_t r = size_t(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32; r < rows; r += warps)
+        for (int x = int(threadIdx.x & 31); x < NX; x += 32) dst[r * size_t(NX) + x] = src[r * size_t(px) + x];
+}
+
 // ------------------------------------------------------------------ reductions
 
 template <int NT>
@@ -1460,6 +1467,19 @@ cudaError_t launch_gather_chunk(const DeviceState &s, int cur, float *stage, siz
         k_gather_chunk<CodecF16><<<grid, dim3(kBX, kBY), 0, st>>>(s, cur, stage, pitch, z0);
     else
         k_gather_chunk<CodecF32><<<grid, dim3(kBX, kBY), 0, st>>>(s, cur, stage, pitch, z0);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_unpad_rows(const DeviceState &s, int cur, cudaStream_t st) {
+    const size_t rows = size_t(s.g.NY) * s.g.NZ * kQ;
+    const void *src = s.pops[cur];
+    void *dst = s.pops[cur ^ 1];
+    if (s.g.storage == kStoreF16)
+        k_unpad_rows<<<8 * 148, 256, 0, st>>>(static_cast<const __half2 *>(src), static_cast<__half2 *>(dst), s.g.NX,
+                                              s.g.px, rows);
+    else
+        k_unpad_rows<<<8 * 148, 256, 0, st>>>(static_cast<const float2 *>(src), static_cast<float2 *>(dst), s.g.NX, s.g.px,
+                                              rows);
     return cudaGetLastError();
 }
 

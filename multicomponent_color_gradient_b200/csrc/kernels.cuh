@@ -94,6 +94,7 @@ struct FusedTiling {
     int alternate; // odd z-chunks march down, so neighbouring chunks pull their shared planes together
     int march;     // how a step runs (StepMarch)
     int interface_ctas, boundary_ctas;  // CTAs of k_step_interface that relax pieces, and after them the jet columns
+    int pitch;     // row pitch the kernels are compiled for (0: runtime)
     int fixed_nx;  // row length the kernel is compiled for (0: runtime geometry)
     int wait_limit;  // k_fused_bulk: tries (about 1 us each) of a wait for a staged row before it gives up
     int boundary;    // jet: the fused step writes the inlet and outlet columns itself (no k_boundary launch)
@@ -160,6 +161,9 @@ cudaError_t launch_scatter_chunk(const DeviceState &s, int wbuf, const float *st
                                  cudaStream_t st);
 cudaError_t launch_gather_chunk(const DeviceState &s, int cur, float *stage, size_t pitch, int z0, int nz,
                                 cudaStream_t st);
+
+// pops[cur], rows of pitch g.px, to pops[cur ^ 1] with rows of NX elements.
+cudaError_t launch_unpad_rows(const DeviceState &s, int cur, cudaStream_t st);
 
 // Diagnostics / mean fields.
 cudaError_t launch_tke(const DeviceState &s, double *out, cudaStream_t st);

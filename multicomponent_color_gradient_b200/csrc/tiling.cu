@@ -69,6 +69,10 @@ FusedTiling fused_tiling(const Geometry &g, int max_smem) {
         split_tiling(g, t);
     else
         march_tiling(g, max_smem, t);
+    // the row pitch the kernels are compiled for (the marches: whole rows)
+    t.pitch = t.march == kMarchSplit ? (g.px % 32 == 0 ? g.px : 0) : t.fixed_nx;
+    if (const char *v = std::getenv("MCG_FUSED_FIXED_NX"))  // tests
+        if (std::atoi(v) == 0) t.pitch = 0;
     // the jet's inlet and outlet columns within the step's launches, instead of
     // a k_boundary launch after them
     t.boundary = g.boundary == kBoundaryJet;
@@ -77,20 +81,21 @@ FusedTiling fused_tiling(const Geometry &g, int max_smem) {
 }
 
 // One object per row pitch instantiates these (fused.cu).
-extern template cudaError_t fused_configure_pitch<0>(const Geometry &, const FusedTiling &);
-extern template cudaError_t fused_configure_pitch<kFusedNX>(const Geometry &, const FusedTiling &);
-extern template cudaError_t fused_configure_pitch<kFusedNX2>(const Geometry &, const FusedTiling &);
-extern template cudaError_t fused_launch_pitch<0>(const DeviceState &, const FusedTiling &, int, int64_t, bool,
-                                                  cudaStream_t);
-extern template cudaError_t fused_launch_pitch<kFusedNX>(const DeviceState &, const FusedTiling &, int, int64_t, bool,
-                                                         cudaStream_t);
-extern template cudaError_t fused_launch_pitch<kFusedNX2>(const DeviceState &, const FusedTiling &, int, int64_t,
-                                                          bool, cudaStream_t);
+#define MCG_EACH_PITCH(F) F(0) F(32) F(64) F(96) F(128) F(160) F(192) F(224) F(256)
+#define MCG_EXTERN(P)                                                                          \
+    extern template cudaError_t fused_configure_pitch<P>(const Geometry &, const FusedTiling &); \
+    extern template cudaError_t fused_launch_pitch<P>(const DeviceState &, const FusedTiling &, int, int64_t, bool, \
+                                                      cudaStream_t);
+MCG_EACH_PITCH(MCG_EXTERN)
 
 cudaError_t fused_configure(const Geometry &g, const FusedTiling &t) {
-    if (t.fixed_nx == kFusedNX) return fused_configure_pitch<kFusedNX>(g, t);
-    if (t.fixed_nx == kFusedNX2) return fused_configure_pitch<kFusedNX2>(g, t);
-    return fused_configure_pitch<0>(g, t);
+    switch (t.pitch) {
+#define MCG_CASE(P) \
+    case P: return fused_configure_pitch<P>(g, t);
+        MCG_EACH_PITCH(MCG_CASE)
+#undef MCG_CASE
+    }
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_fused(const DeviceState &s, const FusedTiling &t_in, int cur, int64_t step, bool stats,
@@ -101,9 +106,13 @@ cudaError_t launch_fused(const DeviceState &s, const FusedTiling &t_in, int cur,
         t.bnd_psi = s.psi[(step + 1) & 1];
         t.bnd_step = step;
     }
-    if (t.fixed_nx == kFusedNX) return fused_launch_pitch<kFusedNX>(s, t, cur, step, stats, st);
-    if (t.fixed_nx == kFusedNX2) return fused_launch_pitch<kFusedNX2>(s, t, cur, step, stats, st);
-    return fused_launch_pitch<0>(s, t, cur, step, stats, st);
+    switch (t.pitch) {
+#define MCG_CASE(P) \
+    case P: return fused_launch_pitch<P>(s, t, cur, step, stats, st);
+        MCG_EACH_PITCH(MCG_CASE)
+#undef MCG_CASE
+    }
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace mcg
