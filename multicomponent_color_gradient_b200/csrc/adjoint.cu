@@ -154,8 +154,7 @@ struct DeviceBuffers {
     ~DeviceBuffers() {
         if (!used.empty()) cudaStreamSynchronize(stream);
         drop_spare();
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && total <= total_b / 16) {
+        if (total <= mcg::device_bytes(device) / 16) {
             std::lock_guard<std::mutex> lock(g_kept_mutex);
             if (g_kept[device].empty()) {
                 g_kept[device].swap(used);

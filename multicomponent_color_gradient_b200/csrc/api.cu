@@ -52,6 +52,16 @@ cudaError_t device_malloc(void **p, size_t bytes) {
     return cudaMalloc(p, bytes);
 }
 
+size_t device_bytes(int device) {
+    static std::mutex m;
+    static std::map<int, size_t> known;
+    std::lock_guard<std::mutex> lock(m);
+    size_t &b = known[device];
+    size_t free_b = 0;
+    if (b == 0 && cudaMemGetInfo(&free_b, &b) != cudaSuccess) b = 0;
+    return b;
+}
+
 namespace {
 std::mutex g_live_mutex;
 std::map<int, int> g_live;  // handles by device
@@ -196,10 +206,9 @@ int row_pitch(const mcg_params &p, int device, size_t *padding) {
     if (px == p.NX || 3 * px > 4 * p.NX || std::getenv("MCG_FUSED_FIXED_NX")) return p.NX;
     if (p.storage == MCG_STORAGE_F32 && p.NX % 8 == 0 && p.NX >= 64) return p.NX;
     const size_t extra = 2 * (pop_buffer_bytes(p, px) - pop_buffer_bytes(p, p.NX));
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return p.NX;
+    const size_t most = mcg::device_bytes(device) / 128;
     std::lock_guard<std::mutex> lock(g_pad_mutex);
-    if (g_pad[device] + extra > total_b / 128) return p.NX;
+    if (g_pad[device] + extra > most) return p.NX;
     g_pad[device] += extra;
     *padding = extra;
     return px;

@@ -571,21 +571,6 @@ __device__ __forceinline__ void unpark_moments(const __half2 *wrow, int px, Node
     m = NodeMoments{v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], v[9], v[10]};
 }
 
-// Both launches start while the one before them drains (programmatic
-// dependent launch): everything before this reads only kernel parameters.
-// The pointers are renewed behind the wait, so that no load of theirs can be
-// moved above it.
-template <class C>
-__device__ __forceinline__ void wait_for_previous_launch(C &codec, const float *&psi) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    auto rd = codec.rd;
-    auto wr = codec.wr;
-    asm volatile("" : "+l"(rd), "+l"(wr), "+l"(psi)::"memory");
-    codec.rd = rd;
-    codec.wr = wr;
-}
-__device__ __forceinline__ void allow_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 template <class C, bool kStats, bool kPeriodic, int kPX>
 __global__ void __launch_bounds__(kSplitThreads, kSplitBlocks) k_step_pull(const DeviceState s_arg, int cur, int64_t step) {
     const DeviceState s = pitch_state<C, kPX>(s_arg);
@@ -713,6 +698,75 @@ __global__ void __launch_bounds__(kInterfaceThreads, kInterfaceBlocks) k_step_in
                 outlet_column<C>(s, T.bnd_dst, T.bnd_psi, x, z, m);
         }
     }
+}
+
+// ------------------------------------------------------------------ granular sequence
+
+// launch_Macros and launch_collistream as the reference drives them, by the
+// pieces of the split step: moments and psi of every interior node to HBM
+// (216 or 108 B read, 48 written a node), and the relaxation from there (48 B
+// read, 216 or 108 written, whole sectors).  A step of the five launchers of the
+// 64x128x64 jet takes 56 us (86 with kernels of runtime pitch that stored the
+// rows in part, each launch after the end of the one before).
+template <class C, bool kPeriodic, int kPX>
+__global__ void __launch_bounds__(kSplitThreads, kSplitBlocks) k_moments(const DeviceState s_arg, int cur, int64_t step) {
+    const DeviceState s = pitch_state<C, kPX>(s_arg);
+    const Geometry &g = s.g;
+    C codec = pitch_codec<C, kPX>(s_arg, cur);
+    const int ppr = pieces_per_row<C>(g);
+    const int piece = int(blockIdx.x) * (kSplitThreads / 32) + int(threadIdx.x >> 5);
+    const int row = piece / ppr, y = 1 + row;
+    const int zi = (step & 1) ? g.NZ - 3 - int(blockIdx.y) : int(blockIdx.y), z = 1 + zi;
+    const int x = (piece - row * ppr) * 32 + int(threadIdx.x & 31);
+    const float *psi_at = s_arg.psi[step & 1];
+    allow_next_launch();
+    wait_for_previous_launch(codec, psi_at);
+    if (y > g.NY - 2 || x < 1 || x > g.NX - 2) return;
+    const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
+    const NodeMoments m = pull_moments<C, kPeriodic>(g, codec, x, y, z);
+    const float v[kMomCount] = {m.rr, m.rb, m.ux, m.uy, m.uz, m.pxx, m.pxy, m.pyy, m.pyz, m.pzz, m.pxz};
+#pragma unroll
+    for (int k = 0; k < kMomCount; ++k) s.mom[size_t(k) * g.N + id] = v[k];
+    const float ps = psi_of(m.rr, m.rb);
+    float *psi = const_cast<float *>(psi_at);
+    psi[id] = ps;
+    if constexpr (kPeriodic) {
+        // ghost mirrors so the unwrapped gradient stencil sees a periodic field
+        const int xs[2] = {x, x == 1 ? g.NX - 1 : (x == g.NX - 2 ? 0 : -1)};
+        const int ys[2] = {y, y == 1 ? g.NY - 1 : (y == g.NY - 2 ? 0 : -1)};
+        const int zs[2] = {z, z == 1 ? g.NZ - 1 : (z == g.NZ - 2 ? 0 : -1)};
+#pragma unroll
+        for (int k = 1; k < 8; ++k) {
+            const int xx = xs[k & 1], yy = ys[(k >> 1) & 1], zz = zs[(k >> 2) & 1];
+            if (xx >= 0 && yy >= 0 && zz >= 0)
+                psi[uint32_t(xx) + uint32_t(g.sy) * uint32_t(yy) + uint32_t(g.sz) * uint32_t(zz)] = ps;
+        }
+    }
+}
+
+template <class C, int kPX>
+__global__ void __launch_bounds__(kInterfaceThreads, kInterfaceBlocks) k_collide(const DeviceState s_arg, int cur,
+                                                                                int64_t step) {
+    const DeviceState s = pitch_state<C, kPX>(s_arg);
+    const Geometry &g = s.g;
+    C codec = pitch_codec<C, kPX>(s_arg, cur);
+    const int ppr = pieces_per_row<C>(g);
+    const int piece = int(blockIdx.x) * (kInterfaceThreads / 32) + int(threadIdx.x >> 5);
+    const int row = piece / ppr, y = 1 + row;
+    const int zi = (step & 1) ? int(blockIdx.y) : g.NZ - 3 - int(blockIdx.y), z = 1 + zi;  // against k_moments
+    const int x = (piece - row * ppr) * 32 + int(threadIdx.x & 31);
+    const float *psi = s_arg.psi[step & 1];
+    allow_next_launch();
+    wait_for_previous_launch(codec, psi);
+    if (y > g.NY - 2 || x >= store_columns<C>(g)) return;
+    const int xn = min(max(x, 1), g.NX - 2);
+    const uint32_t id = uint32_t(xn) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
+    float v[kMomCount];
+#pragma unroll
+    for (int k = 0; k < kMomCount; ++k) v[k] = s.mom[size_t(k) * g.N + id];
+    const NodeMoments m{v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], v[9], v[10]};
+    auto psi_at = [&](int cx, int cy, int cz) { return psi[int(id) + cx + g.sy * cy + g.sz * cz]; };
+    collide_node<false>(g, s.ph, codec, pop_row(g, y, z), x, y, z, m, psi_at);
 }
 
 // ------------------------------------------------------------------ bulk-staged pipelined fused step
@@ -1054,20 +1108,11 @@ cudaError_t fused_launch_one(const DeviceState &s, const FusedTiling &t, int cur
             return cudaGetLastError();
         }
     }
-    cudaLaunchAttribute overlap{};
-    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    overlap.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.blockDim = block;
-    cfg.stream = st;
-    cfg.attrs = &overlap;
-    cfg.numAttrs = 1;
-    cfg.gridDim = grid;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_step_pull<C, kStats, kPeriodic, kPX>, s, cur, step);
+    const cudaError_t e = launch_overlapped(k_step_pull<C, kStats, kPeriodic, kPX>, grid, block, st, s, cur, step);
     if (e != cudaSuccess) return e;
-    cfg.gridDim = dim3(t.interface_ctas + (t.boundary ? t.boundary_ctas : 0));
-    cfg.blockDim = dim3(kInterfaceThreads);
-    return cudaLaunchKernelEx(&cfg, k_step_interface<C, kPeriodic, kPX>, s, t, cur, step);
+    return launch_overlapped(k_step_interface<C, kPeriodic, kPX>,
+                             dim3(t.interface_ctas + (t.boundary ? t.boundary_ctas : 0)), dim3(kInterfaceThreads), st, s,
+                             t, cur, step);
 }
 
 template <int kPX>
@@ -1100,6 +1145,30 @@ cudaError_t fused_launch_pitch(const DeviceState &s, const FusedTiling &t, int c
     if (s.g.storage == kStoreF16)
         return per ? go(CodecF16{}, std::true_type{}) : go(CodecF16{}, std::false_type{});
     return per ? go(CodecF32{}, std::true_type{}) : go(CodecF32{}, std::false_type{});
+}
+
+template <int kPX>
+cudaError_t moments_launch_pitch(const DeviceState &s, int cur, int64_t step, cudaStream_t st) {
+    constexpr int kWarps = kSplitThreads / 32;
+    auto go = [&](auto codec) {
+        using C = decltype(codec);
+        const dim3 grid((pieces_per_row<C>(s.g) * (s.g.NY - 2) + kWarps - 1) / kWarps, s.g.NZ - 2);
+        return s.g.boundary == kBoundaryPeriodic
+                   ? launch_overlapped(k_moments<C, true, kPX>, grid, dim3(kSplitThreads), st, s, cur, step)
+                   : launch_overlapped(k_moments<C, false, kPX>, grid, dim3(kSplitThreads), st, s, cur, step);
+    };
+    return s.g.storage == kStoreF16 ? go(CodecF16{}) : go(CodecF32{});
+}
+
+template <int kPX>
+cudaError_t collide_launch_pitch(const DeviceState &s, int cur, int64_t step, cudaStream_t st) {
+    constexpr int kWarps = kInterfaceThreads / 32;
+    auto go = [&](auto codec) {
+        using C = decltype(codec);
+        const dim3 grid((pieces_per_row<C>(s.g) * (s.g.NY - 2) + kWarps - 1) / kWarps, s.g.NZ - 2);
+        return launch_overlapped(k_collide<C, kPX>, grid, dim3(kInterfaceThreads), st, s, cur, step);
+    };
+    return s.g.storage == kStoreF16 ? go(CodecF16{}) : go(CodecF32{});
 }
 
 }  // namespace mcg

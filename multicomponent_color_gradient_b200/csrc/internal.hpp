@@ -103,6 +103,8 @@ void tke_update(mcg_handle *h, int32_t step, double total);
 mcg_status unpad_rows(mcg_handle *h);  // api.cu
 // adjoint.cu: frees the device memory kept between adjoint runs on `device`.
 void workspace_release(int device) noexcept;
+// Memory of the current device, `device` (0 if unknown).
+size_t device_bytes(int device);
 // cudaMalloc that first gives that memory back where it is in the way.
 cudaError_t device_malloc(void **p, size_t bytes);
 

@@ -12,75 +12,6 @@ namespace {
 
 constexpr int kBX = 32, kBY = 8;
 
-// launch_Macros equivalent: moments and psi of every interior node to HBM.
-template <class C, bool kPeriodic>
-__global__ void __launch_bounds__(kBX * kBY) k_moments(const DeviceState s, const C codec, int64_t step) {
-    const Geometry &g = s.g;
-    const int x = blockIdx.x * kBX + threadIdx.x;
-    const int y = blockIdx.y * kBY + threadIdx.y;
-    const int z = blockIdx.z;
-    if (!(x >= 1 && x <= g.NX - 2 && y >= 1 && y <= g.NY - 2 && z >= 1 && z <= g.NZ - 2)) return;
-    const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
-    const NodeMoments m = pull_moments<C, kPeriodic>(g, codec, x, y, z);
-    const size_t N = g.N;
-    float *mom = s.mom;
-    mom[kMomRR * N + id] = m.rr;
-    mom[kMomRB * N + id] = m.rb;
-    mom[kMomUX * N + id] = m.ux;
-    mom[kMomUY * N + id] = m.uy;
-    mom[kMomUZ * N + id] = m.uz;
-    mom[kMomPXX * N + id] = m.pxx;
-    mom[kMomPXY * N + id] = m.pxy;
-    mom[kMomPYY * N + id] = m.pyy;
-    mom[kMomPYZ * N + id] = m.pyz;
-    mom[kMomPZZ * N + id] = m.pzz;
-    mom[kMomPXZ * N + id] = m.pxz;
-    const float ps = psi_of(m.rr, m.rb);
-    float *psi = s.psi[step & 1];
-    psi[id] = ps;
-    if constexpr (kPeriodic) {
-        // ghost mirrors so the unwrapped gradient stencil sees a periodic field
-        const int xs[2] = {x, x == 1 ? g.NX - 1 : (x == g.NX - 2 ? 0 : -1)};
-        const int ys[2] = {y, y == 1 ? g.NY - 1 : (y == g.NY - 2 ? 0 : -1)};
-        const int zs[2] = {z, z == 1 ? g.NZ - 1 : (z == g.NZ - 2 ? 0 : -1)};
-#pragma unroll
-        for (int k = 1; k < 8; ++k) {
-            const int xx = xs[k & 1], yy = ys[(k >> 1) & 1], zz = zs[(k >> 2) & 1];
-            if (xx >= 0 && yy >= 0 && zz >= 0)
-                psi[uint32_t(xx) + uint32_t(g.sy) * uint32_t(yy) + uint32_t(g.sz) * uint32_t(zz)] = ps;
-        }
-    }
-}
-
-// launch_collistream equivalent: relax from the moment planes and psi in HBM.
-template <class C>
-__global__ void __launch_bounds__(kBX * kBY, 4) k_collide(const DeviceState s, const C codec, int64_t step) {
-    const Geometry &g = s.g;
-    const int x = blockIdx.x * kBX + threadIdx.x;
-    const int y = blockIdx.y * kBY + threadIdx.y;
-    const int z = blockIdx.z;
-    if (!(x >= 1 && x <= g.NX - 2 && y >= 1 && y <= g.NY - 2 && z >= 1 && z <= g.NZ - 2)) return;
-    const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
-    const size_t N = g.N;
-    const float *__restrict__ mom = s.mom;
-    NodeMoments m;
-    m.rr = __ldg(mom + kMomRR * N + id);
-    m.rb = __ldg(mom + kMomRB * N + id);
-    m.ux = __ldg(mom + kMomUX * N + id);
-    m.uy = __ldg(mom + kMomUY * N + id);
-    m.uz = __ldg(mom + kMomUZ * N + id);
-    m.pxx = __ldg(mom + kMomPXX * N + id);
-    m.pxy = __ldg(mom + kMomPXY * N + id);
-    m.pyy = __ldg(mom + kMomPYY * N + id);
-    m.pyz = __ldg(mom + kMomPYZ * N + id);
-    m.pzz = __ldg(mom + kMomPZZ * N + id);
-    m.pxz = __ldg(mom + kMomPXZ * N + id);
-    const float *__restrict__ psi = s.psi[step & 1];
-    auto psi_at = [&](int cx, int cy, int cz) { return __ldg(psi + (int(id) + cx + g.sy * cy + g.sz * cz)); };
-    collide_node<false>(g, s.ph, codec, pop_row(g, y, z), x, y, z, m, psi_at);
-}
-
-
 // Jet boundary of step `step`: blockIdx.z == 0 is the inlet (y=0 plane), 1 the
 // outlet (y=NY-1 plane), unless `which` selects one.  Values go to the ghost
 // planes of buffer `wbuf` (the one the collision of this step writes) and to
@@ -91,6 +22,8 @@ __global__ void __launch_bounds__(256) k_boundary(const DeviceState s, int wbuf,
     const Geometry &g = s.g;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int z = blockIdx.y * blockDim.y + threadIdx.y;
+    allow_next_launch();
+    wait_for_previous_launch();
     if (x < 1 || x > g.NX - 2 || z < 1 || z > g.NZ - 2) return;
     const int side = which >= 0 ? which : int(blockIdx.z);
     float *psi_next = s.psi[(step + 1) & 1];
@@ -110,6 +43,8 @@ __global__ void __launch_bounds__(kBX * kBY) k_accumulate_radial(const DeviceSta
     const int x = blockIdx.x * kBX + threadIdx.x;
     const int y = blockIdx.y * kBY + threadIdx.y;
     const int z = blockIdx.z;
+    allow_next_launch();
+    wait_for_previous_launch();
     const bool active = x >= 1 && x <= g.NX - 2 && y >= 1 && y <= g.NY - 2 && z >= 1 && z <= g.NZ - 2;
     float ux = 0, uy = 0, uz = 0;
     if (active) {
@@ -430,22 +365,11 @@ unsigned grid1(const Geometry &g) {
 
 
 template <class C>
-cudaError_t moments_dispatch(const DeviceState &s, int cur, int64_t step, cudaStream_t st) {
-    const C codec = make_codec<C>(s, cur);
-    if (s.g.boundary == kBoundaryPeriodic)
-        k_moments<C, true><<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s, codec, step);
-    else
-        k_moments<C, false><<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s, codec, step);
-    return cudaGetLastError();
-}
-
-template <class C>
 cudaError_t boundary_dispatch(const DeviceState &s, int wbuf, int64_t step, int which, bool from_bmom,
                               cudaStream_t st) {
     dim3 grid = grid_plane(s.g);
     grid.z = which >= 0 ? 1 : 2;
-    k_boundary<C><<<grid, dim3(32, 8), 0, st>>>(s, wbuf, step, which, from_bmom ? 1 : 0);
-    return cudaGetLastError();
+    return launch_overlapped(k_boundary<C>, grid, dim3(32, 8), st, s, wbuf, step, which, from_bmom ? 1 : 0);
 }
 
 // ------------------------------------------------------------------ discrete adjoint
@@ -1403,21 +1327,6 @@ __global__ void __launch_bounds__(kBX * kBY) k_adj_initial(const DeviceState s, 
 
 // ---------------------------------------------------------------------- host side
 
-cudaError_t launch_moments(const DeviceState &s, int cur, int64_t step, bool stats, cudaStream_t st) {
-    cudaError_t e = s.g.storage == kStoreF16 ? moments_dispatch<CodecF16>(s, cur, step, st)
-                                             : moments_dispatch<CodecF32>(s, cur, step, st);
-    if (e != cudaSuccess || !stats) return e;
-    return launch_accumulate_radial(s, st);
-}
-
-cudaError_t launch_collide(const DeviceState &s, int cur, int64_t step, cudaStream_t st) {
-    if (s.g.storage == kStoreF16)
-        k_collide<CodecF16><<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s, make_codec<CodecF16>(s, cur), step);
-    else
-        k_collide<CodecF32><<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s, make_codec<CodecF32>(s, cur), step);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_boundary(const DeviceState &s, int wbuf, int64_t step, int which, bool from_bmom,
                             cudaStream_t st) {
     if (s.g.storage == kStoreF16) return boundary_dispatch<CodecF16>(s, wbuf, step, which, from_bmom, st);
@@ -1425,8 +1334,7 @@ cudaError_t launch_boundary(const DeviceState &s, int wbuf, int64_t step, int wh
 }
 
 cudaError_t launch_accumulate_radial(const DeviceState &s, cudaStream_t st) {
-    k_accumulate_radial<<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s);
-    return cudaGetLastError();
+    return launch_overlapped(k_accumulate_radial, grid3(s.g), dim3(kBX, kBY), st, s);
 }
 
 cudaError_t launch_init_fields(const DeviceState &s, int mode, int red_inside, float r2, float bx, float by, float bz,

@@ -514,6 +514,38 @@ __device__ __forceinline__ NodeMoments pull_moments(const Geometry &g, const C &
 // (odd) are added per direction.  psi_at(cx,cy,cz) returns the neighbour's
 // psi, read unwrapped like forces.cuh:31 (ghost psi is what the reference
 // sees there).
+// Launches that follow one another on a stream overlap by programmatic dependent
+// launch: each starts while the one before it drains, and everything before the
+// wait reads only kernel parameters.  Every thread of a kernel launched this way
+// waits, so that the end of a launch is also the end of all before it.
+__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The same, renewing the pointers behind the wait, so that no load of theirs can
+// be moved above it.
+template <class C>
+__device__ __forceinline__ void wait_for_previous_launch(C &codec, const float *&psi) {
+    wait_for_previous_launch();
+    auto rd = codec.rd;
+    auto wr = codec.wr;
+    asm volatile("" : "+l"(rd), "+l"(wr), "+l"(psi)::"memory");
+    codec.rd = rd;
+    codec.wr = wr;
+}
+__device__ __forceinline__ void allow_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, const A &...args) {
+    cudaLaunchAttribute overlap{};
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cfg.attrs = &overlap;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Columns of a lattice row whose slots a kernel that relaxes the row stores:
 // the interior ones, ghost column 0 and the columns that complete the last 64
 // bytes (the pitch allowing).  Nothing reads the ghost and pad columns of an

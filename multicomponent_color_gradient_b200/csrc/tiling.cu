@@ -52,6 +52,8 @@ static void split_tiling(const Geometry &g, FusedTiling &t) {
     t.boundary_ctas = int(std::min<long long>((columns + kInterfaceThreads - 1) / kInterfaceThreads, 148));
 }
 
+static int compiled_pitch(const Geometry &g) { return g.px % 32 == 0 ? g.px : 0; }
+
 FusedTiling fused_tiling(const Geometry &g, int max_smem) {
     FusedTiling t{};
     t.tpr = ((g.NX + 31) / 32) * 32;
@@ -70,7 +72,7 @@ FusedTiling fused_tiling(const Geometry &g, int max_smem) {
     else
         march_tiling(g, max_smem, t);
     // the row pitch the kernels are compiled for (the marches: whole rows)
-    t.pitch = t.march == kMarchSplit ? (g.px % 32 == 0 ? g.px : 0) : t.fixed_nx;
+    t.pitch = t.march == kMarchSplit ? compiled_pitch(g) : t.fixed_nx;
     if (const char *v = std::getenv("MCG_FUSED_FIXED_NX"))  // tests
         if (std::atoi(v) == 0) t.pitch = 0;
     // the jet's inlet and outlet columns within the step's launches, instead of
@@ -85,7 +87,9 @@ FusedTiling fused_tiling(const Geometry &g, int max_smem) {
 #define MCG_EXTERN(P)                                                                          \
     extern template cudaError_t fused_configure_pitch<P>(const Geometry &, const FusedTiling &); \
     extern template cudaError_t fused_launch_pitch<P>(const DeviceState &, const FusedTiling &, int, int64_t, bool, \
-                                                      cudaStream_t);
+                                                      cudaStream_t);                           \
+    extern template cudaError_t moments_launch_pitch<P>(const DeviceState &, int, int64_t, cudaStream_t);           \
+    extern template cudaError_t collide_launch_pitch<P>(const DeviceState &, int, int64_t, cudaStream_t);
 MCG_EACH_PITCH(MCG_EXTERN)
 
 cudaError_t fused_configure(const Geometry &g, const FusedTiling &t) {
@@ -109,6 +113,28 @@ cudaError_t launch_fused(const DeviceState &s, const FusedTiling &t_in, int cur,
     switch (t.pitch) {
 #define MCG_CASE(P) \
     case P: return fused_launch_pitch<P>(s, t, cur, step, stats, st);
+        MCG_EACH_PITCH(MCG_CASE)
+#undef MCG_CASE
+    }
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_moments(const DeviceState &s, int cur, int64_t step, bool stats, cudaStream_t st) {
+    cudaError_t e = cudaErrorInvalidValue;
+    switch (compiled_pitch(s.g)) {
+#define MCG_CASE(P) \
+    case P: e = moments_launch_pitch<P>(s, cur, step, st); break;
+        MCG_EACH_PITCH(MCG_CASE)
+#undef MCG_CASE
+    }
+    if (e != cudaSuccess || !stats) return e;
+    return launch_accumulate_radial(s, st);
+}
+
+cudaError_t launch_collide(const DeviceState &s, int cur, int64_t step, cudaStream_t st) {
+    switch (compiled_pitch(s.g)) {
+#define MCG_CASE(P) \
+    case P: return collide_launch_pitch<P>(s, cur, step, st);
         MCG_EACH_PITCH(MCG_CASE)
 #undef MCG_CASE
     }
