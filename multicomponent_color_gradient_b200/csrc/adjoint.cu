@@ -703,11 +703,10 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
         d.pops[0] = work[t & 1];
         d.pops[1] = work[(t + 1) & 1];
         if (rec) {
-            ADJ_CUDA(cudaMemcpyAsync(rec + size_t(mcg::kTapePsi) * N, run.psi[(step0 + t) & 1], N * sizeof(float),
-                                     cudaMemcpyDeviceToDevice, h->stream),
-                     "record psi");
-            ADJ_LAUNCH(h, mcg::launch_copy_outlet_state(d, rec + size_t(mcg::kTapePlanes) * N, h->stream),
-                       "jet adjoint: record outlet state");
+            ADJ_LAUNCH(h,
+                       mcg::launch_record_state(d, run.psi[(step0 + t) & 1], rec, rec + size_t(mcg::kTapePlanes) * N,
+                                                h->stream),
+                       "jet adjoint: record psi and outlet state");
             if (mcg_status st = record_step(h, d, rec, 5 * NP, step0 + t, stats)) return st;
         } else {
             ADJ_LAUNCH(h, mcg::launch_fused(d, h->tiling, 0, step0 + t, stats, h->stream), "jet adjoint: forward step");

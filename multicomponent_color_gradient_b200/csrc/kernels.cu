@@ -11,6 +11,7 @@ namespace {
 // ------------------------------------------------------------------ granular sequence
 
 constexpr int kBX = 32, kBY = 8;
+constexpr int kRedThreads = 256;
 
 // Jet boundary of step `step`: blockIdx.z == 0 is the inlet (y=0 plane), 1 the
 // outlet (y=NY-1 plane), unless `which` selects one.  Values go to the ghost
@@ -105,22 +106,37 @@ __global__ void k_init_fields(const DeviceState s, int mode, int red_inside, flo
 // buffers).  Every other slot of the other buffer is written by the first
 // step before anything reads it.  Directions are unrolled, so the pull
 // source and the equilibrium take compile-time lattice constants.
+// By pieces of 32 columns, the ghost columns of the rows filled with zeros to
+// complete their sectors (store_columns): an initial jet of 128x256x128 float32
+// takes 226 us in all (384 on 32x8 blocks that left them partly written).
 template <class C>
-__global__ void k_init_pops(const DeviceState s, int mode, float noise) {
+__global__ void __launch_bounds__(kRedThreads) k_init_pops(const DeviceState s, const C codec, int mode, float noise) {
     const Geometry &g = s.g;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z = blockIdx.z;
-    if (!(x >= 1 && x <= g.NX - 2 && y >= 1 && y <= g.NY - 2 && z >= 1 && z <= g.NZ - 2)) return;
+    const int ppr = pieces_per_row<C>(g);
+    const int piece = int(blockIdx.x) * (kRedThreads / 32) + int(threadIdx.x >> 5);
+    const int row = piece / ppr, y = 1 + row, z = 1 + int(blockIdx.y);
+    const int x = (piece - row * ppr) * 32 + int(threadIdx.x & 31);
+    if (y > g.NY - 2 || x >= store_columns<C>(g)) return;
+    const bool node = x >= 1 && x <= g.NX - 2;
     const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
     const size_t N = g.N;
-    const float rr = s.mom[kMomRR * N + id], rb = s.mom[kMomRB * N + id];
-    const float ux = s.mom[kMomUX * N + id], uy = s.mom[kMomUY * N + id], uz = s.mom[kMomUZ * N + id];
-    const float usq = ux * ux + uy * uy + uz * uz;
+    float rr = 0.f, rb = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
+    if (node) {
+        rr = s.mom[kMomRR * N + id];
+        rb = s.mom[kMomRB * N + id];
+        ux = s.mom[kMomUX * N + id];
+        uy = s.mom[kMomUY * N + id];
+        uz = s.mom[kMomUZ * N + id];
+    }
+    const float usq = fmaf(uz, uz, fmaf(ux, ux, uy * uy));  // one order of rounding in every build
     const bool periodic = g.boundary == kBoundaryPeriodic;
+    const PullMap<C> pm(g, x, y, z, periodic);
+    typename C::Elem *const other = const_cast<typename C::Elem *>(codec.rd);  // the other buffer
     static_for<kQ>([&](auto I) {
         constexpr int i = decltype(I)::value;
         using D = Dir<i>;
+        const bool ghost = (D::cy == 1 && pm.gy_p) || (D::cy == -1 && pm.gy_m);  // a slot of a y ghost plane
+        if (!node && ghost) return;
         float fr, fb;
         if (mode == 3) {
             // per colour, the third-order equilibrium at the node's velocity (lbm.cuh:16-35)
@@ -141,10 +157,13 @@ __global__ void k_init_pops(const DeviceState s, int mode, float noise) {
                 fb = fb * f;
             }
         }
-        int xs, ys, zs;
-        pull_src_rt(g, x, y, z, i, xs, ys, zs);
-        C::store_to(s.pops[0], g, i, xs, ys, zs, fr, fb, s.ph.f16_rho0);
-        if (!periodic && (ys == 0 || ys == g.NY - 1)) C::store_to(s.pops[1], g, i, xs, ys, zs, fr, fb, s.ph.f16_rho0);
+        size_t grow;
+        int xs;
+        pm.template src<i>(node ? x : x + D::cx, grow, xs);
+        const size_t at = grow + size_t(D::cx + 1) * g.px + xs;
+        const typename C::Elem v = codec.template pack<i>(fr, fb);
+        codec.wr[at] = v;
+        if (ghost) other[at] = v;
     });
 }
 
@@ -177,44 +196,60 @@ __global__ void k_refresh_psi(const DeviceState s) {
 // sources in buffer `wbuf` (the sources of planes z0 and z0+nz-1 lie in the
 // neighbouring chunks' planes; every source is written by exactly one node).
 template <class C>
-__global__ void k_scatter_chunk(const DeviceState s, int wbuf, const float *__restrict__ stage, size_t pitch, int z0) {
+__global__ void __launch_bounds__(kRedThreads) k_scatter_chunk(const DeviceState s, const C codec,
+                                                              const float *__restrict__ stage, size_t pitch, int z0) {
     const Geometry &g = s.g;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z = z0 + int(blockIdx.z);
-    if (!(x >= 1 && x <= g.NX - 2 && y >= 1 && y <= g.NY - 2 && z >= 1 && z <= g.NZ - 2)) return;
-    const size_t lid = size_t(x) + size_t(g.sy) * size_t(y) + size_t(g.sz) * size_t(blockIdx.z);
+    const int ppr = pieces_per_row<C>(g);
+    const int piece = int(blockIdx.x) * (kRedThreads / 32) + int(threadIdx.x >> 5);
+    const int row = piece / ppr, y = 1 + row, z = z0 + int(blockIdx.y);
+    const int x = (piece - row * ppr) * 32 + int(threadIdx.x & 31);
+    if (y > g.NY - 2 || z < 1 || z > g.NZ - 2 || x >= store_columns<C>(g)) return;
+    const bool node = x >= 1 && x <= g.NX - 2;
+    const size_t lid = size_t(x) + size_t(g.sy) * size_t(y) + size_t(g.sz) * size_t(blockIdx.y);
     const float *fr = stage, *fb = stage + size_t(kQ) * pitch;
-    for (int i = 0; i < kQ; ++i) {
-        int xs, ys, zs;
-        pull_src_rt(g, x, y, z, i, xs, ys, zs);
-        C::store_to(s.pops[wbuf], g, i, xs, ys, zs, fr[size_t(i) * pitch + lid], fb[size_t(i) * pitch + lid],
-                    s.ph.f16_rho0);
-    }
+    const PullMap<C> pm(g, x, y, z, g.boundary == kBoundaryPeriodic);
+    static_for<kQ>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        using D = Dir<i>;
+        if (!node && ((D::cy == 1 && pm.gy_p) || (D::cy == -1 && pm.gy_m))) return;
+        float r = 0.f, b = 0.f;
+        if (node) {
+            r = fr[size_t(i) * pitch + lid];
+            b = fb[size_t(i) * pitch + lid];
+        }
+        size_t grow;
+        int xs;
+        pm.template src<i>(node ? x : x + D::cx, grow, xs);
+        codec.wr[grow + size_t(D::cx + 1) * g.px + xs] = codec.template pack<i>(r, b);
+    });
 }
 
 // Gather: f(t) = pops[cur] pulled at the chunk's nodes into the stage; ghost
 // nodes give 0.
-template <class C>
-__global__ void k_gather_chunk(const DeviceState s, int cur, float *__restrict__ stage, size_t pitch, int z0) {
+template <class C, bool kPeriodic>
+__global__ void __launch_bounds__(kRedThreads) k_gather_chunk(const DeviceState s, const C codec,
+                                                             float *__restrict__ stage, size_t pitch, int z0) {
     const Geometry &g = s.g;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z = z0 + int(blockIdx.z);
-    if (x >= g.NX || y >= g.NY) return;
-    const size_t lid = size_t(x) + size_t(g.sy) * size_t(y) + size_t(g.sz) * size_t(blockIdx.z);
-    const bool interior = x >= 1 && x <= g.NX - 2 && y >= 1 && y <= g.NY - 2 && z >= 1 && z <= g.NZ - 2;
+    const int ppr = (g.NX + 31) / 32;
+    const int piece = int(blockIdx.x) * (kRedThreads / 32) + int(threadIdx.x >> 5);
+    const int y = piece / ppr, z = z0 + int(blockIdx.y);
+    const int x = (piece - y * ppr) * 32 + int(threadIdx.x & 31);
+    if (y >= g.NY || x >= g.NX) return;
+    const size_t lid = size_t(x) + size_t(g.sy) * size_t(y) + size_t(g.sz) * size_t(blockIdx.y);
     float *fr = stage, *fb = stage + size_t(kQ) * pitch;
-    for (int i = 0; i < kQ; ++i) {
-        float r = 0.0f, b = 0.0f;
-        if (interior) {
-            int xs, ys, zs;
-            pull_src_rt(g, x, y, z, i, xs, ys, zs);
-            C::load_from(s.pops[cur], g, i, xs, ys, zs, r, b, s.ph.f16_rho0);
-        }
+    if (!(x >= 1 && x <= g.NX - 2 && y >= 1 && y <= g.NY - 2 && z >= 1 && z <= g.NZ - 2)) {
+        for (int i = 0; i < kQ; ++i) fr[size_t(i) * pitch + lid] = fb[size_t(i) * pitch + lid] = 0.0f;
+        return;
+    }
+    RawPull<C> raw;
+    pull_issue<C, kPeriodic>(g, codec, x, y, z, raw);
+    static_for<kQ>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        float r, b;
+        codec.template unpack<i>(raw.v[i], r, b);
         fr[size_t(i) * pitch + lid] = r;
         fb[size_t(i) * pitch + lid] = b;
-    }
+    });
 }
 
 template <class E>
@@ -240,7 +275,6 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     return r;
 }
 
-constexpr int kRedThreads = 256;
 
 // Sum of 0.5|u|^2 over interior nodes (kernels.cu:136-152), float64.
 __global__ void __launch_bounds__(kRedThreads) k_tke(const DeviceState s, double *out) {
@@ -892,8 +926,7 @@ __device__ __forceinline__ void for_flagged_pieces(const Geometry &g, const uint
 // pieces, each other block the unflagged ones among kAdjThreads / 32 neighbours.
 template <bool kPeriodic>
 __global__ void __launch_bounds__(kAdjThreads, kAdjRelaxBlocks) k_adj_relax(const DeviceState s,
-                                                                           const float *__restrict__ M,
-                                                                           const uint8_t *__restrict__ flags,
+                                                                           const float *M, const uint8_t *flags,
                                                                            uint8_t *near_flags, const float *lam,
                                                                            float *lmom, float *lf, float *lam_out,
                                                                            double *acc, AdjObjective obj,
@@ -901,6 +934,8 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjRelaxBlocks) k_adj_relax(cons
     __shared__ double sh[3 * (kAdjThreads / 32)];
     const Geometry &g = s.g;
     double a_omega = 0.0, a_Ah = 0.0, a_J = 0.0;
+    allow_next_launch();
+    wait_for_previous_launch();
     if (int(blockIdx.x) < list_blocks) {
         for_flagged_pieces(g, flags, uint32_t(list_blocks), [&](int w, int y, int z) {
             const int x = w * 32 + int(threadIdx.x & 31);
@@ -947,12 +982,15 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjRelaxBlocks) k_adj_relax(cons
 }
 
 template <bool kPeriodic>
-__global__ void __launch_bounds__(kAdjThreads, kAdjNearBlocks) k_adj_near(const DeviceState s, const float *__restrict__ M,
-                                                                const uint8_t *__restrict__ flags,
-                                                                const uint8_t *__restrict__ near_flags,
-                                                                const float *lmom, const float *lf, float *lam_out) {
+__global__ void __launch_bounds__(kAdjThreads, kAdjNearBlocks) k_adj_near(const DeviceState s, const float *M,
+                                                                             const uint8_t *flags,
+                                                                             const uint8_t *near_flags,
+                                                                             const float *lmom, const float *lf,
+                                                                             float *lam_out) {
     const Geometry &g = s.g;
     const size_t N = g.N;
+    allow_next_launch();
+    wait_for_previous_launch();
     for_flagged_pieces(g, near_flags, gridDim.x, [&](int w, int y, int z) {
         const unsigned around = flags_around<kPeriodic>(g, flags, w, y, z);
         const int x = w * 32 + int(threadIdx.x & 31);
@@ -1064,15 +1102,17 @@ __device__ __forceinline__ float inlet_noise_factor(const Physics &ph, int64_t s
 // One thread per interior column (x, z): the outlet at y = NY-1 (blockIdx.z 0)
 // or, in a jet column, the inlet at y = 0 (1).  A ghost-plane slot enters only if an interior
 // node pulls it (the boundary also writes slots nothing reads).
-__global__ void __launch_bounds__(32) k_adj_boundary(const DeviceState s, int64_t step, const float *__restrict__ M,
-                                                      const float *__restrict__ Bt, const float *__restrict__ lam,
-                                                      const float *__restrict__ lf, float *lmom,
-                                                      const float *__restrict__ LB_in, float *LB_out,
-                                                      const float *__restrict__ bessel, int nb, double *dJdc) {
+__global__ void __launch_bounds__(32) k_adj_boundary(const DeviceState s, int64_t step, const float *M,
+                                                      const float *Bt, const float *lam,
+                                                      const float *lf, float *lmom,
+                                                      const float *LB_in, float *LB_out,
+                                                      const float *bessel, int nb, double *dJdc) {
     const Geometry &g = s.g;
     const Physics &ph = s.ph;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int z = blockIdx.y * blockDim.y + threadIdx.y;
+    allow_next_launch();
+    wait_for_previous_launch();
     const bool col = x >= 1 && x <= g.NX - 2 && z >= 1 && z <= g.NZ - 2;
     const size_t N = g.N;
     const int NP = g.NX * g.NZ;
@@ -1277,6 +1317,23 @@ __global__ void __launch_bounds__(256) k_copy_outlet_state(const DeviceState s, 
     for (int c = 0; c < 5; ++c) dst[c * NP + x + g.NX * z] = s.mom[size_t(c) * g.N + idB];
 }
 
+// What a jet record needs of the state beside what the step writes into it: the
+// psi plane with its ghost values (plane kTapePsi of rec; the step rewrites the
+// interior) and the outlet state (5 planes behind the record's).
+__global__ void __launch_bounds__(256) k_record_state(const DeviceState s, const float *psi, float *rec, float *outlet) {
+    const Geometry &g = s.g;
+    const uint32_t NP = uint32_t(g.NX) * uint32_t(g.NZ), stride = gridDim.x * 256;
+    allow_next_launch();
+    wait_for_previous_launch();
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < g.N; i += stride) rec[size_t(kTapePsi) * g.N + i] = psi[i];
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < NP; i += stride) {
+        const uint32_t z = i / uint32_t(g.NX), x = i - z * uint32_t(g.NX);
+        const uint32_t idB = x + uint32_t(g.sy) * uint32_t(g.NY - 1) + uint32_t(g.sz) * z;
+#pragma unroll
+        for (int c = 0; c < 5; ++c) outlet[size_t(c) * NP + i] = s.mom[size_t(c) * g.N + idB];
+    }
+}
+
 // dJ/du0 for an initial state f0_c,i = feq_i(rho_c, u0): pulls lambda_0 like
 // the forward step pulls populations.
 __global__ void __launch_bounds__(kBX * kBY) k_adj_initial(const DeviceState s, const float *__restrict__ M,
@@ -1344,11 +1401,13 @@ cudaError_t launch_init_fields(const DeviceState &s, int mode, int red_inside, f
 }
 
 cudaError_t launch_init_pops(const DeviceState &s, int mode, float noise, cudaStream_t st) {
-    if (s.g.storage == kStoreF16)
-        k_init_pops<CodecF16><<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s, mode, noise);
-    else
-        k_init_pops<CodecF32><<<grid3(s.g), dim3(kBX, kBY), 0, st>>>(s, mode, noise);
-    return cudaGetLastError();
+    auto go = [&](auto made) {
+        using C = decltype(made);
+        const dim3 grid((pieces_per_row<C>(s.g) * (s.g.NY - 2) + kRedThreads / 32 - 1) / (kRedThreads / 32), s.g.NZ - 2);
+        k_init_pops<C><<<grid, kRedThreads, 0, st>>>(s, made, mode, noise);
+        return cudaGetLastError();
+    };
+    return s.g.storage == kStoreF16 ? go(make_codec<CodecF16>(s, 1)) : go(make_codec<CodecF32>(s, 1));
 }
 
 cudaError_t launch_refresh_psi(const DeviceState &s, cudaStream_t st) {
@@ -1358,24 +1417,27 @@ cudaError_t launch_refresh_psi(const DeviceState &s, cudaStream_t st) {
 
 cudaError_t launch_scatter_chunk(const DeviceState &s, int wbuf, const float *stage, size_t pitch, int z0, int nz,
                                  cudaStream_t st) {
-    dim3 grid = grid3(s.g);
-    grid.z = unsigned(nz);
-    if (s.g.storage == kStoreF16)
-        k_scatter_chunk<CodecF16><<<grid, dim3(kBX, kBY), 0, st>>>(s, wbuf, stage, pitch, z0);
-    else
-        k_scatter_chunk<CodecF32><<<grid, dim3(kBX, kBY), 0, st>>>(s, wbuf, stage, pitch, z0);
-    return cudaGetLastError();
+    auto go = [&](auto made) {
+        using C = decltype(made);
+        const dim3 grid((pieces_per_row<C>(s.g) * (s.g.NY - 2) + kRedThreads / 32 - 1) / (kRedThreads / 32), nz);
+        k_scatter_chunk<C><<<grid, kRedThreads, 0, st>>>(s, made, stage, pitch, z0);
+        return cudaGetLastError();
+    };
+    return s.g.storage == kStoreF16 ? go(make_codec<CodecF16>(s, wbuf ^ 1)) : go(make_codec<CodecF32>(s, wbuf ^ 1));
 }
 
 cudaError_t launch_gather_chunk(const DeviceState &s, int cur, float *stage, size_t pitch, int z0, int nz,
                                 cudaStream_t st) {
-    dim3 grid = grid3(s.g);
-    grid.z = unsigned(nz);
-    if (s.g.storage == kStoreF16)
-        k_gather_chunk<CodecF16><<<grid, dim3(kBX, kBY), 0, st>>>(s, cur, stage, pitch, z0);
-    else
-        k_gather_chunk<CodecF32><<<grid, dim3(kBX, kBY), 0, st>>>(s, cur, stage, pitch, z0);
-    return cudaGetLastError();
+    const dim3 grid(((s.g.NX + 31) / 32 * s.g.NY + kRedThreads / 32 - 1) / (kRedThreads / 32), nz);
+    auto go = [&](auto made) {
+        using C = decltype(made);
+        if (s.g.boundary == kBoundaryPeriodic)
+            k_gather_chunk<C, true><<<grid, kRedThreads, 0, st>>>(s, made, stage, pitch, z0);
+        else
+            k_gather_chunk<C, false><<<grid, kRedThreads, 0, st>>>(s, made, stage, pitch, z0);
+        return cudaGetLastError();
+    };
+    return s.g.storage == kStoreF16 ? go(make_codec<CodecF16>(s, cur)) : go(make_codec<CodecF32>(s, cur));
 }
 
 cudaError_t launch_unpad_rows(const DeviceState &s, int cur, cudaStream_t st) {
@@ -1517,9 +1579,8 @@ cudaError_t adj_relax(const DeviceState &s, const float *M, const uint8_t *flags
     constexpr int kWarps = kAdjThreads / 32;
     const int plane = (adj_pieces_per_row(s.g) * (s.g.NY - 2) + kWarps - 1) / kWarps;
     const int list = int(adj_list_blocks(s.g, kAdjRelaxBlocks));
-    k_adj_relax<kPeriodic><<<list + plane * (s.g.NZ - 2), kAdjThreads, 0, st>>>(s, M, flags, near_flags, lam_in, lmom, lf,
-                                                                               lam_out, acc, obj, list, plane);
-    return cudaGetLastError();
+    return launch_overlapped(k_adj_relax<kPeriodic>, dim3(list + plane * (s.g.NZ - 2)), dim3(kAdjThreads), st, s, M, flags,
+                             near_flags, lam_in, lmom, lf, lam_out, acc, obj, list, plane);
 }
 }  // namespace
 
@@ -1534,11 +1595,10 @@ cudaError_t launch_adj_relax(const DeviceState &s, const float *M, const uint8_t
 cudaError_t launch_adj_near(const DeviceState &s, const float *M, const uint8_t *flags, const uint8_t *near_flags,
                             const float *lmom, const float *lf, float *lam_out, cudaStream_t st) {
     const unsigned n = adj_list_blocks(s.g, kAdjNearBlocks);
-    if (s.g.boundary == kBoundaryPeriodic)
-        k_adj_near<true><<<n, kAdjThreads, 0, st>>>(s, M, flags, near_flags, lmom, lf, lam_out);
-    else
-        k_adj_near<false><<<n, kAdjThreads, 0, st>>>(s, M, flags, near_flags, lmom, lf, lam_out);
-    return cudaGetLastError();
+    return s.g.boundary == kBoundaryPeriodic
+               ? launch_overlapped(k_adj_near<true>, dim3(n), dim3(kAdjThreads), st, s, M, flags, near_flags, lmom, lf, lam_out)
+               : launch_overlapped(k_adj_near<false>, dim3(n), dim3(kAdjThreads), st, s, M, flags, near_flags, lmom, lf,
+                                   lam_out);
 }
 
 cudaError_t launch_piece_flags(const DeviceState &s, const float *M, uint8_t *flags, cudaStream_t st) {
@@ -1554,14 +1614,19 @@ cudaError_t launch_adj_boundary(const DeviceState &s, int64_t step, const float 
     // one warp per block: a column is a long chain of dependent work, and blocks
     // of 8 warps put the 62 x 62 columns of a 64-wide jet on 16 SMs
     const dim3 block(32, 1), grid((s.g.NX + 31) / 32, s.g.NZ, 2);
-    k_adj_boundary<<<grid, block, 0, st>>>(s, step, M, Bt, lam_next, lf, lmom, LB_in, LB_out, bessel, nb, dJdc);
-    return cudaGetLastError();
+    return launch_overlapped(k_adj_boundary, grid, block, st, s, step, M, Bt, lam_next, lf, lmom, LB_in, LB_out, bessel, nb,
+                             dJdc);
 }
 
 cudaError_t launch_restore_outlet_state(const DeviceState &s, const float *src, float *psi, cudaStream_t st) {
     const dim3 block(32, 8), grid((s.g.NX + 31) / 32, (s.g.NZ + 7) / 8);
     k_restore_outlet_state<<<grid, block, 0, st>>>(s, src, psi);
     return cudaGetLastError();
+}
+
+cudaError_t launch_record_state(const DeviceState &s, const float *psi, float *rec, float *outlet, cudaStream_t st) {
+    const unsigned blocks = unsigned(std::min<uint32_t>((s.g.N + 255) / 256, 4 * 148));
+    return launch_overlapped(k_record_state, dim3(blocks), dim3(256), st, s, psi, rec, outlet);
 }
 
 cudaError_t launch_copy_outlet_state(const DeviceState &s, float *dst, cudaStream_t st) {

@@ -244,6 +244,8 @@ cudaError_t launch_adj_boundary(const DeviceState &s, int64_t step, const float 
 // The outlet state (5 planes at y = NY-1, interior columns) to dst[5][NX*NZ],
 // and back (restoring also the outlet-plane psi in `psi`).
 cudaError_t launch_copy_outlet_state(const DeviceState &s, float *dst, cudaStream_t st);
+// psi (with ghosts) and the outlet state of a jet's state into its record.
+cudaError_t launch_record_state(const DeviceState &s, const float *psi, float *rec, float *outlet, cudaStream_t st);
 cudaError_t launch_restore_outlet_state(const DeviceState &s, const float *src, float *psi, cudaStream_t st);
 cudaError_t launch_adj_initial(const DeviceState &s, const float *M, const float *lam0, float *du0, cudaStream_t st);
 

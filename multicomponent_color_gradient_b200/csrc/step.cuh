@@ -68,15 +68,13 @@ struct CodecF32 {
                                                     float b, float) {
         static_cast<float2 *>(buf)[pop_index(g, slot_pair(i), x, y, z)] = make_float2(r, b);
     }
+    template <int I>
+    __device__ __forceinline__ Elem pack(float r, float b) const {
+        return make_float2(r, b);
+    }
     // the colour pair of a pulled element
     template <int I>
     __device__ __forceinline__ void unpack(Raw v, float &r, float &b) const {
-        r = v.x;
-        b = v.y;
-    }
-    __device__ __forceinline__ static void load_from(const void *buf, const Geometry &g, int i, int x, int y, int z,
-                                                     float &r, float &b, float) {
-        const float2 v = static_cast<const float2 *>(buf)[pop_index(g, slot_pair(i), x, y, z)];
         r = v.x;
         b = v.y;
     }
@@ -166,12 +164,12 @@ struct CodecF16 {
         static_cast<__half2 *>(buf)[pop_index(g, slot_pair(i), x, y, z)] = f16_encode(r, b, 1.0f / dir_w(i), rho0);
     }
     template <int I>
+    __device__ __forceinline__ Elem pack(float r, float b) const {
+        return f16_encode(r, b, 1.0f / Dir<I>::w, rho0);
+    }
+    template <int I>
     __device__ __forceinline__ void unpack(Raw h, float &r, float &b) const {
         f16_decode(h, Dir<I>::w, rho0, r, b);
-    }
-    __device__ __forceinline__ static void load_from(const void *buf, const Geometry &g, int i, int x, int y, int z,
-                                                     float &r, float &b, float rho0) {
-        f16_decode(static_cast<const __half2 *>(buf)[pop_index(g, slot_pair(i), x, y, z)], dir_w(i), rho0, r, b);
     }
 };
 
@@ -312,21 +310,6 @@ struct FastPullMap {
         return b + (-(long long)D::cy * step_y + (long long)(dir_group(I) * C::kGroupSlots + D::cx + 1) * px - D::cx);
     }
 };
-
-// Runtime-direction pull source (init/gather/diagnostic kernels): source
-// coordinates of direction i for interior node (x,y,z).
-__device__ __forceinline__ void pull_src_rt(const Geometry &g, int x, int y, int z, int i, int &xs, int &ys, int &zs) {
-    const bool periodic = g.boundary == kBoundaryPeriodic;
-    xs = x - dir_cx(i);
-    ys = y - dir_cy(i);
-    zs = z - dir_cz(i);
-    const bool ghost_plane = !periodic && (ys == 0 || ys == g.NY - 1);
-    if (!ghost_plane) {
-        xs = wrap_interior(xs, g.NX);
-        zs = wrap_interior(zs, g.NZ);
-    }
-    if (periodic) ys = wrap_interior(ys, g.NY);
-}
 
 // ------------------------------------------------------------------ per-node pieces
 
