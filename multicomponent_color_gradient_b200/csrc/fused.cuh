@@ -508,9 +508,10 @@ __global__ void __launch_bounds__(kFusedThreads, PipeBlocks<C>::value) k_fused_p
 //   k_step_pull       one warp per piece of 32 columns of a row: pulls its 32
 //                     nodes, forms moments, psi and statistics, and, when all
 //                     32 are bulk, relaxes and stores them at once.  A piece
-//                     with an interface node leaves its moments in the slots
-//                     it will store (of the buffer the step writes, which no
-//                     one reads yet) and sets its flag.
+//                     (float16: a quarter of one) with an interface node
+//                     leaves its moments in the slots it will store (of the
+//                     buffer the step writes, which no one reads yet) and sets
+//                     its flag.
 //   k_step_interface  relaxes the flagged pieces, with the colour gradient
 //                     from the psi the first launch wrote for every node, and
 //                     writes the jet's inlet and outlet columns.
@@ -539,6 +540,14 @@ constexpr int kInterfaceThreads = 128, kInterfaceBlocks = 5;
 // rows of 128 columns (4 against 1: 174 against 196 us a step for the
 // 128x256x128 float16 jet, 2250 against 2328 for 256x512x256 float32).
 constexpr int kPieceGroup = 4;
+
+// Float16, whose kernels are bound by their instructions, parks and relaxes
+// quarters of 8 columns (32 bytes of a row): fewer bulk nodes go through the
+// interface launch (64x128x64 jet 28.0 us a step against 31.6 by pieces, periodic
+// drops 128x256x128 181 against 195).  Float32 is bound by HBM and takes whole
+// pieces (318 by quarters against 313 for the same drops).
+template <class C>
+constexpr bool relax_by_quarters() { return std::is_same<C, CodecF16>::value; }
 
 // Moments of a node to and from its own element slots in the row it will
 // store: two floats an element in float32, one in float16.
@@ -610,20 +619,20 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitBlocks) k_step_pull(const
     const unsigned interface = __ballot_sync(kFull, xin && !is_bulk(m.rr, m.rb));
     if ((x & 31) == 0) s.piece_flags[(size_t(zi) * (g.NY - 2) + row) * ppr + w] = piece_flag(g, w, interface);
     const size_t at = pop_row(g, y, z);
-    if (interface) {
+    if (interface & (relax_by_quarters<C>() ? 0xffu << (x & 24) : kFull)) {
         if (xin) park_moments(codec.wr + at + x, g.px, m);
     } else if (xst) {
         collide_node<true>(g, s.ph, codec, at, x, y, z, m, [](int, int, int) { return 0.0f; });
     }
 }
 
-// One piece of k_step_interface: moments from where k_step_pull parked them,
-// psi of the neighbours, relaxation and stores.
+// One piece of k_step_interface, or four quarters, one per 8 lanes: moments from
+// where k_step_pull parked them, psi of the neighbours, relaxation and stores.
 template <class C, bool kPeriodic>
-__device__ __forceinline__ void relax_piece(const DeviceState &s, const C &codec, const float *psi, int x, int y,
-                                            int z) {
+__device__ __forceinline__ void relax_parked(const DeviceState &s, const C &codec, const float *psi, bool on, int x,
+                                               int y, int z) {
     const Geometry &g = s.g;
-    const bool xst = x < store_columns<C>(g);
+    const bool xst = on && x < store_columns<C>(g);
     const int xn = min(max(x, 1), g.NX - 2);
     const size_t at = pop_row(g, y, z);
     NodeMoments m{};
@@ -640,16 +649,17 @@ __device__ __forceinline__ void relax_piece(const DeviceState &s, const C &codec
     collide_node<false>(g, s.ph, codec, at, x, y, z, m, psi_at);
 }
 
-// Blocks [0, T.interface_ctas) relax the flagged pieces; each looks at every
-// interface_ctas-th group of neighbouring pieces, so that the pieces of one interface, which lie
-// together, go to different SMs, and its warps share what it finds.  The
-// blocks after them write the jet's inlet and outlet columns from the
-// fluid-plane moments in bmom.
+// Blocks [0, T.interface_ctas) relax what is flagged; each looks at every
+// interface_ctas-th group of neighbouring pieces, so that the pieces of one
+// interface, which lie together, go to different SMs, and its warps share what
+// it finds.  The blocks after them write the jet's inlet and outlet columns from
+// the fluid-plane moments in bmom.
 template <class C, bool kPeriodic, int kPX>
 __global__ void __launch_bounds__(kInterfaceThreads, kInterfaceBlocks) k_step_interface(const DeviceState s_arg,
                                                                                        const FusedTiling T, int cur,
                                                                                        int64_t step) {
-    __shared__ uint32_t list[kInterfaceThreads];
+    constexpr bool kQuarters = relax_by_quarters<C>();
+    __shared__ uint32_t list[(kQuarters ? 4 : 1) * kInterfaceThreads];  // pieces, or 4 * piece + quarter
     __shared__ int found;
     const DeviceState s = pitch_state<C, kPX>(s_arg);
     const Geometry &g = s.g;
@@ -669,17 +679,23 @@ __global__ void __launch_bounds__(kInterfaceThreads, kInterfaceBlocks) k_step_in
                                 threadIdx.x % kPieceGroup + first;
             // against the planes' order of k_step_pull (see there)
             const uint32_t mine = (step & 1) ? uint32_t(at) : pieces - 1 - uint32_t(at);
-            const bool flagged = at < pieces && s.piece_flags[mine];
-            const unsigned hits = __ballot_sync(kFull, flagged);
-            int base = 0;
-            if (lane == 0 && hits) base = atomicAdd(&found, __popc(hits));
-            base = __shfl_sync(kFull, base, 0);
-            if (flagged) list[base + __popc(hits & ((1u << lane) - 1u))] = mine;
+            const unsigned flag = at < pieces ? unsigned(s.piece_flags[mine]) : 0u;
+            if (flag) {
+                unsigned quarters = kQuarters ? flag >> 4 : 1u;
+                int k = atomicAdd(&found, __popc(quarters));
+                for (; quarters; quarters &= quarters - 1)
+                    list[k++] = kQuarters ? 4 * mine + uint32_t(__ffs(int(quarters)) - 1) : mine;
+            }
             __syncthreads();
-            for (int i = warp; i < found; i += kInterfaceThreads / 32) {
-                const uint32_t piece = list[i], row = piece / ppr, zi = row / uint32_t(g.NY - 2);
-                relax_piece<C, kPeriodic>(s, codec, psi, int(piece - row * ppr) * 32 + lane,
-                                          1 + int(row - zi * uint32_t(g.NY - 2)), 1 + int(zi));
+            constexpr int kTake = kQuarters ? 4 : 1;  // entries a warp takes together
+            for (int i = kTake * warp; i < found; i += kTake * (kInterfaceThreads / 32)) {
+                const int k = kQuarters ? i + (lane >> 3) : i;
+                const uint32_t entry = list[k < found ? k : i], piece = kQuarters ? entry >> 2 : entry, row = piece / ppr;
+                const uint32_t zi = row / uint32_t(g.NY - 2);
+                const int column = kQuarters ? int(entry & 3) * 8 + (lane & 7) : lane;
+                relax_parked<C, kPeriodic>(s, codec, psi, k < found, int(piece - row * ppr) * 32 + column,
+                                           1 + int(row - zi * uint32_t(g.NY - 2)), 1 + int(zi));
+                __syncwarp();
             }
             __syncthreads();
         }

@@ -550,10 +550,14 @@ __host__ __device__ __forceinline__ int pieces_per_row(const Geometry &g) {
 }
 
 // Flag of piece w of a row from the lanes that hold interface nodes: bit 0 any,
-// bit 1 its first interior column, bit 2 its last.
+// bit 1 its first interior column, bit 2 its last, bits 4 to 7 its quarters of 8
+// columns.
 __device__ __forceinline__ uint8_t piece_flag(const Geometry &g, int w, unsigned lanes) {
     const int first = w == 0 ? 1 : 0, last = min(31, g.NX - 2 - 32 * w);
-    return uint8_t((lanes != 0 ? 1u : 0u) | (((lanes >> first) & 1u) << 1) | (((lanes >> last) & 1u) << 2));
+    unsigned f = (lanes != 0 ? 1u : 0u) | (((lanes >> first) & 1u) << 1) | (((lanes >> last) & 1u) << 2);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) f |= ((lanes >> (8 * q)) & 0xffu) != 0 ? 16u << q : 0u;
+    return uint8_t(f);
 }
 
 // A node whose interface indicator (lbm.cuh:214-216) is at most 1e-4 takes the
