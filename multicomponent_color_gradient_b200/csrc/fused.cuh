@@ -720,19 +720,21 @@ __global__ void __launch_bounds__(kInterfaceThreads, kInterfaceBlocks) k_step_in
 
 // launch_Macros and launch_collistream as the reference drives them, by the
 // pieces of the split step: moments and psi of every interior node to HBM
-// (216 or 108 B read, 48 written a node), and the relaxation from there (48 B
+// (planes first .. first + planes - 1;
+// 216 or 108 B read, 48 written a node), and the relaxation from there (48 B
 // read, 216 or 108 written, whole sectors).  A step of the five launchers of the
 // 64x128x64 jet takes 56 us (86 with kernels of runtime pitch that stored the
 // rows in part, each launch after the end of the one before).
 template <class C, bool kPeriodic, int kPX>
-__global__ void __launch_bounds__(kSplitThreads, kSplitBlocks) k_moments(const DeviceState s_arg, int cur, int64_t step) {
+__global__ void __launch_bounds__(kSplitThreads, kSplitBlocks) k_moments(const DeviceState s_arg, int cur, int64_t step,
+                                                                           int first, int planes) {
     const DeviceState s = pitch_state<C, kPX>(s_arg);
     const Geometry &g = s.g;
     C codec = pitch_codec<C, kPX>(s_arg, cur);
     const int ppr = pieces_per_row<C>(g);
     const int piece = int(blockIdx.x) * (kSplitThreads / 32) + int(threadIdx.x >> 5);
     const int row = piece / ppr, y = 1 + row;
-    const int zi = (step & 1) ? g.NZ - 3 - int(blockIdx.y) : int(blockIdx.y), z = 1 + zi;
+    const int z = first + ((step & 1) ? planes - 1 - int(blockIdx.y) : int(blockIdx.y));
     const int x = (piece - row * ppr) * 32 + int(threadIdx.x & 31);
     const float *psi_at = s_arg.psi[step & 1];
     allow_next_launch();
@@ -1164,14 +1166,14 @@ cudaError_t fused_launch_pitch(const DeviceState &s, const FusedTiling &t, int c
 }
 
 template <int kPX>
-cudaError_t moments_launch_pitch(const DeviceState &s, int cur, int64_t step, cudaStream_t st) {
+cudaError_t moments_launch_pitch(const DeviceState &s, int cur, int64_t step, int first, int planes, cudaStream_t st) {
     constexpr int kWarps = kSplitThreads / 32;
     auto go = [&](auto codec) {
         using C = decltype(codec);
-        const dim3 grid((pieces_per_row<C>(s.g) * (s.g.NY - 2) + kWarps - 1) / kWarps, s.g.NZ - 2);
+        const dim3 grid((pieces_per_row<C>(s.g) * (s.g.NY - 2) + kWarps - 1) / kWarps, planes);
         return s.g.boundary == kBoundaryPeriodic
-                   ? launch_overlapped(k_moments<C, true, kPX>, grid, dim3(kSplitThreads), st, s, cur, step)
-                   : launch_overlapped(k_moments<C, false, kPX>, grid, dim3(kSplitThreads), st, s, cur, step);
+                   ? launch_overlapped(k_moments<C, true, kPX>, grid, dim3(kSplitThreads), st, s, cur, step, first, planes)
+                   : launch_overlapped(k_moments<C, false, kPX>, grid, dim3(kSplitThreads), st, s, cur, step, first, planes);
     };
     return s.g.storage == kStoreF16 ? go(CodecF16{}) : go(CodecF32{});
 }

@@ -137,6 +137,8 @@ cudaError_t launch_fused(const DeviceState &s, const FusedTiling &t, int cur, in
 // ---- granular launch sequence (launch.cuh order) ----
 // step: the reference loop index of the step being computed.
 cudaError_t launch_moments(const DeviceState &s, int cur, int64_t step, bool stats, cudaStream_t st);
+// The same for interior planes first .. first + planes - 1.
+cudaError_t launch_moments_planes(const DeviceState &s, int cur, int64_t step, int first, int planes, cudaStream_t st);
 cudaError_t launch_collide(const DeviceState &s, int cur, int64_t step, cudaStream_t st);
 // Jet inlet (which=0), outlet (1) or both (-1) of step `step`, into the ghost
 // planes of pops[wbuf] and psi[(step+1)&1].  from_bmom: moments of the fluid

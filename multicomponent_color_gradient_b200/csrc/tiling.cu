@@ -88,7 +88,7 @@ FusedTiling fused_tiling(const Geometry &g, int max_smem) {
     extern template cudaError_t fused_configure_pitch<P>(const Geometry &, const FusedTiling &); \
     extern template cudaError_t fused_launch_pitch<P>(const DeviceState &, const FusedTiling &, int, int64_t, bool, \
                                                       cudaStream_t);                           \
-    extern template cudaError_t moments_launch_pitch<P>(const DeviceState &, int, int64_t, cudaStream_t);           \
+    extern template cudaError_t moments_launch_pitch<P>(const DeviceState &, int, int64_t, int, int, cudaStream_t); \
     extern template cudaError_t collide_launch_pitch<P>(const DeviceState &, int, int64_t, cudaStream_t);
 MCG_EACH_PITCH(MCG_EXTERN)
 
@@ -119,14 +119,18 @@ cudaError_t launch_fused(const DeviceState &s, const FusedTiling &t_in, int cur,
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_moments(const DeviceState &s, int cur, int64_t step, bool stats, cudaStream_t st) {
-    cudaError_t e = cudaErrorInvalidValue;
+cudaError_t launch_moments_planes(const DeviceState &s, int cur, int64_t step, int first, int planes, cudaStream_t st) {
     switch (compiled_pitch(s.g)) {
 #define MCG_CASE(P) \
-    case P: e = moments_launch_pitch<P>(s, cur, step, st); break;
+    case P: return moments_launch_pitch<P>(s, cur, step, first, planes, st);
         MCG_EACH_PITCH(MCG_CASE)
 #undef MCG_CASE
     }
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_moments(const DeviceState &s, int cur, int64_t step, bool stats, cudaStream_t st) {
+    const cudaError_t e = launch_moments_planes(s, cur, step, 1, s.g.NZ - 2, st);
     if (e != cudaSuccess || !stats) return e;
     return launch_accumulate_radial(s, st);
 }

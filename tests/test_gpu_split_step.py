@@ -111,3 +111,30 @@ def test_back_to_back_steps_equal_waited_steps():
             out.append(S.get_populations())
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("boundary", ["jet", "periodic"])
+def test_fields_in_chunks_equal_fields_at_once(storage, boundary):
+    """A field read after a step forms and downloads the moments of a large grid
+    in z-chunks; after launch_Macros of the same state they are there already
+    and come whole.  The ghost planes are the same too."""
+    case = derive(dict(NX=130, NY=131, NZ=270, boundary=boundary, storage=storage, tau=0.6, sigma=0.01,
+                       jet_radius=8.0, bubble_radius=30.0, seed=2, init_noise=1e-3, NSTATS_START_STEP=10 ** 9))
+    with Solver(case) as S:
+        S.init_jet() if boundary == "jet" else S.init_bubble()
+        S.step(3)
+        chunked = S.get_fields()
+        at_once = S.get_fields()
+        for k in chunked:
+            np.testing.assert_array_equal(chunked[k], at_once[k])
+        S.step(1)
+        only = S.get_stress()
+        again = S.get_fields()
+    with Solver(case) as S:
+        S.init_jet() if boundary == "jet" else S.init_bubble()
+        S.step(4)
+        want = S.get_fields()
+        np.testing.assert_array_equal(S.get_stress(), only)
+        for k in want:
+            np.testing.assert_array_equal(want[k], again[k])
