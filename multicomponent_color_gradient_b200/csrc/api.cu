@@ -219,6 +219,18 @@ void give_back_padding(mcg_handle *h) {
     h->padding = 0;
 }
 
+// Whether the elements of a population buffer (without padding) fit L2, which
+// decides how a step pulls them (DecodedPullOnce): 97 x 75 x 131 gains 4 % in
+// float16 (103 MB) and would lose 2 % in float32 (206 MB).
+int fits_l2(const mcg_handle *h) {
+    int l2 = 0;
+    if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return pop_buffer_bytes(h->p, h->p.NX) <= size_t(l2) ? 1 : 0;
+}
+
 size_t piece_flag_bytes(const mcg_params &p) { return size_t(p.NY) * p.NZ * ((p.NX + 31) / 32); }
 
 void release(mcg_handle *h) {
@@ -442,6 +454,7 @@ mcg_status mcg_create(const mcg_params *p, mcg_handle **out) {
         g.storage = p->storage;
         g.slots = mcg::kQ;  // one element (both colours) per direction: float2 or half2
         g.px = row_pitch(*p, h->device, &h->padding);
+        h->s.l2_resident = fits_l2(h);
         fill_physics(h);
         compute_ncols(h);
         const size_t N = g.N;

@@ -522,12 +522,12 @@ __global__ void __launch_bounds__(kFusedThreads, PipeBlocks<C>::value) k_fused_p
 // barriers and leaves columns 0 and NX-1 unwritten (see store_columns); the
 // pull launch runs at the rate of a plain copy of the same elements.
 // us a step, this against the marches chosen before (fraction of the measured
-// copy peak at 432 or 216 B a node): jet 128x256x128 float32 295 (0.90) against
-// 352 (0.76), 256x512x256 2250 (0.97) against 2984 (0.73), 200x301x183 761
-// (0.93) against 1541 (0.46), 64x128x64 42 against 76, 24x40x24 10 against 29;
-// float16 jet 128x400x128 266 against 441, 256x512x256 1247 (0.87) against 2073
-// (0.52).  With every node an interface node it is even: 128x256x128 float32
-// 360 against 352, float16 324 against 365.
+// copy peak at 432 or 216 B a node): jet 128x256x128 float32 296 (0.90) against
+// 352 (0.76), 256x512x256 2264 (0.96) against 2984 (0.73), 200x301x183 769
+// (0.92) against 1541 (0.46), 64x128x64 39 against 76, 24x40x24 8-10 against 29;
+// float16 jet 128x400x128 258 (0.81) against 441, 256x512x256 1216 (0.89)
+// against 2073 (0.52).  With every node an interface node: 128x256x128 float32
+// 359 against 352, float16 324 against 365.
 
 // Threads and CTAs per SM the register budgets are sized for: k_step_pull 72
 // registers (64, with spills in float32, to 96 measured within 1 % in float32;

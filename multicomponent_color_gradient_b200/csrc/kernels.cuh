@@ -122,6 +122,7 @@ struct DeviceState {
     double *partials; // reduction scratch
     uint32_t partials_cap;
     uint8_t *piece_flags;  // [NZ-2][NY-2][pieces of 32 columns]: interface nodes of this step (piece_flag)
+    int l2_resident;  // a population buffer fits L2
     int *flag;        // device flags: [0] non-finite value, [1] a k_fused_bulk wait ran out
     float *tape;      // null, or [kTapePlanes][N]: the fused step records the moments and psi it pulls there
     const float *inlet_profile;  // null (top-hat), or [NZ][NX] multipliers of the inlet velocity per column

@@ -31,6 +31,7 @@ struct CodecF32 {
     const float2 *__restrict__ rd;
     float2 *__restrict__ wr;
     int px;  // row pitch
+    int l2_resident;
     // store through `wrow` = the node's row in the written buffer, offset by x
     template <int I>
     __device__ __forceinline__ void store_row(float2 *wrow, float r, float b) const {
@@ -53,6 +54,12 @@ struct CodecF32 {
         // resident before the launch that writes these elements has ended
         float2 v;
         asm("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+        return v;
+    }
+    template <int I>
+    __device__ __forceinline__ Raw load_raw(const float2 *p, uint64_t policy) const {
+        float2 v;
+        asm("ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(policy));
         return v;
     }
     template <int I>
@@ -113,6 +120,7 @@ struct CodecF16 {
     const __half2 *__restrict__ rd;
     __half2 *__restrict__ wr;
     int px;  // row pitch
+    int l2_resident;
     float rho0;
     template <int I>
     __device__ __forceinline__ void store_row(__half2 *wrow, float r, float b) const {
@@ -149,6 +157,14 @@ struct CodecF16 {
         return h;
     }
     template <int I>
+    __device__ __forceinline__ Raw load_raw(const __half2 *p, uint64_t policy) const {
+        uint32_t u;
+        asm("ld.global.L2::cache_hint.L2::256B.b32 %0, [%1], %2;" : "=r"(u) : "l"(p), "l"(policy));
+        __half2 h;
+        memcpy(&h, &u, sizeof h);
+        return h;
+    }
+    template <int I>
     __device__ __forceinline__ float2 decode(Raw h, float &gi) const {
         const float2 v = __half22float2(h);
         const float gs = fmaf(Dir<I>::w, v.x, Dir<I>::w * rho0);
@@ -177,12 +193,13 @@ template <class C>
 __host__ __device__ C make_codec(const DeviceState &s, int cur);
 template <>
 __host__ __device__ CodecF32 make_codec<CodecF32>(const DeviceState &s, int cur) {
-    return CodecF32{static_cast<const float2 *>(s.pops[cur]), static_cast<float2 *>(s.pops[cur ^ 1]), s.g.px};
+    return CodecF32{static_cast<const float2 *>(s.pops[cur]), static_cast<float2 *>(s.pops[cur ^ 1]), s.g.px,
+                    s.l2_resident};
 }
 template <>
 __host__ __device__ CodecF16 make_codec<CodecF16>(const DeviceState &s, int cur) {
     return CodecF16{static_cast<const __half2 *>(s.pops[cur]), static_cast<__half2 *>(s.pops[cur ^ 1]), s.g.px,
-                    s.ph.f16_rho0};
+                    s.l2_resident, s.ph.f16_rho0};
 }
 
 // ------------------------------------------------------------------ helpers
@@ -468,12 +485,33 @@ struct DecodedPull {
         return codec.template decode<I>(codec.template load_raw<I>(pm.template ptr<I>(codec, x)), gi);
     }
 };
+// The same, of a buffer that fits L2: the pulled sectors, which the step reads
+// once, leave L2 before those that it writes, which the next step reads.
+// 64^3 19.9 -> 19.3 us, 97 x 75 x 131 float16 54.9 -> 52.8.  In larger grids the
+// sectors that neighbouring warps share would leave before they have met
+// (128x256x128 297 -> 304 us, float16 at 256x512x256 1221 -> 1283).
+template <class C, class Map>
+struct DecodedPullOnce {
+    const Map &pm;
+    const C &codec;
+    int x;
+    uint64_t first;
+    template <int I>
+    __device__ __forceinline__ float2 get(float &gi) const {
+        return codec.template decode<I>(codec.template load_raw<I>(pm.template ptr<I>(codec, x), first), gi);
+    }
+};
 template <class C, class Map>
 __device__ __forceinline__ void pull_densities_map(const Map &pm, const C &codec, int x, float &rr, float &rb) {
     densities_from(DecodedPull<C, Map>{pm, codec, x}, rr, rb);
 }
 template <class C, class Map>
 __device__ __forceinline__ NodeMoments pull_moments_map(const Map &pm, const C &codec, int x) {
+    if (codec.l2_resident) {
+        uint64_t first;
+        asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+        return moments_from(DecodedPullOnce<C, Map>{pm, codec, x, first});
+    }
     return moments_from(DecodedPull<C, Map>{pm, codec, x});
 }
 template <class C, bool kPeriodic>
@@ -648,12 +686,13 @@ __device__ __forceinline__ void radial_accumulate_warp(const DeviceState &s, int
         if (rb < unsigned(ph.NRB)) {
             key = (rb << 1) | (dx < 0.0f ? 1u : 0u);
             float ur = 0.0f;
-            if (r > 1.0e-12f) ur = (ux * dx + uz * dz) / r;
+            // rounded as written, whatever kernel this is part of
+            if (r > 1.0e-12f) ur = fmaf(ux, dx, __fmul_rn(uz, dz)) / r;
             v0 = uy;
-            v1 = uy * uy;
+            v1 = __fmul_rn(uy, uy);
             v2 = ur;
-            v3 = ur * ur;
-            v4 = ur * uy;
+            v3 = __fmul_rn(ur, ur);
+            v4 = __fmul_rn(ur, uy);
         }
     }
     if (__all_sync(kFull, key == 0xffffffffu)) return;

@@ -113,6 +113,22 @@ def test_back_to_back_steps_equal_waited_steps():
     np.testing.assert_array_equal(out[0][1], out[1][1])
 
 
+@pytest.mark.parametrize("storage,NY", [("f32", 64), ("f32", 150), ("f16", 64), ("f16", 300)])
+def test_pulls_of_buffers_that_fit_l2(monkeypatch, storage, NY):
+    """Buffers that fit L2 are pulled with a hint that larger ones are not:
+    either way the step is the march's bit for bit."""
+    case = derive(dict(NX=66, NY=NY, NZ=66, boundary="periodic", storage=storage, tau=0.6, sigma=0.01,
+                       NSTATS_START_STEP=10 ** 9))
+    monkeypatch.delenv("MCG_FUSED_PIPE", raising=False)
+    _, pops, fields, _ = _run(case, "drop", 4, False)
+    monkeypatch.setenv("MCG_FUSED_PIPE", "0")
+    _, mpops, mfields, _ = _run(case, "drop", 4, False)
+    for a, b in zip(pops, mpops):
+        np.testing.assert_array_equal(a, b)
+    for k in fields:
+        np.testing.assert_array_equal(fields[k], mfields[k], err_msg=k)
+
+
 @pytest.mark.parametrize("storage", ["f32", "f16"])
 @pytest.mark.parametrize("boundary", ["jet", "periodic"])
 def test_fields_in_chunks_equal_fields_at_once(storage, boundary):
