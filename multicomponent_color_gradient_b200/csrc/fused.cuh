@@ -319,6 +319,11 @@ __device__ __forceinline__ DeviceState pitch_state(const DeviceState &s) {
     }
     return l;
 }
+// Brings the parameters of a step into the constant cache while the launch before
+// runs (8^3 5.7 us a step without, 5.1 with, together with relax_flagged).
+__device__ __forceinline__ void touch_params(const DeviceState &s) {
+    asm volatile("" ::"f"(s.ph.omega), "r"(s.ph.sponge), "l"(s.piece_flags), "l"(s.tape));
+}
 template <class C, int kPX>
 __device__ __forceinline__ C pitch_codec(const DeviceState &s, int cur) {
     return fused_codec<C, kPX>(s, cur);
@@ -524,7 +529,7 @@ __global__ void __launch_bounds__(kFusedThreads, PipeBlocks<C>::value) k_fused_p
 // us a step, this against the marches chosen before (fraction of the measured
 // copy peak at 432 or 216 B a node): jet 128x256x128 float32 296 (0.90) against
 // 352 (0.76), 256x512x256 2264 (0.96) against 2984 (0.73), 200x301x183 769
-// (0.92) against 1541 (0.46), 64x128x64 39 against 76, 24x40x24 8-10 against 29;
+// (0.92) against 1541 (0.46), 64x128x64 39 against 76, 24x40x24 6.6 against 29;
 // float16 jet 128x400x128 258 (0.81) against 441, 256x512x256 1216 (0.89)
 // against 2073 (0.52).  With every node an interface node: 128x256x128 float32
 // 359 against 352, float16 324 against 365.
@@ -540,6 +545,14 @@ constexpr int kInterfaceThreads = 128, kInterfaceBlocks = 5;
 // rows of 128 columns (4 against 1: 174 against 196 us a step for the
 // 128x256x128 float16 jet, 2250 against 2328 for 256x512x256 float32).
 constexpr int kPieceGroup = 4;
+
+// CTAs up to which k_step_pull lets the next launch start only when it runs
+// itself: half of those that fit the chip, so that it and the next one fit
+// together.  Launches that each let the next one start at once go on to pile up,
+// waiting, several deep, and fill the SMs unevenly: 32x48x32 jet 8.6 us a step so
+// and 10.4 at once, float16 24x40x24 jet 7.9 and 11.2; from 48^3 on at once is
+// the faster (float16 128x256x128 jet 168.8 against 172.7).
+constexpr unsigned kSmallPulls = 148 * kSplitBlocks / 2;
 
 // Float16, whose kernels are bound by their instructions, parks and relaxes
 // quarters of 8 columns (32 bytes of a row): fewer bulk nodes go through the
@@ -597,8 +610,11 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitBlocks) k_step_pull(const
     // buffers are many times L2).
     const int y = 1 + row, zi = (step & 1) ? g.NZ - 3 - int(blockIdx.y) : int(blockIdx.y), z = 1 + zi;
     const float *psi = s_arg.psi[step & 1];
-    allow_next_launch();
+    const bool small = gridDim.x * gridDim.y <= kSmallPulls;
+    if (!small) allow_next_launch();
+    touch_params(s_arg);
     wait_for_previous_launch(codec, psi);
+    if (small) allow_next_launch();
     if (y > g.NY - 2) return;
     const int w = piece - row * ppr;
     const int x = w * 32 + int(threadIdx.x & 31);
@@ -626,6 +642,23 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitBlocks) k_step_pull(const
     }
 }
 
+// psi of the neighbours of interior node (x, y, z); a periodic box wraps.
+template <bool kPeriodic>
+struct PsiAround {
+    const float *psi;
+    int xs[3], ys[3], zs[3];
+    __device__ __forceinline__ PsiAround(const Geometry &g, const float *p, int x, int y, int z)
+        : psi(p),
+          xs{kPeriodic ? wrap_interior(x - 1, g.NX) : x - 1, x, kPeriodic ? wrap_interior(x + 1, g.NX) : x + 1},
+          ys{g.sy * (kPeriodic ? wrap_interior(y - 1, g.NY) : y - 1), g.sy * y,
+             g.sy * (kPeriodic ? wrap_interior(y + 1, g.NY) : y + 1)},
+          zs{g.sz * (kPeriodic ? wrap_interior(z - 1, g.NZ) : z - 1), g.sz * z,
+             g.sz * (kPeriodic ? wrap_interior(z + 1, g.NZ) : z + 1)} {}
+    __device__ __forceinline__ float operator()(int cx, int cy, int cz) const {
+        return psi[xs[cx + 1] + ys[cy + 1] + zs[cz + 1]];
+    }
+};
+
 // One piece of k_step_interface, or four quarters, one per 8 lanes: moments from
 // where k_step_pull parked them, psi of the neighbours, relaxation and stores.
 template <class C, bool kPeriodic>
@@ -639,20 +672,38 @@ __device__ __forceinline__ void relax_parked(const DeviceState &s, const C &code
     if (xst) unpark_moments(codec.wr + at + xn, g.px, m);
     __syncwarp();  // every lane has its moments before one of them stores over them
     if (!xst) return;
-    const int xs[3] = {kPeriodic ? wrap_interior(xn - 1, g.NX) : xn - 1, xn,
-                       kPeriodic ? wrap_interior(xn + 1, g.NX) : xn + 1};
-    const int ys[3] = {g.sy * (kPeriodic ? wrap_interior(y - 1, g.NY) : y - 1), g.sy * y,
-                       g.sy * (kPeriodic ? wrap_interior(y + 1, g.NY) : y + 1)};
-    const int zs[3] = {g.sz * (kPeriodic ? wrap_interior(z - 1, g.NZ) : z - 1), g.sz * z,
-                       g.sz * (kPeriodic ? wrap_interior(z + 1, g.NZ) : z + 1)};
-    auto psi_at = [&](int cx, int cy, int cz) { return psi[xs[cx + 1] + ys[cy + 1] + zs[cz + 1]]; };
+    const PsiAround<kPeriodic> psi_at(g, psi, xn, y, z);
     collide_node<false>(g, s.ph, codec, at, x, y, z, m, psi_at);
+}
+
+// The same for the piece that a warp of a small grid has to itself, which is bound
+// by latency: moments and psi are read while the flag is on the way, one round
+// trip to L2 in the place of three and no list (16x24x16 jet 5.5 us a step
+// against 6.4 with the list, 24x40x24 6.5 against 6.9).
+template <class C, bool kPeriodic>
+__device__ __forceinline__ void relax_flagged(const DeviceState &s, const C &codec, const float *psi,
+                                              const uint8_t *flag, int x, int y, int z) {
+    const Geometry &g = s.g;
+    const int xn = min(max(x, 1), g.NX - 2);
+    const size_t at = pop_row(g, y, z);
+    const unsigned f = *flag;
+    NodeMoments m;
+    unpark_moments(codec.wr + at + xn, g.px, m);
+    const PsiAround<kPeriodic> around(g, psi, xn, y, z);
+    float near[27];
+#pragma unroll
+    for (int k = 0; k < 27; ++k) near[k] = k == 13 ? 0.0f : around(k % 3 - 1, k / 3 % 3 - 1, k / 9 - 1);
+    auto psi_at = [&](int cx, int cy, int cz) { return near[cx + 1 + 3 * (cy + 1) + 9 * (cz + 1)]; };
+    __syncwarp();  // every lane has its moments before one of them stores over them
+    const bool on = relax_by_quarters<C>() ? (f >> (4 + (x >> 3 & 3))) & 1u : f & 1u;
+    if (on && x < store_columns<C>(g)) collide_node<false>(g, s.ph, codec, at, x, y, z, m, psi_at);
 }
 
 // Blocks [0, T.interface_ctas) relax what is flagged; each looks at every
 // interface_ctas-th group of neighbouring pieces, so that the pieces of one
 // interface, which lie together, go to different SMs, and its warps share what
-// it finds.  The blocks after them write the jet's inlet and outlet columns from
+// it finds.  Where every piece has a warp of its own, each warp takes its piece
+// (relax_flagged).  The blocks after them write the jet's inlet and outlet columns from
 // the fluid-plane moments in bmom.
 template <class C, bool kPeriodic, int kPX>
 __global__ void __launch_bounds__(kInterfaceThreads, kInterfaceBlocks) k_step_interface(const DeviceState s_arg,
@@ -666,12 +717,20 @@ __global__ void __launch_bounds__(kInterfaceThreads, kInterfaceBlocks) k_step_in
     C codec = pitch_codec<C, kPX>(s_arg, cur);
     const float *psi = s_arg.psi[step & 1];
     const int lane = int(threadIdx.x & 31), warp = int(threadIdx.x >> 5);
+    const uint32_t ctas = uint32_t(T.interface_ctas), ppr = uint32_t(pieces_per_row<C>(g));
+    const uint32_t pieces = ppr * uint32_t(g.NY - 2) * uint32_t(g.NZ - 2);
     allow_next_launch();
+    touch_params(s_arg);
+    const uint32_t own = blockIdx.x * (kInterfaceThreads / 32) + uint32_t(warp);
+    const uint32_t own_row = own / ppr, own_zi = own_row / uint32_t(g.NY - 2);
     wait_for_previous_launch(codec, psi);
-    const uint32_t ctas = uint32_t(T.interface_ctas);
+    if (blockIdx.x < ctas && pieces <= ctas * (kInterfaceThreads / 32)) {
+        if (own < pieces)
+            relax_flagged<C, kPeriodic>(s, codec, psi, s.piece_flags + own, int(own - own_row * ppr) * 32 + lane,
+                                        1 + int(own_row - own_zi * uint32_t(g.NY - 2)), 1 + int(own_zi));
+        return;
+    }
     if (blockIdx.x < ctas) {
-        const uint32_t ppr = uint32_t(pieces_per_row<C>(g));
-        const uint32_t pieces = ppr * uint32_t(g.NY - 2) * uint32_t(g.NZ - 2);
         for (uint32_t first = 0; first < pieces; first += ctas * kInterfaceThreads) {
             if (threadIdx.x == 0) found = 0;
             __syncthreads();

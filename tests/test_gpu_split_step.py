@@ -113,6 +113,25 @@ def test_back_to_back_steps_equal_waited_steps():
     np.testing.assert_array_equal(out[0][1], out[1][1])
 
 
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("boundary", ["jet", "periodic"])
+@pytest.mark.parametrize("NY,NZ", [(47, 46), (48, 49), (56, 54), (58, 56)])
+def test_small_grids_equal_march(monkeypatch, storage, boundary, NY, NZ):
+    """Rows of one piece around the sizes up to which k_step_pull holds back the
+    next launch (518 blocks of 4 pieces) and every piece has a warp of its own
+    in k_step_interface (2960 pieces)."""
+    case = derive(dict(NX=30, NY=NY, NZ=NZ, boundary=boundary, storage=storage, tau=0.6, sigma=0.01, jet_radius=6.0,
+                       inlet_noise=0.01, seed=3, NSTATS_START_STEP=10 ** 9))
+    monkeypatch.delenv("MCG_FUSED_PIPE", raising=False)
+    _, pops, fields, _ = _run(case, "drop", 9, False)
+    monkeypatch.setenv("MCG_FUSED_PIPE", "0")
+    _, mpops, mfields, _ = _run(case, "drop", 9, False)
+    for a, b in zip(pops, mpops):
+        np.testing.assert_array_equal(a, b)
+    for k in fields:
+        np.testing.assert_array_equal(fields[k], mfields[k], err_msg=k)
+
+
 @pytest.mark.parametrize("storage,NY", [("f32", 64), ("f32", 150), ("f16", 64), ("f16", 300)])
 def test_pulls_of_buffers_that_fit_l2(monkeypatch, storage, NY):
     """Buffers that fit L2 are pulled with a hint that larger ones are not:
