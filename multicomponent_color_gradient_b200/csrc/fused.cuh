@@ -546,14 +546,6 @@ constexpr int kInterfaceThreads = 128, kInterfaceBlocks = 5;
 // 128x256x128 float16 jet, 2250 against 2328 for 256x512x256 float32).
 constexpr int kPieceGroup = 4;
 
-// CTAs up to which k_step_pull lets the next launch start only when it runs
-// itself: half of those that fit the chip, so that it and the next one fit
-// together.  Launches that each let the next one start at once go on to pile up,
-// waiting, several deep, and fill the SMs unevenly: 32x48x32 jet 8.6 us a step so
-// and 10.4 at once, float16 24x40x24 jet 7.9 and 11.2; from 48^3 on at once is
-// the faster (float16 128x256x128 jet 168.8 against 172.7).
-constexpr unsigned kSmallPulls = 148 * kSplitBlocks / 2;
-
 // Float16, whose kernels are bound by their instructions, parks and relaxes
 // quarters of 8 columns (32 bytes of a row): fewer bulk nodes go through the
 // interface launch (64x128x64 jet 28.0 us a step against 31.6 by pieces, periodic
@@ -610,7 +602,7 @@ __global__ void __launch_bounds__(kSplitThreads, kSplitBlocks) k_step_pull(const
     // buffers are many times L2).
     const int y = 1 + row, zi = (step & 1) ? g.NZ - 3 - int(blockIdx.y) : int(blockIdx.y), z = 1 + zi;
     const float *psi = s_arg.psi[step & 1];
-    const bool small = gridDim.x * gridDim.y <= kSmallPulls;
+    const bool small = gridDim.x * gridDim.y <= kSmallLaunch;
     if (!small) allow_next_launch();
     touch_params(s_arg);
     wait_for_previous_launch(codec, psi);

@@ -934,8 +934,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjRelaxBlocks) k_adj_relax(cons
     __shared__ double sh[3 * (kAdjThreads / 32)];
     const Geometry &g = s.g;
     double a_omega = 0.0, a_Ah = 0.0, a_J = 0.0;
-    allow_next_launch();
-    wait_for_previous_launch();
+    wait_then_allow_if_small();
     if (int(blockIdx.x) < list_blocks) {
         for_flagged_pieces(g, flags, uint32_t(list_blocks), [&](int w, int y, int z) {
             const int x = w * 32 + int(threadIdx.x & 31);
@@ -989,8 +988,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjNearBlocks) k_adj_near(const 
                                                                              float *lam_out) {
     const Geometry &g = s.g;
     const size_t N = g.N;
-    allow_next_launch();
-    wait_for_previous_launch();
+    wait_then_allow_if_small();
     for_flagged_pieces(g, near_flags, gridDim.x, [&](int w, int y, int z) {
         const unsigned around = flags_around<kPeriodic>(g, flags, w, y, z);
         const int x = w * 32 + int(threadIdx.x & 31);
@@ -1111,8 +1109,7 @@ __global__ void __launch_bounds__(32) k_adj_boundary(const DeviceState s, int64_
     const Physics &ph = s.ph;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int z = blockIdx.y * blockDim.y + threadIdx.y;
-    allow_next_launch();
-    wait_for_previous_launch();
+    wait_then_allow_if_small();
     const bool col = x >= 1 && x <= g.NX - 2 && z >= 1 && z <= g.NZ - 2;
     const size_t N = g.N;
     const int NP = g.NX * g.NZ;
@@ -1323,8 +1320,7 @@ __global__ void __launch_bounds__(256) k_copy_outlet_state(const DeviceState s, 
 __global__ void __launch_bounds__(256) k_record_state(const DeviceState s, const float *psi, float *rec, float *outlet) {
     const Geometry &g = s.g;
     const uint32_t NP = uint32_t(g.NX) * uint32_t(g.NZ), stride = gridDim.x * 256;
-    allow_next_launch();
-    wait_for_previous_launch();
+    wait_then_allow_if_small();
     for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < g.N; i += stride) rec[size_t(kTapePsi) * g.N + i] = psi[i];
     for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < NP; i += stride) {
         const uint32_t z = i / uint32_t(g.NX), x = i - z * uint32_t(g.NX);

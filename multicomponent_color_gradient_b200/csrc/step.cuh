@@ -553,6 +553,23 @@ __device__ __forceinline__ void wait_for_previous_launch(C &codec, const float *
 }
 __device__ __forceinline__ void allow_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Blocks up to which a launch lets the next one start only when it runs itself:
+// half of the blocks of k_step_pull that fit the chip, so that it and the next
+// one fit together.  Launches that each let the next one start at once go on to
+// pile up, waiting, several deep, and fill the SMs unevenly (k_step_pull: 32x48x32
+// jet 8.6 us a step so and 10.4 at once, float16 24x40x24 jet 7.9 and 11.2; the
+// adjoint kernels: a 32x48x32 jet gradient 1500 us and 1605).  For larger ones at
+// once is the faster: the next launch's blocks fill the last wave (float16
+// 128x256x128 jet 168.8 us a step against 172.7).
+constexpr unsigned kSmallLaunch = 148 * 7 / 2;
+
+__device__ __forceinline__ void wait_then_allow_if_small() {
+    const bool small = gridDim.x * gridDim.y * gridDim.z <= kSmallLaunch;
+    if (!small) allow_next_launch();
+    wait_for_previous_launch();
+    if (small) allow_next_launch();
+}
+
 template <class... P, class... A>
 cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, const A &...args) {
     cudaLaunchAttribute overlap{};
