@@ -233,14 +233,34 @@ int fits_l2(const mcg_handle *h) {
 
 size_t piece_flag_bytes(const mcg_params &p) { return size_t(p.NY) * p.NZ * ((p.NX + 31) / 32); }
 
+// The device buffers that mcg_create allocates.
+void free_buffers(mcg_handle *h) {
+    mcg::DeviceState &s = h->s;
+    auto drop = [](auto *&q) {
+        if (q) cudaFree(q);
+        q = nullptr;
+    };
+    drop(s.pops[0]);
+    drop(s.pops[1]);
+    drop(s.mom);
+    drop(s.psi[0]);
+    drop(s.psi[1]);
+    drop(s.radial);
+    drop(s.bmom);
+    drop(s.piece_flags);
+    drop(s.uy_avg);
+    drop(s.partials);
+    drop(s.flag);
+    drop(h->d_scalar);
+}
+
 void release(mcg_handle *h) {
-    give_back_padding(h);
     mcg::async_release(h);
     mcg::io_close(h);
-    void *ptrs[] = {h->s.pops[0], h->s.pops[1], h->s.mom,      h->s.psi[0], h->s.psi[1], h->s.radial,
-                    h->s.uy_avg,  h->s.partials, h->s.piece_flags, h->s.flag, h->d_scalar, h->s.bmom,  h->d_inlet_profile, h->d_vti_text};
-    for (void *q : ptrs)
-        if (q) cudaFree(q);
+    free_buffers(h);
+    give_back_padding(h);
+    if (h->d_inlet_profile) cudaFree(h->d_inlet_profile);
+    if (h->d_vti_text) cudaFree(h->d_vti_text);
     if (h->h_vti_text) cudaFreeHost(h->h_vti_text);
     for (cudaEvent_t e : h->prof_events) cudaEventDestroy(e);
     if (h->ev0) cudaEventDestroy(h->ev0);
@@ -262,6 +282,29 @@ cudaError_t alloc_zero(T **ptr, size_t bytes) {
         return e;
     }
     return cudaMemset(*ptr, 0, bytes);
+}
+
+// The handle's device buffers for its row pitch, and the step's launch shape.
+cudaError_t alloc_buffers(mcg_handle *h) {
+    const mcg_params &p = h->p;
+    mcg::DeviceState &s = h->s;
+    const size_t N = s.g.N, M = size_t(p.NY) * (p.NX / 2), pb = pop_buffer_bytes(h);
+    cudaError_t e = alloc_zero(&s.pops[0], pb);
+    if (e == cudaSuccess) e = alloc_zero(&s.pops[1], pb);
+    if (e == cudaSuccess) e = alloc_zero(&s.mom, size_t(mcg::kMomCount) * N * 4);
+    if (e == cudaSuccess) e = alloc_zero(&s.psi[0], N * 4);
+    if (e == cudaSuccess) e = alloc_zero(&s.psi[1], N * 4);
+    if (e == cudaSuccess) e = alloc_zero(&s.radial, 5 * M * 8);
+    if (e == cudaSuccess) e = alloc_zero(&s.bmom, size_t(2) * p.NZ * mcg::kMomCount * p.NX * 4);
+    h->tiling = mcg::fused_tiling(s.g, kFusedSmemPerBlock);
+    if (e == cudaSuccess) e = mcg::fused_configure(s.g, h->tiling);
+    if (e == cudaSuccess) e = alloc_zero(&s.piece_flags, piece_flag_bytes(p));
+    if (e == cudaSuccess) e = alloc_zero(&s.uy_avg, N * 4);
+    s.partials_cap = mcg::conservation_blocks(s.g);
+    if (e == cudaSuccess) e = alloc_zero(&s.partials, size_t(s.partials_cap) * 5 * 8);
+    if (e == cudaSuccess) e = alloc_zero(&s.flag, sizeof(int) * 4);
+    if (e == cudaSuccess) e = alloc_zero(&h->d_scalar, 8 * sizeof(double));
+    return e;
 }
 
 mcg_status check_handle(const mcg_handle *h) {
@@ -457,25 +500,15 @@ mcg_status mcg_create(const mcg_params *p, mcg_handle **out) {
         h->s.l2_resident = fits_l2(h);
         fill_physics(h);
         compute_ncols(h);
-        const size_t N = g.N;
-        const size_t M = size_t(p->NY) * (p->NX / 2);
-        cudaError_t e = cudaSuccess;
-        const size_t pb = pop_buffer_bytes(h);
-        if (e == cudaSuccess) e = alloc_zero(&h->s.pops[0], pb);
-        if (e == cudaSuccess) e = alloc_zero(&h->s.pops[1], pb);
-        if (e == cudaSuccess) e = alloc_zero(&h->s.mom, size_t(mcg::kMomCount) * N * 4);
-        if (e == cudaSuccess) e = alloc_zero(&h->s.psi[0], N * 4);
-        if (e == cudaSuccess) e = alloc_zero(&h->s.psi[1], N * 4);
-        if (e == cudaSuccess) e = alloc_zero(&h->s.radial, 5 * M * 8);
-        if (e == cudaSuccess) e = alloc_zero(&h->s.bmom, size_t(2) * p->NZ * mcg::kMomCount * p->NX * 4);
-        h->tiling = mcg::fused_tiling(g, kFusedSmemPerBlock);
-        if (e == cudaSuccess) e = mcg::fused_configure(g, h->tiling);
-        if (e == cudaSuccess) e = alloc_zero(&h->s.piece_flags, piece_flag_bytes(*p));
-        if (e == cudaSuccess) e = alloc_zero(&h->s.uy_avg, N * 4);
-        h->s.partials_cap = mcg::conservation_blocks(g);
-        if (e == cudaSuccess) e = alloc_zero(&h->s.partials, size_t(h->s.partials_cap) * 5 * 8);
-        if (e == cudaSuccess) e = alloc_zero(&h->s.flag, sizeof(int) * 4);
-        if (e == cudaSuccess) e = alloc_zero(&h->d_scalar, 8 * sizeof(double));
+        cudaError_t e = alloc_buffers(h);
+        if (e == cudaErrorMemoryAllocation && g.px != p->NX) {
+            // no room for padded rows: the rows as they are
+            (void)cudaGetLastError();
+            free_buffers(h);
+            give_back_padding(h);
+            g.px = p->NX;
+            e = alloc_buffers(h);
+        }
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreate(&h->ev0);
         if (e == cudaSuccess) e = cudaEventCreate(&h->ev1);
