@@ -27,6 +27,9 @@ mcg_status fail(mcg_status s, const std::string &msg) {
 }
 
 mcg_status cuda_fail(cudaError_t e, const char *what) {
+    // reported here: a later launch that asks for the last error does not get it
+    // again (errors that end the context stay)
+    (void)cudaGetLastError();
     g_last_error = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
     return e == cudaErrorMemoryAllocation ? MCG_ERR_OOM : MCG_ERR_CUDA;
 }

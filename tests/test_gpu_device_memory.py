@@ -69,3 +69,14 @@ def test_create_without_room_for_padded_rows():
     # the padding it did without is there for the next handle
     with Solver(case) as S:
         assert device_bytes(S) == padded
+
+
+def test_out_of_memory_does_not_reach_the_next_call():
+    """A call that found no memory leaves nothing behind that a later launch
+    would report as its own failure."""
+    with only_free(64 * MB):
+        with pytest.raises(_lib.McgError) as err:
+            Solver(derive(CASE))
+        assert err.value.status == 2  # MCG_ERR_OOM
+        with Solver(derive(dict(CASE, NX=24, NY=20, NZ=20, bubble_radius=5.0))) as S:
+            walk(S)
