@@ -421,7 +421,7 @@ static mcg_status bubble_adjoint(mcg_handle *h, const float *psi_target, int32_t
                                  double *dJ_dsigma, double *dJ_dtau, float *dJ_du0, int64_t *forward_steps,
                                  float *ms) {
     return mcg::guarded([&]() -> mcg_status {
-        if (!h) return fail(MCG_ERR_INVALID_ARG, "handle is null");
+        if (mcg_status s = mcg::check_handle(h)) return s;
         if (!psi_target) return fail(MCG_ERR_INVALID_ARG, "psi_target is null");
         if (nsteps < 1) return fail(MCG_ERR_INVALID_ARG, "nsteps must be >= 1");
         if (snapshots < 1) return fail(MCG_ERR_INVALID_ARG, "snapshots must be >= 1");
@@ -576,7 +576,7 @@ struct JetObjective {
 
 mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t_end, int32_t segment,
                        const JetObjective &objective, double *J, double *dJ_dc, int64_t *forward_steps, float *ms) {
-    if (!h) return fail(MCG_ERR_INVALID_ARG, "handle is null");
+    if (mcg_status st = mcg::check_handle(h)) return st;
     if (nsteps < 1) return fail(MCG_ERR_INVALID_ARG, "nsteps must be >= 1");
     if (t_begin < 0 || t_end < t_begin || t_end >= nsteps)
         return fail(MCG_ERR_INVALID_ARG, "need 0 <= t_begin <= t_end < nsteps");

@@ -45,6 +45,13 @@ void radial_counts_for(const mcg_handle *h, uint32_t samples, uint64_t *count) {
 
 void radial_counts(const mcg_handle *h, uint64_t *count) { radial_counts_for(h, h->stats_samples, count); }
 
+mcg_status check_handle(const mcg_handle *h) {
+    if (!h) return fail(MCG_ERR_INVALID_ARG, "handle is null");
+    if (!h->s.pops[0] || !h->s.pops[1])
+        return fail(MCG_ERR_STATE, "the handle lost its population buffers when device memory ran out");
+    return MCG_OK;
+}
+
 cudaError_t device_malloc(void **p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation) return e;
@@ -310,10 +317,7 @@ cudaError_t alloc_buffers(mcg_handle *h) {
     return e;
 }
 
-mcg_status check_handle(const mcg_handle *h) {
-    if (!h) return fail(MCG_ERR_INVALID_ARG, "handle is null");
-    return MCG_OK;
-}
+using mcg::check_handle;
 
 // Automatic start of the radial statistics (meanF/meanFieldsRT.cuh:173-190).
 bool stats_for_step(mcg_handle *h) {
@@ -385,19 +389,40 @@ mcg_status ensure_moments(mcg_handle *h) {
 }  // namespace
 
 namespace mcg {
-// Takes the padding out of the rows of both population buffers (their memory
-// stays), for a call that finds no room for buffers of padded rows.
+// Takes the padding out of the rows of both population buffers and gives its
+// memory back, for a call that finds no room beside padded rows.
 mcg_status unpad_rows(mcg_handle *h) {
     if (mcg_status s = ensure_moments(h)) return s;  // the spare buffer holds the last step's input
     MCG_LAUNCH(h, launch_unpad_rows(h->s, h->cur, h->stream), "unpad rows");
-    h->s.g.px = h->p.NX;
-    MCG_CUDA(cudaMemcpyAsync(h->s.pops[h->cur], h->s.pops[h->cur ^ 1], pop_buffer_bytes(h), cudaMemcpyDeviceToDevice,
-                             h->stream),
-             "unpad rows");
     MCG_CUDA(cudaStreamSynchronize(h->stream), "unpad rows");
+    h->cur ^= 1;  // the spare buffer holds the state in plain rows
+    h->s.g.px = h->p.NX;
+    const size_t bytes = pop_buffer_bytes(h);
+    // each buffer in turn makes way for a smaller one with a copy of the state
+    // (ghost-plane slots have to hold the same in both)
+    for (int k = 0; k < 2; ++k) {
+        void *&spare = h->s.pops[h->cur ^ 1];
+        cudaFree(spare);
+        spare = nullptr;
+        if (cudaError_t e = device_malloc(&spare, bytes); e != cudaSuccess) {
+            spare = nullptr;  // check_handle refuses the handle from here on
+            return cuda_fail(e, "unpad rows");
+        }
+        MCG_CUDA(cudaMemcpyAsync(spare, h->s.pops[h->cur], bytes, cudaMemcpyDeviceToDevice, h->stream), "unpad rows");
+        MCG_CUDA(cudaStreamSynchronize(h->stream), "unpad rows");
+        h->cur ^= 1;
+    }
+    give_back_padding(h);
     h->tiling = fused_tiling(h->s.g, kFusedSmemPerBlock);
     MCG_CUDA(fused_configure(h->s.g, h->tiling), "unpad rows");
     return MCG_OK;
+}
+
+cudaError_t device_malloc(mcg_handle *h, void **p, size_t bytes) {
+    cudaError_t e = device_malloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation || h->s.g.px == h->p.NX) return e;
+    (void)cudaGetLastError();
+    return unpad_rows(h) == MCG_OK ? device_malloc(p, bytes) : e;
 }
 }  // namespace mcg
 
@@ -694,7 +719,7 @@ mcg_status mcg_set_inlet_bessel(mcg_handle *h, const float *coeffs, int32_t n) {
                 prof[size_t(z) * NX + x] = float(m);
             }
         if (!h->d_inlet_profile)
-            MCG_CUDA(mcg::device_malloc(reinterpret_cast<void **>(&h->d_inlet_profile), prof.size() * sizeof(float)),
+            MCG_CUDA(mcg::device_malloc(h, reinterpret_cast<void **>(&h->d_inlet_profile), prof.size() * sizeof(float)),
                      "inlet profile allocation");
         MCG_CUDA(cudaMemcpyAsync(h->d_inlet_profile, prof.data(), prof.size() * sizeof(float), cudaMemcpyHostToDevice,
                                  h->stream),

@@ -91,6 +91,8 @@ mcg_status guarded(F &&body) noexcept {
     }
 }
 mcg_status cuda_fail(cudaError_t e, const char *what);
+// Whether h can be worked on.
+mcg_status check_handle(const mcg_handle *h);
 
 // Radial count materialisation: samples * ncols[rb] on interior y rows.
 void radial_counts(const mcg_handle *h, uint64_t *count);
@@ -107,6 +109,9 @@ void workspace_release(int device) noexcept;
 size_t device_bytes(int device);
 // cudaMalloc that first gives that memory back where it is in the way.
 cudaError_t device_malloc(void **p, size_t bytes);
+// The same for a buffer that h needs, which if need be takes the place of the
+// padding of h's rows.
+cudaError_t device_malloc(mcg_handle *h, void **p, size_t bytes);
 
 // io.cpp
 mcg_status io_open(mcg_handle *h, const char *root);

@@ -154,7 +154,7 @@ mcg_status io_write_radial_host(mcg_handle *h, const StatsSnapshot &st, const do
 mcg_status io_write_vti(mcg_handle *h, const std::string &path) {
     const VtiText L = vti_text_layout(uint64_t(h->s.g.N));
     cudaError_t e = cudaSuccess;
-    if (!h->d_vti_text) e = device_malloc(reinterpret_cast<void **>(&h->d_vti_text), L.total);
+    if (!h->d_vti_text) e = device_malloc(h, reinterpret_cast<void **>(&h->d_vti_text), L.total);
     if (e == cudaSuccess && !h->h_vti_text) e = cudaMallocHost(&h->h_vti_text, L.total);
     if (e == cudaSuccess) {
         e = launch_vti_encode(h->s, h->d_vti_text, h->stream);

@@ -92,11 +92,11 @@ mcg_status create_async(mcg_handle *h) {
     const bool vti = h->p.write_vti_output != 0;
     cudaError_t e = cudaStreamCreateWithFlags(&a->io, cudaStreamNonBlocking);
     for (int k = 0; k < AsyncOutput::kSlots && e == cudaSuccess; ++k) {
-        if (vti) e = device_malloc(reinterpret_cast<void **>(&a->d_text[k]), T);
+        if (vti) e = device_malloc(h, reinterpret_cast<void **>(&a->d_text[k]), T);
         if (e == cudaSuccess && vti) e = cudaMallocHost(&a->h_text[k], T);
-        if (e == cudaSuccess) e = device_malloc(reinterpret_cast<void **>(&a->d_radial[k]), 5 * M * sizeof(double));
+        if (e == cudaSuccess) e = device_malloc(h, reinterpret_cast<void **>(&a->d_radial[k]), 5 * M * sizeof(double));
         if (e == cudaSuccess) e = cudaMallocHost(&a->h_radial[k], 5 * M * sizeof(double));
-        if (e == cudaSuccess) e = device_malloc(reinterpret_cast<void **>(&a->d_tke[k]), sizeof(double));
+        if (e == cudaSuccess) e = device_malloc(h, reinterpret_cast<void **>(&a->d_tke[k]), sizeof(double));
         if (e == cudaSuccess) e = cudaMallocHost(&a->h_tke[k], sizeof(double));
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a->staged[k], cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&a->ready[k], cudaEventDisableTiming);
