@@ -37,7 +37,6 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <vector>
 
@@ -126,78 +125,66 @@ int64_t forward_steps_of(const std::vector<Action> &acts) {
         ++(h)->launches;                                     \
     } while (0)
 
-// Device memory of one adjoint run.  Allocating and freeing a run's gigabytes
-// took longer than the run (2 GB in 17 blocks: 10-56 ms and 9-1000 ms), so the
-// blocks of the last run on a device are kept for the next one, up to 1/16 of
-// the device's memory, while any handle lives (workspace_release).  A run takes
-// the kept blocks out, so runs of several threads never share one, and returns
-// its own after its stream has finished with them.  Blocks come with whatever
-// they hold; a buffer that has to start at zero is cleared.
-struct Block {
-    void *p;
-    size_t bytes;
-};
-std::mutex g_kept_mutex;
-std::map<int, std::vector<Block>> g_kept;  // by device
+// Device memory of one adjoint run, from a pool that the handles of a device
+// share.  Allocating and freeing a run's gigabytes took longer than the run
+// (2.9 GB in 17 blocks: cudaMalloc 10-86 ms, cudaFree 10-34 ms), so the pool
+// keeps up to 1/16 of the device's memory between runs, while a handle lives
+// (0.05 ms).  What it keeps without using it the driver takes back for any
+// allocation of the process that finds no other room.  Blocks come with
+// whatever they hold; a buffer that has to start at zero is cleared.
+cudaError_t adjoint_pool(mcg::DeviceShare &share, int device, cudaMemPool_t *pool) {
+    std::lock_guard<std::mutex> lock(share.m);
+    if (!share.pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t made = nullptr;
+        uint64_t keep = share.bytes / 16;
+        cudaError_t e = cudaMemPoolCreate(&made, &props);
+        if (e == cudaSuccess && (e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess)
+            cudaMemPoolDestroy(made);
+        if (e != cudaSuccess) return e;
+        share.pool = made;
+    }
+    *pool = share.pool;
+    return cudaSuccess;
+}
 
 struct DeviceBuffers {
+    mcg_handle *h;
     cudaStream_t stream;  // the run's stream
-    int device = 0;
-    std::vector<Block> used, spare;
+    cudaMemPool_t pool = nullptr;
+    std::vector<void *> used;
     size_t total = 0, limit = SIZE_MAX;  // bytes in use, and the most a run may take (tests)
-    explicit DeviceBuffers(cudaStream_t st) : stream(st) {
+    explicit DeviceBuffers(mcg_handle *handle) : h(handle), stream(handle->stream) {
         if (const char *v = std::getenv("MCG_ADJOINT_MEMORY_MB")) limit = size_t(std::atoll(v)) << 20;
-        cudaGetDevice(&device);
-        std::lock_guard<std::mutex> lock(g_kept_mutex);
-        spare.swap(g_kept[device]);
     }
     ~DeviceBuffers() {
-        if (!used.empty()) cudaStreamSynchronize(stream);
-        drop_spare();
-        if (total <= mcg::device_bytes(device) / 16) {
-            std::lock_guard<std::mutex> lock(g_kept_mutex);
-            if (g_kept[device].empty()) {
-                g_kept[device].swap(used);
-                return;
-            }
-        }
-        for (const Block &b : used) cudaFree(b.p);
+        if (used.empty()) return;
+        for (void *p : used) cudaFreeAsync(p, stream);
+        cudaStreamSynchronize(stream);  // the pool gives back what it does not keep
     }
-    void drop_spare() {
-        for (const Block &b : spare) cudaFree(b.p);
-        spare.clear();
-    }
+    // Bytes that the pool holds without using them.
     size_t spare_bytes() const {
-        size_t s = 0;
-        for (const Block &b : spare) s += b.bytes;
-        return s;
+        uint64_t held = 0, in_use = 0;
+        if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &in_use) != cudaSuccess)
+            return 0;
+        return held > in_use ? size_t(held - in_use) : 0;
     }
     cudaError_t alloc(void **p, size_t bytes, bool zero = false) {
         *p = nullptr;
         if (total + bytes > limit) return cudaErrorMemoryAllocation;
-        size_t best = spare.size();
-        for (size_t k = 0; k < spare.size(); ++k)
-            if (spare[k].bytes >= bytes && spare[k].bytes <= bytes + bytes / 4 + 4096 &&
-                (best == spare.size() || spare[k].bytes < spare[best].bytes))
-                best = k;
+        if (!pool)
+            if (cudaError_t e = adjoint_pool(*h->share, h->device, &pool); e != cudaSuccess) return e;
         used.reserve(used.size() + 1);
-        if (best < spare.size()) {
-            used.push_back(spare[best]);
-            spare.erase(spare.begin() + long(best));
-        } else {
-            void *q = nullptr;
-            cudaError_t e = cudaMalloc(&q, bytes);
-            if (e == cudaErrorMemoryAllocation && !spare.empty()) {
-                cudaGetLastError();
-                drop_spare();
-                e = cudaMalloc(&q, bytes);
-            }
-            if (e != cudaSuccess) return e;
-            used.push_back({q, bytes});
-        }
-        total += used.back().bytes;
-        *p = used.back().p;
-        return zero ? cudaMemsetAsync(*p, 0, bytes, stream) : cudaSuccess;
+        void *q = nullptr;
+        if (cudaError_t e = cudaMallocFromPoolAsync(&q, bytes, pool, stream); e != cudaSuccess) return e;
+        used.push_back(q);
+        total += bytes;
+        *p = q;
+        return zero ? cudaMemsetAsync(q, 0, bytes, stream) : cudaSuccess;
     }
 };
 
@@ -347,29 +334,12 @@ struct Run {
 
 }  // namespace
 
-namespace mcg {
-void workspace_release(int device) noexcept {
-    std::vector<Block> blocks;
-    {
-        std::lock_guard<std::mutex> lock(g_kept_mutex);
-        blocks.swap(g_kept[device]);
-    }
-    int current = 0;
-    cudaGetDevice(&current);
-    if (current != device) cudaSetDevice(device);
-    for (const Block &b : blocks) cudaFree(b.p);
-    if (current != device) cudaSetDevice(current);
-}
-}  // namespace mcg
-
 namespace {
 // A run that finds no room for buffers of padded rows runs with unpadded ones.
 template <class F>
 mcg_status with_rows_that_fit(mcg_handle *h, F &&run) {
     const mcg_status st = run();
     if (st != MCG_ERR_OOM || !h || h->s.g.px == h->p.NX) return st;
-    cudaGetLastError();
-    mcg::workspace_release(h->device);
     if (mcg_status u = mcg::unpad_rows(h)) return u;
     return run();
 }
@@ -441,7 +411,7 @@ static mcg_status bubble_adjoint(mcg_handle *h, const float *psi_target, int32_t
         bool any_taped = false;
         for (const Action &a : acts) any_taped = any_taped || (a.kind == Action::kTaped && a.n > 1);
 
-        DeviceBuffers buf(h->stream);
+        DeviceBuffers buf(h);
         Run run;
         run.h = h;
         run.base = h->s;
@@ -596,7 +566,7 @@ mcg_status jet_adjoint(mcg_handle *h, int32_t nsteps, int32_t t_begin, int32_t t
     const int nb = mcg::kInletBesselMax;
     const bool profile = objective.kind == 1;
 
-    DeviceBuffers buf(h->stream);
+    DeviceBuffers buf(h);
     void *p = nullptr;
     mcg::DeviceState run = h->s;
     void *work[2];

@@ -52,37 +52,23 @@ mcg_status check_handle(const mcg_handle *h) {
     return MCG_OK;
 }
 
-cudaError_t device_malloc(void **p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaErrorMemoryAllocation) return e;
-    cudaGetLastError();
-    int device = 0;
-    cudaGetDevice(&device);
-    workspace_release(device);
-    return cudaMalloc(p, bytes);
-}
-
-size_t device_bytes(int device) {
+// The share of the current device, `device`.
+static std::shared_ptr<DeviceShare> device_share(int device) {
     static std::mutex m;
-    static std::map<int, size_t> known;
+    static std::map<int, std::weak_ptr<DeviceShare>> known;
     std::lock_guard<std::mutex> lock(m);
-    size_t &b = known[device];
-    size_t free_b = 0;
-    if (b == 0 && cudaMemGetInfo(&free_b, &b) != cudaSuccess) b = 0;
-    return b;
-}
-
-namespace {
-std::mutex g_live_mutex;
-std::map<int, int> g_live;  // handles by device
-}
-static void handle_born(int device) {
-    std::lock_guard<std::mutex> lock(g_live_mutex);
-    ++g_live[device];
-}
-static void handle_gone(int device) {
-    std::lock_guard<std::mutex> lock(g_live_mutex);
-    if (--g_live[device] == 0) workspace_release(device);
+    std::weak_ptr<DeviceShare> &k = known[device];
+    std::shared_ptr<DeviceShare> s = k.lock();
+    if (!s) {
+        s = std::make_shared<DeviceShare>();
+        size_t free_b = 0;
+        if (cudaMemGetInfo(&free_b, &s->bytes) != cudaSuccess) {
+            (void)cudaGetLastError();
+            s->bytes = 0;
+        }
+        k = s;
+    }
+    return s;
 }
 
 StatsSnapshot stats_snapshot(const mcg_handle *h) {
@@ -208,24 +194,21 @@ size_t pop_buffer_bytes(const mcg_handle *h) { return pop_buffer_bytes(h->p, h->
 // sectors of 64 bytes already (200x301x183: 761 without, 782 with), nor where it
 // would cost more than a third more memory, nor beyond 1/128 of the device's
 // memory for all handles together.
-std::mutex g_pad_mutex;
-std::map<int, size_t> g_pad;  // bytes of padding in use, by device
-int row_pitch(const mcg_params &p, int device, size_t *padding) {
+int row_pitch(const mcg_params &p, mcg::DeviceShare &share, size_t *padding) {
     *padding = 0;
     const int px = (p.NX + 31) / 32 * 32;
     if (px == p.NX || 3 * px > 4 * p.NX || std::getenv("MCG_FUSED_FIXED_NX")) return p.NX;
     if (p.storage == MCG_STORAGE_F32 && p.NX % 8 == 0 && p.NX >= 64) return p.NX;
     const size_t extra = 2 * (pop_buffer_bytes(p, px) - pop_buffer_bytes(p, p.NX));
-    const size_t most = mcg::device_bytes(device) / 128;
-    std::lock_guard<std::mutex> lock(g_pad_mutex);
-    if (g_pad[device] + extra > most) return p.NX;
-    g_pad[device] += extra;
+    std::lock_guard<std::mutex> lock(share.m);
+    if (share.padding + extra > share.bytes / 128) return p.NX;
+    share.padding += extra;
     *padding = extra;
     return px;
 }
 void give_back_padding(mcg_handle *h) {
-    std::lock_guard<std::mutex> lock(g_pad_mutex);
-    g_pad[h->device] -= h->padding;
+    std::lock_guard<std::mutex> lock(h->share->m);
+    h->share->padding -= h->padding;
     h->padding = 0;
 }
 
@@ -286,7 +269,7 @@ void release(mcg_handle *h) {
 
 template <class T>
 cudaError_t alloc_zero(T **ptr, size_t bytes) {
-    cudaError_t e = mcg::device_malloc(reinterpret_cast<void **>(ptr), bytes);
+    cudaError_t e = cudaMalloc(reinterpret_cast<void **>(ptr), bytes);
     if (e != cudaSuccess) {
         *ptr = nullptr;
         return e;
@@ -404,7 +387,7 @@ mcg_status unpad_rows(mcg_handle *h) {
         void *&spare = h->s.pops[h->cur ^ 1];
         cudaFree(spare);
         spare = nullptr;
-        if (cudaError_t e = device_malloc(&spare, bytes); e != cudaSuccess) {
+        if (cudaError_t e = cudaMalloc(&spare, bytes); e != cudaSuccess) {
             spare = nullptr;  // check_handle refuses the handle from here on
             return cuda_fail(e, "unpad rows");
         }
@@ -419,10 +402,10 @@ mcg_status unpad_rows(mcg_handle *h) {
 }
 
 cudaError_t device_malloc(mcg_handle *h, void **p, size_t bytes) {
-    cudaError_t e = device_malloc(p, bytes);
+    cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation || h->s.g.px == h->p.NX) return e;
     (void)cudaGetLastError();
-    return unpad_rows(h) == MCG_OK ? device_malloc(p, bytes) : e;
+    return unpad_rows(h) == MCG_OK ? cudaMalloc(p, bytes) : e;
 }
 }  // namespace mcg
 
@@ -524,7 +507,8 @@ mcg_status mcg_create(const mcg_params *p, mcg_handle **out) {
         g.boundary = p->boundary;
         g.storage = p->storage;
         g.slots = mcg::kQ;  // one element (both colours) per direction: float2 or half2
-        g.px = row_pitch(*p, h->device, &h->padding);
+        h->share = mcg::device_share(h->device);
+        g.px = row_pitch(*p, *h->share, &h->padding);
         h->s.l2_resident = fits_l2(h);
         fill_physics(h);
         compute_ncols(h);
@@ -553,7 +537,6 @@ mcg_status mcg_create(const mcg_params *p, mcg_handle **out) {
             delete h;
             return s;
         }
-        mcg::handle_born(h->device);
         h->stream = h->own_stream;
         *out = h;
         return MCG_OK;
@@ -564,10 +547,8 @@ mcg_status mcg_destroy(mcg_handle *h) {
     return mcg::guarded([&]() -> mcg_status {
         if (!h) return MCG_OK;
         cudaStreamSynchronize(h->stream);
-        const int device = h->device;
         release(h);
         delete h;
-        mcg::handle_gone(device);
         return MCG_OK;
     });
 }

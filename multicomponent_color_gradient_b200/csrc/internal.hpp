@@ -6,6 +6,8 @@
 #include <cstdint>
 #include <cstdio>
 #include <exception>
+#include <memory>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -22,12 +24,24 @@ struct StatsSnapshot {
     uint32_t samples = 0;
 };
 struct AsyncOutput;  // output_async.cpp
+
+// What the handles of one device share, while one of them lives.
+struct DeviceShare {
+    size_t bytes = 0;  // memory of the device
+    std::mutex m;      // guards what follows
+    size_t padding = 0;            // bytes that pad population rows
+    cudaMemPool_t pool = nullptr;  // of the adjoint runs (adjoint.cu), made by the first
+    ~DeviceShare() {
+        if (pool) cudaMemPoolDestroy(pool);
+    }
+};
 }  // namespace mcg
 
 struct mcg_handle {
     mcg_params p{};
     mcg::DeviceState s{};
     int device = 0;
+    std::shared_ptr<mcg::DeviceShare> share;
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
     int cur = 0;            // pops[cur] holds f(t) in pull layout
@@ -103,13 +117,7 @@ StatsSnapshot stats_snapshot(const mcg_handle *h);
 void tke_update(mcg_handle *h, int32_t step, double total);
 
 mcg_status unpad_rows(mcg_handle *h);  // api.cu
-// adjoint.cu: frees the device memory kept between adjoint runs on `device`.
-void workspace_release(int device) noexcept;
-// Memory of the current device, `device` (0 if unknown).
-size_t device_bytes(int device);
-// cudaMalloc that first gives that memory back where it is in the way.
-cudaError_t device_malloc(void **p, size_t bytes);
-// The same for a buffer that h needs, which if need be takes the place of the
+// cudaMalloc of a buffer that h needs, which if need be takes the place of the
 // padding of h's rows.
 cudaError_t device_malloc(mcg_handle *h, void **p, size_t bytes);
 

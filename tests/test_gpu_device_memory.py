@@ -140,3 +140,20 @@ def test_adjoint_in_the_room_of_the_padding(monkeypatch):
         assert_same_gradient(got, want)
         S.step(1)
         assert_same(S.get_fields(), fields)
+
+
+def test_memory_kept_between_adjoint_runs_is_there_for_others():
+    """What the library keeps between adjoint runs does not stand in the way of
+    an allocation beside it, and the next run does without it."""
+    import torch
+
+    case, target = adjoint_case()
+    with Solver(case) as S:
+        S.init_bubble()
+        torch.cuda.empty_cache()
+        before = torch.cuda.mem_get_info()[0]
+        want = S.adjoint_run(target, 3, 2, tape=2)
+        kept = before - torch.cuda.mem_get_info()[0]
+        with only_free(-kept // 2):
+            pass
+        assert_same_gradient(S.adjoint_run(target, 3, 2, tape=2), want)
