@@ -1,0 +1,39 @@
+// context.cpp - which CUDA context device memory belongs to.
+//
+// A cudaDeviceReset destroys a device's context with all its memory and modules;
+// the next call makes a new one, which the driver hands out under the same
+// pointer.  What tells the two apart is cuCtxGetId, unique for the life of the
+// process.  The driver's functions come from the runtime's entry point table, as
+// the library does not link libcuda, so that it loads on machines without a GPU.
+#include "internal.hpp"
+
+namespace mcg {
+namespace {
+
+using Context = void *;
+template <class F>
+F driver_entry(const char *name) {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    return reinterpret_cast<F>(f);
+}
+
+uint64_t id_of(Context ctx) {
+    static const auto get_id = driver_entry<int (*)(Context, unsigned long long *)>("cuCtxGetId");
+    unsigned long long id = 0;
+    return ctx && get_id && get_id(ctx, &id) == 0 ? uint64_t(id) : 0;
+}
+
+}  // namespace
+
+uint64_t current_context_id() {
+    static const auto get_current = driver_entry<int (*)(Context *)>("cuCtxGetCurrent");
+    Context ctx = nullptr;
+    return get_current && get_current(&ctx) == 0 ? id_of(ctx) : 0;
+}
+
+}  // namespace mcg

@@ -117,6 +117,8 @@ StatsSnapshot stats_snapshot(const mcg_handle *h);
 void tke_update(mcg_handle *h, int32_t step, double total);
 
 mcg_status unpad_rows(mcg_handle *h);  // api.cu
+// Id of the calling thread's CUDA context, 0 where there is none (context.cpp).
+uint64_t current_context_id();
 // cudaMalloc of a buffer that h needs, which if need be takes the place of the
 // padding of h's rows.
 cudaError_t device_malloc(mcg_handle *h, void **p, size_t bytes);

@@ -87,40 +87,17 @@ __global__ void __launch_bounds__(kThreads) k_fold_planes(const double *partials
 
 std::mutex g_setup_mutex;
 struct ScratchAddr {
-    void *ctx = nullptr;  // the context the address belongs to
+    uint64_t ctx = 0;  // the context the address belongs to (current_context_id)
     double *ptr = nullptr;
 };
 ScratchAddr g_partials_addr[kMaxDevices];
-
-// cuCtxGetCurrent through the runtime's driver entry point table (the library
-// does not link libcuda itself, so that it loads on machines without a GPU).
-using CtxGetCurrent = int (*)(void **);
-CtxGetCurrent ctx_get_current() {
-    static CtxGetCurrent fn = [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess) {
-            cudaGetLastError();
-            return CtxGetCurrent(nullptr);
-        }
-        return reinterpret_cast<CtxGetCurrent>(f);
-    }();
-    return fn;
-}
-
-void *current_context() {
-    void *ctx = nullptr;
-    if (CtxGetCurrent f = ctx_get_current()) f(&ctx);
-    return ctx;
-}
 
 // Device address of g_static_partials on the current device.  The host-side
 // name is only a stand-in for the symbol; the address comes from
 // cudaGetSymbolAddress with that device current, once per device and
 // context: a cudaDeviceReset tears the context and its module down, and the
 // next context may load the array elsewhere, so a change of the current
-// context looks the address up again.
+// context's id (its pointer stays the same) looks the address up again.
 mcg_status scratch_on_current_device(double **out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -128,7 +105,7 @@ mcg_status scratch_on_current_device(double **out) {
     if (dev < 0 || dev >= kMaxDevices) return mcg::fail(MCG_ERR_UNSUPPORTED, "device index beyond 64");
     std::lock_guard<std::mutex> lock(g_setup_mutex);
     ScratchAddr &a = g_partials_addr[dev];
-    void *ctx = current_context();
+    const uint64_t ctx = mcg::current_context_id();
     if (!a.ptr || !ctx || ctx != a.ctx) {
         void *p = nullptr;
         e = cudaGetSymbolAddress(&p, g_static_partials);  // initialises the context if needed
@@ -137,7 +114,7 @@ mcg_status scratch_on_current_device(double **out) {
             return mcg::cuda_fail(e, "cudaGetSymbolAddress(static scratch)");
         }
         a.ptr = static_cast<double *>(p);
-        a.ctx = current_context();
+        a.ctx = mcg::current_context_id();
     }
     *out = a.ptr;
     return MCG_OK;
