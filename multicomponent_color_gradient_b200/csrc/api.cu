@@ -7,7 +7,6 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -54,19 +53,14 @@ mcg_status check_handle(const mcg_handle *h) {
 
 // The share of the current device, `device`.
 static std::shared_ptr<DeviceShare> device_share(int device) {
-    static std::mutex m;
-    static std::map<int, std::weak_ptr<DeviceShare>> known;
-    std::lock_guard<std::mutex> lock(m);
-    std::weak_ptr<DeviceShare> &k = known[device];
-    std::shared_ptr<DeviceShare> s = k.lock();
-    if (!s) {
-        s = std::make_shared<DeviceShare>();
-        size_t free_b = 0;
-        if (cudaMemGetInfo(&free_b, &s->bytes) != cudaSuccess) {
-            (void)cudaGetLastError();
-            s->bytes = 0;
-        }
-        k = s;
+    static PerContext<DeviceShare> known;
+    (void)cudaFree(nullptr);  // the context, if this is the device's first call
+    std::shared_ptr<DeviceShare> s = known.get(device, primary_context_id(device));
+    std::lock_guard<std::mutex> lock(s->m);
+    size_t free_b = 0;
+    if (s->bytes == 0 && cudaMemGetInfo(&free_b, &s->bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        s->bytes = 0;
     }
     return s;
 }
@@ -250,8 +244,11 @@ void free_buffers(mcg_handle *h) {
 void release(mcg_handle *h) {
     mcg::async_release(h);
     mcg::io_close(h);
-    free_buffers(h);
     give_back_padding(h);
+    // memory, streams and events of a context that a reset destroyed are gone, and
+    // their addresses may belong to others by now
+    if (h->share->gone()) return;
+    free_buffers(h);
     if (h->d_inlet_profile) cudaFree(h->d_inlet_profile);
     if (h->d_vti_text) cudaFree(h->d_vti_text);
     if (h->h_vti_text) cudaFreeHost(h->h_vti_text);
@@ -546,7 +543,7 @@ mcg_status mcg_create(const mcg_params *p, mcg_handle **out) {
 mcg_status mcg_destroy(mcg_handle *h) {
     return mcg::guarded([&]() -> mcg_status {
         if (!h) return MCG_OK;
-        cudaStreamSynchronize(h->stream);
+        if (!h->share->gone()) cudaStreamSynchronize(h->stream);
         release(h);
         delete h;
         return MCG_OK;

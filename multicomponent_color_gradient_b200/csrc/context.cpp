@@ -28,12 +28,36 @@ uint64_t id_of(Context ctx) {
     return ctx && get_id && get_id(ctx, &id) == 0 ? uint64_t(id) : 0;
 }
 
-}  // namespace
-
-uint64_t current_context_id() {
+Context current_context() {
     static const auto get_current = driver_entry<int (*)(Context *)>("cuCtxGetCurrent");
     Context ctx = nullptr;
-    return get_current && get_current(&ctx) == 0 ? id_of(ctx) : 0;
+    return get_current && get_current(&ctx) == 0 ? ctx : nullptr;
 }
+
+// The device's primary context, the one the runtime works in, or null if it is
+// not active (asking does not activate it).
+Context primary_context(int device) {
+    static const auto get_state = driver_entry<int (*)(int, unsigned *, int *)>("cuDevicePrimaryCtxGetState");
+    static const auto retain = driver_entry<int (*)(Context *, int)>("cuDevicePrimaryCtxRetain");
+    static const auto release = driver_entry<int (*)(int)>("cuDevicePrimaryCtxRelease");
+    unsigned flags = 0;
+    int active = 0;
+    Context ctx = nullptr;
+    if (!get_state || !retain || !release || get_state(device, &flags, &active) != 0 || !active) return nullptr;
+    if (retain(&ctx, device) != 0) return nullptr;
+    release(device);
+    return ctx;
+}
+
+}  // namespace
+
+uint64_t current_context_id() { return id_of(current_context()); }
+
+uint64_t primary_context_id(int device) {
+    const Context ctx = primary_context(device);
+    return ctx && ctx == current_context() ? id_of(ctx) : 0;
+}
+
+bool context_gone(int device, uint64_t id) { return id != 0 && id_of(primary_context(device)) != id; }
 
 }  // namespace mcg

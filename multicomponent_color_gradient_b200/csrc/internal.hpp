@@ -14,6 +14,7 @@
 
 #include "../../include/mcg.h"
 #include "kernels.cuh"
+#include "per_context.hpp"
 
 namespace mcg {
 // The radial-statistics state an output writes (a copy, so that outputs
@@ -25,14 +26,25 @@ struct StatsSnapshot {
 };
 struct AsyncOutput;  // output_async.cpp
 
-// What the handles of one device share, while one of them lives.
+// Id of the calling thread's CUDA context, 0 where there is none (context.cpp).
+uint64_t current_context_id();
+// The same where that is `device`'s primary context, otherwise 0.
+uint64_t primary_context_id(int device);
+// Whether the primary context with that id has been destroyed (id 0: not known).
+bool context_gone(int device, uint64_t id);
+
+// What the handles of one device and context share, while one of them lives.
 struct DeviceShare {
-    size_t bytes = 0;  // memory of the device
+    const int device;
+    const uint64_t context;  // primary_context_id
+    size_t bytes = 0;        // memory of the device
     std::mutex m;      // guards what follows
     size_t padding = 0;            // bytes that pad population rows
     cudaMemPool_t pool = nullptr;  // of the adjoint runs (adjoint.cu), made by the first
+    DeviceShare(int d, uint64_t c) : device(d), context(c) {}
+    bool gone() const { return context_gone(device, context); }
     ~DeviceShare() {
-        if (pool) cudaMemPoolDestroy(pool);
+        if (pool && !gone()) cudaMemPoolDestroy(pool);
     }
 };
 }  // namespace mcg
@@ -117,8 +129,6 @@ StatsSnapshot stats_snapshot(const mcg_handle *h);
 void tke_update(mcg_handle *h, int32_t step, double total);
 
 mcg_status unpad_rows(mcg_handle *h);  // api.cu
-// Id of the calling thread's CUDA context, 0 where there is none (context.cpp).
-uint64_t current_context_id();
 // cudaMalloc of a buffer that h needs, which if need be takes the place of the
 // padding of h's rows.
 cudaError_t device_malloc(mcg_handle *h, void **p, size_t bytes);

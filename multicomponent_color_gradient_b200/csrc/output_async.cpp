@@ -137,7 +137,8 @@ void async_release(mcg_handle *h) {
         a->cv.notify_all();
         a->worker.join();  // the worker drains the queue before it stops
     }
-    for (int k = 0; k < AsyncOutput::kSlots; ++k) {
+    const bool gone = h->share->gone();  // see release (api.cu)
+    for (int k = 0; k < AsyncOutput::kSlots && !gone; ++k) {
         if (a->d_text[k]) cudaFree(a->d_text[k]);
         if (a->h_text[k]) cudaFreeHost(a->h_text[k]);
         if (a->d_radial[k]) cudaFree(a->d_radial[k]);
@@ -147,7 +148,7 @@ void async_release(mcg_handle *h) {
         if (a->staged[k]) cudaEventDestroy(a->staged[k]);
         if (a->ready[k]) cudaEventDestroy(a->ready[k]);
     }
-    if (a->io) cudaStreamDestroy(a->io);
+    if (a->io && !gone) cudaStreamDestroy(a->io);
     delete a;
     h->async_out = nullptr;
 }

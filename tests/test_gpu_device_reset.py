@@ -63,3 +63,37 @@ for _ in range(2):
     call("cudaMalloc", C.byref(p), C.c_size_t(64 << 20))
     sums()
 """)
+
+
+def test_adjoint_runs_and_late_close_after_a_reset():
+    """A handle that is open at the reset leaves nothing to the next one: runs of
+    the new context take new memory, and the old handle's close, though late,
+    frees nothing of it."""
+    run("""
+def start(n=30):
+    S = Solver(case(n))
+    S.init_bubble()
+    return S
+target = np.linspace(-1, 1, 30 * 20 * 18).astype(np.float32)
+old = start()
+want = old.adjoint_run(target, 8, 3, tape=4)
+call("cudaDeviceReset")
+new = start()
+got = new.adjoint_run(target, 8, 3, tape=4)
+np.testing.assert_array_equal(got["dJ_du0"], want["dJ_du0"])
+new.step(2)
+fields = new.get_fields()
+with start() as S:
+    S.step(2)
+    plain = S.get_fields()
+new.close()
+new = start()
+old.close()
+new.step(2)
+after = new.get_fields()
+for k in plain:
+    np.testing.assert_array_equal(fields[k], plain[k])
+    np.testing.assert_array_equal(after[k], plain[k])
+np.testing.assert_allclose(got["J"], want["J"], rtol=1e-9)
+new.close()
+""")
