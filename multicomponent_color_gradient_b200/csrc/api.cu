@@ -393,8 +393,7 @@ mcg_status unpad_rows(mcg_handle *h) {
         h->cur ^= 1;
     }
     give_back_padding(h);
-    h->tiling = fused_tiling(h->s.g, kFusedSmemPerBlock);
-    MCG_CUDA(fused_configure(h->s.g, h->tiling), "unpad rows");
+    retile_plain_rows(h->s.g, h->tiling);
     return MCG_OK;
 }
 

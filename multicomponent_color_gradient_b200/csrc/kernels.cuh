@@ -130,6 +130,9 @@ struct DeviceState {
 
 // ---- the fused step (moments + colour gradient + collision in one pass) ----
 FusedTiling fused_tiling(const Geometry &g, int max_smem_per_block);
+// The shape of t, made for padded rows, for the same grid with plain rows (px = NX,
+// not whole pieces); how the step runs and the limits set on it stay.
+void retile_plain_rows(const Geometry &g, FusedTiling &t);
 cudaError_t fused_configure(const Geometry &g, const FusedTiling &t);
 inline int fused_launches(const FusedTiling &t) { return t.march == kMarchSplit ? 2 : 1; }  // kernels of a step
 cudaError_t launch_fused(const DeviceState &s, const FusedTiling &t, int cur, int64_t step, bool stats,

@@ -54,6 +54,13 @@ static void split_tiling(const Geometry &g, FusedTiling &t) {
 
 static int compiled_pitch(const Geometry &g) { return g.px % 32 == 0 ? g.px : 0; }
 
+void retile_plain_rows(const Geometry &g, FusedTiling &t) {
+    // a march's shape does not depend on the pitch
+    if (t.march != kMarchSplit) return;
+    split_tiling(g, t);
+    t.pitch = 0;
+}
+
 FusedTiling fused_tiling(const Geometry &g, int max_smem) {
     FusedTiling t{};
     t.tpr = ((g.NX + 31) / 32) * 32;

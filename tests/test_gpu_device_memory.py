@@ -157,3 +157,35 @@ def test_memory_kept_between_adjoint_runs_is_there_for_others():
         with only_free(-kept // 2):
             pass
         assert_same_gradient(S.adjoint_run(target, 3, 2, tape=2), want)
+
+
+@pytest.mark.parametrize("at_create", ["0", None])
+def test_giving_padding_up_keeps_how_the_step_runs(monkeypatch, at_create):
+    """How a handle's step runs is settled when the handle is made, not by the
+    environment of the call that takes the padding out."""
+    if at_create is not None:
+        monkeypatch.setenv("MCG_FUSED_PIPE", at_create)
+    else:
+        monkeypatch.delenv("MCG_FUSED_PIPE", raising=False)
+    case = derive(dict(CASE, NY=34, NZ=34, bubble_radius=8.0))
+    N = case["NX"] * case["NY"] * case["NZ"]
+    target = np.linspace(-1, 1, N).astype(np.float32)
+    with Solver(case) as S:
+        how = S.tiling()["pipelined"]
+        assert how == (3 if at_create is None else 0)
+        S.init_bubble()
+        S.step(2)
+        want = S.get_fields()
+        S.init_bubble()
+        if at_create is None:
+            monkeypatch.setenv("MCG_FUSED_PIPE", "1")
+        else:
+            monkeypatch.delenv("MCG_FUSED_PIPE")
+        padded = device_bytes(S)
+        plain_run, padded_run = (11 * 216 * (N // 97 * px) for px in (97, 128))
+        monkeypatch.setenv("MCG_ADJOINT_MEMORY_MB", str((plain_run + padded_run) // 2 + 120 * N >> 20))
+        S.adjoint_run(target, 12, 8, tape=0)
+        assert device_bytes(S) < padded
+        assert S.tiling()["pipelined"] == how
+        S.step(2)
+        assert_same(S.get_fields(), want)
