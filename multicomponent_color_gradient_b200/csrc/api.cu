@@ -185,9 +185,11 @@ size_t pop_buffer_bytes(const mcg_handle *h) { return pop_buffer_bytes(h->p, h->
 // columns are padded to them, so that the step's kernels are compiled for the
 // pitch and rows start on 128 bytes (us a step: 97x75x131 float32 103 -> 78,
 // float16 73 -> 61, 24x40x24 10.5 -> 9.7).  Not where float32 rows are whole
-// sectors of 64 bytes already (200x301x183: 761 without, 782 with), nor where it
-// would cost more than a third more memory, nor beyond 1/128 of the device's
-// memory for all handles together.
+// sectors of 64 bytes already: at 160x130 rows padding costs 11 % at 72 columns,
+// 7 at 104, 5 at 136, 4 at 168 and 200, 1 to 2 where it adds 8 or 16 columns
+// (120, 152, 176, 184, 216, 232), and gains 0.7 to 1 % at 240 and 248 alone.  Nor
+// where it would cost more than a third more memory, nor beyond 1/128 of the
+// device's memory for all handles together.
 int row_pitch(const mcg_params &p, mcg::DeviceShare &share, size_t *padding) {
     *padding = 0;
     const int px = (p.NX + 31) / 32 * 32;

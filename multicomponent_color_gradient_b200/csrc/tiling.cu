@@ -72,7 +72,8 @@ FusedTiling fused_tiling(const Geometry &g, int max_smem) {
     if (const char *v = std::getenv("MCG_FUSED_PIPE")) t.march = std::atoi(v) != 0 ? kMarchPipe : kMarchBlock;
     if (const char *v = std::getenv("MCG_FUSED_BULK"))
         if (std::atoi(v) != 0 && t.march != kMarchBlock && t.fixed_nx == kFusedNX) t.march = kMarchBulk;
-    // planes are blockIdx.y of the split step
+    // planes are blockIdx.y of the split step, whose extent ends at 65535; such a
+    // grid can be set by mcg_set_populations, stepped and summed
     if (t.march == kMarchSplit && g.NZ - 2 > 65535) t.march = kMarchBlock;
     if (t.march == kMarchSplit)
         split_tiling(g, t);
