@@ -531,8 +531,10 @@ __global__ void __launch_bounds__(kFusedThreads, PipeBlocks<C>::value) k_fused_p
 // 352 (0.76), 256x512x256 2264 (0.96) against 2984 (0.73), 200x301x183 769
 // (0.92) against 1541 (0.46), 64x128x64 39 against 76, 24x40x24 6.6 against 29;
 // float16 jet 128x400x128 258 (0.81) against 441, 256x512x256 1216 (0.89)
-// against 2073 (0.52).  With every node an interface node: 128x256x128 float32
-// 359 against 352, float16 324 against 365.
+// against 2073 (0.52).  With an interface at every node, which no flow keeps, float32
+// 128x256x128 takes 358 against 351 and float16 256^3 1256 against 1228; other
+// sizes gain there too (float16 128x256x128 316 against 324, float32 256^3 1450
+// against 1558, 200x301x183 1052 against 1556, 64x128x64 42 against 77).
 
 // Threads and CTAs per SM the register budgets are sized for: k_step_pull 72
 // registers (64, with spills in float32, to 96 measured within 1 % in float32;
@@ -651,8 +653,25 @@ struct PsiAround {
     }
 };
 
+// The same read at once, for use after other loads have been waited for.
+struct PsiNear {
+    float v[27];
+    template <bool kPeriodic>
+    __device__ __forceinline__ explicit PsiNear(const PsiAround<kPeriodic> &around) {
+#pragma unroll
+        for (int k = 0; k < 27; ++k) v[k] = k == 13 ? 0.0f : around(k % 3 - 1, k / 3 % 3 - 1, k / 9 - 1);
+    }
+    __device__ __forceinline__ float operator()(int cx, int cy, int cz) const {
+        return v[cx + 1 + 3 * (cy + 1) + 9 * (cz + 1)];
+    }
+};
+
 // One piece of k_step_interface, or four quarters, one per 8 lanes: moments from
 // where k_step_pull parked them, psi of the neighbours, relaxation and stores.
+// Float16 reads psi together with the moments, one latency instead of two: with
+// an interface at every node 128x256x128 takes 316 us a step against 325,
+// 256^3 1256 against 1302, jets of little interface the same.  In float32 the 26
+// words spill (373 against 357).
 template <class C, bool kPeriodic>
 __device__ __forceinline__ void relax_parked(const DeviceState &s, const C &codec, const float *psi, bool on, int x,
                                                int y, int z) {
@@ -662,10 +681,10 @@ __device__ __forceinline__ void relax_parked(const DeviceState &s, const C &code
     const size_t at = pop_row(g, y, z);
     NodeMoments m{};
     if (xst) unpark_moments(codec.wr + at + xn, g.px, m);
+    const PsiAround<kPeriodic> around(g, psi, xn, y, z);
+    const std::conditional_t<std::is_same<C, CodecF16>::value, PsiNear, const PsiAround<kPeriodic> &> psi_at(around);
     __syncwarp();  // every lane has its moments before one of them stores over them
-    if (!xst) return;
-    const PsiAround<kPeriodic> psi_at(g, psi, xn, y, z);
-    collide_node<false>(g, s.ph, codec, at, x, y, z, m, psi_at);
+    if (xst) collide_node<false>(g, s.ph, codec, at, x, y, z, m, psi_at);
 }
 
 // The same for the piece that a warp of a small grid has to itself, which is bound
@@ -681,11 +700,7 @@ __device__ __forceinline__ void relax_flagged(const DeviceState &s, const C &cod
     const unsigned f = *flag;
     NodeMoments m;
     unpark_moments(codec.wr + at + xn, g.px, m);
-    const PsiAround<kPeriodic> around(g, psi, xn, y, z);
-    float near[27];
-#pragma unroll
-    for (int k = 0; k < 27; ++k) near[k] = k == 13 ? 0.0f : around(k % 3 - 1, k / 3 % 3 - 1, k / 9 - 1);
-    auto psi_at = [&](int cx, int cy, int cz) { return near[cx + 1 + 3 * (cy + 1) + 9 * (cz + 1)]; };
+    const PsiNear psi_at(PsiAround<kPeriodic>(g, psi, xn, y, z));
     __syncwarp();  // every lane has its moments before one of them stores over them
     const bool on = relax_by_quarters<C>() ? (f >> (4 + (x >> 3 & 3))) & 1u : f & 1u;
     if (on && x < store_columns<C>(g)) collide_node<false>(g, s.ph, codec, at, x, y, z, m, psi_at);
