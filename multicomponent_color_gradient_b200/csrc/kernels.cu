@@ -585,184 +585,184 @@ __device__ __forceinline__ void adj_collide_node(const DeviceState &s, const flo
                                                  double &a_omega, double &a_Ah, double &a_J) {
     const Geometry &g = s.g;
     const Physics &ph = s.ph;
-            const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
-            const size_t N = g.N;
-            const float *mom = M;
-            const float rr = mom[kMomRR * N + id], rb = mom[kMomRB * N + id];
-            const float ux = mom[kMomUX * N + id], uy = mom[kMomUY * N + id], uz = mom[kMomUZ * N + id];
-            const NeqTerms n = make_neq(mom[kMomPXX * N + id], mom[kMomPXY * N + id], mom[kMomPYY * N + id],
-                                        mom[kMomPYZ * N + id], mom[kMomPZZ * N + id], mom[kMomPXZ * N + id], ux, uy, uz);
-            const float rho = rr + rb;
-            const float invr = 1.0f / rho;
-            const float aR = rr * invr, aB = rb * invr;
-            const float oms = 1.0f - omega_at(ph, y);
-            const bool interface = kInterface && !is_bulk(rr, rb);
-            float Fx = 0.f, Fy = 0.f, Fz = 0.f, absF = 0.f, K = 0.f;
-            bool has_dir = false;
-            if (interface) {
-                // periodic box: neighbours wrap over the interior; jet: the record's
-                // psi plane holds the ghost values the forward step read unwrapped
-                const float *psi = M + size_t(kTapePsi) * N;
-                const int xn[3] = {kPeriodic ? wrap_interior(x - 1, g.NX) : x - 1, x,
-                                   kPeriodic ? wrap_interior(x + 1, g.NX) : x + 1};
-                const int yn[3] = {g.sy * (kPeriodic ? wrap_interior(y - 1, g.NY) : y - 1), g.sy * y,
-                                   g.sy * (kPeriodic ? wrap_interior(y + 1, g.NY) : y + 1)};
-                const int zn[3] = {g.sz * (kPeriodic ? wrap_interior(z - 1, g.NZ) : z - 1), g.sz * z,
-                                   g.sz * (kPeriodic ? wrap_interior(z + 1, g.NZ) : z + 1)};
-                float sx = 0.f, sy = 0.f, sz = 0.f;
-                static_for<kQ - 1>([&](auto I) {
-                    constexpr int i = decltype(I)::value + 1;
-                    using D = Dir<i>;
-                    const float wp = D::w * psi[xn[D::cx + 1] + yn[D::cy + 1] + zn[D::cz + 1]];
-                    if constexpr (D::cx != 0) sx += D::fx * wp;
-                    if constexpr (D::cy != 0) sy += D::fy * wp;
-                    if constexpr (D::cz != 0) sz += D::fz * wp;
-                });
-                Fx = kInvCs2 * sx;
-                Fy = kInvCs2 * sy;
-                Fz = kInvCs2 * sz;
-                absF = sqrtf(Fx * Fx + Fy * Fy + Fz * Fz);
-                has_dir = !(absF <= 1.0e-4f);
-                K = ph.beta * ((rr * rb) / (rho * rho)) * rho;
-            }
-            const float invF = has_dir ? 1.0f / absF : 0.0f;
-            const float invF2 = invF * invF;
-            [[maybe_unused]] const float Ah = ph.Ah;
-            const size_t row = pop_row(g, y, z);
-            // (lambda_r, lambda_b) of a direction: one float2, as the populations
-            auto lam_at = [&](int slot) {
-                return reinterpret_cast<const float2 *>(lam)[row + size_t(slot) * size_t(g.px) + size_t(x)];
-            };
-            // Bulk part: g_i = w_i P(c_i) with P the collision polynomial, so the
-            // sums over directions are the polynomial's coefficients dotted with
-            // the moments T_k = sum_i w_i lambda_g,i m_k(c_i) (and U_k with
-            // lambda_r - lambda_b for the colour split).  The moments are formed
-            // group by group: per (cy, cz) the three cx values reduce to
-            // (sum, sum cx, sum cx^2), which add into the 17 moments with the
-            // weights cy^b cz^c.
-            float Tm[17], Um[17];
+    const uint32_t id = uint32_t(x) + uint32_t(g.sy) * uint32_t(y) + uint32_t(g.sz) * uint32_t(z);
+    const size_t N = g.N;
+    const float *mom = M;
+    const float rr = mom[kMomRR * N + id], rb = mom[kMomRB * N + id];
+    const float ux = mom[kMomUX * N + id], uy = mom[kMomUY * N + id], uz = mom[kMomUZ * N + id];
+    const NeqTerms n = make_neq(mom[kMomPXX * N + id], mom[kMomPXY * N + id], mom[kMomPYY * N + id],
+                                mom[kMomPYZ * N + id], mom[kMomPZZ * N + id], mom[kMomPXZ * N + id], ux, uy, uz);
+    const float rho = rr + rb;
+    const float invr = 1.0f / rho;
+    const float aR = rr * invr, aB = rb * invr;
+    const float oms = 1.0f - omega_at(ph, y);
+    const bool interface = kInterface && !is_bulk(rr, rb);
+    float Fx = 0.f, Fy = 0.f, Fz = 0.f, absF = 0.f, K = 0.f;
+    bool has_dir = false;
+    if (interface) {
+        // periodic box: neighbours wrap over the interior; jet: the record's
+        // psi plane holds the ghost values the forward step read unwrapped
+        const float *psi = M + size_t(kTapePsi) * N;
+        const int xn[3] = {kPeriodic ? wrap_interior(x - 1, g.NX) : x - 1, x,
+                           kPeriodic ? wrap_interior(x + 1, g.NX) : x + 1};
+        const int yn[3] = {g.sy * (kPeriodic ? wrap_interior(y - 1, g.NY) : y - 1), g.sy * y,
+                           g.sy * (kPeriodic ? wrap_interior(y + 1, g.NY) : y + 1)};
+        const int zn[3] = {g.sz * (kPeriodic ? wrap_interior(z - 1, g.NZ) : z - 1), g.sz * z,
+                           g.sz * (kPeriodic ? wrap_interior(z + 1, g.NZ) : z + 1)};
+        float sx = 0.f, sy = 0.f, sz = 0.f;
+        static_for<kQ - 1>([&](auto I) {
+            constexpr int i = decltype(I)::value + 1;
+            using D = Dir<i>;
+            const float wp = D::w * psi[xn[D::cx + 1] + yn[D::cy + 1] + zn[D::cz + 1]];
+            if constexpr (D::cx != 0) sx += D::fx * wp;
+            if constexpr (D::cy != 0) sy += D::fy * wp;
+            if constexpr (D::cz != 0) sz += D::fz * wp;
+        });
+        Fx = kInvCs2 * sx;
+        Fy = kInvCs2 * sy;
+        Fz = kInvCs2 * sz;
+        absF = sqrtf(Fx * Fx + Fy * Fy + Fz * Fz);
+        has_dir = !(absF <= 1.0e-4f);
+        K = ph.beta * ((rr * rb) / (rho * rho)) * rho;
+    }
+    const float invF = has_dir ? 1.0f / absF : 0.0f;
+    const float invF2 = invF * invF;
+    [[maybe_unused]] const float Ah = ph.Ah;
+    const size_t row = pop_row(g, y, z);
+    // (lambda_r, lambda_b) of a direction: one float2, as the populations
+    auto lam_at = [&](int slot) {
+        return reinterpret_cast<const float2 *>(lam)[row + size_t(slot) * size_t(g.px) + size_t(x)];
+    };
+    // Bulk part: g_i = w_i P(c_i) with P the collision polynomial, so the
+    // sums over directions are the polynomial's coefficients dotted with
+    // the moments T_k = sum_i w_i lambda_g,i m_k(c_i) (and U_k with
+    // lambda_r - lambda_b for the colour split).  The moments are formed
+    // group by group: per (cy, cz) the three cx values reduce to
+    // (sum, sum cx, sum cx^2), which add into the 17 moments with the
+    // weights cy^b cz^c.
+    float Tm[17], Um[17];
     #pragma unroll
-            for (int k = 0; k < 17; ++k) Tm[k] = Um[k] = 0.f;
-            static_for<9>([&](auto G) {
-                constexpr int cy = decltype(G)::value / 3 - 1, cz = decltype(G)::value % 3 - 1;
-                float mv[3], nv[3];
-                static_for<3>([&](auto X) {
-                    constexpr int cx = decltype(X)::value - 1;
-                    constexpr int i = dir_of(cx, cy, cz);
-                    const float2 l = lam_at(slot_pair(i));
-                    mv[cx + 1] = Dir<i>::w * (aR * l.x + aB * l.y);
-                    nv[cx + 1] = Dir<i>::w * (l.x - l.y);
-                });
-                const float m2 = mv[2] + mv[0], n2 = nv[2] + nv[0];
-                const float ms[3] = {m2 + mv[1], mv[2] - mv[0], m2};
-                const float ns[3] = {n2 + nv[1], nv[2] - nv[0], n2};
-                static_for<17>([&](auto K) {
-                    constexpr int k = decltype(K)::value;
-                    constexpr int wgt = ipow1(cy, poly_exp(k, 1)) * ipow1(cz, poly_exp(k, 2));
-                    constexpr int a = poly_exp(k, 0);
-                    if constexpr (wgt == 1) {
-                        Tm[k] += ms[a];
-                        Um[k] += ns[a];
-                    } else if constexpr (wgt == -1) {
-                        Tm[k] -= ms[a];
-                        Um[k] -= ns[a];
-                    }
-                });
-            });
-            const PolyAdjoint pT = poly_adjoint(Tm, ux, uy, uz, n);
-            const PolyAdjoint pU = poly_adjoint(Um, ux, uy, uz, n);
-            const float(&S2)[6] = pT.S2;
-            const float(&S3)[7] = pT.S3;
-            const float l_rhoeq = rho * pT.Phi;  // sum lambda_g feq (feq is proportional to rho)
-            const float l_oms = pT.Psi;          // sum lambda_g fneq
-            float l_d = rho * pU.Phi + oms * pU.Psi;  // sum (lambda_r - lambda_b) g
-            // interface nodes: the perturbation and recolouring terms, direction by direction
-            float sAx = 0.f, sAy = 0.f, sAz = 0.f, sB = 0.f, sDx = 0.f, sDy = 0.f, sDz = 0.f, sE = 0.f, sBB = 0.f,
-                  l_Ah = 0.f;
-            if (interface) {
-                {  // rest direction: even only
-                    const float2 l0 = lam_at(slot_pair(0));
-                    const float lg = aR * l0.x + aB * l0.y, ld = l0.x - l0.y;
-                    const float o2A = -absF * Dir<0>::B;  // Omega2 / (A/2)
-                    l_d += ld * (Ah * o2A);
-                    sBB += lg * Dir<0>::B;
-                    l_Ah += lg * o2A;
-                }
-                static_for<(kQ - 1) / 2>([&](auto P) {
-                    constexpr int i = 2 * decltype(P)::value + 1;
-                    using D = Dir<i>;
-                    const float2 li = lam_at(slot_pair(i)), lo = lam_at(slot_pair(i + 1));
-                    const float lgi = aR * li.x + aB * li.y, lgo = aR * lo.x + aB * lo.y;
-                    const float ldi = li.x - li.y, ldo = lo.x - lo.y;
-                    const float gs = lgi + lgo, ds = ldi + ldo, dd = ldi - ldo;
-                    float fc = 0.f;
-                    if constexpr (D::cx != 0) fc += D::fx * Fx;
-                    if constexpr (D::cy != 0) fc += D::fy * Fy;
-                    if constexpr (D::cz != 0) fc += D::fz * Fz;
-                    const float o2A = absF * (D::w * (fc * fc) * invF2 - D::B);  // Omega2 / (A/2), even
-                    l_d += ds * (Ah * o2A);
-                    sBB += gs * D::B;
-                    l_Ah += gs * o2A;
-                    const float a = gs * D::w * fc, d = dd * D::w * D::invc;
-                    if constexpr (D::cx != 0) { sAx += D::fx * a; sDx += D::fx * d; }
-                    if constexpr (D::cy != 0) { sAy += D::fy * a; sDy += D::fy * d; }
-                    if constexpr (D::cz != 0) { sAz += D::fz * a; sDz += D::fz * d; }
-                    sB += a * fc;
-                    sE += d * fc;
-                });
+    for (int k = 0; k < 17; ++k) Tm[k] = Um[k] = 0.f;
+    static_for<9>([&](auto G) {
+        constexpr int cy = decltype(G)::value / 3 - 1, cz = decltype(G)::value % 3 - 1;
+        float mv[3], nv[3];
+        static_for<3>([&](auto X) {
+            constexpr int cx = decltype(X)::value - 1;
+            constexpr int i = dir_of(cx, cy, cz);
+            const float2 l = lam_at(slot_pair(i));
+            mv[cx + 1] = Dir<i>::w * (aR * l.x + aB * l.y);
+            nv[cx + 1] = Dir<i>::w * (l.x - l.y);
+        });
+        const float m2 = mv[2] + mv[0], n2 = nv[2] + nv[0];
+        const float ms[3] = {m2 + mv[1], mv[2] - mv[0], m2};
+        const float ns[3] = {n2 + nv[1], nv[2] - nv[0], n2};
+        static_for<17>([&](auto K) {
+            constexpr int k = decltype(K)::value;
+            constexpr int wgt = ipow1(cy, poly_exp(k, 1)) * ipow1(cz, poly_exp(k, 2));
+            constexpr int a = poly_exp(k, 0);
+            if constexpr (wgt == 1) {
+                Tm[k] += ms[a];
+                Um[k] += ns[a];
+            } else if constexpr (wgt == -1) {
+                Tm[k] -= ms[a];
+                Um[k] -= ns[a];
             }
-            // fneq: Pi enters directly (H2) and through the third-order terms a3
-            const float c2 = oms * kInv2Cs4, c3 = oms * kInv2Cs6;
-            float lPxx = S2[0] * c2, lPxy = 2.0f * S2[1] * c2, lPyy = S2[2] * c2;
-            float lPyz = 2.0f * S2[3] * c2, lPzz = S2[4] * c2, lPxz = 2.0f * S2[5] * c2;
-            const float la_xxy = S3[0] * c3, la_xxz = S3[1] * c3, la_xyy = S3[2] * c3, la_xzz = S3[3] * c3;
-            const float la_yyz = S3[4] * c3, la_yzz = S3[5] * c3, la_xyz = 2.0f * S3[6] * c3;
-            lPxx += la_xxy * uy + la_xxz * uz;
-            lPyy += la_xyy * ux + la_yyz * uz;
-            lPzz += la_xzz * ux + la_yzz * uy;
-            lPxy += 2.0f * la_xxy * ux + 2.0f * la_xyy * uy + la_xyz * uz;
-            lPxz += 2.0f * la_xxz * ux + 2.0f * la_xzz * uz + la_xyz * uy;
-            lPyz += 2.0f * la_yyz * uy + 2.0f * la_yzz * uz + la_xyz * ux;
-            float lux = 2.0f * la_xxy * n.pxy + 2.0f * la_xxz * n.pxz + la_xyy * n.pyy + la_xzz * n.pzz + la_xyz * n.pyz;
-            float luy = la_xxy * n.pxx + 2.0f * la_xyy * n.pxy + 2.0f * la_yyz * n.pyz + la_yzz * n.pzz + la_xyz * n.pxz;
-            float luz = la_xxz * n.pxx + 2.0f * la_xzz * n.pxz + la_yyz * n.pyy + 2.0f * la_yzz * n.pyz + la_xyz * n.pxy;
-            // feq: rho times the u-gradient of the feq polynomial against T
-            lux += rho * pT.dPhi[0];
-            luy += rho * pT.dPhi[1];
-            luz += rho * pT.dPhi[2];
-            // colour gradient: perturbation and recolouring
-            float lFx = 0.f, lFy = 0.f, lFz = 0.f, lK = 0.f;
-            if (interface) {
-                if (has_dir) {
-                    const float i3 = invF2 * invF;
-                    lFx = Ah * (2.0f * invF * sAx - Fx * i3 * sB - Fx * invF * sBB) + K * (sDx * invF - Fx * i3 * sE);
-                    lFy = Ah * (2.0f * invF * sAy - Fy * i3 * sB - Fy * invF * sBB) + K * (sDy * invF - Fy * i3 * sE);
-                    lFz = Ah * (2.0f * invF * sAz - Fz * i3 * sB - Fz * invF * sBB) + K * (sDz * invF - Fz * i3 * sE);
-                    lK = sE * invF;
-                } else if (absF > 0.0f) {
-                    const float q = -Ah * sBB / absF;
-                    lFx = q * Fx;
-                    lFy = q * Fy;
-                    lFz = q * Fz;
-                }
-            }
-            const float inv2 = invr * invr;
-            const float l_rho = l_rhoeq * invr;  // feq is proportional to rho
-            o.rr = l_rho + l_d * rb * inv2 + lK * ph.beta * rb * rb * inv2;
+        });
+    });
+    const PolyAdjoint pT = poly_adjoint(Tm, ux, uy, uz, n);
+    const PolyAdjoint pU = poly_adjoint(Um, ux, uy, uz, n);
+    const float(&S2)[6] = pT.S2;
+    const float(&S3)[7] = pT.S3;
+    const float l_rhoeq = rho * pT.Phi;  // sum lambda_g feq (feq is proportional to rho)
+    const float l_oms = pT.Psi;          // sum lambda_g fneq
+    float l_d = rho * pU.Phi + oms * pU.Psi;  // sum (lambda_r - lambda_b) g
+    // interface nodes: the perturbation and recolouring terms, direction by direction
+    float sAx = 0.f, sAy = 0.f, sAz = 0.f, sB = 0.f, sDx = 0.f, sDy = 0.f, sDz = 0.f, sE = 0.f, sBB = 0.f,
+          l_Ah = 0.f;
+    if (interface) {
+        {  // rest direction: even only
+            const float2 l0 = lam_at(slot_pair(0));
+            const float lg = aR * l0.x + aB * l0.y, ld = l0.x - l0.y;
+            const float o2A = -absF * Dir<0>::B;  // Omega2 / (A/2)
+            l_d += ld * (Ah * o2A);
+            sBB += lg * Dir<0>::B;
+            l_Ah += lg * o2A;
+        }
+        static_for<(kQ - 1) / 2>([&](auto P) {
+            constexpr int i = 2 * decltype(P)::value + 1;
+            using D = Dir<i>;
+            const float2 li = lam_at(slot_pair(i)), lo = lam_at(slot_pair(i + 1));
+            const float lgi = aR * li.x + aB * li.y, lgo = aR * lo.x + aB * lo.y;
+            const float ldi = li.x - li.y, ldo = lo.x - lo.y;
+            const float gs = lgi + lgo, ds = ldi + ldo, dd = ldi - ldo;
+            float fc = 0.f;
+            if constexpr (D::cx != 0) fc += D::fx * Fx;
+            if constexpr (D::cy != 0) fc += D::fy * Fy;
+            if constexpr (D::cz != 0) fc += D::fz * Fz;
+            const float o2A = absF * (D::w * (fc * fc) * invF2 - D::B);  // Omega2 / (A/2), even
+            l_d += ds * (Ah * o2A);
+            sBB += gs * D::B;
+            l_Ah += gs * o2A;
+            const float a = gs * D::w * fc, d = dd * D::w * D::invc;
+            if constexpr (D::cx != 0) { sAx += D::fx * a; sDx += D::fx * d; }
+            if constexpr (D::cy != 0) { sAy += D::fy * a; sDy += D::fy * d; }
+            if constexpr (D::cz != 0) { sAz += D::fz * a; sDz += D::fz * d; }
+            sB += a * fc;
+            sE += d * fc;
+        });
+    }
+    // fneq: Pi enters directly (H2) and through the third-order terms a3
+    const float c2 = oms * kInv2Cs4, c3 = oms * kInv2Cs6;
+    float lPxx = S2[0] * c2, lPxy = 2.0f * S2[1] * c2, lPyy = S2[2] * c2;
+    float lPyz = 2.0f * S2[3] * c2, lPzz = S2[4] * c2, lPxz = 2.0f * S2[5] * c2;
+    const float la_xxy = S3[0] * c3, la_xxz = S3[1] * c3, la_xyy = S3[2] * c3, la_xzz = S3[3] * c3;
+    const float la_yyz = S3[4] * c3, la_yzz = S3[5] * c3, la_xyz = 2.0f * S3[6] * c3;
+    lPxx += la_xxy * uy + la_xxz * uz;
+    lPyy += la_xyy * ux + la_yyz * uz;
+    lPzz += la_xzz * ux + la_yzz * uy;
+    lPxy += 2.0f * la_xxy * ux + 2.0f * la_xyy * uy + la_xyz * uz;
+    lPxz += 2.0f * la_xxz * ux + 2.0f * la_xzz * uz + la_xyz * uy;
+    lPyz += 2.0f * la_yyz * uy + 2.0f * la_yzz * uz + la_xyz * ux;
+    float lux = 2.0f * la_xxy * n.pxy + 2.0f * la_xxz * n.pxz + la_xyy * n.pyy + la_xzz * n.pzz + la_xyz * n.pyz;
+    float luy = la_xxy * n.pxx + 2.0f * la_xyy * n.pxy + 2.0f * la_yyz * n.pyz + la_yzz * n.pzz + la_xyz * n.pxz;
+    float luz = la_xxz * n.pxx + 2.0f * la_xzz * n.pxz + la_yyz * n.pyy + 2.0f * la_yzz * n.pyz + la_xyz * n.pxy;
+    // feq: rho times the u-gradient of the feq polynomial against T
+    lux += rho * pT.dPhi[0];
+    luy += rho * pT.dPhi[1];
+    luz += rho * pT.dPhi[2];
+    // colour gradient: perturbation and recolouring
+    float lFx = 0.f, lFy = 0.f, lFz = 0.f, lK = 0.f;
+    if (interface) {
+        if (has_dir) {
+            const float i3 = invF2 * invF;
+            lFx = Ah * (2.0f * invF * sAx - Fx * i3 * sB - Fx * invF * sBB) + K * (sDx * invF - Fx * i3 * sE);
+            lFy = Ah * (2.0f * invF * sAy - Fy * i3 * sB - Fy * invF * sBB) + K * (sDy * invF - Fy * i3 * sE);
+            lFz = Ah * (2.0f * invF * sAz - Fz * i3 * sB - Fz * invF * sBB) + K * (sDz * invF - Fz * i3 * sE);
+            lK = sE * invF;
+        } else if (absF > 0.0f) {
+            const float q = -Ah * sBB / absF;
+            lFx = q * Fx;
+            lFy = q * Fy;
+            lFz = q * Fz;
+        }
+    }
+    const float inv2 = invr * invr;
+    const float l_rho = l_rhoeq * invr;  // feq is proportional to rho
+    o.rr = l_rho + l_d * rb * inv2 + lK * ph.beta * rb * rb * inv2;
     o.rb = l_rho - l_d * rr * inv2 + lK * ph.beta * rr * rr * inv2;
     // the objective's source: J_t = (w/2) sum uy^2 over nodes with y >= y_obs,
-            // or the profile objective's dJ/duy of the node's radial bin (the bin of
-            // radial_accumulate_warp, same float arithmetic)
-            float lobj = 0.f;
-            if (obj.table) {
-                const float dx = float(x) - ph.jet_x0, dz = float(z) - ph.jet_z0;
-                const unsigned rbin = unsigned(sqrtf(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dz, dz))));
-                if (rbin < unsigned(ph.NRB)) lobj = obj.table[size_t(y) * ph.NRB + rbin];
-            } else if (obj.weight != 0.0f && y >= obj.y_obs) {
-                lobj = obj.weight * uy;
-                a_J += 0.5 * double(obj.weight) * double(uy) * double(uy);
-            }
-            o.ux = lux;
+    // or the profile objective's dJ/duy of the node's radial bin (the bin of
+    // radial_accumulate_warp, same float arithmetic)
+    float lobj = 0.f;
+    if (obj.table) {
+        const float dx = float(x) - ph.jet_x0, dz = float(z) - ph.jet_z0;
+        const unsigned rbin = unsigned(sqrtf(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dz, dz))));
+        if (rbin < unsigned(ph.NRB)) lobj = obj.table[size_t(y) * ph.NRB + rbin];
+    } else if (obj.weight != 0.0f && y >= obj.y_obs) {
+        lobj = obj.weight * uy;
+        a_J += 0.5 * double(obj.weight) * double(uy) * double(uy);
+    }
+    o.ux = lux;
     o.uy = luy + lobj;
     o.uz = luz;
     o.pxx = lPxx; o.pxy = lPxy; o.pyy = lPyy; o.pyz = lPyz; o.pzz = lPzz; o.pxz = lPxz;

@@ -528,13 +528,6 @@ __device__ __forceinline__ NodeMoments pull_moments(const Geometry &g, const C &
     return pull_moments_map(PullMap<C>(g, x, y, z, kPeriodic), codec, x);
 }
 
-// Relax one node and store its 54 post-collision values (lbm.cuh:184-293).
-// The bulk part feq + (1-omega) fneq of all 27 directions comes from
-// collision_poly (lattice.cuh).  At interface nodes the perturbation Omega2
-// (even in c: one evaluation per opposite pair) and the recolouring Delta
-// (odd) are added per direction.  psi_at(cx,cy,cz) returns the neighbour's
-// psi, read unwrapped like forces.cuh:31 (ghost psi is what the reference
-// sees there).
 // Launches that follow one another on a stream overlap by programmatic dependent
 // launch: each starts while the one before it drains, and everything before the
 // wait reads only kernel parameters.  Every thread of a kernel launched this way
@@ -621,6 +614,13 @@ __device__ __forceinline__ bool is_bulk(float rr, float rb) {
     const float invrT = 1.0f / (rr + rb);
     return 4.0f * rr * rb * invrT * invrT <= 1e-4f;
 }
+// Relax one node and store its 54 post-collision values (lbm.cuh:184-293).
+// The bulk part feq + (1-omega) fneq of all 27 directions comes from
+// collision_poly (lattice.cuh).  At interface nodes the perturbation Omega2
+// (even in c: one evaluation per opposite pair) and the recolouring Delta
+// (odd) are added per direction.  psi_at(cx,cy,cz) returns the neighbour's
+// psi, read unwrapped like forces.cuh:31 (ghost psi is what the reference
+// sees there).
 // kBulk: the caller knows that the node is_bulk (psi_at is not called).
 template <bool kBulk, class C, class PsiAt>
 __device__ __forceinline__ void collide_node(const Geometry &g, const Physics &ph, const C &codec, size_t row, int x,
