@@ -55,7 +55,7 @@ mcg_status check_handle(const mcg_handle *h) {
 static std::shared_ptr<DeviceShare> device_share(int device) {
     static PerContext<DeviceShare> known;
     (void)cudaFree(nullptr);  // the context, if this is the device's first call
-    std::shared_ptr<DeviceShare> s = known.get(device, primary_context_id(device));
+    std::shared_ptr<DeviceShare> s = known.get(device, current_context_id());
     std::lock_guard<std::mutex> lock(s->m);
     size_t free_b = 0;
     if (s->bytes == 0 && cudaMemGetInfo(&free_b, &s->bytes) != cudaSuccess) {

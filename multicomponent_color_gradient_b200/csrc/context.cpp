@@ -34,8 +34,7 @@ Context current_context() {
     return get_current && get_current(&ctx) == 0 ? ctx : nullptr;
 }
 
-// The device's primary context, the one the runtime works in, or null if it is
-// not active (asking does not activate it).
+// Null while it is not active; asking does not activate it.
 Context primary_context(int device) {
     static const auto get_state = driver_entry<int (*)(int, unsigned *, int *)>("cuDevicePrimaryCtxGetState");
     static const auto retain = driver_entry<int (*)(Context *, int)>("cuDevicePrimaryCtxRetain");
@@ -53,11 +52,6 @@ Context primary_context(int device) {
 
 uint64_t current_context_id() { return id_of(current_context()); }
 
-uint64_t primary_context_id(int device) {
-    const Context ctx = primary_context(device);
-    return ctx && ctx == current_context() ? id_of(ctx) : 0;
-}
-
-bool context_gone(int device, uint64_t id) { return id != 0 && id_of(primary_context(device)) != id; }
+uint64_t primary_context_id(int device) { return id_of(primary_context(device)); }
 
 }  // namespace mcg

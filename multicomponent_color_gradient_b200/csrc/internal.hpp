@@ -28,21 +28,21 @@ struct AsyncOutput;  // output_async.cpp
 
 // Id of the calling thread's CUDA context, 0 where there is none (context.cpp).
 uint64_t current_context_id();
-// The same where that is `device`'s primary context, otherwise 0.
+// Id of the device's primary context, the one the runtime works in by itself, 0
+// while there is none.
 uint64_t primary_context_id(int device);
-// Whether the primary context with that id has been destroyed (id 0: not known).
-bool context_gone(int device, uint64_t id);
 
 // What the handles of one device and context share, while one of them lives.
 struct DeviceShare {
     const int device;
-    const uint64_t context;  // primary_context_id
+    const uint64_t context;  // current_context_id of those who share it
+    const bool primary;      // it is the device's primary context, whose end can be seen
     size_t bytes = 0;        // memory of the device
     std::mutex m;      // guards what follows
     size_t padding = 0;            // bytes that pad population rows
     cudaMemPool_t pool = nullptr;  // of the adjoint runs (adjoint.cu), made by the first
-    DeviceShare(int d, uint64_t c) : device(d), context(c) {}
-    bool gone() const { return context_gone(device, context); }
+    DeviceShare(int d, uint64_t c) : device(d), context(c), primary(c != 0 && primary_context_id(d) == c) {}
+    bool gone() const { return primary && primary_context_id(device) != context; }
     ~DeviceShare() {
         if (pool && !gone()) cudaMemPoolDestroy(pool);
     }

@@ -10,7 +10,7 @@ namespace mcg {
 
 // Objects made as T(device, context) that live while someone holds them.
 // `context` identifies a device's context for the life of the process
-// (primary_context_id): after a cudaDeviceReset the next holder gets a new
+// (current_context_id): after a cudaDeviceReset the next holder gets a new
 // object, and those of the old context keep theirs.
 template <class T>
 class PerContext {
