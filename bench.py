@@ -55,14 +55,16 @@ def load_peaks():
         return 6650.0, "fallback"
 
 
-def traffic_per_launch(cells: int, kernel: str):
-    """DRAM bytes (read + write) of one launch of `kernel` (e.g.
-    "k_fused_pipe<CodecF32>"): the per-node figure of its ncu capture in
-    profiles/traffic.json scaled to `cells` nodes, with the capture it came
-    from; (None, None) when the kernel has no capture there."""
+def traffic_per_launch(cells: int, interior: int, kernel: str):
+    """DRAM bytes (read + write) of one step by `kernel` (e.g.
+    "k_fused_pipe<CodecF32>"): the figure per interior node or per node of its
+    ncu capture in profiles/traffic.json scaled to this grid, with the capture
+    it came from; (None, None) when the kernel has no capture there."""
     try:
         with open(os.path.join(ROOT, "profiles", "traffic.json")) as fh:
             rec = json.load(fh)["kernels"][kernel]
+        if "dram_bytes_per_interior_node" in rec:
+            return int(float(rec["dram_bytes_per_interior_node"]) * interior), rec.get("workload")
         return int(float(rec["dram_bytes_per_node"]) * cells), rec.get("workload")
     except (OSError, KeyError, ValueError):
         return None, None
@@ -383,16 +385,19 @@ def main():
         clocks = sampler.stop()
         cells = case["NX"] * case["NY"] * case["NZ"]
         ms = float(np.median(regions))
-        step_bytes = 432 if storage == "f32" else 216  # algorithmic bytes per lattice update
+        # a step pulls and relaxes the interior nodes: MLUPS count every node, as the
+        # reference does, bytes only these
+        interior = (case["NX"] - 2) * (case["NY"] - 2) * (case["NZ"] - 2)
+        step_bytes = 432 if storage == "f32" else 216  # algorithmic bytes of a relaxed node
         n_launch = args.steps * len(regions)
-        r = {"case": case, "cells": cells, "ms": ms, "mlups": world * cells * args.steps / (ms * 1e3),
+        r = {"case": case, "cells": cells, "interior": interior, "ms": ms, "mlups": world * cells * args.steps / (ms * 1e3),
              "step_bytes": step_bytes, "t_fused": kernel_ms["fused"] / n_launch,
              "t_bc": kernel_ms["boundary"] / n_launch, "launches": launches, "clocks": clocks,
              "tiling": S.tiling(),
              "spread": {"regions": len(regions), "min_ms_per_step": round(min(regions) / args.steps, 6),
                         "max_ms_per_step": round(max(regions) / args.steps, 6)}}
-        r["achieved"] = step_bytes * cells / (r["t_fused"] * 1e-3) / 1e9  # GB/s of the fused kernel
-        r["step_gbs"] = step_bytes * cells / (ms / args.steps * 1e-3) / 1e9
+        r["achieved"] = step_bytes * interior / (r["t_fused"] * 1e-3) / 1e9  # GB/s of the fused kernel
+        r["step_gbs"] = step_bytes * interior / (ms / args.steps * 1e-3) / 1e9
         return S, r
 
     S, m = measure(args.storage, args.case, args.repeats, args.seconds)
@@ -401,10 +406,10 @@ def main():
     # the kernel(s) of the step that ran
     kname = {0: "k_fused", 1: "k_fused_pipe", 2: "k_fused_bulk", 3: "k_step_pull+k_step_interface"}[tiling["pipelined"]]
     codec = "CodecF32" if args.storage == "f32" else "CodecF16"
-    traffic, traffic_src = traffic_per_launch(cells, f"{kname}<{codec}>")
+    traffic, traffic_src = traffic_per_launch(cells, m["interior"], f"{kname}<{codec}>")
     roofline = {"bound": "hbm", "kernel": kname, "achieved": round(m["achieved"], 1), "peak": hbm_peak,
                 "unit": "GB/s", "frac": round(m["achieved"] / hbm_peak, 4), "peak_kind": peak_kind,
-                "traffic": traffic, "traffic_capture": traffic_src, "algorithmic_bytes_per_node": m["step_bytes"],
+                "traffic": traffic, "traffic_capture": traffic_src, "algorithmic_bytes_per_node": m["step_bytes"], "interior_nodes": m["interior"],
                 "step_achieved": round(m["step_gbs"], 1), "step_frac": round(m["step_gbs"] / hbm_peak, 4),
                 "tiling": tiling,
                 "kernels": {kname: {"ms_per_launch": round(m["t_fused"], 6)}}}
