@@ -140,7 +140,7 @@ cudaError_t adjoint_pool(mcg::DeviceShare &share, int device, cudaMemPool_t *poo
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
         cudaMemPool_t made = nullptr;
-        uint64_t keep = share.bytes / 16;
+        uint64_t keep = share.bytes() / 16;
         cudaError_t e = cudaMemPoolCreate(&made, &props);
         if (e == cudaSuccess && (e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess)
             cudaMemPoolDestroy(made);

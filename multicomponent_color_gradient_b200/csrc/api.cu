@@ -55,14 +55,7 @@ mcg_status check_handle(const mcg_handle *h) {
 static std::shared_ptr<DeviceShare> device_share(int device) {
     static PerContext<DeviceShare> known;
     (void)cudaFree(nullptr);  // the context, if this is the device's first call
-    std::shared_ptr<DeviceShare> s = known.get(device, current_context_id());
-    std::lock_guard<std::mutex> lock(s->m);
-    size_t free_b = 0;
-    if (s->bytes == 0 && cudaMemGetInfo(&free_b, &s->bytes) != cudaSuccess) {
-        (void)cudaGetLastError();
-        s->bytes = 0;
-    }
-    return s;
+    return known.get(device, current_context_id());
 }
 
 StatsSnapshot stats_snapshot(const mcg_handle *h) {
@@ -197,7 +190,7 @@ int row_pitch(const mcg_params &p, mcg::DeviceShare &share, size_t *padding) {
     if (p.storage == MCG_STORAGE_F32 && p.NX % 8 == 0 && p.NX >= 64) return p.NX;
     const size_t extra = 2 * (pop_buffer_bytes(p, px) - pop_buffer_bytes(p, p.NX));
     std::lock_guard<std::mutex> lock(share.m);
-    if (share.padding + extra > share.bytes / 128) return p.NX;
+    if (share.padding + extra > share.bytes() / 128) return p.NX;
     share.padding += extra;
     *padding = extra;
     return px;

@@ -37,11 +37,20 @@ struct DeviceShare {
     const int device;
     const uint64_t context;  // current_context_id of those who share it
     const bool primary;      // it is the device's primary context, whose end can be seen
-    size_t bytes = 0;        // memory of the device
-    std::mutex m;      // guards what follows
+    std::mutex m;                  // guards what follows
+    size_t memory = 0;             // bytes of the device, once asked for (bytes)
     size_t padding = 0;            // bytes that pad population rows
     cudaMemPool_t pool = nullptr;  // of the adjoint runs (adjoint.cu), made by the first
     DeviceShare(int d, uint64_t c) : device(d), context(c), primary(c != 0 && primary_context_id(d) == c) {}
+    // Memory of the device, 0 where it cannot be told; with m held.
+    size_t bytes() {
+        size_t free_b = 0;
+        if (memory == 0 && cudaMemGetInfo(&free_b, &memory) != cudaSuccess) {
+            (void)cudaGetLastError();
+            memory = 0;
+        }
+        return memory;
+    }
     bool gone() const { return primary && primary_context_id(device) != context; }
     ~DeviceShare() {
         if (pool && !gone()) cudaMemPoolDestroy(pool);
