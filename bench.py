@@ -19,8 +19,8 @@ reference's initial condition with seeded noise; no dataset is involved.
              downloaded.  `e2e.restart` is the same with the whole state
              uploaded instead (mcg_set_fields + mcg_set_populations, 990 MB).
   roofline   live per-launch event times of the dominant kernel against its
-             algorithmic bytes (216 B/node of populations per pass in float32,
-             108 B in float16) and the measured HBM copy peak.
+             algorithmic bytes (216 B of populations per interior node and pass
+             in float32, 108 B in float16) and the measured HBM copy peak.
   cpu_baseline  the float64 OpenMP oracle (oracle/) on a bounded sample of the
              same workload, rank 0 only.
 

@@ -121,7 +121,9 @@ mcg_status mcg_write_constants_header(const mcg_params *p, const char *path);
 /* ---------------- lifetime (memory.cuh:58-133) ---------------- */
 
 /* allocate_device_memory() + allocate_mean_fields_device() equivalent.
- * All device memory is owned by the handle and zero-filled like memory.cuh:79-95. */
+ * All device memory is owned by the handle and zero-filled like memory.cuh:79-95.
+ * Population rows are padded where that fits (mcg_device_bytes counts it); a later
+ * call that needs the room takes the padding out. */
 mcg_status mcg_create(const mcg_params *p, mcg_handle **out);
 /* free_device_memory() + free_mean_fields_runtime() equivalent. */
 mcg_status mcg_destroy(mcg_handle *h);
@@ -278,6 +280,11 @@ mcg_status mcg_set_inlet_bessel(mcg_handle *h, const float *coeffs, int32_t n);
 mcg_status mcg_get_inlet_profile(mcg_handle *h, float *profile);
 
 /* ---------------- discrete adjoint (no counterpart in the reference) ---------------- */
+
+/* The runs below take device memory beyond the handle's from a CUDA memory pool,
+ * which keeps up to a sixteenth of the device's memory for the next run until the
+ * last handle of the device is destroyed.  The driver takes what the pool keeps for
+ * any other allocation of the process that finds no room. */
 
 /* Initial state with a velocity field: every interior node gets, per colour,
  * the third-order equilibrium feq_i(rho_c, u) of lbm.cuh:16-35 (the
