@@ -181,13 +181,38 @@ struct DeviceBuffers {
         if (total + bytes > limit) return cudaErrorMemoryAllocation;
         if (!pool)
             if (cudaError_t e = adjoint_pool(*h->share, h->device, &pool); e != cudaSuccess) return e;
-        used.reserve(used.size() + 1);
+        const size_t need = (bytes + 255) / 256 * 256;
         void *q = nullptr;
-        if (cudaError_t e = cudaMallocFromPoolAsync(&q, bytes, pool, stream); e != cudaSuccess) return e;
-        used.push_back(q);
+        if (need > chunk_left && need < kChunk / 2 && take(&q, kChunk) == cudaSuccess) {
+            chunk = static_cast<char *>(q);
+            chunk_left = kChunk;
+        }
+        if (need <= chunk_left) {
+            q = chunk;
+            chunk += need;
+            chunk_left -= need;
+        } else if (cudaError_t e = take(&q, bytes); e != cudaSuccess) {
+            return e;
+        }
         total += bytes;
         *p = q;
         return zero ? cudaMemsetAsync(q, 0, bytes, stream) : cudaSuccess;
+    }
+
+private:
+    // Small blocks share chunks: a call of the pool costs 0.7 us, and a jet run has
+    // 28 blocks (34x48x16: 1.51 ms in all).
+    static constexpr size_t kChunk = size_t(32) << 20;
+    char *chunk = nullptr;
+    size_t chunk_left = 0;
+    cudaError_t take(void **q, size_t bytes) {
+        used.reserve(used.size() + 1);
+        const cudaError_t e = cudaMallocFromPoolAsync(q, bytes, pool, stream);
+        if (e == cudaSuccess)
+            used.push_back(*q);
+        else
+            (void)cudaGetLastError();
+        return e;
     }
 };
 
